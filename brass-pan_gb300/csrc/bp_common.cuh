@@ -155,7 +155,66 @@ struct SimConsts {
     // walk_planes_order).
     const float *walk_xyz;
     int walk_stride;
+    // Substep lists (sl_pos == nullptr: off): one neighbour search per substep.
+    // The substep's first lambda pass (without a fluid stage, a launch ahead of
+    // its first contact pass) records into nbr every candidate within
+    // h + skin of each particle, in walk order, its own entry included
+    // (nbr_count[t] = entries | index of the own entry << 16); every later
+    // pass of the substep (the position passes, the other lambda passes, the
+    // post passes) reads that list and drops the entries further than h at its
+    // own positions, which leaves the hits of the walk it stands for, in the
+    // walk's order.  That holds while the particle is in the cell it was
+    // recorded in (sl_cell[t], by list slot; negative: no list to read) and
+    // its displacement since then (from sl_pos, by sorted index) and that of
+    // any particle stored in its 27 cells add up to no more than the skin.
+    // Writers of P keep track of that in quarters of the skin
+    // (track_displacement): the first particle of a cell to move more than
+    // k quarters sets bits k of the 27 cells around its stored cell.
+    // Particles that may not read their list go to sl_queue and walk
+    // their cells in a launch of their own (a warp each).
+    // sl_count[kSlMoved]: *cls_moved when the lists were recorded; where it
+    // differs later, the slots have changed meaning and every particle walks.
+    int *sl_cell;
+    float4 *sl_pos;
+    // bit sets over the cell keys, sl_words words each: sl_bits[k - 1] holds the
+    // cells storing a particle that moved more than k quarters of the skin,
+    // sl_bits[kSlLevels + k - 1] the cells with one among their 27
+    unsigned *sl_bits;
+    int sl_words;
+    int *sl_queue;
+    // [0], [1]: queue lengths, by the parity of the pass (a list pass clears the
+    // other one); [kSlMoved]; [kSlDisplaced]: particles that the last list pass
+    // of a substep queued because something near them moved
+    int *sl_count;
+    float *sl_skin;   // [0] the skin in use, adapted after each substep (adapt_skin), [1] the last that was too small
+    float sl_fixed;   // > 0: this skin instead
+    int sl_pass;      // parity of this list pass
+    int sl_adapt;     // this pass is the substep's last over the lists
+    int sl_fluid;     // the lists reach h + skin (the fluid passes read them)
+    // Contact partners of slot t (nullptr: off), the candidates within two radii
+    // + skin when the lists were recorded: cl_count[t] of them (-1: more than
+    // kContactCap) as sorted indices in walk order, entry k at cl_list[k n + t].
+    // cl_near: nullptr, or the cells with a solid in their 27 cells (fluid
+    // elsewhere has no partner).
+    int *cl_list, *cl_count;
+    const unsigned long long *cl_near;
 };
+constexpr int kContactCap = 32;
+constexpr int kSlLevels = 3;
+constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlCounts = 4;
+// Bounds of the adapted skin and where it starts, as fractions of h.
+constexpr float kMinSkin = 0.02f, kMaxSkin = 0.1f, kStartSkin = 0.09f;
+// sl_cell where there is no list to read: something near moved, or another reason.
+constexpr int kListMoved = -1, kListNone = -2;
+
+__device__ __forceinline__ float substep_skin(const SimConsts &C) { return C.sl_fixed > 0.f ? C.sl_fixed : __ldg(C.sl_skin); }
+// The square of a quarter of the skin, less what the rounding of the distance
+// tests may take (k quarters: k * k times it).
+__device__ __forceinline__ float substep_quarter2(const SimConsts &C)
+{
+    const float q = __fmul_rn(0.2495f, substep_skin(C));
+    return __fmul_rn(q, q);
+}
 
 // The walks use the alias classes for the rest of the substep (uniform
 // over a launch: the flag is written by k_class_refresh before it).
@@ -350,12 +409,68 @@ __device__ __forceinline__ int list_state(const SimConsts &C, int i, int3 c, flo
     return 0;
 }
 
+// Substep lists: particle i moved more than `level` quarters of the skin.
+__device__ __forceinline__ void flag_moved(const SimConsts &C, int i, int level)
+{
+    const unsigned key = (unsigned)__ldg(C.cell_keys + i);
+    const unsigned bit = 1u << (key & 31u);
+#pragma unroll 1
+    for (int k = 0; k < level; ++k) {
+        unsigned *far = C.sl_bits + (size_t)k * C.sl_words, *near = far + (size_t)kSlLevels * C.sl_words;
+        // the first particle of a cell to be flagged flags the cells around it
+        if ((far[key >> 5] & bit) || (atomicOr(far + (key >> 5), bit) & bit)) continue;
+        const int s = scene_index(C, i);
+        const unsigned D = s < 0 ? (unsigned)C.D : (unsigned)C.scn[s].D, base = s < 0 ? 0u : (unsigned)C.scn[s].base;
+        const unsigned m = D - 1u, c = key - base, x = c / (D * D), y = (c / D) & m, z = c & m;
+#pragma unroll 1
+        for (unsigned q = 0; q < 27u; ++q) {
+            const unsigned a = base + ((x + q / 9u - 1u) & m) * D * D + ((y + (q / 3u) % 3u - 1u) & m) * D +
+                               ((z + q % 3u - 1u) & m);
+            atomicOr(near + (a >> 5), 1u << (a & 31u));
+        }
+    }
+}
+
+// Substep lists: 0 when the particle of slot t (sorted index i, at p, in cell
+// `key` of its scene's range) may read its list; otherwise why not, as
+// list_state.
+__device__ __forceinline__ int substep_list_state(const SimConsts &C, int t, int i, float3 p, int key)
+{
+    if (C.cls_perm && __ldg(C.cls_moved) != __ldg(C.sl_count + kSlMoved)) return 1;
+    const int built = C.sl_cell[t];
+    if (built < 0) return built == kListMoved ? 3 : 1;
+    if (built != key) return 2;
+    const unsigned *near = C.sl_bits + (size_t)kSlLevels * C.sl_words + (key >> 5);
+    auto moved = [&](int k) { return ((__ldg(near + (size_t)(k - 1) * C.sl_words) >> (key & 31)) & 1u) != 0u; };
+    // nothing near (itself included) moved more than a quarter, or it moved
+    // one quarter at most and the others three, or each two
+    if (!moved(1)) return 0;
+    const float d2 = len2(p - f3(C.sl_pos[i])), q2 = substep_quarter2(C);
+    if (d2 <= q2) return moved(3) ? 3 : 0;
+    if (d2 <= 4.0f * q2) return moved(2) ? 3 : 0;
+    return 3;
+}
+
+// Its own displacement flags the cells around its stored cell: a particle that
+// left those has no list.
+__device__ __forceinline__ bool near_stored_cell(const SimConsts &C, int i, int3 c, const GridView &v)
+{
+    const unsigned m = v.mask, D = (unsigned)v.D, k = (unsigned)(__ldg(C.cell_keys + i) - v.base);
+    return (((unsigned)c.x - k / (D * D) + 1u) & m) <= 2u && (((unsigned)c.y - k / D + 1u) & m) <= 2u &&
+           (((unsigned)c.z - k + 1u) & m) <= 2u;
+}
+
 // Records that particle i moved more than half the skin since the list
 // build: flags its stored cell (the cell its sorted index belongs to) so the
 // particles whose 27 cells include it walk their cells.  Writers of P call it
 // with the new position.
 __device__ __forceinline__ void track_displacement(const SimConsts &C, int i, float3 p, bool active)
 {
+    if (C.sl_pos) {
+        const float d2 = len2(p - f3(C.sl_pos[i])), q2 = substep_quarter2(C);
+        if (!(d2 <= q2)) flag_moved(C, i, d2 <= 4.0f * q2 ? 1 : (d2 <= 9.0f * q2 ? 2 : 3));  // NaN counts as moved
+        return;
+    }
     if (!C.nl_pos || !active) return;
     if (!(len2(p - f3(C.nl_pos[i])) <= C.nl_half_skin2)) {  // NaN counts as moved
         const unsigned key = (unsigned)__ldg(C.cell_keys + i);

@@ -16,7 +16,7 @@
 #include <algorithm>
 
 #include "bp_internal.h"
-#include "bp_walk.cuh"
+#include "bp_lists.cuh"
 
 namespace bp {
 
@@ -376,9 +376,59 @@ __device__ __forceinline__ void walk_solids(float3 pi, const float4 *__restrict_
 // Solid contacts: pairs of different phase with at least one solid, closer
 // than two radii; mass-weighted projection plus friction averaged over the
 // counted contacts; only particle i moves (the reference's j update is
-// commented out).  Reads P, writes Pout = P + delta.  A fluid particle only
-// meets solids, so it walks the compacted solids of its 27 cells (same
-// candidates in the same order; the others contribute nothing).
+// commented out).
+struct Contacts {
+    float3 sd, sf;
+    int count;
+};
+__device__ __forceinline__ bool contact_phases(int phi, int phj) { return phi != phj && (phi > 0 || phj > 0); }
+__device__ __forceinline__ bool contact_near(const SimConsts &C, float d2)
+{
+    const float r = C.radius;
+    return d2 < r * r * 4.0f && d2 > 1e-5f;
+}
+// The pair's projection (dxi) and, where it counts, its friction move (rub):
+// true where it counts.
+__device__ __forceinline__ bool contact_pair(const SimConsts &C, float3 xip, float3 xi, float wi, int j, float3 xjp,
+                                             const float4 *__restrict__ Xs, const float *__restrict__ w, float3 &dxi,
+                                             float3 &rub)
+{
+    const float r = C.radius;
+    const float3 diff = xip - xjp;
+    const float d2 = len2(diff);
+    const float dist = __fsqrt_rn(d2);
+    const float wj = w[j];
+    const float w1 = __fdiv_rn(wi, __fadd_rn(wi, wj));
+    const float w2 = __fdiv_rn(wj, __fadd_rn(wi, wj));
+    const float3 proj = diff * __fsub_rn(__fdiv_rn(2.0f * r, dist), 1.0f);
+    dxi = w1 * proj;
+    const float3 xistar = dxi + xip;
+    const float3 dxj = -w2 * proj;
+    const float dxi2 = len2(dxi);
+    if (!(dxi2 > r * r * 0.001f * 0.001f)) return false;
+    const float3 xj = f3(Xs[j]);
+    const float3 xjstar = dxj + xjp;
+    const float3 t1 = (xistar - xi) - (xjstar - xj);
+    const float3 nn = diff / dist;
+    const float3 tdx = t1 - dot3(t1, nn) * nn;
+    const float tl2 = len2(tdx);
+    rub = w1 * tdx;
+    if (!(tl2 <= __fmul_rn(C.fs * C.fs, dxi2)))
+        rub = rub * fminf(__fmul_rn(C.fd, __fsqrt_rn(__fdiv_rn(dxi2, tl2))), 1.0f);
+    return true;
+}
+__device__ __forceinline__ void contact_finish(const SimConsts &C, int i, float4 pi4, const Contacts &s,
+                                               float4 *__restrict__ Pout)
+{
+    const float3 d = (s.count == 0) ? s.sd : s.sd + s.sf / (float)s.count;
+    const float3 p = f3(pi4) + d;
+    Pout[i] = make_float4(p.x, p.y, p.z, pi4.w);
+    track_displacement(C, i, p, true);
+}
+
+// Reads P, writes Pout = P + delta.  A fluid particle only meets solids, so it
+// walks the compacted solids of its 27 cells (same candidates in the same
+// order; the others contribute nothing).
 template <bool Split>
 __device__ __forceinline__ void collide_one(const SimConsts &C, int i, const float4 *__restrict__ P,
                                             const float4 *__restrict__ Xs, const float *__restrict__ w,
@@ -389,51 +439,121 @@ __device__ __forceinline__ void collide_one(const SimConsts &C, int i, const flo
     const float4 pi4 = P[i];
     const float3 xip = f3(pi4);
     const int phi = phase_of(pi4);
-    const float r = C.radius;
     const float3 xi = f3(Xs[i]);
     const float wi = w[i];
-    float3 sd = make_float3(0.f, 0.f, 0.f), sf = make_float3(0.f, 0.f, 0.f);
-    int count = 0;
+    Contacts s{make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), 0};
     auto test = [&](int j, float4 pj4) {
-        const int phj = phase_of(pj4);
-        const float d2 = len2(xip - f3(pj4));
-        return j != i && phi != phj && (phi > 0 || phj > 0) && d2 < r * r * 4.0f && d2 > 1e-5f;
+        return j != i && contact_phases(phi, phase_of(pj4)) && contact_near(C, len2(xip - f3(pj4)));
     };
     auto body = [&](int j, float4 pj4) {
-            const float3 xjp = f3(pj4);
-            const float3 diff = xip - xjp;
-            const float d2 = len2(diff);
-            const float dist = __fsqrt_rn(d2);
-            const float wj = w[j];
-            const float w1 = __fdiv_rn(wi, __fadd_rn(wi, wj));
-            const float w2 = __fdiv_rn(wj, __fadd_rn(wi, wj));
-            const float3 proj = diff * __fsub_rn(__fdiv_rn(2.0f * r, dist), 1.0f);
-            const float3 dxi = w1 * proj;
-            const float3 xistar = dxi + xip;
-            sd += dxi;
-            const float3 dxj = -w2 * proj;
-            const float dxi2 = len2(dxi);
-            if (dxi2 > r * r * 0.001f * 0.001f) {
-                count += 1;
-                const float3 xj = f3(Xs[j]);
-                const float3 xjstar = dxj + xjp;
-                const float3 t1 = (xistar - xi) - (xjstar - xj);
-                const float3 nn = diff / dist;
-                const float3 tdx = t1 - dot3(t1, nn) * nn;
-                const float tl2 = len2(tdx);
-                if (tl2 <= __fmul_rn(C.fs * C.fs, dxi2))
-                    sf -= w1 * tdx;
-                else
-                    sf -= (w1 * tdx) * fminf(__fmul_rn(C.fd, __fsqrt_rn(__fdiv_rn(dxi2, tl2))), 1.0f);
-            }
+        float3 dxi, rub;
+        const bool counts = contact_pair(C, xip, xi, wi, j, f3(pj4), Xs, w, dxi, rub);
+        s.sd += dxi;
+        if (counts) {
+            s.count += 1;
+            s.sf -= rub;
+        }
     };
     const CellRange rg = contact_range(C, xip, phi < 0 && solid_prefix);
     if (phi < 0 && solid_prefix) walk_solids(xip, solid_pos, v, C, solid_prefix, solid_list, test, body, rg);
     else walk_neighbors<Split, true>(i, xip, 0, P, v, C, S, g, test, body, rg);
-    const float3 d = (count == 0) ? sd : sd + sf / (float)count;
-    const float3 p = xip + d;
-    Pout[i] = make_float4(p.x, p.y, p.z, pi4.w);
-    track_displacement(C, i, p, true);
+    contact_finish(C, i, pi4, s, Pout);
+}
+
+// ---- contacts over the substep lists ----
+
+// A pass over the contact lists that the substep's search left
+// (SimConsts::cl_list: the partners within two radii + skin, sorted indices in
+// walk order), one thread per slot: the pairs of the 27-cell walk in its
+// order.  Most particles have none and only copy their position, so the pass
+// is bound by that copy (40 bytes a particle).
+__global__ void __launch_bounds__(256) k_contacts_lists(SimConsts C, const float4 *__restrict__ P,
+                                                        const float4 *__restrict__ Xs, const float *__restrict__ w,
+                                                        const int *__restrict__ off, float4 *__restrict__ Pout)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) C.sl_count[C.sl_pass ^ 1] = 0;  // the next pass's queue
+    if (t >= C.n) return;
+    const int i = walker_index(C, t);
+    const float4 pi4 = P[i];
+    const float3 xip = f3(pi4);
+    const int cnt = __ldg(C.cl_count + t);
+    if (!reads_substep_list(C, t, i, xip, cell_of(xip, C), grid_view(C, scene_index(C, i), off), cnt >= 0)) return;
+    const int phi = phase_of(pi4);
+    Contacts s{make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), 0};
+    if (cnt > 0) {
+        const float3 xi = f3(Xs[i]);
+        const float wi = w[i];
+        for (int k = 0; k < cnt; ++k) {
+            const int j = __ldg(C.cl_list + (size_t)k * C.n + t);
+            const float4 pj4 = P[j];
+            if (!(contact_phases(phi, phase_of(pj4)) && contact_near(C, len2(xip - f3(pj4))))) continue;
+            float3 dxi, rub;
+            const bool counts = contact_pair(C, xip, xi, wi, j, f3(pj4), Xs, w, dxi, rub);
+            s.sd += dxi;
+            if (counts) {
+                s.count += 1;
+                s.sf -= rub;
+            }
+        }
+    }
+    contact_finish(C, i, pi4, s, Pout);
+}
+
+// The particles that may not read their contact list, a warp each, over whole
+// table cells (the same pairs in the same order as the alias classes give).
+constexpr int kContactThreads = 128;
+__global__ void __launch_bounds__(kContactThreads) k_contacts_queued(SimConsts C, const float4 *__restrict__ P,
+                                                                     const float4 *__restrict__ Xs,
+                                                                     const float *__restrict__ w,
+                                                                     const int *__restrict__ off,
+                                                                     float4 *__restrict__ Pout)
+{
+    __shared__ WarpRows rows[kContactThreads / 32];
+    __shared__ WarpHits hits[kContactThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int queued = C.sl_count[C.sl_pass];
+    adapt_skin(C);
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) / 32; k < queued; k += gridDim.x * blockDim.x / 32) {
+        const int i = walker_index(C, C.sl_queue[k]);
+        const float4 pi4 = P[i];
+        const float3 xip = f3(pi4), xi = f3(Xs[i]);
+        const int phi = phase_of(pi4);
+        const float wi = w[i];
+        float sd = 0.f, sf = 0.f;  // lanes 0..2: the components
+        int count = 0;
+        auto test = [&](int j, float4 pj4) {
+            return j != i && contact_phases(phi, phase_of(pj4)) && contact_near(C, len2(xip - f3(pj4)));
+        };
+        auto batch = [&](int, int n, int j, float4 pj4) {
+            float3 dxi = make_float3(0.f, 0.f, 0.f), rub = dxi;
+            const bool counts = lane < n && contact_pair(C, xip, xi, wi, j, f3(pj4), Xs, w, dxi, rub);
+            const unsigned counted = __ballot_sync(0xffffffffu, counts);
+            const float push[3] = {dxi.x, dxi.y, dxi.z}, drag[3] = {-rub.x, -rub.y, -rub.z};
+            warp_add(rows[threadIdx.x >> 5], n == 32 ? 0xffffffffu : (1u << n) - 1u, push, 1.f, sd);
+            warp_add(rows[threadIdx.x >> 5], counted, drag, 1.f, sf);
+            count += __popc(counted);
+        };
+        warp_neighbors(C, false, cell_of(xip, C), P, grid_view(C, scene_index(C, i), off), hits[threadIdx.x >> 5], test,
+                       batch);
+        Contacts s;
+        s.sd = make_float3(__shfl_sync(0xffffffffu, sd, 0), __shfl_sync(0xffffffffu, sd, 1),
+                           __shfl_sync(0xffffffffu, sd, 2));
+        s.sf = make_float3(__shfl_sync(0xffffffffu, sf, 0), __shfl_sync(0xffffffffu, sf, 1),
+                           __shfl_sync(0xffffffffu, sf, 2));
+        s.count = count;
+        if (lane == 0) contact_finish(C, i, pi4, s, Pout);
+    }
+}
+
+void launch_contacts_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *Xs, const float *w,
+                           const int *off, float4 *Pout, LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    k_contacts_lists<<<(C.n + 255) / 256, 256, 0, st>>>(C, P, Xs, w, off, Pout);
+    L->done("launch_contacts_lists");
+    k_contacts_queued<<<queue_blocks(C.n, kContactThreads), kContactThreads, 0, st>>>(C, P, Xs, w, off, Pout);
+    L->done("launch_contacts_queued");
 }
 
 // Fluid particles (and, without a solid list, everything), one CTA per 256

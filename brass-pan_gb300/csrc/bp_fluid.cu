@@ -13,8 +13,10 @@
 // pairs in a fixed order, so results are deterministic run to run.  The pair
 // term for (k, j) is bit-identical to the reference's term for (j, k) up to
 // sign, because the spiky gradient is odd in the difference vector.
+#include <algorithm>
+
 #include "bp_internal.h"
-#include "bp_walk.cuh"
+#include "bp_lists.cuh"
 
 namespace bp {
 
@@ -104,7 +106,7 @@ __device__ __forceinline__ void k_lambda_tile(
     // Verlet lists are kept per particle, the position pass's lists per slot
     ListWriter list(build ? C.vl : C.nbr, build ? C.vl_cap : C.nbr_cap, C.n, build ? i : t);
     auto finish = [&]() {
-        const int cnt = list.finish();
+        const int cnt = list.finish(i);
         if (build) finish_verlet(C, i, pi4, cnt);
         else C.nbr_count[t] = cnt;
     };
@@ -133,7 +135,7 @@ __device__ __forceinline__ void k_lambda_tile(
         } else {
             walk_neighbors<Split>(i, pi, 0, P, v, C, Stage ? &S : nullptr, g, test, push);
         }
-        const int cnt = list.finish();
+        const int cnt = list.finish(slots ? t : i);
         C.nbr_count[t] = cnt;
         return cnt;
     };
@@ -275,6 +277,260 @@ void launch_lambda(cudaStream_t st, const SimConsts &C, const float4 *P, const f
     L->done(__func__);
 }
 
+// ---- the passes over the substep lists (bp_lists.cuh) ----
+
+// Writes a fluid particle's density and lambda, and their copies.
+__device__ __forceinline__ void finish_lambda(const SimConsts &C, bool slots, int i, int t, float density, float rho0,
+                                              float den, const float *__restrict__ mass, float *__restrict__ lam,
+                                              float *__restrict__ rho)
+{
+    float c = density / rho0 - 1.0f;
+    if (C.clamp_c) c = fmaxf(c, 0.0f);
+    const float l = -c / den;
+    lam[i] = l;
+    if (slots) {
+        C.cls_lm[t] = make_float2(l, __ldg(mass + i));
+        C.cls_rho[t] = density;
+    } else {
+        C.lm[i] = make_float2(l, __ldg(mass + i));
+    }
+    rho[i] = density;
+}
+
+// Records slot t's contact partners (SimConsts::cl_list) from its list just
+// recorded.
+__device__ __forceinline__ void record_contacts(const SimConsts &C, const float4 *__restrict__ P, bool slots, int t,
+                                                int i, float4 pi4, int3 c, const GridView &v, int packed, float touch2)
+{
+    const int phi = phase_of(pi4);
+    const int addr = cell_addr(c.x, c.y, c.z, v.D, v.mask);
+    int n = 0;
+    if (packed < 0) {
+        n = kContactCap + 1;
+    } else if (phi > 0 || !C.cl_near || ((__ldg(C.cl_near + (addr >> 6)) >> (addr & 63)) & 1ull)) {
+        auto none = [](int) { return 0; };
+        for_each_padded<false>(C.nbr, C.n, t, packed & 0xffff, slots ? C.cls_pos : P, none, [&](int q, float4 pj4, int) {
+            const int phj = phase_of(pj4);  // the own entry: the same phase
+            if (phi == phj || !(phi > 0 || phj > 0) || !(len2(f3(pi4) - f3(pj4)) <= touch2)) return;
+            if (n < kContactCap) C.cl_list[(size_t)n * C.n + t] = slots ? __ldg(C.cls_perm + q) : q;
+            ++n;
+        });
+    }
+    C.cl_count[t] = n <= kContactCap ? n : -1;
+}
+
+// The lambda pass over the substep lists: the density (and, in textbook mode,
+// the denominator) of k_lambda, from the same pairs in the same order.
+// What bounds it: a list read is latency-bound on its gathers, like k_deltap;
+// the recording walk is issue-bound, like k_lambda.
+template <ListPass Pass>
+__device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const float4 *__restrict__ P,
+                                                    const float *__restrict__ mass, const int *__restrict__ off,
+                                                    float *__restrict__ lam, float *__restrict__ rho, int t)
+{
+    const bool slots = classes_on(C);
+    const int i = slots ? __ldg(C.cls_perm + t) : t;
+    const float4 pi4 = slots ? C.cls_pos[t] : P[i];
+    const float3 pi = f3(pi4);
+    const bool solid = phase_of(pi4) > 0;
+    if (Pass == kRecordLists) {
+        C.sl_pos[i] = pi4;
+        if (solid && C.sl_fluid) {  // solids carry lambda 0 (read by the position pass)
+            lam[i] = 0.f;
+            (slots ? C.cls_lm[t] : C.lm[i]) = make_float2(0.f, __ldg(mass + i));
+        }
+    }
+    // textbook mode: no pass but the contacts moves a solid by its neighbours
+    if (solid && C.textbook && !(Pass == kRecordLists && C.cl_list)) return;
+    const int sc = scene_index(C, i);
+    const GridView v = grid_view(C, sc, off);
+    const int3 c = cell_of(pi, C);
+    int packed;
+    if (Pass == kReadLists) {
+        if (!reads_substep_list(C, t, i, pi, c, v) || solid) return;
+        packed = __ldg(C.nbr_count + t);
+    } else {
+        const float skin = substep_skin(C), touch = 2.0f * C.radius + skin;
+        const float reach = fmaxf(C.sl_fluid ? C.h + skin : 0.f, C.cl_list ? touch : 0.f);
+        packed = record_substep_list(C, P, slots, t, i, pi, c, __fmul_rn(reach, reach), v);
+        const bool fits = packed >= 0;
+        if (C.cl_list) record_contacts(C, P, slots, t, i, pi4, c, v, packed, __fmul_rn(touch, touch));
+        // the neighbours within h alone may still fit; later passes then walk
+        if (!fits && C.sl_fluid) packed = record_substep_list(C, P, slots, t, i, pi, c, C.h2, v);
+        C.nbr_count[t] = packed;
+        C.sl_cell[t] = (fits && near_stored_cell(C, i, c, v)) ? v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask) : kListNone;
+        if (!C.sl_fluid) return;
+    }
+    if (solid) return;
+    const int cnt = packed & 0xffff, self = packed >> 16;
+    const float4 *__restrict__ src = slots ? C.cls_pos : P;
+    const float *__restrict__ ms = slots ? C.cls_mass : mass;
+    const float rho0 = rest_density(C, sc);
+    float density = 0.f, den = C.lambda_den;
+    // the records were written by the calling thread, except in a reading pass
+    constexpr bool kReadOnly = Pass == kReadLists;
+    auto fetch = [&](int j) { return __ldg(ms + j); };
+    if (!C.textbook) {
+        auto add = [&](float mj, float4 pj, float d2) {
+            const float ld = __fmul_rn(mj, poly6(C, d2));
+            density = __fadd_rn(density, (phase_of(pj) < 0) ? ld : __fmul_rn(C.solid_scale, ld));
+        };
+        if (packed >= 0) {
+            // j >= i: where no column run wraps around the table the walk is
+            // in ascending j, so these are the entries from the own one on
+            auto inner = [&](int a) {
+                const unsigned u = (unsigned)a & v.mask;
+                return u != 0u && u != v.mask;
+            };
+            const bool ascending = inner(c.x) && inner(c.y) && inner(c.z);
+            int e = ascending ? (self & ~3) : 0;
+            const int first = e;
+            for_each_padded<kReadOnly>(C.nbr, C.n, t, cnt, src, fetch, [&](int j, float4 pj, float mj) {
+                const float d2 = len2(pi - f3(pj));
+                bool take = d2 <= C.h2;
+                if (ascending) take = take && (unsigned)(e - self) < (unsigned)(cnt - self);
+                else take = take && e < cnt && (slots ? __ldg(C.cls_perm + j) : j) >= i;
+                ++e;
+                if (take) add(mj, pj, d2);
+            }, first);
+        } else {
+            auto test = [&](int, float4 pj) { return len2(pi - f3(pj)) <= C.h2; };
+            walk_neighbors<true>(i, pi, i, P, v, C, nullptr, -1, test,
+                                 [&](int j, float4 pj) { add(__ldg(mass + j), pj, len2(pi - f3(pj))); });
+        }
+    } else {
+        const float inv_rho0 = inv_rest_density(C, sc);
+        float sum_g2 = 0.f;
+        float3 gi = make_float3(0.f, 0.f, 0.f);
+        auto term = [&](float mj, float4 pj) {
+            const float3 diff = pi - f3(pj);
+            const float d2 = len2(diff);
+            if (!(d2 <= C.h2)) return;
+            const float ld = __fmul_rn(mj, poly6(C, d2));
+            density = __fadd_rn(density, (phase_of(pj) < 0) ? ld : __fmul_rn(C.solid_scale, ld));
+            if (d2 > 0.f) {
+                const float3 g = __fmul_rn(-mj, inv_rho0) * spiky_grad_r(C, diff, d2, rsqrtf(d2));
+                sum_g2 = __fadd_rn(sum_g2, dot3(g, g));
+                gi -= g;
+            }
+        };
+        if (packed >= 0) {
+            int e = 0;
+            for_each_padded<kReadOnly>(C.nbr, C.n, t, cnt, src, fetch, [&](int, float4 pj, float mj) {
+                if (e++ < cnt) term(mj, pj);
+            });
+        } else {
+            auto test = [&](int, float4 pj) { return len2(pi - f3(pj)) <= C.h2; };
+            walk_neighbors<true>(i, pi, 0, P, v, C, nullptr, -1, test,
+                                 [&](int j, float4 pj) { term(__ldg(mass + j), pj); });
+        }
+        sum_g2 += dot3(gi, gi);
+        den = sum_g2 + C.relaxation;
+    }
+    finish_lambda(C, slots, i, t, density, rho0, den, mass, lam, rho);
+}
+
+template <ListPass Pass>
+__global__ void __launch_bounds__(kScanThreads, BP_SCAN_MIN_BLOCKS) k_lambda_lists(
+    SimConsts C, const float4 *__restrict__ P, const float *__restrict__ mass, const int *__restrict__ off,
+    float *__restrict__ lam, float *__restrict__ rho)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) {
+        C.sl_count[C.sl_pass ^ 1] = 0;  // the next pass's queue
+        if (Pass == kRecordLists) {
+            C.sl_count[C.sl_pass] = 0;
+            C.sl_count[kSlDisplaced] = 0;
+            C.sl_count[kSlMoved] = C.cls_perm ? *C.cls_moved : 0;
+        }
+    }
+    if (t < C.n) lambda_substep_list<Pass>(C, P, mass, off, lam, rho, t);
+}
+
+// The queued particles' lambda pass, a warp per particle: walks the
+// cells, leaves the neighbours within h in the list for this iteration's
+// position pass, and adds the pair terms, computed a candidate per lane, in
+// walk order.
+constexpr int kQueueThreads = 128;
+__global__ void __launch_bounds__(kQueueThreads) k_lambda_queued(SimConsts C, const float4 *__restrict__ P,
+                                                                const float *__restrict__ mass,
+                                                                const int *__restrict__ off, float *__restrict__ lam,
+                                                                float *__restrict__ rho)
+{
+    __shared__ WarpRows rows[kQueueThreads / 32];
+    __shared__ WarpHits hits[kQueueThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int queued = C.sl_count[C.sl_pass];
+    adapt_skin(C);
+    const bool slots = classes_on(C);
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) / 32; k < queued; k += gridDim.x * blockDim.x / 32) {
+        const int t = C.sl_queue[k];
+        const int i = slots ? __ldg(C.cls_perm + t) : t;
+        const float4 pi4 = slots ? C.cls_pos[t] : P[i];
+        const float3 pi = f3(pi4);
+        const bool solid = phase_of(pi4) > 0;  // its list only (reference mode)
+        const int sc = scene_index(C, i);
+        const GridView v = grid_view(C, sc, off);
+        const float inv_rho0 = inv_rest_density(C, sc);
+        if (C.nl_stats && slots && lane == 0) atomicAdd(C.nl_stats + 4, 1u);
+        float acc = 0.f;  // lane 0: the density; textbook, lanes 1..4: sum of g^2, -sum of g
+        int self = 0;
+        const int me = slots ? t : i;
+        auto test = [&](int, float4 pj) { return len2(pi - f3(pj)) <= C.h2; };
+        auto batch = [&](int k0, int n, int q, float4 pj) {
+            const bool in = lane < n;
+            if (in) put_entry(C, t, k0 + lane, q);
+            const unsigned own = __ballot_sync(kWarp, in && q == me);
+            if (own) self = k0 + __ffs(own) - 1;
+            if (solid) return;
+            bool take = in;
+            float value[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+            if (in) {
+                const int j = slots ? __ldg(C.cls_perm + q) : q;
+                const float mj = __ldg((slots ? C.cls_mass : mass) + q);
+                const float3 diff = pi - f3(pj);
+                const float d2 = len2(diff);
+                take = C.textbook || j >= i;
+                value[0] = __fmul_rn(mj, poly6(C, d2));
+                if (phase_of(pj) >= 0) value[0] = __fmul_rn(C.solid_scale, value[0]);
+                if (C.textbook && d2 > 0.f) {  // the pair at r = 0 adds zeros
+                    const float3 g = __fmul_rn(-mj, inv_rho0) * spiky_grad_r(C, diff, d2, rsqrtf(d2));
+                    value[1] = dot3(g, g);
+                    value[2] = -g.x;
+                    value[3] = -g.y;
+                    value[4] = -g.z;
+                }
+            }
+            warp_add(rows[threadIdx.x >> 5], __ballot_sync(kWarp, take), value, 1.f, acc);
+        };
+        const int cnt = warp_neighbors(C, slots, cell_of(pi, C), P, v, hits[threadIdx.x >> 5], test, batch);
+        warp_pad(C, t, cnt, slots ? t : i);
+        const float sum_g2 = __shfl_sync(kWarp, acc, 1);
+        const float3 gi = make_float3(__shfl_sync(kWarp, acc, 2), __shfl_sync(kWarp, acc, 3), __shfl_sync(kWarp, acc, 4));
+        if (lane != 0) continue;
+        C.nbr_count[t] = cnt <= C.nbr_cap ? cnt | (self << 16) : -1;
+        if (solid) continue;
+        finish_lambda(C, slots, i, t, acc, rest_density(C, sc),
+                      C.textbook ? (sum_g2 + dot3(gi, gi)) + C.relaxation : C.lambda_den, mass, lam, rho);
+    }
+}
+
+void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const float *mass,
+                         const int *off, float *lam, float *rho, LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    const int grid = (C.n + C.scan_block - 1) / C.scan_block;
+    if (record) {
+        k_lambda_lists<kRecordLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+        L->done("launch_lambda");
+        return;
+    }
+    k_lambda_lists<kReadLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+    L->done("launch_lambda_lists");
+    k_lambda_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, mass, off, lam, rho);
+    L->done("launch_lambda_queued");
+}
+
 // Position correction.  Reference mode: the pair (a, b), a < b, contributes
 // when a is a fluid particle (only fluid threads run fluidPosition and they
 // only visit b > a), to both ends.  In gather form particle k includes j when
@@ -295,8 +551,12 @@ __device__ __forceinline__ void k_deltap_tile(
     const float4 pk4 = valid ? a.P[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int phk = phase_of(pk4);
     const bool moves = valid && !(C.textbook && phk > 0);
-    const int listed = (moves && C.nbr) ? __ldg(C.nbr_count + t) : -1;
+    int listed = (moves && C.nbr) ? __ldg(C.nbr_count + t) : -1;
     const bool walk = moves && listed < 0;
+    listed &= 0xffff;  // substep lists: above it, the own entry's index
+    // substep lists also hold entries past h (the test changes nothing for
+    // lists of the neighbours within h); r = 0 excludes k itself
+    auto near = [&](float d2) { return d2 > 0.f && d2 <= C.h2; };
     const int g = (Stage && __syncthreads_or(walk)) ? stage_block(C, a.P, a.off, i0, S) : -1;
     if (!valid) return;
     const float3 pk = f3(pk4);
@@ -304,18 +564,21 @@ __device__ __forceinline__ void k_deltap_tile(
     float3 sum = make_float3(0.f, 0.f, 0.f);
     if (moves) {
         const float lk = a.lam[k];
-        auto pair = [&](float4 pj4, float lj, float mj) {
-            const float3 diff = pk - f3(pj4);
-            const float d2 = len2(diff);
+        // adds the pair term where ok; the rest of it has no condition
+        auto pair_at = [&](bool ok, float3 diff, float d2, float lj, float mj) {
             float sl = __fadd_rn(lk, lj);
             if (C.scorr_on)
                 sl = __fsub_rn(sl, __fmul_rn(C.scorr_k, ipowf(__fmul_rn(poly6(C, d2), C.scorr_inv_wq), C.scorr_ni)));
             float3 delta = sl * spiky_grad_r(C, diff, d2, rsqrtf(d2));
             if (C.delta_clamp > 0.f) {  // per-pair clamp; the length is only needed past it
                 const float l2 = len2(delta);
-                if (!(l2 < C.delta_clamp2)) delta = delta * __fmul_rn(C.delta_clamp, rsqrtf(l2));
+                if (ok && !(l2 < C.delta_clamp2)) delta = delta * __fmul_rn(C.delta_clamp, rsqrtf(l2));
             }
-            sum = fma3(mj, delta, sum);
+            if (ok) sum = fma3(mj, delta, sum);
+        };
+        auto pair = [&](float4 pj4, float lj, float mj) {
+            const float3 diff = pk - f3(pj4);
+            pair_at(true, diff, len2(diff), lj, mj);
         };
         auto body = [&](int j, float4 pj4) {
             if (!C.textbook && !((j > k) ? (phk < 0) : (phase_of(pj4) < 0))) return;
@@ -329,27 +592,26 @@ __device__ __forceinline__ void k_deltap_tile(
         // four pair terms of a record
         if (!walk && slots) {
             auto fetch = [&](int q) { return __ldg(C.cls_lm + q); };
-            for_each_in_list_with(C.nbr, C.n, t, listed, C.cls_pos, fetch, [&](int q, float4 pj4, float2 lm) {
-                if (!(len2(pk - f3(pj4)) > 0.f)) return;  // r = 0 excludes k itself
-                if (!C.textbook) {
-                    const bool fj = phase_of(pj4) < 0;
-                    if (!(phk < 0 && fj)) {
-                        const int j = __ldg(C.cls_perm + q);
-                        if (!((j > k) ? (phk < 0) : fj)) return;
-                    }
-                }
-                pair(pj4, lm.x, lm.y);
+            for_each_padded(C.nbr, C.n, t, listed, C.cls_pos, fetch, [&](int q, float4 pj4, float2 lm) {
+                const float3 diff = pk - f3(pj4);
+                const float d2 = len2(diff);
+                bool ok = near(d2);
+                const bool fj = phase_of(pj4) < 0;
+                if (!C.textbook && !(phk < 0 && fj)) ok = ok && ((__ldg(C.cls_perm + q) > k) ? (phk < 0) : fj);
+                pair_at(ok, diff, d2, lm.x, lm.y);
             });
         } else if (!walk && C.lm) {
             auto fetch = [&](int j) { return __ldg(C.lm + j); };
-            for_each_in_list_with(C.nbr, C.n, t, listed, a.P, fetch, [&](int j, float4 pj4, float2 lm) {
-                if (!(len2(pk - f3(pj4)) > 0.f)) return;  // r = 0 excludes k itself
-                if (!C.textbook && !((j > k) ? (phk < 0) : (phase_of(pj4) < 0))) return;
-                pair(pj4, lm.x, lm.y);
+            for_each_padded(C.nbr, C.n, t, listed, a.P, fetch, [&](int j, float4 pj4, float2 lm) {
+                const float3 diff = pk - f3(pj4);
+                const float d2 = len2(diff);
+                bool ok = near(d2);
+                if (!C.textbook) ok = ok && ((j > k) ? (phk < 0) : (phase_of(pj4) < 0));
+                pair_at(ok, diff, d2, lm.x, lm.y);
             });
         } else if (!walk) {
-            auto listed_body = [&](int j, float4 pj4) {  // r = 0 excludes k itself
-                if (len2(pk - f3(pj4)) > 0.f) body(j, pj4);
+            auto listed_body = [&](int j, float4 pj4) {
+                if (near(len2(pk - f3(pj4)))) body(j, pj4);
             };
             for_each_in_list(C.nbr, C.n, t, listed, a.P, listed_body);
         } else {
@@ -488,7 +750,7 @@ __device__ __forceinline__ void k_post_a_tile(
                 if (j != i && phase_of(pj4) == phi) list.push(j);
             });
         }
-        cnt = list.finish();
+        cnt = list.finish(slots ? t : i);
         C.nbr_count[t] = cnt;
         // the records just written come back through the coherent path (plain loads)
         if (cnt >= 0 && slots)
@@ -542,7 +804,7 @@ __device__ __forceinline__ int post_list_count(const SimConsts &C, const float4 
     if (i >= C.n || phase_of(P[i]) >= 0) return 0;
     if (!C.nbr || !C.nbr_count) return kWalkCells;
     const int cnt = __ldg(C.nbr_count + t);
-    return cnt >= 0 ? cnt : kWalkCells;
+    return cnt >= 0 ? cnt & 0xffff : kWalkCells;  // substep lists: above it, the own entry's index
 }
 
 // Pass B: vorticity confinement (fluidVorticity) then Akinci tension
@@ -596,10 +858,12 @@ __device__ __forceinline__ void k_post_b_tile(
     auto pair_terms = [&](float4 pj4, const Nb &nb) {
         const float3 diff = pi - f3(pj4);
         const float d2 = len2(diff);
-        if (!(d2 > 0.f)) return;
+        // the last two hold for the lists pass A records, not for substep lists
+        const bool ok = d2 > 0.f && d2 <= C.h2 && phase_of(pj4) == phi;
         const float inv_r = rsqrtf(d2);
-        if (want_v) eta = fma3(nb.om, spiky_grad_r(C, diff, d2, inv_r), eta);
-        if (want_t) {
+        const float3 g = spiky_grad_r(C, diff, d2, inv_r);
+        if (ok && want_v) eta = fma3(nb.om, g, eta);
+        if (ok && want_t) {
             const float4 nj4 = nb.nm;
             const float dist = __fmul_rn(d2, inv_r);
             const float3 fco = __fmul_rn(__fmul_rn(-C.tension, akinci_spline(C, dist)), inv_r) * diff;
@@ -613,10 +877,9 @@ __device__ __forceinline__ void k_post_b_tile(
     // pair terms of a record
     auto listed = [&](int, float4 pj4, const Nb &nb) { pair_terms(pj4, nb); };
     if (cnt != kWalkCells && slots) {
-        for_each_in_list_with(C.nbr, C.n, t, cnt, C.cls_pos,
-                              [&](int q) { return fetch_at(C.cls_om, C.cls_nm, q); }, listed);
+        for_each_padded(C.nbr, C.n, t, cnt, C.cls_pos, [&](int q) { return fetch_at(C.cls_om, C.cls_nm, q); }, listed);
     } else if (cnt != kWalkCells) {
-        for_each_in_list_with(C.nbr, C.n, t, cnt, P, [&](int j) { return fetch_at(Om, Nm, j); }, listed);
+        for_each_padded(C.nbr, C.n, t, cnt, P, [&](int j) { return fetch_at(Om, Nm, j); }, listed);
     } else {
         walk_neighbors<Split>(
             i, pi, 0, P, grid_view(C, sc, off), C, Stage ? &S : nullptr, g,
@@ -696,16 +959,26 @@ __device__ __forceinline__ void k_post_c_tile(
     int own = -1;
     // reference mode: each entry's velocity loads with its position, before
     // the four pair terms of a record
-    auto listed = [&](int, float4 pj4, float4 vj4) { vn = fma3(poly6(C, len2(pi - f3(pj4))), f3(vj4) - vi, vn); };
+    // substep lists also hold the own entry, other phases and entries past h
+    const int me = post_slots(C, Stage) ? t : i;
+    auto keep = [&](int j, float4 pj4, float d2) { return j != me && phase_of(pj4) == phi && d2 <= C.h2; };
+    auto listed = [&](int j, float4 pj4, float4 vj4) {
+        const float d2 = len2(pi - f3(pj4));
+        if (keep(j, pj4, d2)) vn = fma3(poly6(C, d2), f3(vj4) - vi, vn);
+    };
     if (cnt != kWalkCells && post_slots(C, Stage) && !C.textbook) {  // V: pass B's output, in class order
-        for_each_in_list_with(C.nbr, C.n, t, cnt, C.cls_pos, [&](int q) { return C.cls_vb[q]; }, listed);
+        for_each_padded(C.nbr, C.n, t, cnt, C.cls_pos, [&](int q) { return C.cls_vb[q]; }, listed);
     } else if (cnt != kWalkCells && !C.textbook) {
-        for_each_in_list_with(C.nbr, C.n, t, cnt, P, [&](int j) { return V[j]; }, listed);
+        for_each_padded(C.nbr, C.n, t, cnt, P, [&](int j) { return V[j]; }, listed);
     } else if (cnt != kWalkCells && post_slots(C, Stage)) {
         for_each_in_list(C.nbr, C.n, t, cnt, C.cls_pos,
-                         [&](int q, float4 pj4) { body_at(C.cls_vb, C.cls_mass, C.cls_rho, q, pj4); });
+                         [&](int q, float4 pj4) {
+                             if (keep(q, pj4, len2(pi - f3(pj4)))) body_at(C.cls_vb, C.cls_mass, C.cls_rho, q, pj4);
+                         });
     } else if (cnt != kWalkCells) {
-        for_each_in_list(C.nbr, C.n, t, cnt, P, body);
+        for_each_in_list(C.nbr, C.n, t, cnt, P, [&](int j, float4 pj4) {
+            if (keep(j, pj4, len2(pi - f3(pj4)))) body(j, pj4);
+        });
     } else if (C.nbr && !C.nbr_count) {
         // no pass A before it: record the walk's pairs, then sum over them
         ListWriter list(C.nbr, C.nbr_cap, C.n, t);
@@ -737,6 +1010,140 @@ __global__ void __launch_bounds__(kScanThreads, BP_POSTBC_MIN_BLOCKS) k_post_c(
     } else {
         k_post_c_tile<Split, Stage>(C, P, V, off, mass, rho, Vout, blockIdx.x * blockDim.x);
     }
+}
+
+// A neighbour's velocity and density, as pass A's pair terms read them.
+struct PostANeighbour {
+    float3 v;
+    float rho;
+};
+__device__ __forceinline__ PostANeighbour post_a_neighbour(const SimConsts &C, const float4 *__restrict__ V,
+                                                           const float *__restrict__ rho, int j)
+{
+    PostANeighbour r;
+    r.v = C.use_vort ? f3(V[j]) : make_float3(0.f, 0.f, 0.f);
+    r.rho = C.use_akinci ? __ldg(rho + j) : 0.f;
+    return r;
+}
+__device__ __forceinline__ void finish_post_a(const SimConsts &C, bool slots, int i, int t, float3 om, float3 nn,
+                                              const float *__restrict__ rho, float4 *__restrict__ Om,
+                                              float4 *__restrict__ Nm)
+{
+    const float4 om4 = make_float4(om.x, om.y, om.z, len3(om));
+    const float3 n = C.h * nn;
+    const float4 nm4 = make_float4(n.x, n.y, n.z, rho[i]);
+    Om[i] = om4;
+    Nm[i] = nm4;
+    if (slots) {
+        C.cls_om[t] = om4;
+        C.cls_nm[t] = nm4;
+    }
+}
+
+// Pass A over the substep lists: the sums of k_post_a, from the same pairs in
+// the same order (post_slots() equals classes_on() with them).
+__global__ void __launch_bounds__(kScanThreads, BP_POSTBC_MIN_BLOCKS) k_post_a_lists(
+    SimConsts C, const float4 *__restrict__ P, const float4 *__restrict__ V, const float *__restrict__ rho,
+    const int *__restrict__ off, float4 *__restrict__ Om, float4 *__restrict__ Nm)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= C.n) return;
+    const bool slots = post_slots(C, false);
+    const int i = slots ? __ldg(C.cls_perm + t) : t;
+    const float4 pi4 = slots ? C.cls_pos[t] : P[i];
+    const int phi = phase_of(pi4);
+    if (phi >= 0) return;
+    const float3 pi = f3(pi4);
+    if (!reads_substep_list(C, t, i, pi, cell_of(pi, C), grid_view(C, scene_index(C, i), off))) return;
+    const int cnt = __ldg(C.nbr_count + t) & 0xffff;
+    const float4 *__restrict__ src = slots ? C.cls_pos : P;
+    const float4 *__restrict__ vs = slots ? C.cls_vel : V;
+    const float *__restrict__ rs = slots ? C.cls_rho : rho;
+    const float3 vi = f3(vs[t]);
+    float3 om = make_float3(0.f, 0.f, 0.f), nn = make_float3(0.f, 0.f, 0.f);
+    for_each_padded(
+        C.nbr, C.n, t, cnt, src, [&](int j) { return post_a_neighbour(C, vs, rs, j); },
+        [&](int, float4 pj4, const PostANeighbour &nb) {
+            const float3 diff = pi - f3(pj4);
+            const float d2 = len2(diff);
+            const bool ok = d2 > 0.f && d2 <= C.h2 && phase_of(pj4) == phi;
+            const float3 g = spiky_grad_r(C, diff, d2, rsqrtf(d2));
+            const float3 w = cross3(nb.v - vi, g);
+            if (ok && C.use_vort) om += w;
+            if (ok && C.use_akinci) nn = fma3(__frcp_rn(nb.rho), g, nn);
+        });
+    finish_post_a(C, slots, i, t, om, nn, rho, Om, Nm);
+}
+
+// The queued particles' pass A, as k_lambda_queued: a queued particle leaves
+// its neighbours within h in its list for passes B and C.
+__global__ void __launch_bounds__(kQueueThreads) k_post_a_queued(SimConsts C, const float4 *__restrict__ P,
+                                                                const float4 *__restrict__ V,
+                                                                const float *__restrict__ rho,
+                                                                const int *__restrict__ off, float4 *__restrict__ Om,
+                                                                float4 *__restrict__ Nm)
+{
+    __shared__ WarpRows rows[kQueueThreads / 32];
+    __shared__ WarpHits hits[kQueueThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int queued = C.sl_count[C.sl_pass];
+    adapt_skin(C);
+    const bool slots = post_slots(C, false);
+    const float4 *__restrict__ vs = slots ? C.cls_vel : V;
+    const float *__restrict__ rs = slots ? C.cls_rho : rho;
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) / 32; k < queued; k += gridDim.x * blockDim.x / 32) {
+        const int t = C.sl_queue[k];
+        const int i = slots ? __ldg(C.cls_perm + t) : t;
+        const float4 pi4 = slots ? C.cls_pos[t] : P[i];
+        const int phi = phase_of(pi4);
+        const float3 pi = f3(pi4), vi = f3(vs[t]);
+        if (C.nl_stats && slots && lane == 0) atomicAdd(C.nl_stats + 4, 1u);
+        float acc = 0.f;  // lanes 0..2: omega, 3..5: the normal
+        auto test = [&](int q, float4 pj) { return len2(pi - f3(pj)) <= C.h2 && phase_of(pj) == phi && q != t; };
+        auto batch = [&](int k0, int n, int q, float4 pj) {
+            const bool in = lane < n;
+            if (in) put_entry(C, t, k0 + lane, q);
+            float value[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            float scale = 0.f;
+            const float3 diff = pi - f3(pj);
+            const float d2 = len2(diff);
+            const bool apart = in && d2 > 0.f;
+            if (apart) {
+                const PostANeighbour nb = post_a_neighbour(C, vs, rs, q);
+                const float3 g = spiky_grad_r(C, diff, d2, rsqrtf(d2));
+                const float3 w = cross3(nb.v - vi, g);
+                value[0] = w.x;
+                value[1] = w.y;
+                value[2] = w.z;
+                value[3] = g.x;
+                value[4] = g.y;
+                value[5] = g.z;
+                scale = __frcp_rn(nb.rho);
+            }
+            warp_add<6, true>(rows[threadIdx.x >> 5], __ballot_sync(kWarp, apart), value, scale, acc);
+        };
+        const int cnt = warp_neighbors(C, slots, cell_of(pi, C), P, grid_view(C, scene_index(C, i), off),
+                                       hits[threadIdx.x >> 5], test, batch);
+        warp_pad(C, t, cnt, t);
+        float sum[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sum[q] = __shfl_sync(kWarp, acc, q);
+        if (lane != 0) continue;
+        C.nbr_count[t] = cnt <= C.nbr_cap ? cnt : -1;
+        const float3 zero = make_float3(0.f, 0.f, 0.f);
+        finish_post_a(C, slots, i, t, C.use_vort ? make_float3(sum[0], sum[1], sum[2]) : zero,
+                      C.use_akinci ? make_float3(sum[3], sum[4], sum[5]) : zero, rho, Om, Nm);
+    }
+}
+
+void launch_post_a_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,
+                         const int *off, float4 *Om, float4 *Nm, LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    k_post_a_lists<<<(C.n + C.scan_block - 1) / C.scan_block, C.scan_block, 0, st>>>(C, P, V, rho, off, Om, Nm);
+    L->done("launch_post_a_lists");
+    k_post_a_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, V, rho, off, Om, Nm);
+    L->done("launch_post_a_queued");
 }
 
 void launch_post_a(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,

@@ -131,6 +131,15 @@ void launch_walk_planes(cudaStream_t st, int n, const float4 *P, float *planes, 
 // ---- fluid kernels ----
 void launch_lambda(cudaStream_t st, const SimConsts &C, const float4 *P, const float *mass, const int *off,
                    float *lam, float *rho, LaunchLog *L);
+// The same over the substep lists (SimConsts::sl_pos): record them (and the
+// contact partners; without a fluid stage nothing else), or read them (then
+// also a launch over the particles that may not).
+void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const float *mass,
+                         const int *off, float *lam, float *rho, LaunchLog *L);
+void launch_post_a_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,
+                         const int *off, float4 *Om, float4 *Nm, LaunchLog *L);
+void launch_contacts_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *Xs, const float *w,
+                           const int *off, float4 *Pout, LaunchLog *L);
 struct DeltaArgs {
     const float4 *P;
     const float *mass, *lam;

@@ -1,0 +1,257 @@
+// bp_lists.cuh -- substep lists: one neighbour search per substep
+// (SimConsts::sl_pos).  What the passes over them share: who may read a list,
+// the queue of those that may not, the walk of a queued particle by a whole
+// warp, and the skin.
+#pragma once
+
+#include <algorithm>
+
+#include "bp_internal.h"
+#include "bp_walk.cuh"
+
+namespace bp {
+
+constexpr unsigned kWarp = 0xffffffffu;
+
+// What a pass over the substep lists does: records them (the substep's first
+// lambda pass) or reads them (and queues the particles that may not).
+enum ListPass { kRecordLists, kReadLists };
+
+// Appends t to a queue (nullptr: only counts it).
+__device__ __forceinline__ void append_to(int *count, int *queue, int t)
+{
+    const unsigned m = __activemask();
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(count, __popc(m));
+    if (!queue) return;
+    base = __shfl_sync(m, base, leader);
+    queue[base + __popc(m & ((1u << lane) - 1u))] = t;
+}
+
+// May the particle of slot t, at pi, read its list in this pass?  Queues it
+// where not.
+// (fits: its list holds all it should.)
+__device__ __forceinline__ bool reads_substep_list(const SimConsts &C, int t, int i, float3 p, int3 c,
+                                                   const GridView &v, bool fits = true)
+{
+    int state = substep_list_state(C, t, i, p, v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask));
+    if (state != 0) C.sl_cell[t] = state == 3 ? kListMoved : kListNone;
+    else if (!fits) state = 1;
+    if (C.nl_stats) atomicAdd(C.nl_stats + state, 1u);
+    if (state == 0) return true;
+    append_to(C.sl_count + C.sl_pass, C.sl_queue, t);
+    if (C.sl_adapt && state == 3) append_to(C.sl_count + kSlDisplaced, nullptr, t);
+    return false;
+}
+
+// The skin of the next substep's lists, from how many particles the last pass
+// over this one's could not read theirs because something near them had moved
+// too far.  A list read costs about (1 + skin / h)^3 and a queued walk about
+// ten reads, so the break-even lies at a few queued particles in a hundred;
+// their share falls steeply with the skin (1M-particle dam break, frame 20:
+// 45 % at 0.03 h, 24 % at 0.05 h, 0.6 % at 0.1 h), so it shrinks slowly and
+// stays off the last value that was too small, which it forgets slowly too.
+// The results do not depend on the skin.
+__device__ __forceinline__ void adapt_skin(const SimConsts &C)
+{
+    if (!C.sl_adapt || blockIdx.x != 0 || threadIdx.x != 0) return;
+    const long long moved = C.sl_count[kSlDisplaced];
+    float skin = C.sl_skin[0], bad = C.sl_skin[1] * 0.998f;
+    if (moved * 25 > C.n) {
+        bad = skin;
+        skin = fminf(skin * 1.3f, C.h * kMaxSkin);
+    } else if (moved * 100 < C.n) {
+        skin = fmaxf(skin * 0.9f, fmaxf(fminf(bad * 1.15f, skin), C.h * kMinSkin));
+    }
+    C.sl_skin[0] = skin;
+    C.sl_skin[1] = bad;
+}
+
+// Records the candidates within sqrt(r2) of slot t's particle (sorted index
+// i) into its list, in walk order and its own entry included; returns what
+// nbr_count holds (entries | own entry's index << 16, or -1: overflow).
+__device__ __forceinline__ int record_substep_list(const SimConsts &C, const float4 *__restrict__ P, bool slots, int t,
+                                                   int i, float3 pi, int3 c, float r2, const GridView &v)
+{
+    ListWriter list(C.nbr, C.nbr_cap, C.n, t);
+    int self = 0;
+    const int me = slots ? t : i;
+    // the walk planes hold the order this walk reads, except where a particle
+    // left the classes' reach after they were written
+    const int planes = walk_planes_order(C);
+    if (planes == (slots ? 2 : 1)) {
+        record_walk_planes(planes, pi, r2, v, C, [&](int c0, unsigned bits) {
+            const unsigned d = (unsigned)(me - c0);
+            if (d < 32u && ((bits >> d) & 1u)) self = list.cnt + __popc(bits & ((1u << d) - 1u));
+            list.push_bits(c0, bits);
+        });
+    } else {
+        if (C.nl_stats) atomicAdd(C.nl_stats + 1, 1u);
+        auto push = [&](int j, float4) {
+            if (j == me) self = list.cnt;
+            list.push(j);
+        };
+        auto test = [&](int, float4 pj) { return len2(pi - f3(pj)) <= r2; };
+        walk_table<true>(c, 0, P, v, nullptr, -1, test, push);
+    }
+    const int cnt = list.finish(me);
+    return cnt < 0 ? -1 : cnt | (self << 16);
+}
+
+// ---- walks by a whole warp ----
+
+// The candidates of the 27-cell walk of real cell c, in walk order, 32 at a
+// time: chunk(q, p, in) on every lane, q = the lane's candidate and p its
+// position (in: it has one).  slots: the class walk (q a class position, read
+// from C.cls_pos), else the table walk (q a sorted index, read from P).  Every
+// lane of the warp takes part, with the same particle.
+// One thread's walk is a serial chain of about 30 dependent loads and 9 loops
+// whose length bounds a launch with few walkers; a warp takes a run's
+// candidates at once, five runs' loads in flight (32,768-particle dam break,
+// 1000 walkers: 59 us a launch with a thread each, 43 us with 8 lanes each,
+// whose four groups diverge).
+template <class F>
+__device__ __forceinline__ void warp_walk(const SimConsts &C, bool slots, int3 c, const float4 *__restrict__ P,
+                                          const GridView &v, F &&chunk)
+{
+    constexpr int kAhead = 5;  // runs
+    const int lane = threadIdx.x & 31;
+    const unsigned m = v.mask, D = (unsigned)v.D;
+    const int sh = __ffs(v.D) - 1;
+    const unsigned z0 = (unsigned)(c.z - 1) & m, z2 = (unsigned)(c.z + 1) & m;
+    const bool wrap = !(z0 < z2);
+    const int runs = wrap ? 18 : 9;  // 9 columns, two pieces each where z wraps around the table
+    const float4 *__restrict__ src = slots ? C.cls_pos : P;
+    int rb = 0, re = 0;  // lane r finds the ends of run r
+    if (lane < runs) {
+        const int col = wrap ? lane >> 1 : lane, piece = wrap ? lane & 1 : 0;
+        const int xr = c.x + col / 3 - 1, yr = c.y + col % 3 - 1;
+        const unsigned base = ((unsigned)xr & m) * D * D + ((unsigned)yr & m) * D;
+        const unsigned za = piece ? 0u : z0, zb = wrap ? (piece ? z2 : D - 1u) : z2;
+        const int *__restrict__ o = v.off + base;
+        if (slots) {
+            const int zr = piece ? c.z + 1 : c.z - 1;
+            const int cls = ((xr >> sh) & 1) | (((yr >> sh) & 1) << 1) | (((zr >> sh) & 1) << 2);
+            o = C.cls_off + v.base + (size_t)cls * (size_t)C.cls_T + base;
+        }
+        rb = __ldg(o + za);
+        re = __ldg(o + zb + 1);
+    }
+#pragma unroll 1
+    for (int r = 0; r < runs; r += kAhead) {
+        int b[kAhead], e[kAhead];
+        float4 p[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            b[u] = __shfl_sync(0xffffffffu, rb, r + u);  // lanes past the last run hold an empty one
+            e[u] = __shfl_sync(0xffffffffu, re, r + u);
+            p[u] = b[u] + lane < e[u] ? src[b[u] + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+#pragma unroll 1
+            for (int q0 = b[u]; q0 < e[u]; q0 += 32) {
+                const int q = q0 + lane;
+                if (q0 != b[u]) p[u] = q < e[u] ? src[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+                chunk(q, p[u], q < e[u]);
+            }
+    }
+}
+
+// Sums of up to kWarpTerms quantities over a warp walk's pairs, in walk order:
+// lane c adds quantity c of each pair of a chunk from a row in shared memory
+// (a load and an add a pair for all of them together, instead of a shuffle a
+// quantity).
+constexpr int kWarpTerms = 7;  // odd: a warp's rows fall into different banks
+using WarpRows = float[32][kWarpTerms];
+// The lanes of `take` add value[0..N) to acc of lanes 0..N, in lane order;
+// lanes 3..5 add scale * value with one rounding where Scaled.
+template <int N, bool Scaled = false>
+__device__ __forceinline__ void warp_add(WarpRows &rows, unsigned take, const float (&value)[N], float scale, float &acc)
+{
+    static_assert(N + (Scaled ? 1 : 0) <= kWarpTerms, "a row holds kWarpTerms quantities");
+    const int lane = threadIdx.x & 31;
+    if ((take >> lane) & 1u) {
+        float *row = rows[__popc(take & ((1u << lane) - 1u))];
+#pragma unroll
+        for (int k = 0; k < N; ++k) row[k] = value[k];
+        if (Scaled) row[N] = scale;
+    }
+    __syncwarp();
+    if (lane < N) {
+        const int n = __popc(take);
+#pragma unroll 4
+        for (int r = 0; r < n; ++r)
+            acc = (Scaled && lane >= 3) ? __fmaf_rn(rows[r][N], rows[r][lane], acc) : __fadd_rn(acc, rows[r][lane]);
+    }
+    __syncwarp();
+}
+
+// The candidates of the 27-cell walk of real cell c that pass test(q, p), in
+// walk order, in batches of up to 32: batch(k0, n, q, p) on every lane, the
+// lanes below n holding hits k0 + lane.  Hits collect in shared memory until a
+// batch is full, so that what batch() gathers for them is one round of loads
+// for 32 hits instead of one for each run (mixed scene of 150k particles, 13k
+// walkers: 28 us a launch with a gather per run).
+struct WarpHits {
+    float4 p[64];
+    int q[64];
+};
+template <class T, class B>
+__device__ __forceinline__ int warp_neighbors(const SimConsts &C, bool slots, int3 c, const float4 *__restrict__ P,
+                                              const GridView &v, WarpHits &buf, T &&test, B &&batch)
+{
+    const int lane = threadIdx.x & 31;
+    int done = 0, held = 0;
+    warp_walk(C, slots, c, P, v, [&](int q, float4 p, bool in) {
+        const bool hit = in && test(q, p);
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (!hits) return;
+        if (hit) {
+            const int k = held + __popc(hits & ((1u << lane) - 1u));
+            buf.p[k] = p;
+            buf.q[k] = q;
+        }
+        held += __popc(hits);
+        __syncwarp();
+        if (held < 32) return;
+        batch(done, 32, buf.q[lane], buf.p[lane]);
+        done += 32;
+        held -= 32;
+        const float4 rp = buf.p[32 + lane];
+        const int rq = buf.q[32 + lane];
+        __syncwarp();
+        buf.p[lane] = rp;
+        buf.q[lane] = rq;
+        __syncwarp();
+    });
+    if (held) batch(done, held, buf.q[lane], buf.p[lane]);
+    __syncwarp();
+    return done + held;
+}
+
+// Writes entry k of slot t's list (layout of ListWriter) where it fits.
+__device__ __forceinline__ void put_entry(const SimConsts &C, int t, int k, int q)
+{
+    if (k < C.nbr_cap) C.nbr[((size_t)(k >> 2) * C.n + t) * 4 + (k & 3)] = q;
+}
+// Fills up the last record of a list of cnt entries (ListWriter::finish(pad)).
+__device__ __forceinline__ void warp_pad(const SimConsts &C, int t, int cnt, int pad)
+{
+    const int k = cnt + (threadIdx.x & 31);
+    if ((cnt & 3) && k < ((cnt + 3) & ~3) && k < C.nbr_cap) C.nbr[((size_t)(k >> 2) * C.n + t) * 4 + (k & 3)] = pad;
+}
+
+// CTAs of `threads` for a launch over the queue, a warp per entry, whose length
+// only the device knows.
+inline int queue_blocks(int n, int threads)
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int per = threads / 32;
+    return std::min((n + per - 1) / per, std::max(sms, 1) * 8);
+}
+
+}  // namespace bp

@@ -137,6 +137,14 @@ struct bp_solver {
     float2 *lm = nullptr;  // (lambda, mass) per sorted particle (SimConsts::lm)
     float *walk_xyz = nullptr;  // walk planes (SimConsts::walk_xyz): 4 planes of walk_stride floats
     int walk_stride = 0;
+    // substep lists (SimConsts::sl_pos): the cell each was recorded in, the
+    // queue of the particles that may not read theirs, the counts, the cell
+    // bits (sl_words each: moved, then near) and the skin
+    int *sl_cell = nullptr, *sl_queue = nullptr, *sl_count = nullptr;
+    unsigned *sl_bits = nullptr;
+    float *sl_skin = nullptr;
+    int *cl_list = nullptr, *cl_count = nullptr;  // contact partners (SimConsts::cl_list), with solids
+    size_t sl_words = 0;
     SortScratch sort{};
     // alias classes (SimConsts::cls_perm); cls.perm == nullptr: not allocated
     // (key spaces above kClassMaxCells cells)

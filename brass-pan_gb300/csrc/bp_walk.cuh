@@ -347,6 +347,15 @@ struct ListWriter {
         if ((cnt & 3) && cnt < cap) rec[(size_t)(cnt >> 2) * stride] = buf;
         return cnt <= cap ? cnt : -1;
     }
+    // The same, the last record filled up with `pad` (for_each_padded).
+    __device__ __forceinline__ int finish(int pad)
+    {
+        const int q = cnt & 3;
+        if (q < 2) buf.y = pad;
+        if (q < 3) buf.z = pad;
+        buf.w = pad;
+        return finish();
+    }
 };
 
 // The cnt entries of particle i's list, in order: f(j, P[j]).  Each record's
@@ -413,6 +422,45 @@ __device__ __forceinline__ void for_each_in_list_with(const int *base, int n, in
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             if (q < m) f(j[q], pj[q], xj[q]);
+    }
+}
+
+#ifndef BP_LIST_AHEAD
+#define BP_LIST_AHEAD 2
+#endif
+// As for_each_in_list_with, for lists whose last record is filled up with
+// entries that f drops (ListWriter::finish(pad)): every record is read whole,
+// without a test per entry, f(j, P[j], fetch(j)) for the entries and the
+// padding.
+template <bool ReadOnly = true, class G, class F>
+__device__ __forceinline__ void for_each_padded(const int *base, int n, int i, int cnt, const float4 *__restrict__ P,
+                                                G &&fetch, F &&f, int first = 0)
+{
+    using T = decltype(fetch(0));
+    const int4 *rec = reinterpret_cast<const int4 *>(base) + i;
+    const size_t stride = (size_t)n;
+    auto load = [&](int k) {
+        const int4 *rp = rec + (size_t)(k >> 2) * stride;
+        return ReadOnly ? __ldg(rp) : *rp;
+    };
+    int4 next = first < cnt ? load(first) : make_int4(0, 0, 0, 0);
+#pragma unroll 1
+    for (int k = first; k < cnt; k += 4) {
+        const int j[4] = {next.x, next.y, next.z, next.w};
+        if (k + 4 < cnt) next = load(k + 4);
+#if BP_LIST_AHEAD
+        if (k + 4 * BP_LIST_AHEAD < cnt)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + (size_t)((k >> 2) + BP_LIST_AHEAD) * stride));
+#endif
+        float4 pj[4];
+        T xj[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            pj[q] = P[j[q]];
+            xj[q] = fetch(j[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) f(j[q], pj[q], xj[q]);
     }
 }
 
@@ -509,6 +557,39 @@ __device__ __forceinline__ void walk_classes(int i, int3 c, int lo, const GridVi
     }
 }
 
+// The 27-cell walk of real cell c over whole table cells: 9 column runs,
+// split where z wraps around the table, candidates j >= lo.  S != nullptr:
+// read from the CTA's staged runs (column group g) where they hold the run.
+template <bool Split, bool Ranged = false, class T, class B>
+__device__ __forceinline__ void walk_table(int3 c, int lo, const float4 *__restrict__ P, const GridView &v,
+                                           const StageShared *S, int g, T &test, B &body, CellRange rg = CellRange{})
+{
+    const unsigned m = v.mask;
+    const unsigned D = (unsigned)v.D;
+    const int *__restrict__ off = v.off;
+    const unsigned z0 = (unsigned)(c.z + (Ranged ? rg.loz : -1)) & m;
+    const unsigned z2 = (unsigned)(c.z + (Ranged ? rg.hiz : 1)) & m;
+    const bool wrap = (Ranged && rg.hiz - rg.loz != 2) ? z0 > z2 : !(z0 < z2);
+#pragma unroll 1
+    for (int col = 0; col < 9; ++col) {
+        if constexpr (Ranged) {
+            const int dx = col / 3 - 1, dy = col % 3 - 1;
+            if (dx < rg.lox || dx > rg.hix || dy < rg.loy || dy > rg.hiy) continue;
+        }
+        const unsigned x = (unsigned)(c.x + col / 3 - 1) & m, y = (unsigned)(c.y + col % 3 - 1) & m;
+        const unsigned base = x * D * D + y * D;
+#pragma unroll 1
+        for (int piece = 0; piece < (wrap ? 2 : 1); ++piece) {
+            const unsigned za = (wrap && piece == 1) ? 0u : z0;
+            const unsigned zb = wrap ? (piece == 0 ? D - 1 : z2) : z2;
+            const int b = __ldg(off + base + za), e = __ldg(off + base + zb + 1);
+            const int sidx = S ? staged_index(*S, g, col, b, e) : -1;
+            const float4 *src = sidx >= 0 ? S->pos + sidx : P + b;
+            walk_run<Split>(max(b, lo), b, e, src, test, body);
+        }
+    }
+}
+
 // Walk of particle i (sorted index) at position pi over the candidates
 // j >= lo of its 27 cells on grid v: body(j, P[j]) for every j with
 // test(j, P[j]).  S / g come from stage_block (S == nullptr or g < 0: no
@@ -524,9 +605,6 @@ __device__ __forceinline__ void walk_neighbors(int i, float3 pi, int lo, const f
                                                T &&test, B &&body, CellRange rg = CellRange{})
 {
     const int3 c = cell_of(pi, C);
-    const unsigned m = v.mask;
-    const unsigned D = (unsigned)v.D;
-    const int *__restrict__ off = v.off;
     const bool staged = walks_staged(C, v, i, c, S, g);
     const int state = (C.vl && !C.vl_build) ? list_state(C, i, c, pi) : 1;
     if (C.nl_stats) atomicAdd(C.nl_stats + state, 1u);
@@ -536,35 +614,13 @@ __device__ __forceinline__ void walk_neighbors(int i, float3 pi, int lo, const f
         });
         return;
     }
-    const unsigned z0 = (unsigned)(c.z + (Ranged ? rg.loz : -1)) & m;
-    const unsigned z2 = (unsigned)(c.z + (Ranged ? rg.hiz : 1)) & m;
 
     if (C.cls_perm && !staged && __ldg(C.cls_moved) == 0) {
         if (C.nl_stats) atomicAdd(C.nl_stats + 4, 1u);
         walk_classes<Split, false, Ranged>(i, c, lo, v, C, test, body, rg);
         return;
     }
-
-    // 27-cell walk: 9 column runs, split where z wraps around the table
-    const bool wrap = (Ranged && rg.hiz - rg.loz != 2) ? z0 > z2 : !(z0 < z2);
-#pragma unroll 1
-    for (int col = 0; col < 9; ++col) {
-        if constexpr (Ranged) {
-            const int dx = col / 3 - 1, dy = col % 3 - 1;
-            if (dx < rg.lox || dx > rg.hix || dy < rg.loy || dy > rg.hiy) continue;
-        }
-        const unsigned x = (unsigned)(c.x + col / 3 - 1) & m, y = (unsigned)(c.y + col % 3 - 1) & m;
-        const unsigned base = x * D * D + y * D;
-#pragma unroll 1
-        for (int piece = 0; piece < (wrap ? 2 : 1); ++piece) {
-            const unsigned za = (wrap && piece == 1) ? 0u : z0;
-            const unsigned zb = wrap ? (piece == 0 ? D - 1 : z2) : z2;
-            const int b = __ldg(off + base + za), e = __ldg(off + base + zb + 1);
-            const int sidx = staged ? staged_index(*S, g, col, b, e) : -1;
-            const float4 *src = sidx >= 0 ? S->pos + sidx : P + b;
-            walk_run<Split>(max(b, lo), b, e, src, test, body);
-        }
-    }
+    walk_table<Split, Ranged>(c, lo, P, v, staged ? S : nullptr, g, test, body, rg);
 }
 
 // ---- recording walks over the walk planes (SimConsts::walk_xyz) ----

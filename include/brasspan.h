@@ -141,8 +141,10 @@ typedef struct bp_params {
     float wind_drag;             /* 10 (wind.cuh:40) */
     float wind_lift;             /* 100 (wind.cuh:43) */
     int32_t rotation_iterations; /* 20 (shapematching.cuh:72) */
-    float neighbor_skin;         /* skin of the per-substep Verlet lists, as a fraction of h
-                                    (0 disables them; results are identical either way): 0 */
+    float neighbor_skin;         /* skin of the per-substep neighbour lists, as a fraction of h
+                                    (results are identical under any): 0, which lets the unstaged
+                                    split walks over the walk planes adapt it to the displacements
+                                    they meet and turns the lists off for the other walks */
     int32_t walk_options;        /* BP_WALK_* tuning switches of the neighbour walks:
                                     BP_WALK_NO_STAGING | BP_WALK_NO_CONTACT_CULLING */
     float bending_stiffness;     /* 0.8 (bending.cuh:71) */
@@ -294,12 +296,12 @@ bp_status bp_solver_profile(bp_solver *s, int32_t num_substeps, float dt, int32_
                             int32_t capacity, bp_stage_time *out, int32_t *count);
 
 /* One real update that also counts the neighbour walks of every scan pass:
- * out_walks[0] walks over the per-substep Verlet lists; 27-cell walks
- * because [1] no list was built for the particle (lists are off, the pass
- * builds them, its column runs wrap around the table, or its list held more
- * than 256 candidates), [2] the particle left the cell its list was built
- * for, [3] it or a particle stored in its 27 cells moved more than half the
- * skin; [4] of the cell walks, those restricted to the alias classes. */
+ * out_walks[0] walks over the per-substep lists; 27-cell walks
+ * because [1] there is no list for the particle (lists are off, the pass
+ * builds them, its candidates did not fit, or an earlier pass found it had
+ * left its cell), [2] the particle left the cell its list was built
+ * for, [3] it and a particle stored in its 27 cells moved more than the
+ * skin allows; [4] of the cell walks, those restricted to the alias classes. */
 bp_status bp_solver_walk_stats(bp_solver *s, int32_t num_substeps, float dt, int32_t iterations,
                                uint64_t out_walks[5]);
 
