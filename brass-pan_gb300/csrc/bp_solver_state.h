@@ -32,6 +32,7 @@ using namespace bp;
 
 namespace bp {
 void destroy_tape(Tape *t);  // frees a recording (bp_backward.cu)
+void retire_tape(bp_solver *s);  // ends s->tape; its buffers and graphs wait in s->spare for the next recording
 
 // Stages of a substep as recorded for the adjoint.
 enum TapeStage : int {
@@ -177,11 +178,13 @@ struct bp_solver {
     int64_t last_launches = 0;
 
     bp::Tape *tape = nullptr;  // recording for bp_solver_backward (nullptr: not recording)
+    bp::Tape *spare = nullptr;  // an ended recording's buffers and graphs (retire_tape)
     bool tape_empty() const;   // no update recorded yet
 
     ~bp_solver()
     {
         if (tape) bp::destroy_tape(tape);
+        if (spare) bp::destroy_tape(spare);
         if (exec) cudaGraphExecDestroy(exec);
         for (void *p : allocs) cudaFree(p);
         if (own_stream && stream) cudaStreamDestroy(stream);
@@ -250,14 +253,18 @@ struct StateSnapshot {
     {
         for (void *p : copies) cudaFree(p);
     }
+    // the buffers of an earlier take() of the same solver are used again
     bp_status take(bp_solver *s)
     {
         bufs = state_buffers(s);
-        for (auto &b : bufs) {
-            void *p = nullptr;
-            if (cudaMalloc(&p, b.second) != cudaSuccess) return bp::fail_with(BP_ERR_OUT_OF_MEMORY, "state snapshot");
-            copies.push_back(p);
-            cudaMemcpyAsync(p, b.first, b.second, cudaMemcpyDeviceToDevice, s->stream);
+        for (size_t k = 0; k < bufs.size(); ++k) {
+            if (k == copies.size()) {
+                void *p = nullptr;
+                if (cudaMalloc(&p, bufs[k].second) != cudaSuccess)
+                    return bp::fail_with(BP_ERR_OUT_OF_MEMORY, "state snapshot");
+                copies.push_back(p);
+            }
+            cudaMemcpyAsync(copies[k], bufs[k].first, bufs[k].second, cudaMemcpyDeviceToDevice, s->stream);
         }
         pcur = s->Pcur;
         return BP_OK;
