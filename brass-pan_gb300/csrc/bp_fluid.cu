@@ -1168,27 +1168,65 @@ void launch_post_c(cudaStream_t st, const SimConsts &C, const float4 *P, const f
     L->done(__func__);
 }
 
-// Same count on caller buffers in the reference's start/end format.
-__global__ void k_neighbor_counts_f3(int n, const float *__restrict__ pos3, float cell, int D, float h2,
-                                     const int *__restrict__ start, const int *__restrict__ end,
-                                     int *__restrict__ counts)
+// Same count on caller buffers in the reference's start/end format.  The three
+// cells of a column that do not wrap around the table are one run of sorted
+// positions (their keys are consecutive), from the first occupied one's start
+// to the last one's end: two loads find it where both ends are occupied, and
+// its positions are read in order, the twelve floats of four at a time.  Bound
+// by the latency and number of those loads (1,000,003 points, 128^3 table: 87
+// us; cell by cell, 27 pairs of loads a point, 154 us; three 16-byte loads for
+// four positions from the boundary below the run, 97 us).
+__device__ __forceinline__ int count_run(int b, int e, const float *__restrict__ pos3, float3 pi, float h2)
+{
+    int cnt = 0;
+    for (; b + 4 <= e; b += 4) {
+        float v[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k) v[k] = __ldg(pos3 + 3 * (size_t)b + k);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            cnt += len2(pi - make_float3(v[3 * k], v[3 * k + 1], v[3 * k + 2])) <= h2 ? 1 : 0;
+    }
+    for (; b < e; ++b) {
+        const float *p = pos3 + 3 * (size_t)b;
+        cnt += len2(pi - make_float3(__ldg(p), __ldg(p + 1), __ldg(p + 2))) <= h2 ? 1 : 0;
+    }
+    return cnt;
+}
+
+__global__ void __launch_bounds__(128) k_neighbor_counts_f3(int n, const float *__restrict__ pos3, float cell, int D,
+                                                            float h2, const int *__restrict__ start,
+                                                            const int *__restrict__ end, int *__restrict__ counts)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float3 pi = make_float3(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2]);
+    const float *pp = pos3 + 3 * (size_t)i;
+    const float3 pi = make_float3(pp[0], pp[1], pp[2]);
     const unsigned m = (unsigned)D - 1u;
     const int cx = cell_coord(pi.x, cell), cy = cell_coord(pi.y, cell), cz = cell_coord(pi.z, cell);
+    const unsigned z = (unsigned)cz & m;
     int cnt = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-                const int a = cell_addr(cx + dx, cy + dy, cz + dz, D, m);
-                const int b = start[a], e = end[a];
-                for (int j = b; j < e; ++j) {
-                    const float3 pj = make_float3(pos3[3 * j], pos3[3 * j + 1], pos3[3 * j + 2]);
-                    if (len2(pi - pj) <= h2) ++cnt;
-                }
+    for (int col = 0; col < 9; ++col) {
+        const int x = cx + col / 3 - 1, y = cy + col % 3 - 1;
+        if (z != 0u && z != m) {
+            const int a = cell_addr(x, y, cz - 1, D, m);
+            int b = __ldg(start + a), e = __ldg(end + a + 2);
+            if (b < 0) {
+                b = __ldg(start + a + 1);
+                if (b < 0) b = __ldg(start + a + 2);
             }
+            if (e < 0) {
+                e = __ldg(end + a + 1);
+                if (e < 0) e = __ldg(end + a);
+            }
+            if (b >= 0) cnt += count_run(b, e, pos3, pi, h2);
+        } else {
+            for (int dz = -1; dz <= 1; ++dz) {
+                const int a = cell_addr(x, y, cz + dz, D, m);
+                cnt += count_run(__ldg(start + a), __ldg(end + a), pos3, pi, h2);
+            }
+        }
+    }
     counts[i] = cnt;
 }
 
