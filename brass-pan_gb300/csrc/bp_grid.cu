@@ -8,7 +8,10 @@
 //   reorderParticlesData (kernel/grid.cuh:134-163)
 //   + inverseMapping    (kernel/util.cuh:348-358) -> k_reorder (float4 records, fused predict,
 //                                                    mass scaling and plane stabilisation)
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <type_traits>
 
 #include "bp_internal.h"
 
@@ -274,20 +277,21 @@ __device__ __forceinline__ float3 predict(float3 x, float3 v, float3 gr, const S
 // Cell key of the predicted position; in a batched ensemble the key of the
 // particle's scene grid, offset by the scene's first key.  Every particle of
 // a scene keeps its scene's index segment, so X/V index i has scene_of[i].
+__device__ __forceinline__ int state_key(const SimConsts &C, const float4 *__restrict__ X, const float4 *__restrict__ V,
+                                         int i)
+{
+    const int s = scene_index(C, i);
+    const float3 p = predict(f3(X[i]), f3(V[i]), gravity_of(C, s), C);
+    if (s < 0) return hash_key(p, C.cell, C.D, C.mask);
+    const SceneConsts &S = C.scn[s];
+    return S.base + hash_key(p, C.cell, S.D, S.mask);
+}
+
 __global__ void __launch_bounds__(kSortThreads) k_hash_state(SimConsts C, const float4 *__restrict__ X,
                                                              const float4 *__restrict__ V, int *__restrict__ keys,
                                                              int *__restrict__ hist, int tiles)
 {
-    hash_tile(
-        C.n,
-        [&](int i) {
-            const int s = scene_index(C, i);
-            const float3 p = predict(f3(X[i]), f3(V[i]), gravity_of(C, s), C);
-            if (s < 0) return hash_key(p, C.cell, C.D, C.mask);
-            const SceneConsts &S = C.scn[s];
-            return S.base + hash_key(p, C.cell, S.D, S.mask);
-        },
-        keys, hist, tiles);
+    hash_tile(C.n, [&](int i) { return state_key(C, X, V, i); }, keys, hist, tiles);
 }
 
 void launch_hash_f3(cudaStream_t st, int n, const float *pos3, float cell, int D, int *keys, int *hist,
@@ -306,6 +310,203 @@ void launch_hash_state(cudaStream_t st, const SimConsts &C, const float4 *X, con
     const int tiles = sort_tiles(C.n);
     k_hash_state<<<tiles, kSortThreads, 0, st>>>(C, X, V, keys, hist, tiles);
     L->done(__func__);
+}
+
+// ------------------------------------------------------------------------
+// hash and sort in one launch
+// ------------------------------------------------------------------------
+
+// Up to kClusterSortMax keys are hashed and sorted by one cluster of at most 8
+// CTAs: the same 9-bit digits, tiles, warp segments and ranks as the
+// hash / upsweep / scan / downsweep chain, with the tiles' digit counts
+// exchanged through distributed shared memory and cluster barriers in place of
+// the launches between.  Such sorts are bound by those launches: a substep's
+// hash and sort on a 64^3 table took 6 of them, 33 us and the gaps between
+// them for 32,768 particles, now one of 22 us (1,728 particles: 9 us; 128 x
+// 128 flag, a frame 219 -> 188 us).  Above it a cluster's 8 SMs are too few.
+constexpr int kClusterSortCtas = 8;  // the portable cluster size
+
+template <int Items, class KeyOf>
+__device__ __forceinline__ void sort_cluster(int n, int passes, KeyOf key_of, int *__restrict__ keys, int *keys_out,
+                                             int *vals_out, const SortScratch &s)
+{
+    namespace cg = cooperative_groups;
+    constexpr int W = kSortThreads / 32;
+    __shared__ __align__(16) int cnt[W][kRadixBins];
+    __shared__ int hist[kRadixBins], dbase[kRadixBins];
+    __shared__ int wsum[W];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tiles = (int)cluster.num_blocks(), tile = (int)cluster.block_rank();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;  // kSortThreads == kRadixBins
+    const int seg0 = (tile * W + warp) * 32 * Items;
+    const unsigned lt = (1u << lane) - 1u;
+    const int *ksrc = nullptr, *vsrc = nullptr;
+    for (int p = 0; p < passes; ++p) {
+        int *kdst = p == passes - 1 ? keys_out : s.keys_alt[p & 1];
+        int *vdst = p == passes - 1 ? vals_out : s.vals_alt[p & 1];
+        int key[Items], val[Items], loc[Items];
+        if (p == 0) {
+#pragma unroll
+            for (int r = 0; r < Items; ++r) {
+                const int idx = seg0 + r * 32 + lane;
+                key[r] = key_of(min(idx, n - 1));
+                val[r] = idx;
+            }
+#pragma unroll
+            for (int r = 0; r < Items; ++r)
+                if (val[r] < n) keys[val[r]] = key[r];
+        } else {
+#pragma unroll
+            for (int r = 0; r < Items; ++r) {  // written by other SMs: past the L1 cache
+                const int idx = min(seg0 + r * 32 + lane, n - 1);
+                key[r] = __ldcg(ksrc + idx);
+                val[r] = __ldcg(vsrc + idx);
+            }
+        }
+        int4 *zero = reinterpret_cast<int4 *>(&cnt[0][0]);
+        for (int e = threadIdx.x; e < W * kRadixBins / 4; e += kSortThreads) zero[e] = make_int4(0, 0, 0, 0);
+        __syncthreads();
+        const int shift = p * kRadixBits;
+#pragma unroll
+        for (int r = 0; r < Items; ++r) {
+            const bool valid = seg0 + r * 32 + lane < n;
+            const int dig = valid ? (key[r] >> shift) & (kRadixBins - 1) : kRadixBins;
+            const unsigned peers = __match_any_sync(0xffffffffu, dig);
+            const int before = __popc(peers & lt);
+            int base = 0;
+            if (valid) base = cnt[warp][dig];
+            __syncwarp();
+            if (valid && before == 0) cnt[warp][dig] = base + __popc(peers);
+            __syncwarp();
+            loc[r] = base + before;
+        }
+        __syncthreads();
+        int run = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const int c = cnt[w][d];
+            cnt[w][d] = run;
+            run += c;
+        }
+        hist[d] = run;
+        cluster.sync();
+        // all tiles' keys of this digit, and those of the tiles before this one
+        int total = 0, before = 0;
+        for (int q = 0; q < tiles; ++q) {
+            const int v = *cluster.map_shared_rank(&hist[d], q);
+            before += q < tile ? v : 0;
+            total += v;
+        }
+        int incl = total;  // exclusive prefix over the digits
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        int wp = 0;
+#pragma unroll
+        for (int k = 0; k < W; ++k) wp += k < warp ? wsum[k] : 0;
+        dbase[d] = wp + incl - total + before;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < Items; ++r) {
+            if (seg0 + r * 32 + lane >= n) continue;
+            const int dig = (key[r] >> shift) & (kRadixBins - 1);
+            const int pos = dbase[dig] + cnt[warp][dig] + loc[r];
+            kdst[pos] = key[r];
+            vdst[pos] = val[r];
+        }
+        cluster.sync();  // the keys are in place, and no CTA still reads this one's counts
+        ksrc = kdst;
+        vsrc = vdst;
+    }
+}
+
+template <int Items>
+__global__ void __launch_bounds__(kSortThreads) k_sort_state(SimConsts C, const float4 *__restrict__ X,
+                                                             const float4 *__restrict__ V, int passes,
+                                                             int *__restrict__ keys, int *keys_out, int *vals_out,
+                                                             SortScratch s)
+{
+    sort_cluster<Items>(C.n, passes, [&](int i) { return state_key(C, X, V, i); }, keys, keys_out, vals_out, s);
+}
+
+template <int Items>
+__global__ void __launch_bounds__(kSortThreads) k_sort_f3(int n, const float *__restrict__ pos3, float cell, int D,
+                                                          int passes, int *__restrict__ keys, int *keys_out,
+                                                          int *vals_out, SortScratch s)
+{
+    const unsigned m = (unsigned)D - 1u;
+    sort_cluster<Items>(
+        n, passes, [&](int i) { return hash_key(make_float3(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2]), cell, D, m); },
+        keys, keys_out, vals_out, s);
+}
+
+// A launch of one cluster: the fewest CTAs (a power of two) that hold n keys.
+template <class... K, class... A>
+static void launch_cluster(void (*kernel)(K...), int n, int items, cudaStream_t st, A &&...args)
+{
+    int ctas = 1;
+    while (ctas * kSortThreads * items < n) ctas *= 2;
+    cudaLaunchAttribute shape[1];
+    shape[0].id = cudaLaunchAttributeClusterDimension;
+    shape[0].val.clusterDim = {(unsigned)ctas, 1u, 1u};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kSortThreads);
+    cfg.stream = st;
+    cfg.attrs = shape;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
+// f(keys per thread): the fewest that let 8 CTAs hold n keys, as a thread ranks
+// its keys one after another (16,384 particles: 8 keys a thread in 4 CTAs 197
+// us a flag frame, 4 keys in 8 CTAs 188 us).
+constexpr int kClusterSortMax = kClusterSortCtas * kSortThreads * 16;
+template <class F>
+static void with_cluster_items(int n, F &&f)
+{
+    const int per = (n + kClusterSortCtas * kSortThreads - 1) / (kClusterSortCtas * kSortThreads);
+    if (per <= 1) f(std::integral_constant<int, 1>{});
+    else if (per <= 2) f(std::integral_constant<int, 2>{});
+    else if (per <= 4) f(std::integral_constant<int, 4>{});
+    else if (per <= 8) f(std::integral_constant<int, 8>{});
+    else f(std::integral_constant<int, 16>{});
+}
+
+void hash_sort_state(cudaStream_t st, const SimConsts &C, int dim, const float4 *X, const float4 *V, int *keys,
+                     int *keys_out, int *vals_out, const SortScratch &s, LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    if (C.n > kClusterSortMax) {
+        launch_hash_state(st, C, X, V, keys, s.hist, L);
+        radix_sort_pairs(st, C.n, dim, keys, nullptr, keys_out, vals_out, s, true, L);
+        return;
+    }
+    const int passes = sort_passes(dim);
+    with_cluster_items(C.n, [&](auto items) {
+        launch_cluster(k_sort_state<items.value>, C.n, items.value, st, C, X, V, passes, keys, keys_out, vals_out, s);
+    });
+    L->done("k_sort_state");
+}
+
+void hash_sort_f3(cudaStream_t st, int n, const float *pos3, float cell, int D, int *keys, int *keys_out,
+                  int *vals_out, const SortScratch &s, LaunchLog *L)
+{
+    if (n <= 0) return;
+    if (n > kClusterSortMax) {
+        launch_hash_f3(st, n, pos3, cell, D, keys, s.hist, L);
+        radix_sort_pairs(st, n, D, keys, nullptr, keys_out, vals_out, s, true, L);
+        return;
+    }
+    const int passes = sort_passes(D);
+    with_cluster_items(n, [&](auto items) {
+        launch_cluster(k_sort_f3<items.value>, n, items.value, st, n, pos3, cell, D, passes, keys, keys_out, vals_out, s);
+    });
+    L->done("k_sort_f3");
 }
 
 // ------------------------------------------------------------------------
@@ -335,8 +536,11 @@ __global__ void k_reset_start_end(int n, const int *__restrict__ sorted, int *__
 }
 
 // Dense prefix: off[c] = number of particles whose key is below c, for
-// c in [0, ncells].  Dense or small tables (per == 1): one cell per thread,
-// found by a binary search over all keys.  Large tables with many more cells
+// c in [0, ncells].  Dense or small tables (per == 1): one cell per thread;
+// the warp finds its first cell's by probing 32 keys at a time and holds the
+// 32 keys from there on, or, where its cells hold more, each lane bisects from
+// there (a bisection over all keys for every cell: 7.3 us a launch on 32,768
+// keys and 64^3 cells, now 6.3).  Large tables with many more cells
 // than particles (mostly empty cells) give each warp 32 * per consecutive cells:
 // lanes 0 and 31 search the keys at the ends of that range, the warp copies
 // the keys between them into shared memory, and lane l takes cells l,
@@ -356,17 +560,45 @@ __device__ __forceinline__ int lower_bound_key(const int *__restrict__ sorted, i
     return lo;
 }
 
+// The same over a warp, which probes 32 places at a time: every lane gets the
+// number of keys below c.
+__device__ __forceinline__ int warp_lower_bound(const int *__restrict__ sorted, int lo, int hi, long long c, int lane)
+{
+    while (hi - lo > 32) {
+        const int step = (hi - lo + 31) >> 5;
+        const int at = lo + (lane + 1) * step - 1;
+        const unsigned below = __ballot_sync(0xffffffffu, at < hi && __ldg(sorted + at) < c);
+        lo += __popc(below) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo + __popc(__ballot_sync(0xffffffffu, lo + lane < hi && __ldg(sorted + lo + lane) < c));
+}
+
 __global__ void __launch_bounds__(256) k_cell_offsets(int n, int ncells, int per, const int *__restrict__ sorted,
                                                       int *__restrict__ off, Gate gate)
 {
     __shared__ int keys[256 / 32][kOffsetKeysPerWarp];
     if (gate_closed(gate)) return;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
     if (per == 1) {
-        if (t <= ncells) off[t] = lower_bound_key(sorted, 0, n, t);
+        const long long w0 = t - lane;
+        const int a = warp_lower_bound(sorted, 0, n, w0, lane);
+        // the warp's keys: mostly few enough to hold, one per lane
+        const int mine = a + lane < n ? __ldg(sorted + a + lane) : 0x7fffffff;
+        int lo = 0;
+        if (__all_sync(0xffffffffu, mine < w0 + 32)) {
+            lo = lower_bound_key(sorted, a, warp_lower_bound(sorted, a + 32, n, w0 + 32, lane), t);
+        } else {
+            // keys below cell t, by bisection over the lanes' keys (the last is not below)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (__shfl_sync(0xffffffffu, mine, lo + o - 1) < t) lo += o;
+            lo += a;
+        }
+        if (t <= ncells) off[t] = lo;
         return;
     }
-    const int lane = threadIdx.x & 31;
     int *wk = keys[threadIdx.x >> 5];
     const long long w0 = (t - lane) * per, w1 = w0 + 32LL * per;  // the warp's cells [w0, w1)
     int a = 0, b = n;

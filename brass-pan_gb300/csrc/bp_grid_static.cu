@@ -90,8 +90,7 @@ extern "C" bp_status bp_grid_build_static(void *stream, int32_t n, const float *
     cudaStream_t st = (cudaStream_t)stream;
     LaunchLog L;
     L.stream = st;
-    launch_hash_f3(st, n, pos, cell, D, cell_ids, sc.hist, &L);
-    radix_sort_pairs(st, n, D, cell_ids, nullptr, sorted_cell_ids, sorted_ids, sc, true, &L);
+    hash_sort_f3(st, n, pos, cell, D, cell_ids, sorted_cell_ids, sorted_ids, sc, &L);
     launch_find_start_end(st, n, sorted_cell_ids, start, end, &L);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(BP_ERR_CUDA, std::string("bp_grid_build_static: ") + cudaGetErrorString(e));

@@ -74,6 +74,11 @@ void launch_hash_f3(cudaStream_t st, int n, const float *pos3, float cell, int D
                     LaunchLog *L);
 void launch_hash_state(cudaStream_t st, const SimConsts &C, const float4 *X, const float4 *V, int *keys,
                        int *hist, LaunchLog *L);
+// Cell keys and their stable sort: keys, then keys_out / vals_out sorted.
+void hash_sort_state(cudaStream_t st, const SimConsts &C, int dim, const float4 *X, const float4 *V, int *keys,
+                     int *keys_out, int *vals_out, const SortScratch &s, LaunchLog *L);
+void hash_sort_f3(cudaStream_t st, int n, const float *pos3, float cell, int D, int *keys, int *keys_out,
+                  int *vals_out, const SortScratch &s, LaunchLog *L);
 void launch_find_start_end(cudaStream_t st, int n, const int *sorted, int *start, int *end, LaunchLog *L);
 void launch_reset_start_end(cudaStream_t st, int n, const int *sorted, int *start, int *end,
                             LaunchLog *L);

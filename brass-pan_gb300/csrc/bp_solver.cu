@@ -774,8 +774,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     const bool tail = distance || bending || rigid || immov;  // stages after the fluid position pass
     if (picking) launch_pick(st, picked, s->to_new, s->Xc, ppos, 1, s->Vc, make_float3(0.f, 0.f, 0.f), L);
 
-    launch_hash_state(st, C, s->Xc, s->Vc, s->keys, s->sort.hist, L);
-    radix_sort_pairs(st, s->n, s->sort_dim, s->keys, nullptr, s->sorted_keys, s->order, s->sort, true, L);
+    hash_sort_state(st, C, s->sort_dim, s->Xc, s->Vc, s->keys, s->sorted_keys, s->order, s->sort, L);
     launch_cell_offsets(st, s->n, (int)s->ncells, s->sorted_keys, s->off, L);
 
     // iteration fusion: the reorder takes iteration 0's plane collision, and the
@@ -1440,8 +1439,7 @@ extern "C" bp_status bp_grid_build(void *stream, int32_t n, const float *pos, fl
     sort_scratch_carve(ws, n, D, &sc);
     LaunchLog L;
     L.stream = st;
-    launch_hash_f3(st, n, pos, cell, D, cell_ids, sc.hist, &L);
-    radix_sort_pairs(st, n, D, cell_ids, nullptr, sorted_cell_ids, sorted_ids, sc, true, &L);
+    hash_sort_f3(st, n, pos, cell, D, cell_ids, sorted_cell_ids, sorted_ids, sc, &L);
     launch_find_start_end(st, n, sorted_cell_ids, start, end, &L);
     BP_CUDA(cudaGetLastError());
     return BP_OK;
