@@ -756,6 +756,113 @@ void launch_distance(cudaStream_t st, const SimConsts &C, const DistanceArgs &a,
     L->done("k_distance_apply");
 }
 
+__global__ void k_step_entries(int entries, DistanceArgs a, int2 *__restrict__ range, int4 *__restrict__ inc)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < a.num_nodes) range[a.node_ids[q]] = make_int2(a.node_ptr[q], a.node_ptr[q + 1]);
+    if (q >= entries) return;
+    const int edge = a.node_inc[q] >> 1, side = a.node_inc[q] & 1;
+    const int2 pr = a.pairs[edge];
+    const float2 prm = a.params[edge];
+    inc[q] = make_int4((side ? pr.x : pr.y) * 2 + side, __float_as_int(prm.x), __float_as_int(prm.y), edge);
+}
+
+void build_distance_step(const DistanceArgs &a, int entries, int2 *range, int4 *inc)
+{
+    const int threads = std::max(entries, a.num_nodes);
+    if (threads > 0) k_step_entries<<<(threads + 255) / 256, 256>>>(entries, a, range, inc);
+}
+
+// A cloth iteration's end in one launch, four lanes per particle: its edges'
+// corrections in CSR order, evaluated by both ends (the same operations and so
+// the same bits as k_distance_edges, from the positions before), the
+// immovables, the next iteration's planes or the commit.  Where most particles
+// are cloth the four launches it replaces are bound by their own latency; the
+// edges' second evaluation is cheaper than the gather of the first.  Each lane
+// has the loads of two edges in flight and evaluates them, and the four add
+// them up in order (128 x 128 flag, a frame: 188 us with the four launches,
+// 165 with one thread per particle, 136 with four lanes).
+constexpr int kStepLanes = 4;
+__global__ void __launch_bounds__(128) k_distance_step(SimConsts C, DistanceStep a, const float4 *__restrict__ P,
+                                                       float4 *__restrict__ Pout)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x % kStepLanes;
+    const int i = (int)min(t / kStepLanes, (long long)C.n - 1);  // lanes past the end repeat the last particle, without its stores
+    const float4 p4 = P[i];
+    const float4 xs = a.Xs[i];
+    const int id = a.orig_s[i];
+    const float wi = a.w[i];
+    const int2 range = __ldg(a.range + id);
+    const int b = range.x, e = range.y;
+    const bool pinned = a.pinned && a.pinned[id];
+    const float3 pi = f3(p4);
+    float3 d = make_float3(0.f, 0.f, 0.f);
+    const int rounds = __reduce_max_sync(0xffffffffu, (e - b + 2 * kStepLanes - 1) / (2 * kStepLanes));
+    for (int r = 0; r < rounds; ++r) {
+        int4 c[2];
+        float4 po[2];
+        float wo[2];
+        float3 term[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int q = b + (2 * r + k) * kStepLanes + lane;
+            c[k] = q < e ? __ldg(a.inc + q) : make_int4(2 * id, 0, 0, 0);  // an edge to itself: no correction
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int j = __ldg(a.to_new + (c[k].x >> 1));
+            po[k] = P[j];
+            wo[k] = __ldg(a.w + j);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const bool second = (c[k].x & 1) != 0;
+            const float3 x12 = second ? f3(po[k]) - pi : pi - f3(po[k]);
+            const float d12 = len3(x12);
+            float3 g = make_float3(0.f, 0.f, 0.f);
+            if (!(d12 <= 1e-5f)) {
+                const float3 nn = x12 / d12;
+                const float sw = wi + wo[k];
+                g = (nn * ((d12 - __int_as_float(c[k].y)) / sw)) * __int_as_float(c[k].z);
+            }
+            term[k] = second ? wi * g : -wi * g;
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int l = 0; l < kStepLanes; ++l) {
+                const float3 u = make_float3(__shfl_sync(0xffffffffu, term[k].x, l, kStepLanes),
+                                             __shfl_sync(0xffffffffu, term[k].y, l, kStepLanes),
+                                             __shfl_sync(0xffffffffu, term[k].z, l, kStepLanes));
+                if (b + (2 * r + k) * kStepLanes + l < e) d += u;
+            }
+    }
+    if (lane != 0 || t / kStepLanes >= C.n) return;
+    float3 p = pi;
+    if (b < e) p = make_float3(p.x + d.x, p.y + d.y, p.z + d.z);
+    if (pinned) p = f3(xs);
+    if (a.epilogue == 1) {
+        plane_collide(C, scene_index(C, i), f3(xs), p);
+    } else if (a.epilogue == 2) {  // updateVelocity + updatePositions, as k_commit
+        const float3 v = (p - f3(xs)) * C.inv_dt;
+        a.Xc[i] = make_float4(p.x, p.y, p.z, xs.w);
+        a.Vc[i] = make_float4(v.x, v.y, v.z, a.Vs[i].w);
+        a.orig_c[i] = id;
+    }
+    Pout[i] = make_float4(p.x, p.y, p.z, p4.w);
+    track_displacement(C, i, p, true);
+}
+
+void launch_distance_step(cudaStream_t st, const SimConsts &C, const DistanceStep &a, const float4 *P, float4 *Pout,
+                          LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    const long long threads = (long long)C.n * kStepLanes;
+    k_distance_step<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(C, a, P, Pout);
+    L->done(__func__);
+}
+
 // ---- dihedral bending ----
 
 // bendingConstraints (K/bending.cuh:3-75): the dihedral angle of the two

@@ -218,6 +218,26 @@ struct DistanceArgs {
     const int *node_inc;     // edge*2 + side
     float4 *edge_k;          // per-edge correction vector
 };
+// The constraints as one particle sees them, for the launch that does a whole
+// cloth iteration's end (launch_distance_step): by original id, CSR.
+struct DistanceStep {
+    const int2 *range;       // [n]: the particle's entries of inc
+    const int4 *inc;         // the other end's original id << 1 | side, rest length and stiffness (bits), edge
+    const unsigned char *pinned;  // [n], nullptr: no immovables
+    const int *orig_s, *to_new;
+    const float *w;
+    int epilogue;            // as DeltaArgs::epilogue
+    const float4 *Xs, *Vs;
+    float4 *Xc, *Vc;
+    int *orig_c;
+};
+// Fills range (zero before) and inc, on the default stream.
+void build_distance_step(const DistanceArgs &a, int entries, int2 *range, int4 *inc);
+// Reads P, writes Pout: the distance constraints' corrections (each particle
+// evaluates its own edges), the immovables put back, then the next iteration's
+// plane collision or the commit.
+void launch_distance_step(cudaStream_t st, const SimConsts &C, const DistanceStep &a, const float4 *P, float4 *Pout,
+                          LaunchLog *L);
 void launch_distance(cudaStream_t st, const SimConsts &C, const DistanceArgs &a, float4 *P, const float *w,
                      const int *to_new, unsigned *err, LaunchLog *L);
 struct BendingArgs {

@@ -510,6 +510,17 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         s->dist.node_ptr = nptr;
         s->dist.node_inc = ninc;
         s->dist.edge_k = ek;
+        // launch_distance_step touches every particle: worth it where at least
+        // a quarter of them have constraints
+        if (4LL * s->dist.num_nodes >= n) {
+            int2 *p1;
+            int4 *p2;
+            if ((st = s->alloc(&p1, N)) || (st = s->alloc(&p2, inc.size()))) return bail(st);
+            BP_CUDA_BAIL(cudaMemset(p1, 0, N * sizeof(int2)));
+            build_distance_step(s->dist, (int)inc.size(), p1, p2);
+            s->dist_step.range = p1;
+            s->dist_step.inc = p2;
+        }
     }
     if (sc->num_bendings > 0) {
         const int q = sc->num_bendings;
@@ -569,6 +580,11 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
     if (sc->num_immovables > 0) {
         s->nimm = sc->num_immovables;
         if ((st = s->upload(&s->imm, sc->immovables, s->nimm))) return bail(st);
+        std::vector<unsigned char> pinned(N, 0);
+        for (int k = 0; k < s->nimm; ++k) pinned[sc->immovables[k]] = 1;
+        unsigned char *pp;
+        if ((st = s->upload(&pp, pinned.data(), N))) return bail(st);
+        s->dist_step.pinned = pp;
     }
     if (batch) {
         const int S = (int)batch->scenes.size();
@@ -781,6 +797,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // position pass the next iteration's or the final commit (BP_WALK_NO_FUSION:
     // launches of their own; bit-identical either way)
     const bool fuse = !tape && !(s->prm.walk_options & BP_WALK_NO_FUSION);
+    const bool distance_step = fuse && distance && !bending && !rigid && s->dist_step.range;
     const bool fuse_first_planes = planes && !wind && !picking && iterations > 0 && fuse;
     ReorderArgs ra;
     ra.order = s->order;
@@ -984,6 +1001,29 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             }
             launch_deltap(st, (verlet && it == 0) ? Cpost : Cf, da, L);
             std::swap(cur, other);
+        }
+        if (distance_step) {
+            DistanceStep ds = s->dist_step;
+            if (!immov) ds.pinned = nullptr;
+            ds.orig_s = s->orig_s;
+            ds.to_new = s->to_new;
+            ds.w = s->w;
+            ds.Xs = s->Xs;
+            ds.Vs = s->Vs;
+            ds.Xc = s->Xc;
+            ds.Vc = s->Vc;
+            ds.orig_c = s->orig_c;
+            ds.epilogue = 0;
+            if (it == iterations - 1) {
+                ds.epilogue = 2;
+                committed = true;
+            } else if (planes && !picking) {
+                ds.epilogue = 1;
+                planes_done = true;
+            }
+            launch_distance_step(st, Cpost, ds, cur, other, L);
+            std::swap(cur, other);
+            continue;
         }
         if (distance) {
             if (tape) tape->push(TS_DISTANCE, cur);

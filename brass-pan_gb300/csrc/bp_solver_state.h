@@ -162,6 +162,7 @@ struct bp_solver {
     SceneConsts *scn = nullptr;
     int *scene_of = nullptr;
     DistanceArgs dist{};
+    DistanceStep dist_step{};  // range == nullptr: the scene is not mostly cloth
     BendingArgs bend{};
     WindArgs wind{};
     RigidArgs rigid{};
