@@ -515,20 +515,22 @@ __global__ void __launch_bounds__(kQueueThreads) k_lambda_queued(SimConsts C, co
     }
 }
 
-void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const float *mass,
-                         const int *off, float *lam, float *rho, LaunchLog *L)
+// Moves particle k by its summed corrections, then the pass's epilogue.
+__device__ __forceinline__ void finish_deltap(const SimConsts &C, const DeltaArgs &a, int sc, int k, float4 pk4,
+                                              float3 sum)
 {
-    if (C.n <= 0) return;
-    const int grid = (C.n + C.scan_block - 1) / C.scan_block;
-    if (record) {
-        k_lambda_lists<kRecordLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
-        L->done("launch_lambda");
-        return;
+    float3 p = f3(pk4) + sum * inv_rest_density(C, sc);
+    if (a.epilogue == 1) {
+        plane_collide(C, sc, f3(a.Xs[k]), p);
+    } else if (a.epilogue == 2) {  // updateVelocity + updatePositions (PS:71-81, 121-137)
+        const float4 xs = a.Xs[k];
+        const float3 v = (p - f3(xs)) * C.inv_dt;
+        a.Xc[k] = make_float4(p.x, p.y, p.z, xs.w);
+        a.Vc[k] = make_float4(v.x, v.y, v.z, pk4.w);
+        a.orig_c[k] = a.orig_s[k];
     }
-    k_lambda_lists<kReadLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
-    L->done("launch_lambda_lists");
-    k_lambda_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, mass, off, lam, rho);
-    L->done("launch_lambda_queued");
+    a.Pout[k] = make_float4(p.x, p.y, p.z, pk4.w);
+    track_displacement(C, k, p, true);
 }
 
 // Position correction.  Reference mode: the pair (a, b), a < b, contributes
@@ -624,18 +626,7 @@ __device__ __forceinline__ void k_deltap_tile(
                 body);
         }
     }
-    float3 p = pk + sum * inv_rest_density(C, sc);
-    if (a.epilogue == 1) {
-        plane_collide(C, sc, f3(a.Xs[k]), p);
-    } else if (a.epilogue == 2) {  // updateVelocity + updatePositions (PS:71-81, 121-137)
-        const float4 xs = a.Xs[k];
-        const float3 v = (p - f3(xs)) * C.inv_dt;
-        a.Xc[k] = make_float4(p.x, p.y, p.z, xs.w);
-        a.Vc[k] = make_float4(v.x, v.y, v.z, pk4.w);
-        a.orig_c[k] = a.orig_s[k];
-    }
-    a.Pout[k] = make_float4(p.x, p.y, p.z, pk4.w);
-    track_displacement(C, k, p, true);
+    finish_deltap(C, a, sc, k, pk4, sum);
 }
 
 template <bool Split, bool Stage, bool Persist = false>
@@ -652,13 +643,6 @@ __global__ void __launch_bounds__(kScanThreads, BP_DELTAP_MIN_BLOCKS) k_deltap(
     } else {
         k_deltap_tile<Split, Stage>(C, a, blockIdx.x * blockDim.x);
     }
-}
-
-void launch_deltap(cudaStream_t st, const SimConsts &C, const DeltaArgs &a, LaunchLog *L)
-{
-    if (C.n <= 0) return;
-    BP_LAUNCH_SPLIT(k_deltap, st, C, a);
-    L->done(__func__);
 }
 
 // The post passes keep class positions in their lists (SimConsts::cls_post):
@@ -807,6 +791,22 @@ __device__ __forceinline__ int post_list_count(const SimConsts &C, const float4 
     return cnt >= 0 ? cnt & 0xffff : kWalkCells;  // substep lists: above it, the own entry's index
 }
 
+// Particle i's velocity from its pass B sums.
+__device__ __forceinline__ void finish_post_b(const SimConsts &C, bool slots, int i, int t, float4 vi4, float3 eta,
+                                              float3 ft, const float4 *__restrict__ Om, float4 *__restrict__ Vout)
+{
+    float3 v = f3(vi4);
+    if (C.use_vort && len2(eta) > 1e-3f) {
+        const float inv = 1.0f / sqrtf(dot3(eta, eta));
+        const float3 nrm = eta * inv;
+        v += (C.vort_eps * cross3(nrm, f3(Om[i]))) * C.dt;
+    }
+    if (C.use_akinci) v = v + ft * C.dt;
+    const float4 v4 = make_float4(v.x, v.y, v.z, vi4.w);
+    Vout[i] = v4;
+    if (slots) C.cls_vb[t] = v4;  // pass C's neighbour velocities
+}
+
 // Pass B: vorticity confinement (fluidVorticity) then Akinci tension
 // (fluidAkinciTension), both on the same neighbours.  v' = v + eps (N x w) dt,
 // v'' = v' + F dt, exactly the reference's sequence (in-place update followed
@@ -886,16 +886,7 @@ __device__ __forceinline__ void k_post_b_tile(
             [&](int j, float4 pj4) { return j != i && phase_of(pj4) == phi && len2(pi - f3(pj4)) <= C.h2; },
             body);
     }
-    float3 v = f3(vi4);
-    if (want_v && len2(eta) > 1e-3f) {
-        const float inv = 1.0f / sqrtf(dot3(eta, eta));
-        const float3 nrm = eta * inv;
-        v += (C.vort_eps * cross3(nrm, f3(Om[i]))) * C.dt;
-    }
-    if (want_t) v = v + ft * C.dt;
-    const float4 v4 = make_float4(v.x, v.y, v.z, vi4.w);
-    Vout[i] = v4;
-    if (slots) C.cls_vb[t] = v4;  // pass C's neighbour velocities
+    finish_post_b(C, slots, i, t, vi4, eta, ft, Om, Vout);
 }
 
 template <bool Split, bool Stage, bool Persist = false>
@@ -1136,16 +1127,548 @@ __global__ void __launch_bounds__(kQueueThreads) k_post_a_queued(SimConsts C, co
     }
 }
 
+// The recording pass of small scenes, a warp per particle (k_lambda_lists<
+// kRecordLists> takes a thread's whole walk, about 28 us whatever the number of
+// particles): the candidates within the lists' reach, from the position
+// records, the contact partners among them and, for fluid, the lambda pass's
+// sums over those within h.
+// Measured, a frame (a thread each, a warp each): 1,728 particles 188 -> 157
+// us, 5,832 200 -> 177, 13,824 232 -> 233 (textbook mode 327 -> 315), 21,952
+// 276 -> 296: the line lies at kWarpRecordMax.
+constexpr int kWarpRecordMax = 14000;
+__global__ void __launch_bounds__(kQueueThreads) k_lambda_record(SimConsts C, const float4 *__restrict__ P,
+                                                                 const float *__restrict__ mass,
+                                                                 const int *__restrict__ off, float *__restrict__ lam,
+                                                                 float *__restrict__ rho)
+{
+    __shared__ WarpRows rows[kQueueThreads / 32];
+    __shared__ WarpHits hits[kQueueThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = 0;
+        C.sl_count[kSlMoved] = C.cls_perm ? *C.cls_moved : 0;
+    }
+    if (t >= C.n) return;  // whole warps
+    const bool slots = classes_on(C);
+    const int i = slots ? __ldg(C.cls_perm + t) : t;
+    const float4 pi4 = slots ? C.cls_pos[t] : P[i];
+    const float3 pi = f3(pi4);
+    const int phi = phase_of(pi4);
+    const bool solid = phi > 0;
+    if (lane == 0) {
+        C.sl_pos[i] = pi4;
+        if (solid && C.sl_fluid) {  // solids carry lambda 0 (read by the position pass)
+            lam[i] = 0.f;
+            (slots ? C.cls_lm[t] : C.lm[i]) = make_float2(0.f, __ldg(mass + i));
+        }
+    }
+    if (solid && C.textbook && !C.cl_list) return;  // as lambda_substep_list
+    const int sc = scene_index(C, i);
+    const GridView v = grid_view(C, sc, off);
+    const int3 c = cell_of(pi, C);
+    if (C.nl_stats && lane == 0) {
+        atomicAdd(C.nl_stats + 1, 1u);
+        if (slots) atomicAdd(C.nl_stats + 4, 1u);
+    }
+    const float skin = substep_skin(C), touch = 2.0f * C.radius + skin;
+    const float reach = fmaxf(C.sl_fluid ? C.h + skin : 0.f, C.cl_list ? touch : 0.f);
+    const float reach2 = __fmul_rn(reach, reach), touch2 = __fmul_rn(touch, touch);
+    const float inv_rho0 = inv_rest_density(C, sc);
+    const int me = slots ? t : i;
+    const bool sums = C.sl_fluid && !solid;
+    float acc = 0.f;  // lane 0: the density; textbook, lanes 1..4: sum of g^2, -sum of g
+    int self = 0, touching = 0;
+    auto batch = [&](int k0, int n, int q, float4 pj) {
+        const bool in = lane < n;
+        if (in) put_entry(C, t, k0 + lane, q);
+        const unsigned own = __ballot_sync(kWarp, in && q == me);
+        if (own) self = k0 + __ffs(own) - 1;
+        const float3 diff = pi - f3(pj);
+        const float d2 = len2(diff);
+        if (C.cl_list) {
+            const int phj = phase_of(pj);
+            const bool near = in && phi != phj && (solid || phj > 0) && d2 <= touch2;
+            const unsigned b = __ballot_sync(kWarp, near);
+            const int k = touching + __popc(b & ((1u << lane) - 1u));
+            if (near && k < kContactCap) C.cl_list[(size_t)k * C.n + t] = slots ? __ldg(C.cls_perm + q) : q;
+            touching += __popc(b);
+        }
+        if (!sums) return;
+        bool take = in && d2 <= C.h2;
+        float value[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        if (take) {
+            const int j = slots ? __ldg(C.cls_perm + q) : q;
+            const float mj = __ldg((slots ? C.cls_mass : mass) + q);
+            take = C.textbook || j >= i;
+            value[0] = __fmul_rn(mj, poly6(C, d2));
+            if (phase_of(pj) >= 0) value[0] = __fmul_rn(C.solid_scale, value[0]);
+            if (C.textbook && d2 > 0.f) {  // the pair at r = 0 adds zeros
+                const float3 g = __fmul_rn(-mj, inv_rho0) * spiky_grad_r(C, diff, d2, rsqrtf(d2));
+                value[1] = dot3(g, g);
+                value[2] = -g.x;
+                value[3] = -g.y;
+                value[4] = -g.z;
+            }
+        }
+        warp_add(rows[threadIdx.x >> 5], __ballot_sync(kWarp, take), value, 1.f, acc);
+    };
+    int cnt = warp_neighbors(C, slots, c, P, v, hits[threadIdx.x >> 5],
+                             [&](int, float4 pj) { return len2(pi - f3(pj)) <= reach2; }, batch);
+    const bool fits = cnt <= C.nbr_cap;
+    if (!fits && C.sl_fluid)  // the neighbours within h alone may still fit; later passes then walk
+        cnt = warp_neighbors(C, slots, c, P, v, hits[threadIdx.x >> 5],
+                             [&](int, float4 pj) { return len2(pi - f3(pj)) <= C.h2; },
+                             [&](int k0, int n, int q, float4) {
+                                 if (lane < n) put_entry(C, t, k0 + lane, q);
+                                 const unsigned own = __ballot_sync(kWarp, lane < n && q == me);
+                                 if (own) self = k0 + __ffs(own) - 1;
+                             });
+    warp_pad(C, t, cnt, me);
+    const float sum_g2 = __shfl_sync(kWarp, acc, 1);
+    const float3 gi = make_float3(__shfl_sync(kWarp, acc, 2), __shfl_sync(kWarp, acc, 3), __shfl_sync(kWarp, acc, 4));
+    if (lane != 0) return;
+    C.nbr_count[t] = cnt <= C.nbr_cap ? cnt | (self << 16) : -1;
+    C.sl_cell[t] = (fits && near_stored_cell(C, i, c, v)) ? v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask) : kListNone;
+    if (C.cl_list) C.cl_count[t] = fits && touching <= kContactCap ? touching : -1;
+    if (sums)
+        finish_lambda(C, slots, i, t, acc, rest_density(C, sc),
+                      C.textbook ? (sum_g2 + dot3(gi, gi)) + C.relaxation : C.lambda_den, mass, lam, rho);
+}
+
+// ---- the list readers of small scenes: four lanes per particle ----
+
+// A reading pass's thread takes its list's records one after another, a round
+// of gathers and four pair terms each, and in a scene whose particles do not
+// fill the GPU nothing hides that chain.  Four lanes per particle take four
+// records at once and add their terms up in turn, in list order and with the
+// same operations, so to the same bits (fma(1, v, s) rounds as v + s).
+// Measured, a frame (one thread each, four lanes): 1,728 particles 244 -> 184
+// us, 21,952 particles 307 -> 275, 32,768 301 -> 306; textbook mode, whose
+// lambda pass has more to add up, 421 -> 274, 505 -> 387, 510 -> 448 and 46,656
+// particles 567 -> 566: the lines lie just below.
+constexpr int kGroupLanes = 4, kGroupThreads = 128;
+constexpr int kGroupMax = 30000, kGroupMaxTextbook = 45000;
+
+// A pair's addends: component k adds s[k / 3] * v[k].
+template <int NV>
+struct GroupTerm {
+    float v[NV];
+    float s[2];
+};
+struct GroupParticle {
+    int t, i, lane;  // slot, sorted index, lane in the group
+    bool slots, real;
+    float4 p4;
+};
+// Lanes past the end repeat the last particle and store nothing (real).
+__device__ __forceinline__ GroupParticle group_particle(const SimConsts &C, const float4 *__restrict__ P, bool slots)
+{
+    GroupParticle g;
+    const int t = (blockIdx.x * kGroupThreads + threadIdx.x) / kGroupLanes;
+    g.lane = threadIdx.x % kGroupLanes;
+    g.real = t < C.n;
+    g.t = min(t, C.n - 1);
+    g.slots = slots;
+    g.i = slots ? __ldg(C.cls_perm + g.t) : g.t;
+    g.p4 = slots ? C.cls_pos[g.t] : P[g.i];
+    return g;
+}
+
+// acc += the terms of entries [4 * first, cnt) of the particle's list, in
+// order, on every lane: term(j, e, P[j], fetch(j), out) is false where entry e
+// adds nothing.  All lanes of the warp take part (cnt 0: none to add).
+template <int NV, class G, class F>
+__device__ __forceinline__ void group_sum(const SimConsts &C, const GroupParticle &me, int first, int cnt,
+                                          const float4 *__restrict__ P, G &&fetch, F &&term, float (&acc)[NV])
+{
+    using X = decltype(fetch(0));
+    const int recs = (cnt + 3) >> 2;
+    const int4 *rec = reinterpret_cast<const int4 *>(C.nbr) + me.t;
+    const size_t stride = (size_t)C.n;
+    const int own = me.slots ? me.t : me.i;
+    const int rounds = __reduce_max_sync(kWarp, max(recs - first + kGroupLanes - 1, 0) / kGroupLanes);
+    int at = first + me.lane;
+    int4 next = at < recs ? __ldg(rec + (size_t)at * stride) : make_int4(own, own, own, own);
+    for (int r = 0; r < rounds; ++r, at += kGroupLanes) {
+        const int j[4] = {next.x, next.y, next.z, next.w};
+        next = at + kGroupLanes < recs ? __ldg(rec + (size_t)(at + kGroupLanes) * stride) : make_int4(own, own, own, own);
+        float4 pj[4];
+        X xj[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            pj[q] = P[j[q]];
+            xj[q] = fetch(j[q]);
+        }
+        GroupTerm<NV> g[4];
+        bool ok[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ok[q] = term(j[q], 4 * at + q, pj[q], xj[q], g[q]) && at < recs;
+#pragma unroll
+        for (int l = 0; l < kGroupLanes; ++l) {
+            if (me.lane == l) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (ok[q]) {
+#pragma unroll
+                        for (int k = 0; k < NV; ++k) acc[k] = __fmaf_rn(g[q].s[k / 3], g[q].v[k], acc[k]);
+                    }
+            }
+#pragma unroll
+            for (int k = 0; k < NV; ++k) acc[k] = __shfl_sync(kWarp, acc[k], l, kGroupLanes);
+        }
+    }
+}
+
+// One lane of the group asks whether the particle reads its list (and queues it where not).
+__device__ __forceinline__ bool group_reads(const SimConsts &C, const GroupParticle &me, bool wanted, int3 c,
+                                            const GridView &v)
+{
+    bool reads = false;
+    if (me.lane == 0 && me.real && wanted) reads = reads_substep_list(C, me.t, me.i, f3(me.p4), c, v);
+    return __shfl_sync(kWarp, reads, 0, kGroupLanes);
+}
+
+template <bool Textbook>
+__global__ void __launch_bounds__(kGroupThreads) k_lambda_group(SimConsts C, const float4 *__restrict__ P,
+                                                                const float *__restrict__ mass,
+                                                                const int *__restrict__ off, float *__restrict__ lam,
+                                                                float *__restrict__ rho)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) C.sl_count[C.sl_pass ^ 1] = 0;  // the next pass's queue
+    const GroupParticle me = group_particle(C, P, classes_on(C));
+    const bool solid = phase_of(me.p4) > 0;
+    const float3 pi = f3(me.p4);
+    const int sc = scene_index(C, me.i);
+    const GridView v = grid_view(C, sc, off);
+    const int3 c = cell_of(pi, C);
+    const bool reads = group_reads(C, me, !(solid && Textbook), c, v) && !solid;
+    const int packed = reads ? __ldg(C.nbr_count + me.t) : 0;
+    const int cnt = packed & 0xffff, self = packed >> 16;
+    const float *__restrict__ ms = me.slots ? C.cls_mass : mass;
+    const float4 *__restrict__ src = me.slots ? C.cls_pos : P;
+    auto fetch = [&](int j) { return __ldg(ms + j); };
+    auto weight = [&](float mj, float4 pj, float d2) {
+        const float ld = __fmul_rn(mj, poly6(C, d2));
+        return (phase_of(pj) < 0) ? ld : __fmul_rn(C.solid_scale, ld);
+    };
+    float density, den = C.lambda_den;
+    if (!Textbook) {
+        auto inner = [&](int a) {
+            const unsigned u = (unsigned)a & v.mask;
+            return u != 0u && u != v.mask;
+        };
+        const bool ascending = inner(c.x) && inner(c.y) && inner(c.z);  // as lambda_substep_list
+        float acc[1] = {0.f};
+        group_sum<1>(C, me, ascending ? self >> 2 : 0, cnt, src, fetch,
+                     [&](int j, int e, float4 pj, float mj, GroupTerm<1> &out) {
+            const float d2 = len2(pi - f3(pj));
+            out.s[0] = 1.f;
+            out.v[0] = weight(mj, pj, d2);
+            if (!(d2 <= C.h2) || e >= cnt) return false;
+            return ascending ? e >= self : (me.slots ? __ldg(C.cls_perm + j) : j) >= me.i;
+        }, acc);
+        density = acc[0];
+    } else {
+        const float inv_rho0 = inv_rest_density(C, sc);
+        float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        group_sum<5>(C, me, 0, cnt, src, fetch, [&](int, int e, float4 pj, float mj, GroupTerm<5> &out) {
+            const float3 diff = pi - f3(pj);
+            const float d2 = len2(diff);
+            out.s[0] = out.s[1] = 1.f;
+            out.v[0] = weight(mj, pj, d2);
+            out.v[1] = out.v[2] = out.v[3] = out.v[4] = 0.f;  // r = 0 adds zeros
+            if (d2 > 0.f) {
+                const float3 g = __fmul_rn(-mj, inv_rho0) * spiky_grad_r(C, diff, d2, rsqrtf(d2));
+                out.v[1] = dot3(g, g);
+                out.v[2] = -g.x;
+                out.v[3] = -g.y;
+                out.v[4] = -g.z;
+            }
+            return d2 <= C.h2 && e < cnt;
+        }, acc);
+        density = acc[0];
+        const float3 gi = make_float3(acc[2], acc[3], acc[4]);
+        den = (acc[1] + dot3(gi, gi)) + C.relaxation;
+    }
+    if (reads && me.lane == 0) finish_lambda(C, me.slots, me.i, me.t, density, rest_density(C, sc), den, mass, lam, rho);
+}
+
+__global__ void __launch_bounds__(kGroupThreads) k_deltap_group(SimConsts C, DeltaArgs a)
+{
+    const GroupParticle me = group_particle(C, a.P, classes_on(C));
+    const int phk = phase_of(me.p4);
+    const float3 pk = f3(me.p4);
+    const bool moves = !(C.textbook && phk > 0);
+    const int listed = moves ? __ldg(C.nbr_count + me.t) : 0;
+    const float lk = a.lam[me.i];
+    const float2 *__restrict__ lms = me.slots ? C.cls_lm : C.lm;
+    float3 sum;
+    auto pair = [&](float3 diff, float d2, float lj) {
+        float sl = __fadd_rn(lk, lj);
+        if (C.scorr_on)
+            sl = __fsub_rn(sl, __fmul_rn(C.scorr_k, ipowf(__fmul_rn(poly6(C, d2), C.scorr_inv_wq), C.scorr_ni)));
+        float3 delta = sl * spiky_grad_r(C, diff, d2, rsqrtf(d2));
+        if (C.delta_clamp > 0.f) {
+            const float l2 = len2(delta);
+            if (!(l2 < C.delta_clamp2)) delta = delta * __fmul_rn(C.delta_clamp, rsqrtf(l2));
+        }
+        return delta;
+    };
+    // reference mode: the lower-indexed of the pair is fluid
+    auto admits = [&](int j, bool fj) { return C.textbook || ((j > me.i) ? (phk < 0) : fj); };
+    float acc[3] = {0.f, 0.f, 0.f};
+    group_sum<3>(C, me, 0, listed >= 0 ? listed & 0xffff : 0, me.slots ? C.cls_pos : a.P,
+                 [&](int j) { return __ldg(lms + j); },
+                 [&](int j, int, float4 pj, float2 lm, GroupTerm<3> &out) {
+        const float3 diff = pk - f3(pj);
+        const float d2 = len2(diff);
+        const float3 delta = pair(diff, d2, lm.x);
+        out.s[0] = lm.y;
+        out.v[0] = delta.x;
+        out.v[1] = delta.y;
+        out.v[2] = delta.z;
+        const bool fj = phase_of(pj) < 0;
+        return d2 > 0.f && d2 <= C.h2 && ((phk < 0 && fj) || admits(me.slots ? __ldg(C.cls_perm + j) : j, fj));
+    }, acc);
+    if (me.lane != 0 || !me.real) return;
+    sum = make_float3(acc[0], acc[1], acc[2]);
+    const int sc = scene_index(C, me.i);
+    if (listed < 0)  // overflowed
+        walk_neighbors<true>(
+            me.i, pk, 0, a.P, grid_view(C, sc, a.off), C, nullptr, -1,
+            [&](int, float4 pj) {
+                const float d2 = len2(pk - f3(pj));
+                return d2 <= C.h2 && d2 > 0.f;
+            },
+            [&](int j, float4 pj) {
+                if (!admits(j, phase_of(pj) < 0)) return;
+                const float3 diff = pk - f3(pj);
+                sum = fma3(__ldg(a.mass + j), pair(diff, len2(diff), __ldg(a.lam + j)), sum);
+            });
+    finish_deltap(C, a, sc, me.i, me.p4, sum);
+}
+
+__global__ void __launch_bounds__(kGroupThreads) k_post_a_group(SimConsts C, const float4 *__restrict__ P,
+                                                                const float4 *__restrict__ V,
+                                                                const float *__restrict__ rho,
+                                                                const int *__restrict__ off, float4 *__restrict__ Om,
+                                                                float4 *__restrict__ Nm)
+{
+    const GroupParticle me = group_particle(C, P, post_slots(C, false));
+    const int phi = phase_of(me.p4);
+    const float3 pi = f3(me.p4);
+    const bool reads = group_reads(C, me, phi < 0, cell_of(pi, C), grid_view(C, scene_index(C, me.i), off));
+    const int cnt = reads ? __ldg(C.nbr_count + me.t) & 0xffff : 0;
+    const float4 *__restrict__ vs = me.slots ? C.cls_vel : V;
+    const float *__restrict__ rs = me.slots ? C.cls_rho : rho;
+    const float3 vi = f3(vs[me.t]);
+    float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    group_sum<6>(C, me, 0, cnt, me.slots ? C.cls_pos : P, [&](int j) { return post_a_neighbour(C, vs, rs, j); },
+                 [&](int, int, float4 pj, const PostANeighbour &nb, GroupTerm<6> &out) {
+        const float3 diff = pi - f3(pj);
+        const float d2 = len2(diff);
+        const float3 g = spiky_grad_r(C, diff, d2, rsqrtf(d2));
+        const float3 w = cross3(nb.v - vi, g);
+        out.s[0] = 1.f;
+        out.s[1] = __frcp_rn(nb.rho);
+        out.v[0] = w.x;
+        out.v[1] = w.y;
+        out.v[2] = w.z;
+        out.v[3] = g.x;
+        out.v[4] = g.y;
+        out.v[5] = g.z;
+        return d2 > 0.f && d2 <= C.h2 && phase_of(pj) == phi;
+    }, acc);
+    if (!reads || me.lane != 0) return;
+    const float3 zero = make_float3(0.f, 0.f, 0.f);
+    finish_post_a(C, me.slots, me.i, me.t, C.use_vort ? make_float3(acc[0], acc[1], acc[2]) : zero,
+                  C.use_akinci ? make_float3(acc[3], acc[4], acc[5]) : zero, rho, Om, Nm);
+}
+
+__global__ void __launch_bounds__(kGroupThreads) k_post_b_group(SimConsts C, const float4 *__restrict__ P,
+                                                                const float4 *__restrict__ V,
+                                                                const float4 *__restrict__ Om,
+                                                                const float4 *__restrict__ Nm,
+                                                                const int *__restrict__ off, float4 *__restrict__ Vout)
+{
+    const GroupParticle me = group_particle(C, P, post_slots(C, false));
+    const int phi = phase_of(me.p4);
+    const float3 pi = f3(me.p4);
+    const float4 vi4 = V[me.i];
+    const float4 ni4 = Nm[me.i];
+    const int sc = scene_index(C, me.i);
+    const float two_rho0 = 2.0f * rest_density(C, sc);
+    const int listed = phi < 0 ? __ldg(C.nbr_count + me.t) : 0;
+    const bool want_v = C.use_vort, want_t = C.use_akinci;
+    struct Nb {
+        float om;
+        float4 nm;
+    };
+    auto fetch_at = [&](const float4 *__restrict__ Omp, const float4 *__restrict__ Nmp, int j) {
+        Nb r;
+        r.om = want_v ? Omp[j].w : 0.f;
+        r.nm = want_t ? Nmp[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        return r;
+    };
+    auto term = [&](float4 pj, const Nb &nb, GroupTerm<6> &out) {
+        const float3 diff = pi - f3(pj);
+        const float d2 = len2(diff);
+        const float inv_r = rsqrtf(d2);
+        const float3 g = spiky_grad_r(C, diff, d2, inv_r);
+        const float dist = __fmul_rn(d2, inv_r);
+        const float3 fco = __fmul_rn(__fmul_rn(-C.tension, akinci_spline(C, dist)), inv_r) * diff;
+        const float3 f = fco + (-C.tension) * (f3(ni4) - f3(nb.nm));
+        out.s[0] = nb.om;
+        out.s[1] = __fmul_rn(two_rho0, __frcp_rn(__fadd_rn(ni4.w, nb.nm.w)));
+        out.v[0] = g.x;
+        out.v[1] = g.y;
+        out.v[2] = g.z;
+        out.v[3] = f.x;
+        out.v[4] = f.y;
+        out.v[5] = f.z;
+        return d2 > 0.f && d2 <= C.h2 && phase_of(pj) == phi;
+    };
+    const float4 *__restrict__ oms = me.slots ? C.cls_om : Om;
+    const float4 *__restrict__ nms = me.slots ? C.cls_nm : Nm;
+    float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    group_sum<6>(C, me, 0, listed >= 0 ? listed & 0xffff : 0, me.slots ? C.cls_pos : P,
+                 [&](int j) { return fetch_at(oms, nms, j); },
+                 [&](int, int, float4 pj, const Nb &nb, GroupTerm<6> &out) { return term(pj, nb, out); }, acc);
+    if (me.lane != 0 || !me.real) return;
+    if (phi >= 0) {
+        Vout[me.i] = vi4;
+        return;
+    }
+    if (listed < 0)  // overflowed
+        walk_neighbors<true>(
+            me.i, pi, 0, P, grid_view(C, sc, off), C, nullptr, -1,
+            [&](int j, float4 pj) { return j != me.i && phase_of(pj) == phi && len2(pi - f3(pj)) <= C.h2; },
+            [&](int j, float4 pj) {
+                GroupTerm<6> out;
+                if (!term(pj, fetch_at(Om, Nm, j), out)) return;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) acc[k] = __fmaf_rn(out.s[k / 3], out.v[k], acc[k]);
+            });
+    finish_post_b(C, me.slots, me.i, me.t, vi4, make_float3(acc[0], acc[1], acc[2]),
+                  make_float3(acc[3], acc[4], acc[5]), Om, Vout);
+}
+
+__global__ void __launch_bounds__(kGroupThreads) k_post_c_group(SimConsts C, const float4 *__restrict__ P,
+                                                                const float4 *__restrict__ V,
+                                                                const int *__restrict__ off,
+                                                                const float *__restrict__ mass,
+                                                                const float *__restrict__ rho,
+                                                                float4 *__restrict__ Vout)
+{
+    const GroupParticle me = group_particle(C, P, post_slots(C, false));
+    const int phi = phase_of(me.p4);
+    const float3 pi = f3(me.p4);
+    const float4 vi4 = V[me.i];
+    const float3 vi = f3(vi4);
+    const int listed = phi < 0 ? __ldg(C.nbr_count + me.t) : 0;
+    const int own = me.slots ? me.t : me.i;
+    struct Nb {
+        float3 v;
+        float m, rho;
+    };
+    auto fetch_at = [&](const float4 *__restrict__ Vp, const float *__restrict__ mp, const float *__restrict__ rp, int j) {
+        Nb r;
+        r.v = f3(Vp[j]);
+        r.m = C.textbook ? __ldg(mp + j) : 0.f;
+        r.rho = C.textbook ? __ldg(rp + j) : 1.f;
+        return r;
+    };
+    auto term = [&](float4 pj, const Nb &nb, GroupTerm<3> &out) {
+        const float d2 = len2(pi - f3(pj));
+        float wgt = poly6(C, d2);
+        if (C.textbook) wgt = __fmul_rn(wgt, __fdiv_rn(nb.m, nb.rho));
+        const float3 dv = nb.v - vi;
+        out.s[0] = wgt;
+        out.v[0] = dv.x;
+        out.v[1] = dv.y;
+        out.v[2] = dv.z;
+        return phase_of(pj) == phi && d2 <= C.h2;
+    };
+    const float4 *__restrict__ vs = me.slots ? C.cls_vb : V;
+    const float *__restrict__ ms = me.slots ? C.cls_mass : mass;
+    const float *__restrict__ rs = me.slots ? C.cls_rho : rho;
+    float acc[3] = {0.f, 0.f, 0.f};
+    group_sum<3>(C, me, 0, listed >= 0 ? listed & 0xffff : 0, me.slots ? C.cls_pos : P,
+                 [&](int j) { return fetch_at(vs, ms, rs, j); },
+                 [&](int j, int, float4 pj, const Nb &nb, GroupTerm<3> &out) { return term(pj, nb, out) && j != own; }, acc);
+    if (me.lane != 0 || !me.real) return;
+    if (phi >= 0) {
+        Vout[me.i] = vi4;
+        return;
+    }
+    if (listed < 0)  // overflowed
+        walk_neighbors<true>(
+            me.i, pi, 0, P, grid_view(C, scene_index(C, me.i), off), C, nullptr, -1,
+            [&](int j, float4 pj) { return j != me.i && phase_of(pj) == phi && len2(pi - f3(pj)) <= C.h2; },
+            [&](int j, float4 pj) {
+                GroupTerm<3> out;
+                if (!term(pj, fetch_at(V, mass, rho, j), out)) return;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) acc[k] = __fmaf_rn(out.s[0], out.v[k], acc[k]);
+            });
+    const float3 v = vi + C.xsph_c * make_float3(acc[0], acc[1], acc[2]);
+    Vout[me.i] = make_float4(v.x, v.y, v.z, vi4.w);
+}
+
+static bool use_groups(const SimConsts &C)
+{
+    return C.sl_pos && C.n <= (C.textbook ? kGroupMaxTextbook : kGroupMax);
+}
+static unsigned group_blocks(const SimConsts &C)
+{
+    return (unsigned)(((long long)C.n * kGroupLanes + kGroupThreads - 1) / kGroupThreads);
+}
+
+bool records_from_planes(int n) { return n > kWarpRecordMax; }
+
+void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const float *mass,
+                         const int *off, float *lam, float *rho, LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    const int grid = (C.n + C.scan_block - 1) / C.scan_block;
+    if (record && C.n <= kWarpRecordMax) {
+        k_lambda_record<<<(C.n * 32 + kQueueThreads - 1) / kQueueThreads, kQueueThreads, 0, st>>>(C, P, mass, off, lam,
+                                                                                               rho);
+        L->done("launch_lambda");
+        return;
+    }
+    if (record) {
+        k_lambda_lists<kRecordLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+        L->done("launch_lambda");
+        return;
+    }
+    if (use_groups(C) && C.textbook)
+        k_lambda_group<true><<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, mass, off, lam, rho);
+    else if (use_groups(C))
+        k_lambda_group<false><<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, mass, off, lam, rho);
+    else k_lambda_lists<kReadLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+    L->done("launch_lambda_lists");
+    k_lambda_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, mass, off, lam, rho);
+    L->done("launch_lambda_queued");
+}
+void launch_deltap(cudaStream_t st, const SimConsts &C, const DeltaArgs &a, LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    if (use_groups(C)) k_deltap_group<<<group_blocks(C), kGroupThreads, 0, st>>>(C, a);
+    else BP_LAUNCH_SPLIT(k_deltap, st, C, a);
+    L->done(__func__);
+}
 void launch_post_a_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,
                          const int *off, float4 *Om, float4 *Nm, LaunchLog *L)
 {
     if (C.n <= 0) return;
-    k_post_a_lists<<<(C.n + C.scan_block - 1) / C.scan_block, C.scan_block, 0, st>>>(C, P, V, rho, off, Om, Nm);
+    if (use_groups(C)) k_post_a_group<<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, V, rho, off, Om, Nm);
+    else k_post_a_lists<<<(C.n + C.scan_block - 1) / C.scan_block, C.scan_block, 0, st>>>(C, P, V, rho, off, Om, Nm);
     L->done("launch_post_a_lists");
     k_post_a_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, V, rho, off, Om, Nm);
     L->done("launch_post_a_queued");
 }
-
 void launch_post_a(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,
                    const int *off, float4 *Om, float4 *Nm, LaunchLog *L)
 {
@@ -1157,14 +1680,16 @@ void launch_post_b(cudaStream_t st, const SimConsts &C, const float4 *P, const f
                    const float4 *Nm, const int *off, float4 *Vout, LaunchLog *L)
 {
     if (C.n <= 0) return;
-    BP_LAUNCH_SPLIT(k_post_b, st, C, P, V, Om, Nm, off, Vout);
+    if (use_groups(C)) k_post_b_group<<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, V, Om, Nm, off, Vout);
+    else BP_LAUNCH_SPLIT(k_post_b, st, C, P, V, Om, Nm, off, Vout);
     L->done(__func__);
 }
 void launch_post_c(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const int *off,
                    const float *mass, const float *rho, float4 *Vout, LaunchLog *L)
 {
     if (C.n <= 0) return;
-    BP_LAUNCH_SPLIT(k_post_c, st, C, P, V, off, mass, rho, Vout);
+    if (use_groups(C) && C.nbr_count) k_post_c_group<<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, V, off, mass, rho, Vout);
+    else BP_LAUNCH_SPLIT(k_post_c, st, C, P, V, off, mass, rho, Vout);
     L->done(__func__);
 }
 

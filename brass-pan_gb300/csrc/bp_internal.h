@@ -141,6 +141,7 @@ void launch_lambda(cudaStream_t st, const SimConsts &C, const float4 *P, const f
 // also a launch over the particles that may not).
 void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const float *mass,
                          const int *off, float *lam, float *rho, LaunchLog *L);
+bool records_from_planes(int n);  // the recording launch reads the walk planes
 void launch_post_a_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,
                          const int *off, float4 *Om, float4 *Nm, LaunchLog *L);
 void launch_contacts_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *Xs, const float *w,

@@ -878,7 +878,8 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     const bool walk_planes = lists && !verlet && s->walk_xyz && C.split && !C.stage &&
                         !(s->prm.walk_options & BP_WALK_NO_PLANES);
     auto refresh_planes = [&](const float4 *P) {
-        if (classes) launch_class_refresh(st, s->n, P, ca, L, nullptr, s->walk_xyz, s->walk_stride);
+        if (shared && !records_from_planes(s->n)) refresh(P);
+        else if (classes) launch_class_refresh(st, s->n, P, ca, L, nullptr, s->walk_xyz, s->walk_stride);
         else launch_walk_planes(st, s->n, P, s->walk_xyz, s->walk_stride, L);
     };
     SimConsts Cf = Cpost;

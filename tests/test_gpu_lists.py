@@ -86,3 +86,25 @@ def test_substep_lists_in_a_batch_with_solids(bp, gpu):
         g.close()
     for a, b in zip(*outs):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("mode", ["reference", "textbook"])
+@pytest.mark.parametrize("side", [24, 31, 36])
+def test_readers_and_recorders_by_size(bp, gpu, side, mode):
+    """Scenes around the sizes where the recording launch takes a warp or a
+    thread per particle and the readers four lanes or one: lists against
+    walks, with a cloth's contacts and lists of every length at the walls."""
+    abi = bp.abi
+    m = abi.BP_MODE_TEXTBOOK if mode == "textbook" else abi.BP_MODE_REFERENCE
+    scene = fluid_scene(bp, (side, side, side), seed=side, grid_dim=64, box=(4.0, 4.0, 4.0))
+    scene.add_cloth((0.5, 0.1 * side + 0.15, 0.5), (0.1, 0, 0), (0, 0, 0.1), 9, 9, 1.0)
+    scene.velocities[-81:, 1] = -2.0
+    outs = []
+    for walk in (abi.BP_WALK_NO_STAGING, abi.BP_WALK_NO_STAGING | abi.BP_WALK_NO_LISTS):
+        g = bp.ParticleSolver(scene, bp.make_params(scene, mode=m, walk_options=walk))
+        for _ in range(3):
+            g.update(2, DT, 3)
+        outs.append((g.positions(), g.velocities(), g.field(abi.BP_FIELD_DENSITIES), g.field(abi.BP_FIELD_LAMBDAS)))
+        g.close()
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
