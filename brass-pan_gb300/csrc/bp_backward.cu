@@ -118,7 +118,7 @@ struct Tape {
     std::vector<std::vector<char>> key_fwd, key_bwd, key_warm;
     // adjoint buffers
     bool grads_ready = false;
-    float4 *gX = nullptr, *gV = nullptr, *gXn = nullptr, *gVn = nullptr, *gP = nullptr, *gP2 = nullptr;
+    float4 *gX = nullptr, *gV = nullptr, *gVn = nullptr, *gP = nullptr, *gP2 = nullptr;
     float4 *gXs = nullptr, *gVs = nullptr, *gPart = nullptr;
     float *gW = nullptr, *gLam = nullptr;
     float4 *G1 = nullptr, *G2 = nullptr, *FG = nullptr, *FV = nullptr, *FW = nullptr, *g_wind = nullptr;
@@ -176,9 +176,8 @@ void retire_tape(bp_solver *s)
     s->spare = t;
 }
 
-int SubstepTape::snap4(const float4 *src, size_t count)
+int SubstepTape::fresh4()
 {
-    if (count == 0) count = (size_t)s->n;
     if (used4 == (int)pool4.size()) {
         void *p = nullptr;
         if (cudaMalloc(&p, (size_t)std::max(s->n, 1) * sizeof(float4)) != cudaSuccess) {
@@ -187,8 +186,16 @@ int SubstepTape::snap4(const float4 *src, size_t count)
         }
         pool4.push_back((float4 *)p);
     }
-    cudaMemcpyAsync(pool4[used4], src, count * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
     return used4++;
+}
+
+int SubstepTape::snap4(const float4 *src, size_t count)
+{
+    if (count == 0) count = (size_t)s->n;
+    const int slot = fresh4();
+    if (slot >= 0)
+        cudaMemcpyAsync(pool4[slot], src, count * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+    return slot;
 }
 
 int SubstepTape::snap1(const float *src)
@@ -233,17 +240,23 @@ void save_state(const bp_solver *s, const StateBuf &b)
     }
 }
 
-void load_state(bp_solver *s, const StateBuf &b)
+void copy_state(bp_solver *s, const StateBuf &from, float4 *X, float4 *V, int *orig, int *to_new)
 {
     const size_t n = (size_t)s->n;
-    cudaMemcpyAsync(s->Xc, b.X, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
-    cudaMemcpyAsync(s->Vc, b.V, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
-    cudaMemcpyAsync(s->orig_c, b.orig, n * sizeof(int), cudaMemcpyDeviceToDevice, s->stream);
-    cudaMemcpyAsync(s->to_new, b.to_new, n * sizeof(int), cudaMemcpyDeviceToDevice, s->stream);
+    cudaMemcpyAsync(X, from.X, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+    cudaMemcpyAsync(V, from.V, n * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+    cudaMemcpyAsync(orig, from.orig, n * sizeof(int), cudaMemcpyDeviceToDevice, s->stream);
+    cudaMemcpyAsync(to_new, from.to_new, n * sizeof(int), cudaMemcpyDeviceToDevice, s->stream);
+}
+
+// The checkpoint c as the start of the segment's first substep.
+void load_state(bp_solver *s, const StateBuf &c, const StateBuf &first)
+{
+    copy_state(s, c, first.X, first.V, first.orig, first.to_new);
     if (s->rigid.num_bodies > 0) {
         const size_t nb = (size_t)s->rigid.num_bodies;
-        cudaMemcpyAsync(s->rigid.rot, b.rot, nb * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
-        cudaMemcpyAsync(s->rigid.cm, b.cm, nb * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+        cudaMemcpyAsync(s->rigid.rot, c.rot, nb * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
+        cudaMemcpyAsync(s->rigid.cm, c.cm, nb * sizeof(float4), cudaMemcpyDeviceToDevice, s->stream);
     }
 }
 
@@ -260,22 +273,62 @@ bool alloc_ctx(Tape &t, const bp_solver *s, SubCtx &c)
     return c.Xs && c.order && c.to_new && c.keys && c.off && c.mass && c.w;
 }
 
-// direction: true saves the solver's buffers into c, false loads them back
-void copy_ctx(bp_solver *s, const SubCtx &c, bool save)
+// The solver's buffers that a substep leaves for its adjoint.
+void save_ctx(bp_solver *s, const SubCtx &c)
 {
     const size_t n = (size_t)s->n;
-    auto cp = [&](void *solver_buf, void *ctx_buf, size_t bytes) {
-        cudaMemcpyAsync(save ? ctx_buf : solver_buf, save ? solver_buf : ctx_buf, bytes, cudaMemcpyDeviceToDevice,
-                        s->stream);
+    auto cp = [&](void *to, const void *from, size_t bytes) {
+        cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, s->stream);
     };
-    cp(s->Xs, c.Xs, n * sizeof(float4));
-    cp(s->order, c.order, n * sizeof(int));
-    cp(s->to_new, c.to_new, n * sizeof(int));
-    cp(s->sorted_keys, c.keys, n * sizeof(int));
-    cp(s->off, c.off, (s->ncells + 1) * sizeof(int));
-    cp(s->mass, c.mass, n * sizeof(float));
-    cp(s->w, c.w, n * sizeof(float));
+    cp(c.Xs, s->Xs, n * sizeof(float4));
+    cp(c.order, s->order, n * sizeof(int));
+    cp(c.to_new, s->to_new, n * sizeof(int));
+    cp(c.keys, s->sorted_keys, n * sizeof(int));
+    cp(c.off, s->off, (s->ncells + 1) * sizeof(int));
+    cp(c.mass, s->mass, n * sizeof(float));
+    cp(c.w, s->w, n * sizeof(float));
 }
+
+// While it lives, the solver works on the buffers of c (and its committed
+// state is st, where given) instead of its own: a substep leaves them filled,
+// or its adjoint reads them, without a copy.
+struct OnBuffers {
+    bp_solver *s;
+    float4 *Xs, *Vs, *Xc, *Vc;
+    int *order, *to_new, *keys, *off, *orig_c;
+    float *mass, *w;
+    OnBuffers(bp_solver *s_, const SubCtx &c, const StateBuf *st)
+        : s(s_), Xs(s->Xs), Vs(s->Vs), Xc(s->Xc), Vc(s->Vc), order(s->order), to_new(s->to_new), keys(s->sorted_keys),
+          off(s->off), orig_c(s->orig_c), mass(s->mass), w(s->w)
+    {
+        s->Xs = c.Xs;
+        s->order = c.order;
+        s->to_new = c.to_new;
+        s->sorted_keys = c.keys;
+        s->off = c.off;
+        s->mass = c.mass;
+        s->w = c.w;
+        if (st) {
+            s->Xc = st->X;
+            s->Vc = st->V;
+            s->orig_c = st->orig;
+        }
+    }
+    ~OnBuffers()
+    {
+        s->Xs = Xs;
+        s->Vs = Vs;
+        s->Xc = Xc;
+        s->Vc = Vc;
+        s->order = order;
+        s->to_new = to_new;
+        s->sorted_keys = keys;
+        s->off = off;
+        s->orig_c = orig_c;
+        s->mass = mass;
+        s->w = w;
+    }
+};
 
 bool stage_on(const bp_params &p, int bit) { return (p.stage_mask & bit) != 0; }
 
@@ -286,7 +339,6 @@ bp_status ensure_grads(Tape &t, const bp_solver *s)
     const size_t m = (size_t)s->dist.num_edges, f = (size_t)s->wind.num_faces;
     t.gX = t.pool.get<float4>(n);
     t.gV = t.pool.get<float4>(n);
-    t.gXn = t.pool.get<float4>(n);
     t.gVn = t.pool.get<float4>(n);
     t.gP = t.pool.get<float4>(n);
     t.gP2 = t.pool.get<float4>(n);
@@ -311,7 +363,7 @@ bp_status ensure_grads(Tape &t, const bp_solver *s)
     t.nmb = t.pool.get<float4>(n);
     t.GD = t.pool.get<float4>(n);
     t.rhob = t.pool.get<float>(n);
-    if (!(t.gX && t.gV && t.gXn && t.gVn && t.gP && t.gP2 && t.gXs && t.gVs && t.gPart && t.gW && t.gLam && t.G1 &&
+    if (!(t.gX && t.gV && t.gVn && t.gP && t.gP2 && t.gXs && t.gVs && t.gPart && t.gW && t.gLam && t.G1 &&
           t.G2 && t.FG && t.FV && t.FW && t.g_wind && t.g_stiff && t.g_rest && t.contacts && t.gRho && t.etab &&
           t.omb && t.ombo && t.nmb && t.GD && t.rhob))
         return fail_with(BP_ERR_OUT_OF_MEMORY, "backward: gradient buffers");
@@ -321,15 +373,17 @@ bp_status ensure_grads(Tape &t, const bp_solver *s)
 
 // The adjoint of one substep whose taped re-run just finished; (gX, gV) are
 // the gradients w.r.t. its committed state on entry and w.r.t. its start
-// state (start.X, start.V, in the previous order) on exit.  Every buffer
-// keeps its role (results are copied back rather than swapped), so the
-// sequence can be captured once and replayed for every substep.
+// state (start.X, start.V, in the previous order) on exit.  Both keep their
+// buffers (t.gX, t.gV) from substep to substep, so the sequence can be captured
+// once and replayed for every substep.
 void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &start, const SubstepTape &T)
 {
     const cudaStream_t st = s->stream;
     SimConsts C = u.C;  // the adjoint walks take the 27 cells, recording their pairs in the list buffer
     C.vl = nullptr;
     C.nl_pos = nullptr;
+    C.sl_pos = nullptr;
+    C.cell_keys = s->sorted_keys;
     C.nl_stats = nullptr;
     // nor the alias classes: their class-order positions are gathered only
     // for the forward walks (the same candidates in the same order remain)
@@ -348,8 +402,11 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
     // the post passes' and XSPH's density gradient, for the last fluid stage (the density they read)
     cudaMemsetAsync(t.gRho, 0, (size_t)s->n * sizeof(float), st);
     bool last_fluid = true;
+    // the gradient of the positions, and of the velocities, as the stages are
+    // undone, and the buffer of each that the next one writes
+    float4 *gP = t.gP, *gP2 = t.gP2, *gV = t.gV, *gVn = t.gVn;
     // the velocity the update gave the picked particle after its last substep
-    if (u.last && u.picked >= 0) adj_unpick(st, u.picked, s->to_new, t.gV, nullptr);
+    if (u.last && u.picked >= 0) adj_unpick(st, u.picked, s->to_new, gV, nullptr);
     for (int r = (int)T.recs.size() - 1; r >= 0; --r) {
         const TapeRec &rec = T.recs[r];
         switch (rec.stage) {
@@ -357,59 +414,58 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
             int c = r - 1;
             while (c >= 0 && T.recs[c].stage != TS_COMMIT) --c;
             const float4 *Pc = T.pool4[T.recs[c].slot];
-            const size_t bytes = (size_t)s->n * sizeof(float4);
             const float *rho = T.pool1[rec.aux1];
             if (C.use_xsph) {  // pass C first: gV -> the gradient of pass B's velocities
-                adj_xsph(st, C, Pc, T.pool4[rec.aux + 2], s->off, s->mass, rho, t.gV, t.gVn, t.gX, t.gRho);
-                cudaMemcpyAsync(t.gV, t.gVn, bytes, cudaMemcpyDeviceToDevice, st);
+                adj_xsph(st, C, Pc, T.pool4[rec.aux + 2], s->off, s->mass, rho, gV, gVn, t.gX, t.gRho);
+                std::swap(gV, gVn);
             }
-            adj_post(st, C, Pc, T.pool4[rec.slot], T.pool4[rec.aux], T.pool4[rec.aux + 1], rho, s->off, t.gV, t.gVn,
+            adj_post(st, C, Pc, T.pool4[rec.slot], T.pool4[rec.aux], T.pool4[rec.aux + 1], rho, s->off, gV, gVn,
                      t.gX, t.gRho, t.etab, t.omb, t.ombo, t.nmb);
-            cudaMemcpyAsync(t.gV, t.gVn, bytes, cudaMemcpyDeviceToDevice, st);
+            std::swap(gV, gVn);
             break;
         }
         case TS_PICK:  // the iteration's target position
-            adj_unpick(st, u.picked, s->to_new, t.gP, nullptr);
+            adj_unpick(st, u.picked, s->to_new, gP, nullptr);
             break;
         case TS_BENDING:
-            adj_bending(st, s->bend, p.bending_stiffness, T.pool4[rec.slot], s->w, s->to_new, t.gP, t.gW);
+            adj_bending(st, s->bend, p.bending_stiffness, T.pool4[rec.slot], s->w, s->to_new, gP, t.gW);
             break;
         case TS_XSPH: {  // velocities before XSPH in the slot; positions: the commit's input
             int c = r - 1;
             while (c >= 0 && T.recs[c].stage != TS_COMMIT) --c;
-            adj_xsph(st, C, T.pool4[T.recs[c].slot], T.pool4[rec.slot], s->off, s->mass, T.pool1[rec.aux1], t.gV,
-                     t.gVn, t.gX, t.gRho);
-            cudaMemcpyAsync(t.gV, t.gVn, (size_t)s->n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
+            adj_xsph(st, C, T.pool4[T.recs[c].slot], T.pool4[rec.slot], s->off, s->mass, T.pool1[rec.aux1], gV,
+                     gVn, t.gX, t.gRho);
+            std::swap(gV, gVn);
             break;
         }
         case TS_COMMIT:
-            adj_commit(st, s->n, C.inv_dt, t.gX, t.gV, t.gP, t.gXs, t.gVs, t.gW);
+            adj_commit(st, s->n, C.inv_dt, t.gX, gV, gP, t.gXs, t.gVs, t.gW);
             break;
         case TS_IMMOVABLE:
-            adj_immovable(st, s->nimm, s->imm, s->to_new, t.gP, t.gXs);
+            adj_immovable(st, s->nimm, s->imm, s->to_new, gP, t.gXs);
             break;
         case TS_DISTANCE:
-            adj_distance(st, s->dist, T.pool4[rec.slot], s->w, s->to_new, t.gP, t.gW, t.G1, t.G2, t.g_stiff,
+            adj_distance(st, s->dist, T.pool4[rec.slot], s->w, s->to_new, gP, t.gW, t.G1, t.G2, t.g_stiff,
                          t.g_rest);
             break;
         case TS_FLUID:
-            adj_fluid(st, C, T.pool4[rec.slot], s->mass, T.pool1[rec.aux], T.pool1[rec.aux + 1], s->off, t.gP,
-                      last_fluid ? t.gRho : nullptr, t.gLam, t.gPart, t.GD, t.rhob, t.gP2);
+            adj_fluid(st, C, T.pool4[rec.slot], s->mass, T.pool1[rec.aux], T.pool1[rec.aux + 1], s->off, gP,
+                      last_fluid ? t.gRho : nullptr, t.gLam, t.gPart, t.GD, t.rhob, gP2);
             last_fluid = false;
-            cudaMemcpyAsync(t.gP, t.gP2, (size_t)s->n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
+            std::swap(gP, gP2);
             break;
         case TS_PLANES:
-            adj_planes(st, C, s->Xs, T.pool4[rec.slot], t.gP, t.gXs);
+            adj_planes(st, C, s->Xs, T.pool4[rec.slot], gP, t.gXs);
             break;
         case TS_PCOLL:
-            adj_contacts(st, C, T.pool4[rec.slot], s->Xs, s->w, s->off, t.contacts, t.gP, t.gP2, t.gXs, t.gW);
-            cudaMemcpyAsync(t.gP, t.gP2, (size_t)s->n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
+            adj_contacts(st, C, T.pool4[rec.slot], s->Xs, s->w, s->off, t.contacts, gP, gP2, t.gXs, t.gW);
+            std::swap(gP, gP2);
             break;
         case TS_SHAPE:
-            adj_shape_matching(st, s->rigid, T.pool4[rec.aux], T.pool4[rec.slot], s->to_new, t.gP);
+            adj_shape_matching(st, s->rigid, T.pool4[rec.aux], T.pool4[rec.slot], s->to_new, gP);
             break;
         case TS_WIND:
-            adj_wind(st, C, s->wind, T.pool4[rec.slot], T.pool4[T.vs_slot], s->mass, s->to_new, t.gP, t.gVs, t.FG,
+            adj_wind(st, C, s->wind, T.pool4[rec.slot], T.pool4[T.vs_slot], s->mass, s->to_new, gP, t.gVs, t.FG,
                      t.FV, t.FW, t.g_wind);
             break;
         default:  // excluded by check_supported
@@ -417,10 +473,8 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
         }
     }
     const int inv_scaled = (distance || bending || pcoll) ? 1 : 0;  // the stages that read w
-    adj_reorder(st, C, s->order, start.X, start.V, planes ? 1 : 0, inv_scaled, t.gP, t.gXs, t.gVs, t.gW, t.gXn,
-                t.gVn);
-    cudaMemcpyAsync(t.gX, t.gXn, (size_t)s->n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(t.gV, t.gVn, (size_t)s->n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
+    // (gX, gV) were read by the commit's adjoint, the last to need them
+    adj_reorder(st, C, s->order, start.X, start.V, planes ? 1 : 0, inv_scaled, gP, t.gXs, t.gVs, t.gW, t.gX, t.gV);
     // the substep began by setting the picked particle's position and velocity
     if (u.picked >= 0) adj_unpick_orig(st, s->n, u.picked, start.orig, t.gX, t.gV);
 }
@@ -478,7 +532,8 @@ bp_status tape_record_update(bp_solver *s, int nsub, float dt, int iterations, i
         save_state(s, t.ckpts[ck]);
         t.since = 0;
     }
-    const SimConsts C = make_consts(s, dt / (float)nsub);
+    SimConsts C = make_consts(s, dt / (float)nsub);
+    if (picked >= 0) C.sl_pos = nullptr;  // as the update itself (enqueue_update)
     for (int k = 0; k < nsub; ++k)
         t.subs.push_back(Tape::Sub{C, s->prm, iterations, k == 0 ? ck : -1, picked, ppos, pvel, k == nsub - 1});
     t.since += nsub;
@@ -554,16 +609,20 @@ extern "C" bp_status bp_solver_backward(bp_solver *s, const float *grad_position
         int seg_begin = seg_end - 1;
         while (t.subs[seg_begin].ckpt < 0) --seg_begin;  // substep 0 always holds checkpoint 0
         const int len = seg_end - seg_begin;
-        while ((int)t.seg.size() < len) {
+        // seg[q] is the start of the segment's substep q, so seg[len] its end
+        while ((int)t.seg.size() < len + 1) {
             StateBuf b;
+            if (!alloc_state(t, s, b)) return bail(BP_ERR_OUT_OF_MEMORY, "backward: segment buffers");
+            t.seg.push_back(b);
+        }
+        while ((int)t.tapes.size() < len) {
             SubCtx c;
             SubstepTape *tp = new (std::nothrow) SubstepTape();
-            if (!tp || !alloc_state(t, s, b) || !alloc_ctx(t, s, c)) {
+            if (!tp || !alloc_ctx(t, s, c)) {
                 delete tp;
                 return bail(BP_ERR_OUT_OF_MEMORY, "backward: segment buffers");
             }
             tp->s = s;
-            t.seg.push_back(b);
             t.ctxs.push_back(c);
             t.tapes.push_back(tp);
             t.g_fwd.push_back(nullptr);
@@ -574,18 +633,37 @@ extern "C" bp_status bp_solver_backward(bp_solver *s, const float *grad_position
         }
         // forward from the checkpoint, recording every substep: its start
         // state, each stage's input and the grid it ran with
-        load_state(s, t.ckpts[t.subs[seg_begin].ckpt]);
+        load_state(s, t.ckpts[t.subs[seg_begin].ckpt], t.seg[0]);
         for (int k = seg_begin; k < seg_end; ++k) {
             const int q = k - seg_begin;
             const Tape::Sub &u = t.subs[k];
             s->prm = u.prm;
             auto body = [&] {
-                save_state(s, t.seg[q]);
-                t.tapes[q]->reset();
-                enqueue_substep(s, u.C, u.iterations, u.picked, u.ppos, &L, t.tapes[q]);
-                if (u.last && u.picked >= 0)  // the end of its update: the picked particle's velocity
+                SubstepTape &T = *t.tapes[q];
+                const StateBuf &from = t.seg[q], &to = t.seg[q + 1];
+                T.reset();
+                SimConsts C = u.C;
+                if (u.picked < 0) {  // straight from and into the segment's buffers
+                    OnBuffers on(s, t.ctxs[q], &from);
+                    T.next_X = to.X;
+                    T.next_V = to.V;
+                    T.next_orig = to.orig;
+                    C.cell_keys = s->sorted_keys;
+                    enqueue_substep(s, C, u.iterations, u.picked, u.ppos, &L, &T);
+                    return;
+                }
+                // the pick changes the start state in place and finds its
+                // particle through the map of the substep before
+                copy_state(s, from, s->Xc, s->Vc, s->orig_c, s->to_new);
+                if (q > 0)
+                    cudaMemcpyAsync(s->to_new, t.ctxs[q - 1].to_new, N * sizeof(int), cudaMemcpyDeviceToDevice, st);
+                T.next_X = T.next_V = nullptr;
+                T.next_orig = nullptr;
+                enqueue_substep(s, C, u.iterations, u.picked, u.ppos, &L, &T);
+                if (u.last)  // the end of its update: the picked particle's velocity
                     launch_pick(s->stream, u.picked, s->to_new, s->Xc, u.ppos, 0, s->Vc, u.pvel, &L);
-                copy_ctx(s, t.ctxs[q], true);
+                save_ctx(s, t.ctxs[q]);
+                save_state(s, to);
             };
             if (sub_key(u) != t.key_warm[q]) {  // a new configuration runs once directly, growing
                 body();                          // the record pool outside any capture
@@ -602,7 +680,7 @@ extern "C" bp_status bp_solver_backward(bp_solver *s, const float *grad_position
             const Tape::Sub &u = t.subs[k];
             s->prm = u.prm;
             const bp_status e = replay(s, t.g_bwd[q], t.key_bwd[q], u, [&] {
-                copy_ctx(s, t.ctxs[q], false);
+                OnBuffers on(s, t.ctxs[q], nullptr);
                 adjoint_substep(s, t, u, t.seg[q], *t.tapes[q]);
             });
             if (e != BP_OK) return bail(e, "backward: adjoint graph");

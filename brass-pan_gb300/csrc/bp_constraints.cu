@@ -20,21 +20,21 @@
 
 namespace bp {
 
-__global__ void k_planes(SimConsts C, const float4 *__restrict__ Xs, float4 *__restrict__ P)
+__global__ void k_planes(SimConsts C, const float4 *__restrict__ Xs, const float4 *P, float4 *Pout)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= C.n) return;
     const float4 p4 = P[i];
     float3 p = f3(p4);
     plane_collide(C, scene_index(C, i), f3(Xs[i]), p);
-    P[i] = make_float4(p.x, p.y, p.z, p4.w);
+    Pout[i] = make_float4(p.x, p.y, p.z, p4.w);
     track_displacement(C, i, p, true);
 }
 
-void launch_planes(cudaStream_t st, const SimConsts &C, const float4 *Xs, float4 *P, LaunchLog *L)
+void launch_planes(cudaStream_t st, const SimConsts &C, const float4 *Xs, const float4 *P, float4 *Pout, LaunchLog *L)
 {
-    if (C.n <= 0 || C.nplanes <= 0) return;
-    k_planes<<<(C.n + 255) / 256, 256, 0, st>>>(C, Xs, P);
+    if (C.n <= 0 || (C.nplanes <= 0 && Pout == P)) return;
+    k_planes<<<(C.n + 255) / 256, 256, 0, st>>>(C, Xs, P, Pout);
     L->done(__func__);
 }
 

@@ -169,7 +169,8 @@ void launch_neighbor_counts_f3(cudaStream_t st, int n, const float *pos3, float 
                                const int *start, const int *end, int *counts);
 
 // ---- per-particle and constraint kernels ----
-void launch_planes(cudaStream_t st, const SimConsts &C, const float4 *Xs, float4 *P, LaunchLog *L);
+// Pout: P itself, or another buffer.
+void launch_planes(cudaStream_t st, const SimConsts &C, const float4 *Xs, const float4 *P, float4 *Pout, LaunchLog *L);
 void launch_commit(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *Xs, const float4 *Vs,
                    const int *orig_s, float4 *Xc, float4 *Vc, int *orig_c, LaunchLog *L);
 // tile_solid: nullptr, or one flag per 256 sorted particles (the tile holds a solid);

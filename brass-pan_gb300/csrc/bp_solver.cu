@@ -144,14 +144,13 @@ static bool planes_confine(const bp_solver *s, int D, float cell)
 // in place of five searches and six reads (1M-particle dam break at 4
 // iterations and 3 post passes: 4.73 -> 3.04 ms a frame of 2 substeps; mixed
 // scene late 12.4 -> 8.85 ms; 1,728 particles 0.45 -> 0.32 ms).  The lists
-// come from the split, unstaged recording walk over the walk planes; a taped
-// update keeps the separate passes its adjoint re-runs.  neighbor_skin sets
-// the skin; with 0 it adapts (adapt_skin), up to the kMaxSkin of h returned.
+// come from the split, unstaged recording walk.  neighbor_skin sets the skin;
+// with 0 it adapts (adapt_skin), up to the kMaxSkin of h returned.
 static float largest_skin(const bp_solver *s)
 {
     const bp_params &p = s->prm;
     const int32_t other = BP_WALK_NO_SPLIT | BP_WALK_NO_LISTS | BP_WALK_NO_PLANES;
-    if (s->tape || !(p.walk_options & BP_WALK_NO_STAGING) || (p.walk_options & other) || p.scan_persistent ||
+    if (!(p.walk_options & BP_WALK_NO_STAGING) || (p.walk_options & other) || p.scan_persistent ||
         !((p.stage_mask & BP_STAGE_FLUID) || ((p.stage_mask & BP_STAGE_PARTICLE_COLLISION) && s->has_solid)))
         return 0.f;
     return p.kernel_radius * (p.neighbor_skin > 0.f ? p.neighbor_skin : kMaxSkin);
@@ -797,7 +796,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // position pass the next iteration's or the final commit (BP_WALK_NO_FUSION:
     // launches of their own; bit-identical either way)
     const bool fuse = !tape && !(s->prm.walk_options & BP_WALK_NO_FUSION);
-    const bool distance_step = fuse && distance && !bending && !rigid && s->dist_step.range;
+    const bool distance_step = (tape || fuse) && distance && !bending && !rigid && s->dist_step.range;
     const bool fuse_first_planes = planes && !wind && !picking && iterations > 0 && fuse;
     ReorderArgs ra;
     ra.order = s->order;
@@ -806,7 +805,8 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     ra.orig_c = s->orig_c;
     ra.Xs = s->Xs;
     ra.Vs = s->Vs;
-    ra.P = s->Pa;
+    const int tape0 = tape ? tape->fresh4() : -1;
+    ra.P = tape0 >= 0 ? tape->pool4[tape0] : s->Pa;
     ra.mass = s->mass;
     ra.orig_s = s->orig_s;
     ra.to_new = s->to_new;
@@ -846,9 +846,33 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     auto refresh = [&](const float4 *P) {
         if (classes) launch_class_refresh(st, s->n, P, ca, L);
     };
-    if (tape) tape->vs_slot = tape->snap4(s->Vs);
+    if (tape && tape->next_X) {  // the commit writes the next substep's start
+        s->Xc = tape->next_X;
+        s->Vc = tape->next_V;
+        s->orig_c = tape->next_orig;
+    }
 
     float4 *cur = s->Pa, *other = s->Pb;
+    int slot = tape0;  // of cur, in the tape's pool
+    if (tape && tape0 >= 0) cur = ra.P;
+    // where a stage that does not work in place writes, and its result as the
+    // next one's input
+    auto stage_out = [&]() -> float4 * {
+        const int k = tape ? tape->fresh4() : -1;
+        return k >= 0 ? tape->pool4[k] : other;
+    };
+    auto stage_done = [&](float4 *out) {
+        if (out == other) std::swap(cur, other);
+        else cur = out;
+        slot = tape ? tape->used4 - 1 : -1;
+    };
+    // a stage that works in place: taped, on a copy of its input
+    auto in_place = [&]() {
+        if (!tape) return;
+        float4 *out = stage_out();
+        cudaMemcpyAsync(out, cur, (size_t)s->n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
+        stage_done(out);
+    };
     // Verlet lists (SimConsts::vl): iteration 0's lambda builds them and every
     // later walk of the substep may read them; the kernels before the build
     // neither read them nor track displacements.
@@ -910,7 +934,11 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
                               C.cell, solid_culling ? s->solid_walk : nullptr);
     }
     if (wind) {
-        if (tape) tape->push(TS_WIND, cur);
+        if (tape) {
+            tape->vs_slot = tape->snap4(s->Vs);
+            tape->push(TS_WIND, slot);
+        }
+        in_place();
         launch_wind(st, Cpre, s->wind, cur, s->Vs, s->mass, s->to_new, L);
     }
 
@@ -928,8 +956,14 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             launch_pick(st, picked, s->to_new, cur, ppos, 1, nullptr, make_float3(0.f, 0.f, 0.f), L);
         }
         if (planes && !planes_done) {
-            if (tape) tape->push(TS_PLANES, cur);
-            launch_planes(st, Cit, s->Xs, cur, L);
+            if (tape) {
+                tape->push(TS_PLANES, slot);
+                float4 *out = stage_out();
+                launch_planes(st, Cit, s->Xs, cur, out, L);
+                stage_done(out);
+            } else {
+                launch_planes(st, Cit, s->Xs, cur, cur, L);
+            }
         }
         planes_done = false;
         if (listed_contacts && !(fluid && it == 0)) {
@@ -938,12 +972,15 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
                 cudaMemsetAsync(s->sl_bits, 0, 2 * kSlLevels * s->sl_words * sizeof(unsigned), st);
                 launch_lambda_lists(st, Cf, true, cur, s->mass, s->off, s->lam, s->rho, L);
             }
+            if (tape) tape->push(TS_PCOLL, slot);
             SimConsts Cc = Cpost;
             next_list_pass(Cc, !fluid && it == iterations - 1);
-            launch_contacts_lists(st, Cc, cur, s->Xs, s->w, s->off, other, L);
-            std::swap(cur, other);
+            float4 *out = stage_out();
+            launch_contacts_lists(st, Cc, cur, s->Xs, s->w, s->off, out, L);
+            stage_done(out);
         } else if (pcoll) {
-            if (tape) tape->push(TS_PCOLL, cur);
+            if (tape) tape->push(TS_PCOLL, slot);
+            float4 *out = stage_out();
             // solids walk in a launch of their own, in full warps (measured
             // faster than walking them in the staged CTAs, whether solids are
             // scattered through fluid or the whole scene)
@@ -956,8 +993,8 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             }
             launch_particle_collision(st, Cc, cur, s->Xs, s->w, s->off, s->tile_solid, s->solid_prefix,
                                       s->solid_list, solid_culling ? s->solid_walk : nullptr, s->num_solids, true,
-                                      s->solid_near, s->solid_pos, other, L);
-            std::swap(cur, other);
+                                      s->solid_near, s->solid_pos, out, L);
+            stage_done(out);
         }
         if (fluid) {
             // lambda and delta-p read the same positions
@@ -976,14 +1013,15 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             if (tape) {
                 const int aux = tape->snap1(s->lam);
                 tape->snap1(s->rho);
-                tape->push(TS_FLUID, cur, aux);
+                tape->push(TS_FLUID, slot, aux);
             }
+            float4 *out = stage_out();
             DeltaArgs da;
             da.P = cur;
             da.mass = s->mass;
             da.lam = s->lam;
             da.off = s->off;
-            da.Pout = other;
+            da.Pout = out;
             da.epilogue = 0;
             da.Xs = s->Xs;
             da.Xc = s->Xc;
@@ -1001,7 +1039,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
                 }
             }
             launch_deltap(st, (verlet && it == 0) ? Cpost : Cf, da, L);
-            std::swap(cur, other);
+            stage_done(out);
         }
         if (distance_step) {
             DistanceStep ds = s->dist_step;
@@ -1015,46 +1053,54 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             ds.Vc = s->Vc;
             ds.orig_c = s->orig_c;
             ds.epilogue = 0;
-            if (it == iterations - 1) {
+            if (tape) {
+                tape->push(TS_DISTANCE, slot);
+                if (immov) tape->push(TS_IMMOVABLE, -1);
+            } else if (it == iterations - 1) {
                 ds.epilogue = 2;
                 committed = true;
             } else if (planes && !picking) {
                 ds.epilogue = 1;
                 planes_done = true;
             }
-            launch_distance_step(st, Cpost, ds, cur, other, L);
-            std::swap(cur, other);
+            float4 *out = stage_out();
+            launch_distance_step(st, Cpost, ds, cur, out, L);
+            stage_done(out);
             continue;
         }
         if (distance) {
-            if (tape) tape->push(TS_DISTANCE, cur);
+            if (tape) tape->push(TS_DISTANCE, slot);
+            in_place();
             launch_distance(st, Cpost, s->dist, cur, s->w, s->to_new, s->err, L);
         }
         if (bending) {  // PS:956-969
-            if (tape) tape->push(TS_BENDING, cur);
+            if (tape) tape->push(TS_BENDING, slot);
+            in_place();
             BendingArgs ba = s->bend;
             ba.stiffness = s->prm.bending_stiffness;
             launch_bending(st, Cpost, ba, cur, s->w, s->to_new, L);
         }
         if (rigid) {
-            if (tape) tape->push(TS_SHAPE, cur);
+            if (tape) tape->push(TS_SHAPE, slot);
+            in_place();
             launch_shape_matching(st, Cpost, s->rigid, cur, s->to_new, L);
             if (tape) tape->recs.back().aux = tape->snap4(s->rigid.rot, (size_t)s->rigid.num_bodies);
         }
         if (immov) {
-            if (tape) tape->push(TS_IMMOVABLE, cur);
+            if (tape) tape->push(TS_IMMOVABLE, slot);
+            in_place();
             launch_immovable(st, Cpost, s->nimm, s->imm, s->to_new, s->Xs, cur, L);
         }
     }
     if (!committed) {
-        if (tape) tape->push(TS_COMMIT, cur);
+        if (tape) tape->push(TS_COMMIT, slot);
         launch_commit(st, Cpost, cur, s->Xs, s->Vs, s->orig_s, s->Xc, s->Vc, s->orig_c, L);
     }
     s->Pcur = cur;
 
-    if (tape && post_ab) tape->push(TS_POST_AB, s->Vc);
+    if (tape && post_ab) tape->push(TS_POST_AB, tape->snap4(s->Vc));
     if (tape && !post_ab && C.use_xsph) {
-        tape->push(TS_XSPH, s->Vc);
+        tape->push(TS_XSPH, tape->snap4(s->Vc));
         tape->recs.back().aux1 = tape->snap1(s->rho);  // the density textbook XSPH weighs with
     }
     // The post passes keep class positions in their lists where lambda left

@@ -59,25 +59,31 @@ struct TapeRec {
     int aux1 = -1;  // TS_POST_AB, TS_XSPH: the density the passes read (pool1)
 };
 
-// The intermediates of one substep re-run for its adjoint: each stage's
-// input, copied into a pool of device buffers that persists across substeps.
+// The intermediates of one substep re-run for its adjoint, in a pool of device
+// buffers that persists across substeps: a stage that writes elsewhere than it
+// reads goes from one buffer of the pool to the next, and one that works in
+// place does so on a copy of its input.
 struct SubstepTape {
     bp_solver *s = nullptr;
     std::vector<float4 *> pool4;
     std::vector<float *> pool1;
     int used4 = 0, used1 = 0;
     std::vector<TapeRec> recs;
-    int vs_slot = -1;  // velocities after the reorder
+    int vs_slot = -1;  // velocities after the reorder (wind reads them)
     bool ok = true;    // false after a failed allocation
+    // where the substep's committed state goes (nullptr: back into the solver's buffers)
+    float4 *next_X = nullptr, *next_V = nullptr;
+    int *next_orig = nullptr;
     void reset()
     {
         used4 = used1 = 0;
         recs.clear();
         vs_slot = -1;
     }
+    int fresh4();  // a buffer of the pool to write to (-1: out of memory)
     int snap4(const float4 *src, size_t count = 0);  // count 0: one per particle (count <= particles)
     int snap1(const float *src);
-    void push(int stage, const float4 *src, int aux = -1) { recs.push_back(TapeRec{stage, snap4(src), aux, -1}); }
+    void push(int stage, int slot, int aux = -1) { recs.push_back(TapeRec{stage, slot, aux, -1}); }
     void mark(int stage) { recs.push_back(TapeRec{stage, -1, -1, -1}); }
 };
 }  // namespace bp
