@@ -166,6 +166,35 @@ __global__ void k_adj_immovable(int k, const int *__restrict__ ids, const int *_
 // p1 -= w1 k, p2 += w2 k.  Per edge: the gradient contributions to both
 // endpoints (xyz: position, w: inverse scaled mass) and to s and L.
 
+struct EdgeAdj {
+    float3 x;           // gradient of the first end's position (the second's: its negative)
+    float w1, w2;       // of the ends' inverse scaled masses
+    float stiff, rest;
+};
+// Ends at p1, p2 with inverse scaled masses w1, w2 and outgoing gradients g1, g2.
+__device__ __forceinline__ EdgeAdj adj_edge(float3 p1, float3 p2, float w1, float w2, float3 g1, float3 g2, float2 prm)
+{
+    EdgeAdj o{make_float3(0.f, 0.f, 0.f), 0.f, 0.f, 0.f, 0.f};
+    const float3 x12 = sub3(p1, p2);
+    const float d = sqrtf(dotf(x12, x12));
+    if (d <= 1e-5f) return o;
+    const float sw = w1 + w2;
+    const float3 n = mul3(x12, 1.0f / d);
+    const float sc = (d - prm.x) / sw * prm.y;
+    const float3 k = mul3(n, sc);
+    const float3 kb = add3(mul3(g1, -w1), mul3(g2, w2));
+    const float3 nb = mul3(kb, sc);
+    const float sb = dotf(kb, n);
+    const float db = sb * prm.y / sw;
+    const float swb = -sb * (d - prm.x) * prm.y / (sw * sw);
+    o.w1 = -dotf(k, g1) + swb;
+    o.w2 = dotf(k, g2) + swb;
+    o.x = add3(mul3(sub3(nb, mul3(n, dotf(n, nb))), 1.0f / d), mul3(n, db));
+    o.stiff = sb * (d - prm.x) / sw;
+    o.rest = -sb * prm.y / sw;
+    return o;
+}
+
 __global__ void k_adj_distance_edges(int m, const int2 *__restrict__ pairs, const float2 *__restrict__ params,
                                      const float4 *__restrict__ Pin, const float *__restrict__ w,
                                      const int *__restrict__ to_new, const float4 *__restrict__ gOut,
@@ -177,31 +206,102 @@ __global__ void k_adj_distance_edges(int m, const int2 *__restrict__ pairs, cons
     const int2 pr = pairs[e];
     const float2 prm = params[e];
     const int id1 = to_new[pr.x], id2 = to_new[pr.y];
-    const float3 x12 = sub3(ld3(Pin, id1), ld3(Pin, id2));
-    const float d = sqrtf(dotf(x12, x12));
-    if (d <= 1e-5f) {
-        G1[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-        G2[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
+    const EdgeAdj o = adj_edge(ld3(Pin, id1), ld3(Pin, id2), w[id1], w[id2], ld3(gOut, id1), ld3(gOut, id2), prm);
+    G1[e] = f4(o.x, o.w1);
+    G2[e] = f4(mul3(o.x, -1.f), o.w2);
+    g_stiff[e] += o.stiff;
+    g_rest[e] += o.rest;
+}
+
+// The adjoint of a cloth iteration's end (k_distance_step) and of the planes
+// before it, four lanes per particle as there: the immovables' gradient goes to
+// their start positions, each edge's is evaluated from both ends and added in
+// CSR order, its first end's lane writes the parameters' gradients, and
+// Pplanes (nullptr: no planes directly before) are undone.  One launch where
+// four bound by their latency were (128 x 128 flag, 10 frames and their
+// gradients: 4315 -> 4090 us; with 2 edges of a lane in flight 4310, with 8
+// lanes 4205, with 16 4540).
+constexpr int kStepLanes = 4, kStepAhead = 3;  // edges of a lane in flight
+__global__ void __launch_bounds__(128) k_adj_distance_step(SimConsts C, DistanceStep a, const float4 *__restrict__ Pin,
+                                                           const float4 *__restrict__ Pplanes,
+                                                           const float4 *__restrict__ gOut, float4 *__restrict__ gIn,
+                                                           float4 *__restrict__ gXs, float *__restrict__ gW,
+                                                           float *__restrict__ g_stiff, float *__restrict__ g_rest)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x % kStepLanes;
+    const int i = (int)min(t / kStepLanes, (long long)C.n - 1);  // lanes past the end repeat the last particle
+    const bool real = t / kStepLanes < C.n;
+    const int id = a.orig_s[i];
+    const int2 range = __ldg(a.range + id);
+    const int b = range.x, e = range.y;
+    const float3 zero = make_float3(0.f, 0.f, 0.f);
+    const bool pinned = a.pinned && a.pinned[id];
+    const float3 out = ld3(gOut, i), gi = pinned ? zero : out;  // the immovables' adjoint
+    const float3 pi = ld3(Pin, i);
+    const float wi = a.w[i];
+    float3 g = gi;
+    float gw = gW[i];
+    const int rounds =
+        __reduce_max_sync(0xffffffffu, (e - b + kStepAhead * kStepLanes - 1) / (kStepAhead * kStepLanes));
+    for (int r = 0; r < rounds; ++r) {
+        const int q0 = b + r * kStepAhead * kStepLanes;
+        int4 c[kStepAhead];
+        float3 po[kStepAhead], go[kStepAhead], x[kStepAhead];
+        float wo[kStepAhead], wb[kStepAhead];
+#pragma unroll
+        for (int k = 0; k < kStepAhead; ++k) {
+            const int q = q0 + k * kStepLanes + lane;
+            c[k] = q < e ? __ldg(a.inc + q) : make_int4(2 * id, 0, 0, 0);  // an edge to itself: nothing
+        }
+#pragma unroll
+        for (int k = 0; k < kStepAhead; ++k) {
+            const int other = c[k].x >> 1, j = __ldg(a.to_new + other);
+            po[k] = ld3(Pin, j);
+            go[k] = (a.pinned && a.pinned[other]) ? zero : ld3(gOut, j);
+            wo[k] = a.w[j];
+        }
+#pragma unroll
+        for (int k = 0; k < kStepAhead; ++k) {
+            const float2 prm = make_float2(__int_as_float(c[k].y), __int_as_float(c[k].z));
+            const bool second = (c[k].x & 1) != 0;
+            const EdgeAdj o = adj_edge(second ? po[k] : pi, second ? pi : po[k], second ? wo[k] : wi,
+                                       second ? wi : wo[k], second ? go[k] : gi, second ? gi : go[k], prm);
+            x[k] = second ? mul3(o.x, -1.f) : o.x;
+            wb[k] = second ? o.w2 : o.w1;
+            if (!second && q0 + k * kStepLanes + lane < e && real) {
+                g_stiff[c[k].w] += o.stiff;
+                g_rest[c[k].w] += o.rest;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kStepAhead; ++k)
+#pragma unroll
+            for (int l = 0; l < kStepLanes; ++l) {
+                const float3 u = make_float3(__shfl_sync(0xffffffffu, x[k].x, l, kStepLanes),
+                                             __shfl_sync(0xffffffffu, x[k].y, l, kStepLanes),
+                                             __shfl_sync(0xffffffffu, x[k].z, l, kStepLanes));
+                const float uw = __shfl_sync(0xffffffffu, wb[k], l, kStepLanes);
+                if (q0 + k * kStepLanes + l < e) {
+                    g = add3(g, u);
+                    gw += uw;
+                }
+            }
     }
-    const float w1 = w[id1], w2 = w[id2], sw = w1 + w2;
-    const float3 n = mul3(x12, 1.0f / d);
-    const float sc = (d - prm.x) / sw * prm.y;
-    const float3 k = mul3(n, sc);
-    const float3 g1 = ld3(gOut, id1), g2 = ld3(gOut, id2);
-    const float3 kb = add3(mul3(g1, -w1), mul3(g2, w2));
-    float wb1 = -dotf(k, g1), wb2 = dotf(k, g2);
-    const float3 nb = mul3(kb, sc);
-    const float sb = dotf(kb, n);
-    const float db = sb * prm.y / sw;
-    const float swb = -sb * (d - prm.x) * prm.y / (sw * sw);
-    wb1 += swb;
-    wb2 += swb;
-    const float3 xb = add3(mul3(sub3(nb, mul3(n, dotf(n, nb))), 1.0f / d), mul3(n, db));
-    G1[e] = f4(xb, wb1);
-    G2[e] = f4(mul3(xb, -1.f), wb2);
-    g_stiff[e] += sb * (d - prm.x) / sw;
-    g_rest[e] += -sb * prm.y / sw;
+    if (lane != 0 || !real) return;
+    gW[i] = gw;
+    float3 gx = f3(gXs[i]);
+    if (pinned) gx = add3(gx, out);
+    if (Pplanes) {
+        const int s = scene_index(C, i);
+        const V3<Dual<6>> x = dv3var<6>(f3(a.Xs[i]), 0);
+        V3<Dual<6>> p = dv3var<6>(f3(Pplanes[i]), 3);
+        BP_PLANES_OF(C, s, dplane_collide<6>(C, np, planes, x, p));
+        gx = make_float3(gx.x + vjp(p, g, 0), gx.y + vjp(p, g, 1), gx.z + vjp(p, g, 2));
+        g = make_float3(vjp(p, g, 3), vjp(p, g, 4), vjp(p, g, 5));
+    }
+    if (pinned || Pplanes) gXs[i] = f4(gx);
+    gIn[i] = f4(g);
 }
 
 __global__ void k_adj_distance_apply(int nn_, const int *__restrict__ node_ids, const int *__restrict__ ptr,
@@ -1271,6 +1371,15 @@ void adj_distance(cudaStream_t st, const DistanceArgs &a, const float4 *Pin, con
                                                               G2, g_stiff, g_rest);
     k_adj_distance_apply<<<blocks(a.num_nodes), 256, 0, st>>>(a.num_nodes, a.node_ids, a.node_ptr, a.node_inc, G1, G2,
                                                               to_new, gP, gW);
+}
+void adj_distance_step(cudaStream_t st, const SimConsts &C, const DistanceStep &a, const float4 *Pin,
+                       const float4 *Pplanes, const float4 *gOut, float4 *gIn, float4 *gXs, float *gW, float *g_stiff,
+                       float *g_rest)
+{
+    if (C.n <= 0) return;
+    const long long threads = (long long)C.n * kStepLanes;
+    k_adj_distance_step<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(C, a, Pin, Pplanes, gOut, gIn, gXs, gW,
+                                                                         g_stiff, g_rest);
 }
 void adj_wind(cudaStream_t st, const SimConsts &C, const WindArgs &a, const float4 *Pin, const float4 *Vs,
               const float *mass, const int *to_new, float4 *gP, float4 *gVs, float4 *FG, float4 *FV, float4 *FW,

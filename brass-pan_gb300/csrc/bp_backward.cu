@@ -31,6 +31,9 @@ void adj_commit(cudaStream_t st, int n, float inv_dt, const float4 *gX, const fl
 void adj_immovable(cudaStream_t st, int k, const int *ids, const int *to_new, float4 *gP, float4 *gXs);
 void adj_distance(cudaStream_t st, const DistanceArgs &a, const float4 *Pin, const float *w, const int *to_new,
                   float4 *gP, float *gW, float4 *G1, float4 *G2, float *g_stiff, float *g_rest);
+void adj_distance_step(cudaStream_t st, const SimConsts &C, const DistanceStep &a, const float4 *Pin,
+                       const float4 *Pplanes, const float4 *gOut, float4 *gIn, float4 *gXs, float *gW, float *g_stiff,
+                       float *g_rest);
 void adj_wind(cudaStream_t st, const SimConsts &C, const WindArgs &a, const float4 *Pin, const float4 *Vs,
               const float *mass, const int *to_new, float4 *gP, float4 *gVs, float4 *FG, float4 *FV, float4 *FW,
               float4 *g_wind);
@@ -371,12 +374,14 @@ bp_status ensure_grads(Tape &t, const bp_solver *s)
     return BP_OK;
 }
 
-// The adjoint of one substep whose taped re-run just finished; (gX, gV) are
+// The adjoint of one substep whose taped re-run just finished (orig: the
+// original id of each sorted particle, as it committed them); (gX, gV) are
 // the gradients w.r.t. its committed state on entry and w.r.t. its start
 // state (start.X, start.V, in the previous order) on exit.  Both keep their
 // buffers (t.gX, t.gV) from substep to substep, so the sequence can be captured
 // once and replayed for every substep.
-void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &start, const SubstepTape &T)
+void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &start, const int *orig,
+                     const SubstepTape &T)
 {
     const cudaStream_t st = s->stream;
     SimConsts C = u.C;  // the adjoint walks take the 27 cells, recording their pairs in the list buffer
@@ -408,6 +413,22 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
     // the velocity the update gave the picked particle after its last substep
     if (u.last && u.picked >= 0) adj_unpick(st, u.picked, s->to_new, gV, nullptr);
     for (int r = (int)T.recs.size() - 1; r >= 0; --r) {
+        // a cloth iteration's end and the planes directly before it in one launch
+        const int imm = T.recs[r].stage == TS_IMMOVABLE ? 1 : 0, d = r - imm;
+        if (s->dist_step.range && d >= 0 && T.recs[d].stage == TS_DISTANCE) {
+            const bool pl = d > 0 && T.recs[d - 1].stage == TS_PLANES;
+            DistanceStep ds = s->dist_step;
+            if (!imm) ds.pinned = nullptr;
+            ds.orig_s = orig;
+            ds.to_new = s->to_new;
+            ds.w = s->w;
+            ds.Xs = s->Xs;
+            adj_distance_step(st, C, ds, T.pool4[T.recs[d].slot], pl ? T.pool4[T.recs[d - 1].slot] : nullptr, gP, gP2,
+                              t.gXs, t.gW, t.g_stiff, t.g_rest);
+            std::swap(gP, gP2);
+            r = pl ? d - 1 : d;
+            continue;
+        }
         const TapeRec &rec = T.recs[r];
         switch (rec.stage) {
         case TS_POST_AB: {  // positions: the commit's input; velocities before pass A in the slot
@@ -681,7 +702,7 @@ extern "C" bp_status bp_solver_backward(bp_solver *s, const float *grad_position
             s->prm = u.prm;
             const bp_status e = replay(s, t.g_bwd[q], t.key_bwd[q], u, [&] {
                 OnBuffers on(s, t.ctxs[q], nullptr);
-                adjoint_substep(s, t, u, t.seg[q], *t.tapes[q]);
+                adjoint_substep(s, t, u, t.seg[q], t.seg[q + 1].orig, *t.tapes[q]);
             });
             if (e != BP_OK) return bail(e, "backward: adjoint graph");
         }

@@ -782,7 +782,7 @@ void build_distance_step(const DistanceArgs &a, int entries, int2 *range, int4 *
 // has the loads of two edges in flight and evaluates them, and the four add
 // them up in order (128 x 128 flag, a frame: 188 us with the four launches,
 // 165 with one thread per particle, 136 with four lanes).
-constexpr int kStepLanes = 4;
+constexpr int kStepLanes = 4, kStepAhead = 2;  // edges of a lane in flight
 __global__ void __launch_bounds__(128) k_distance_step(SimConsts C, DistanceStep a, const float4 *__restrict__ P,
                                                        float4 *__restrict__ Pout)
 {
@@ -798,25 +798,25 @@ __global__ void __launch_bounds__(128) k_distance_step(SimConsts C, DistanceStep
     const bool pinned = a.pinned && a.pinned[id];
     const float3 pi = f3(p4);
     float3 d = make_float3(0.f, 0.f, 0.f);
-    const int rounds = __reduce_max_sync(0xffffffffu, (e - b + 2 * kStepLanes - 1) / (2 * kStepLanes));
+    const int rounds = __reduce_max_sync(0xffffffffu, (e - b + kStepAhead * kStepLanes - 1) / (kStepAhead * kStepLanes));
     for (int r = 0; r < rounds; ++r) {
-        int4 c[2];
-        float4 po[2];
-        float wo[2];
-        float3 term[2];
+        int4 c[kStepAhead];
+        float4 po[kStepAhead];
+        float wo[kStepAhead];
+        float3 term[kStepAhead];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int q = b + (2 * r + k) * kStepLanes + lane;
+        for (int k = 0; k < kStepAhead; ++k) {
+            const int q = b + (kStepAhead * r + k) * kStepLanes + lane;
             c[k] = q < e ? __ldg(a.inc + q) : make_int4(2 * id, 0, 0, 0);  // an edge to itself: no correction
         }
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < kStepAhead; ++k) {
             const int j = __ldg(a.to_new + (c[k].x >> 1));
             po[k] = P[j];
             wo[k] = __ldg(a.w + j);
         }
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < kStepAhead; ++k) {
             const bool second = (c[k].x & 1) != 0;
             const float3 x12 = second ? f3(po[k]) - pi : pi - f3(po[k]);
             const float d12 = len3(x12);
@@ -829,13 +829,13 @@ __global__ void __launch_bounds__(128) k_distance_step(SimConsts C, DistanceStep
             term[k] = second ? wi * g : -wi * g;
         }
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
+        for (int k = 0; k < kStepAhead; ++k)
 #pragma unroll
             for (int l = 0; l < kStepLanes; ++l) {
                 const float3 u = make_float3(__shfl_sync(0xffffffffu, term[k].x, l, kStepLanes),
                                              __shfl_sync(0xffffffffu, term[k].y, l, kStepLanes),
                                              __shfl_sync(0xffffffffu, term[k].z, l, kStepLanes));
-                if (b + (2 * r + k) * kStepLanes + l < e) d += u;
+                if (b + (kStepAhead * r + k) * kStepLanes + l < e) d += u;
             }
     }
     if (lane != 0 || t / kStepLanes >= C.n) return;

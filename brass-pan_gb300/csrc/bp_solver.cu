@@ -352,6 +352,21 @@ struct BatchSpec {
     int max_planes = 0;
 };
 
+// The Verlet lists' buffers (1 KB a particle), for parameters that ask for
+// them; single scenes only.
+static bp_status verlet_buffers(bp_solver *s, const bp_params &p)
+{
+    if (!(p.neighbor_skin > 0.f) || s->vl) return BP_OK;
+    const size_t N = (size_t)std::max(s->n, 1), D = (size_t)p.grid_dim;
+    bp_status st;
+    int *lists = nullptr;
+    if ((st = s->alloc(&s->vl_count, N)) || (st = s->alloc(&s->nl_cell, N)) ||
+        (st = s->alloc(&s->nl_outlier, D * D * ((D + 63) / 64))) || (st = s->alloc(&lists, N * kVerletCap)))
+        return st;
+    s->vl = lists;
+    return BP_OK;
+}
+
 static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, void *stream, const BatchSpec *batch,
                                bp_solver **out)
 {
@@ -392,7 +407,6 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
     const size_t ncells = batch ? batch->ncells : (size_t)D * D * D;
     s->ncells = ncells;
     s->sort_dim = batch ? batch->sort_dim : D;
-    const size_t NM = batch ? 1 : N;  // Verlet lists: single scenes only
     s->sl_words = (ncells + 31) / 32;
     if ((st = s->alloc(&s->Xc, N)) || (st = s->alloc(&s->Vc, N)) || (st = s->alloc(&s->Xs, N)) ||
         (st = s->alloc(&s->Vs, N)) || (st = s->alloc(&s->Pa, N)) || (st = s->alloc(&s->Pb, N)) ||
@@ -401,12 +415,10 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         (st = s->alloc(&s->keys, N)) || (st = s->alloc(&s->sorted_keys, N)) || (st = s->alloc(&s->order, N)) ||
         (st = s->alloc(&s->off, ncells + 1)) || (st = s->alloc(&s->mass, N)) || (st = s->alloc(&s->lam, N)) || (st = s->alloc(&s->lm, N)) ||
         (st = s->alloc(&s->rho, N)) || (st = s->alloc(&s->w, N)) || (st = s->alloc(&s->err, 1)) ||
-        (st = s->alloc(&s->staging, 6 * N)) || (st = s->alloc(&s->vl, NM * kVerletCap)) ||
-        (st = s->alloc(&s->nl_cell, NM)) || (st = s->alloc(&s->nl_pos, N)) || (st = s->alloc(&s->sl_cell, N)) ||
+        (st = s->alloc(&s->staging, 6 * N)) || (st = s->alloc(&s->nl_pos, N)) || (st = s->alloc(&s->sl_cell, N)) ||
         (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 2)) ||
         (st = s->alloc(&s->sl_bits, 2 * kSlLevels * s->sl_words)) ||
-        (st = s->alloc(&s->nl_outlier, (size_t)D * D * ((D + 63) / 64))) ||
-        (st = s->alloc(&s->vl_count, NM)) || (st = s->alloc(&s->nl_stats, 5)))
+        (st = s->alloc(&s->nl_stats, 5)) || (!batch && (st = verlet_buffers(s, *prm))))
         return bail(st);
     {
         char *scratch = nullptr;
@@ -765,6 +777,7 @@ extern "C" bp_status bp_solver_set_params(bp_solver *s, const bp_params *prm)
     } else {
         if (prm->grid_dim != s->prm.grid_dim)
             return fail(BP_ERR_INVALID_ARGUMENT, "grid_dim cannot change after creation");
+        if ((st = verlet_buffers(s, *prm)) != BP_OK) return st;
         s->prm = *prm;
     }
     s->params_version++;
