@@ -224,15 +224,9 @@ __device__ __forceinline__ bool classes_on(const SimConsts &C)
     return C.cls_perm && __ldg(C.cls_moved) == 0;
 }
 
-// Quads of candidates a recording walk over the walk planes tests per loop
-// trip (loads in flight: three per quad).
-#ifndef BP_PLANE_QUADS
-#define BP_PLANE_QUADS 1
-#endif
-constexpr int kPlaneQuads = BP_PLANE_QUADS;
-// Floats past n a walk-plane read may reach: the last trip of a chunk reads
-// up to kPlaneQuads quads from an aligned start below the run's end.
-constexpr int kPlanePad = 4 * kPlaneQuads + 4;
+// Floats past n a walk-plane read may reach: the last quad of a run starts at
+// an aligned index below the run's end.
+constexpr int kPlanePad = 8;
 
 // Order of the walk planes: 2 class order (the classes are on), 1 sorted
 // order (no classes, or their gate is closed: k_class_refresh then writes

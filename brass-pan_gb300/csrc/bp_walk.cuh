@@ -637,39 +637,34 @@ __device__ __forceinline__ void walk_neighbors(int i, float3 pi, int lo, const f
 template <class H>
 __device__ __forceinline__ void record_run_planes(int b, int e, const float *__restrict__ X,
                                                   const float *__restrict__ Y, const float *__restrict__ Z,
-                                                  float2 nx, float2 ny, float2 nz, float r2, H &chunk)
+                                                  float2 nx, float2 ny, float2 nz, float above, H &chunk)
 {
     if (b >= e) return;
+    const float2 nr = make_float2(-above, -above);
 #pragma unroll 1
     for (int c0 = b & ~3; c0 < e; c0 += 32) {
         const int cnt = min(32, e - c0);
-        unsigned bits = 0u;
+        unsigned bits = 0u;  // the candidates' sign bits, the last one's lowest
+        int t = 0;
 #pragma unroll 1
-        for (int t = 0; t < cnt; t += 4 * kPlaneQuads) {
-            float4 x[kPlaneQuads], y[kPlaneQuads], z[kPlaneQuads];
-#pragma unroll
-            for (int u = 0; u < kPlaneQuads; ++u) {
-                x[u] = __ldg(reinterpret_cast<const float4 *>(X + c0 + t + 4 * u));
-                y[u] = __ldg(reinterpret_cast<const float4 *>(Y + c0 + t + 4 * u));
-                z[u] = __ldg(reinterpret_cast<const float4 *>(Z + c0 + t + 4 * u));
-            }
-            unsigned nib = 0u;
-#pragma unroll
-            for (int u = 0; u < kPlaneQuads; ++u) {
-                const float2 xa = __fadd2_rn(make_float2(x[u].x, x[u].y), nx);
-                const float2 xb = __fadd2_rn(make_float2(x[u].z, x[u].w), nx);
-                const float2 ya = __fadd2_rn(make_float2(y[u].x, y[u].y), ny);
-                const float2 yb = __fadd2_rn(make_float2(y[u].z, y[u].w), ny);
-                const float2 za = __fadd2_rn(make_float2(z[u].x, z[u].y), nz);
-                const float2 zb = __fadd2_rn(make_float2(z[u].z, z[u].w), nz);
-                const float2 da = __ffma2_rn(za, za, __ffma2_rn(ya, ya, __fmul2_rn(xa, xa)));
-                const float2 db = __ffma2_rn(zb, zb, __ffma2_rn(yb, yb, __fmul2_rn(xb, xb)));
-                nib |= ((da.x <= r2 ? 1u : 0u) | (da.y <= r2 ? 2u : 0u) | (db.x <= r2 ? 4u : 0u) |
-                        (db.y <= r2 ? 8u : 0u))
-                       << (4 * u);
-            }
-            bits |= nib << t;
+        for (; t < cnt; t += 4) {
+            const float4 x = __ldg(reinterpret_cast<const float4 *>(X + c0 + t));
+            const float4 y = __ldg(reinterpret_cast<const float4 *>(Y + c0 + t));
+            const float4 z = __ldg(reinterpret_cast<const float4 *>(Z + c0 + t));
+            const float2 xa = __fadd2_rn(make_float2(x.x, x.y), nx);
+            const float2 xb = __fadd2_rn(make_float2(x.z, x.w), nx);
+            const float2 ya = __fadd2_rn(make_float2(y.x, y.y), ny);
+            const float2 yb = __fadd2_rn(make_float2(y.z, y.w), ny);
+            const float2 za = __fadd2_rn(make_float2(z.x, z.y), nz);
+            const float2 zb = __fadd2_rn(make_float2(z.z, z.w), nz);
+            const float2 da = __fadd2_rn(__ffma2_rn(za, za, __ffma2_rn(ya, ya, __fmul2_rn(xa, xa))), nr);
+            const float2 db = __fadd2_rn(__ffma2_rn(zb, zb, __ffma2_rn(yb, yb, __fmul2_rn(xb, xb))), nr);
+            bits = __funnelshift_l(__float_as_uint(da.x), bits, 1);
+            bits = __funnelshift_l(__float_as_uint(da.y), bits, 1);
+            bits = __funnelshift_l(__float_as_uint(db.x), bits, 1);
+            bits = __funnelshift_l(__float_as_uint(db.y), bits, 1);
         }
+        bits = __brev(bits) >> (32 - t);  // bit k: candidate c0 + k
         bits &= ~0u << max(b - c0, 0);        // below the run (first chunk only)
         if (cnt < 32) bits &= (1u << cnt) - 1u;  // past its end
         if (bits) chunk(c0, bits);
@@ -691,6 +686,7 @@ __device__ __forceinline__ void record_walk_planes(int order, float3 pi, float r
     const float *__restrict__ Y = X + st;
     const float *__restrict__ Z = Y + st;
     const float2 nx = make_float2(-pi.x, -pi.x), ny = make_float2(-pi.y, -pi.y), nz = make_float2(-pi.z, -pi.z);
+    const float above = __uint_as_float(__float_as_uint(r2) + 1u);  // the float above r2: d2 <= r2 is d2 < above
     if (C.nl_stats) {
         atomicAdd(C.nl_stats + 1, 1u);
         if (order == 2) atomicAdd(C.nl_stats + 4, 1u);
@@ -717,7 +713,7 @@ __device__ __forceinline__ void record_walk_planes(int order, float3 pi, float r
                 const unsigned zb = wrap ? (piece == 0 ? D - 1 : z2) : z2;
                 const int k = kxy | ((piece == 1 ? kz2 : kz0) << 2);
                 const int *o = off + (size_t)k * keys + base;
-                record_run_planes(__ldg(o + za), __ldg(o + zb + 1), X, Y, Z, nx, ny, nz, r2, chunk);
+                record_run_planes(__ldg(o + za), __ldg(o + zb + 1), X, Y, Z, nx, ny, nz, above, chunk);
             }
         }
     } else {
@@ -730,7 +726,7 @@ __device__ __forceinline__ void record_walk_planes(int order, float3 pi, float r
             for (int piece = 0; piece < (wrap ? 2 : 1); ++piece) {
                 const unsigned za = (wrap && piece == 1) ? 0u : z0;
                 const unsigned zb = wrap ? (piece == 0 ? D - 1 : z2) : z2;
-                record_run_planes(__ldg(off + base + za), __ldg(off + base + zb + 1), X, Y, Z, nx, ny, nz, r2, chunk);
+                record_run_planes(__ldg(off + base + za), __ldg(off + base + zb + 1), X, Y, Z, nx, ny, nz, above, chunk);
             }
         }
     }
