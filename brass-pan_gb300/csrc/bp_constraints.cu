@@ -477,9 +477,14 @@ __global__ void __launch_bounds__(256) k_contacts_lists(SimConsts C, const float
     const int i = walker_index(C, t);
     const float4 pi4 = P[i];
     const float3 xip = f3(pi4);
-    const int cnt = __ldg(C.cl_count + t);
-    if (!reads_substep_list(C, t, i, xip, cell_of(xip, C), grid_view(C, scene_index(C, i), off), cnt >= 0)) return;
     const int phi = phase_of(pi4);
+    const int3 c = cell_of(xip, C);
+    const GridView v = grid_view(C, scene_index(C, i), off);
+    // fluid whose 27 cells store no solid has no partner, list or not
+    const int addr = cell_addr(c.x, c.y, c.z, v.D, v.mask);
+    const bool alone = phi < 0 && C.cl_near && !((__ldg(C.cl_near + (addr >> 6)) >> (addr & 63)) & 1ull);
+    const int cnt = alone ? 0 : __ldg(C.cl_count + t);
+    if (!alone && !reads_substep_list(C, t, i, xip, c, v, cnt >= 0)) return;
     Contacts s{make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), 0};
     if (cnt > 0) {
         const float3 xi = f3(Xs[i]);
