@@ -235,7 +235,8 @@ SimConsts bp::make_consts(const bp_solver *s, float sdt)
     if (skin > 0.f) {  // substep lists (enqueue_substep decides per launch)
         C.sl_cell = s->sl_cell;
         C.sl_pos = s->nl_pos;
-        C.sl_bits = s->sl_bits;
+        C.sl_near = s->sl_bits;
+        C.sl_far = s->sl_bits + kSlLevels * s->sl_words;
         C.sl_words = (int)s->sl_words;
         C.sl_queue = s->sl_queue;
         C.sl_count = s->sl_count;
@@ -352,6 +353,9 @@ struct BatchSpec {
     int max_planes = 0;
 };
 
+// Words of SimConsts::sl_near and sl_far.
+static size_t sl_bit_words(const bp_solver *s) { return (kSlLevels + 4) * s->sl_words; }
+
 // The Verlet lists' buffers (1 KB a particle), for parameters that ask for
 // them; single scenes only.
 static bp_status verlet_buffers(bp_solver *s, const bp_params &p)
@@ -417,7 +421,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         (st = s->alloc(&s->rho, N)) || (st = s->alloc(&s->w, N)) || (st = s->alloc(&s->err, 1)) ||
         (st = s->alloc(&s->staging, 6 * N)) || (st = s->alloc(&s->nl_pos, N)) || (st = s->alloc(&s->sl_cell, N)) ||
         (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 2)) ||
-        (st = s->alloc(&s->sl_bits, 2 * kSlLevels * s->sl_words)) ||
+        (st = s->alloc(&s->sl_bits, sl_bit_words(s))) ||
         (st = s->alloc(&s->nl_stats, 5)) || (!batch && (st = verlet_buffers(s, *prm))))
         return bail(st);
     {
@@ -982,7 +986,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         if (listed_contacts && !(fluid && it == 0)) {
             if (it == 0) {
                 refresh_planes(cur);
-                cudaMemsetAsync(s->sl_bits, 0, 2 * kSlLevels * s->sl_words * sizeof(unsigned), st);
+                cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), st);
                 launch_lambda_lists(st, Cf, true, cur, s->mass, s->off, s->lam, s->rho, L);
             }
             if (tape) tape->push(TS_PCOLL, slot);
@@ -1018,7 +1022,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
                 cudaMemsetAsync(s->nl_outlier, 0, (size_t)C.D * C.D * C.nl_zwords * sizeof(unsigned long long), st);
             if (shared) {
                 next_list_pass(Cf, !record && it == iterations - 1 && !post_ab);
-                if (record) cudaMemsetAsync(s->sl_bits, 0, 2 * kSlLevels * s->sl_words * sizeof(unsigned), st);
+                if (record) cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), st);
                 launch_lambda_lists(st, Cf, record, cur, s->mass, s->off, s->lam, s->rho, L);
             } else {
                 launch_lambda(st, it == 0 ? Cbuild : Cf, cur, s->mass, s->off, s->lam, s->rho, L);

@@ -145,8 +145,8 @@ struct bp_solver {
     float *walk_xyz = nullptr;  // walk planes (SimConsts::walk_xyz): 4 planes of walk_stride floats
     int walk_stride = 0;
     // substep lists (SimConsts::sl_pos): the cell each was recorded in, the
-    // queue of the particles that may not read theirs, the counts, the cell
-    // bits (sl_words each: moved, then near) and the skin
+    // queue of the particles that may not read theirs, the counts, the cells'
+    // displacement bits (SimConsts::sl_near, then sl_far) and the skin
     int *sl_cell = nullptr, *sl_queue = nullptr, *sl_count = nullptr;
     unsigned *sl_bits = nullptr;
     float *sl_skin = nullptr;
