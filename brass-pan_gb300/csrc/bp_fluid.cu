@@ -151,7 +151,7 @@ __device__ __forceinline__ void k_lambda_tile(
             // mass gathers overlap there); an overflowed list walks again.
             // Where no column run wraps around the table the walk visits j in
             // ascending order, so the j >= i are the entries from i itself on.
-            int self = 0;
+            int self = kNoOwnEntry;
             const int cnt = record(self);
             if (solid) return;
             const int3 c = cell_of(pi, C);
@@ -159,7 +159,7 @@ __device__ __forceinline__ void k_lambda_tile(
                 const unsigned u = (unsigned)a & v.mask;
                 return u != 0u && u != v.mask;
             };
-            const bool ascending = inner(c.x) && inner(c.y) && inner(c.z);
+            const bool ascending = self != kNoOwnEntry && inner(c.x) && inner(c.y) && inner(c.z);
             const int first = ascending ? (self & ~3) : 0;
             if (cnt >= 0 && slots) {
                 int e = first;  // entry index: ascending, the j >= i are the entries from self on
@@ -208,7 +208,7 @@ __device__ __forceinline__ void k_lambda_tile(
         };
         auto test = [&](int, float4 pj) { return len2(pi - f3(pj)) <= r2; };
         if (C.nbr && !build) {  // record first, then sum over the list (as above)
-            int self = 0;
+            int self = kNoOwnEntry;
             const int cnt = record(self);
             if (cnt >= 0) {
                 for_each_in_list<false>(C.nbr, C.n, t, cnt, slots ? C.cls_pos : P, term);
@@ -382,7 +382,7 @@ __device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const fl
                 const unsigned u = (unsigned)a & v.mask;
                 return u != 0u && u != v.mask;
             };
-            const bool ascending = inner(c.x) && inner(c.y) && inner(c.z);
+            const bool ascending = self != kNoOwnEntry && inner(c.x) && inner(c.y) && inner(c.z);
             int e = ascending ? (self & ~3) : 0;
             const int first = e;
             for_each_padded<kReadOnly>(C.nbr, C.n, t, cnt, src, fetch, [&](int j, float4 pj, float mj) {
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kQueueThreads) k_lambda_queued(SimConsts C, co
         const float inv_rho0 = inv_rest_density(C, sc);
         if (C.nl_stats && slots && lane == 0) atomicAdd(C.nl_stats + 4, 1u);
         float acc = 0.f;  // lane 0: the density; textbook, lanes 1..4: sum of g^2, -sum of g
-        int self = 0;
+        int self = kNoOwnEntry;
         const int me = slots ? t : i;
         auto test = [&](int, float4 pj) { return len2(pi - f3(pj)) <= C.h2; };
         auto batch = [&](int k0, int n, int q, float4 pj) {
@@ -1178,7 +1178,7 @@ __global__ void __launch_bounds__(kQueueThreads) k_lambda_record(SimConsts C, co
     const int me = slots ? t : i;
     const bool sums = C.sl_fluid && !solid;
     float acc = 0.f;  // lane 0: the density; textbook, lanes 1..4: sum of g^2, -sum of g
-    int self = 0, touching = 0;
+    int self = kNoOwnEntry, touching = 0;
     auto batch = [&](int k0, int n, int q, float4 pj) {
         const bool in = lane < n;
         if (in) put_entry(C, t, k0 + lane, q);
@@ -1358,7 +1358,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_lambda_group(SimConsts C, con
             const unsigned u = (unsigned)a & v.mask;
             return u != 0u && u != v.mask;
         };
-        const bool ascending = inner(c.x) && inner(c.y) && inner(c.z);  // as lambda_substep_list
+        // as lambda_substep_list
+        const bool ascending = self != kNoOwnEntry && inner(c.x) && inner(c.y) && inner(c.z);
         float acc[1] = {0.f};
         group_sum<1>(C, me, ascending ? self >> 2 : 0, cnt, src, fetch,
                      [&](int j, int e, float4 pj, float mj, GroupTerm<1> &out) {

@@ -70,12 +70,13 @@ __device__ __forceinline__ void adapt_skin(const SimConsts &C)
 
 // Records the candidates within sqrt(r2) of slot t's particle (sorted index
 // i) into its list, in walk order and its own entry included; returns what
-// nbr_count holds (entries | own entry's index << 16, or -1: overflow).
+// nbr_count holds (entries | own entry's index or kNoOwnEntry << 16, or -1:
+// overflow).
 __device__ __forceinline__ int record_substep_list(const SimConsts &C, const float4 *__restrict__ P, bool slots, int t,
                                                    int i, float3 pi, int3 c, float r2, const GridView &v)
 {
     ListWriter list(C.nbr, C.nbr_cap, C.n, t);
-    int self = 0;
+    int self = kNoOwnEntry;
     const int me = slots ? t : i;
     // the walk planes hold the order this walk reads, except where a particle
     // left the classes' reach after they were written

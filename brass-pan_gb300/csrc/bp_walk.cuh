@@ -358,6 +358,11 @@ struct ListWriter {
     }
 };
 
+// Where a recorded list's own entry is: kNoOwnEntry in lists without one, of a
+// particle whose walk does not cover the cell it is stored in (a plane can
+// move it further than a cell).
+constexpr int kNoOwnEntry = 0x7fff;
+
 // The cnt entries of particle i's list, in order: f(j, P[j]).  Each record's
 // four indices come in one 16-byte load and their positions are loaded
 // before the first of the four calls, so the gathers overlap.  ReadOnly:

@@ -108,3 +108,22 @@ def test_readers_and_recorders_by_size(bp, gpu, side, mode):
         g.close()
     for a, b in zip(*outs):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("mode", ["reference", "textbook"])
+@pytest.mark.parametrize("grid_dim", [16, 64])
+@pytest.mark.parametrize("n", [(20, 12, 16), (40, 36, 20), (40, 36, 34)])
+def test_lists_of_particles_far_from_their_stored_cells(bp, gpu, n, grid_dim, mode):
+    """A block partly outside its box: the planes move particles cells away from
+    the ones they are stored in, so that their walks do not meet themselves."""
+    abi = bp.abi
+    m = abi.BP_MODE_TEXTBOOK if mode == "textbook" else abi.BP_MODE_REFERENCE
+    scene = fluid_scene(bp, n, seed=8, grid_dim=grid_dim, box=(0.05 * n[0], 3.0, 0.06 * n[2]))
+    outs = []
+    for walk in (abi.BP_WALK_NO_STAGING, abi.BP_WALK_NO_STAGING | abi.BP_WALK_NO_LISTS):
+        g = bp.ParticleSolver(scene, bp.make_params(scene, mode=m, walk_options=walk))
+        g.update(1, DT, 3)
+        outs.append((g.positions(), g.velocities(), g.field(abi.BP_FIELD_DENSITIES)))
+        g.close()
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
