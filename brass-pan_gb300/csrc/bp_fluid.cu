@@ -912,7 +912,8 @@ __global__ void __launch_bounds__(kScanThreads, BP_POSTBC_MIN_BLOCKS) k_post_b(
 
 // Pass C: XSPH viscosity (fluidXSph): same phase, j != i, r^2 <= h^2 (r = 0
 // included).  Textbook mode weights each neighbour by its volume m_j / rho_j.
-template <bool Split, bool Stage>
+// First: no pass A or B before it, over the substep lists (k_post_c_lists).
+template <bool Split, bool Stage, bool First = false>
 __device__ __forceinline__ void k_post_c_tile(
     const SimConsts &C,
     const float4 *__restrict__ P,
@@ -926,7 +927,8 @@ __device__ __forceinline__ void k_post_c_tile(
     StageShared &S = stage_shared();
     const int t = i0 + threadIdx.x;
     const int i = (Stage || t >= C.n) ? t : walker_index(C, t);
-    const int cnt = post_list_count(C, P, i, t);
+    const float4 *__restrict__ vslots = First ? C.cls_vel : C.cls_vb;  // the velocities in class order
+    int cnt = First ? 0 : post_list_count(C, P, i, t);
     const int g = (Stage && __syncthreads_or(cnt == kWalkCells)) ? stage_block(C, P, off, i0, S) : -1;
     if (i >= C.n) return;
     const float4 pi4 = P[i];
@@ -937,6 +939,11 @@ __device__ __forceinline__ void k_post_c_tile(
         return;
     }
     const float3 pi = f3(pi4), vi = f3(vi4);
+    const GridView gv = grid_view(C, scene_index(C, i), off);
+    if constexpr (First) {
+        if (!reads_substep_list(C, t, i, pi, cell_of(pi, C), gv)) return;
+        cnt = __ldg(C.nbr_count + t) & 0xffff;
+    }
     float3 vn = make_float3(0.f, 0.f, 0.f);
     auto body_at = [&](const float4 *__restrict__ Vp, const float *__restrict__ mp, const float *__restrict__ rp,
                        int j, float4 pj4) {
@@ -946,7 +953,6 @@ __device__ __forceinline__ void k_post_c_tile(
     };
     auto body = [&](int j, float4 pj4) { body_at(V, mass, rho, j, pj4); };
     auto test = [&](int j, float4 pj4) { return j != i && phase_of(pj4) == phi && len2(pi - f3(pj4)) <= C.h2; };
-    const GridView gv = grid_view(C, scene_index(C, i), off);
     int own = -1;
     // reference mode: each entry's velocity loads with its position, before
     // the four pair terms of a record
@@ -957,14 +963,14 @@ __device__ __forceinline__ void k_post_c_tile(
         const float d2 = len2(pi - f3(pj4));
         if (keep(j, pj4, d2)) vn = fma3(poly6(C, d2), f3(vj4) - vi, vn);
     };
-    if (cnt != kWalkCells && post_slots(C, Stage) && !C.textbook) {  // V: pass B's output, in class order
-        for_each_padded(C.nbr, C.n, t, cnt, C.cls_pos, [&](int q) { return C.cls_vb[q]; }, listed);
+    if (cnt != kWalkCells && post_slots(C, Stage) && !C.textbook) {  
+        for_each_padded(C.nbr, C.n, t, cnt, C.cls_pos, [&](int q) { return vslots[q]; }, listed);
     } else if (cnt != kWalkCells && !C.textbook) {
         for_each_padded(C.nbr, C.n, t, cnt, P, [&](int j) { return V[j]; }, listed);
     } else if (cnt != kWalkCells && post_slots(C, Stage)) {
         for_each_in_list(C.nbr, C.n, t, cnt, C.cls_pos,
                          [&](int q, float4 pj4) {
-                             if (keep(q, pj4, len2(pi - f3(pj4)))) body_at(C.cls_vb, C.cls_mass, C.cls_rho, q, pj4);
+                             if (keep(q, pj4, len2(pi - f3(pj4)))) body_at(vslots, C.cls_mass, C.cls_rho, q, pj4);
                          });
     } else if (cnt != kWalkCells) {
         for_each_in_list(C.nbr, C.n, t, cnt, P, [&](int j, float4 pj4) {
@@ -1111,7 +1117,7 @@ __global__ void __launch_bounds__(kQueueThreads) k_post_a_queued(SimConsts C, co
                 value[5] = g.z;
                 scale = __frcp_rn(nb.rho);
             }
-            warp_add<6, true>(rows[threadIdx.x >> 5], __ballot_sync(kWarp, apart), value, scale, acc);
+            warp_add<6, 3>(rows[threadIdx.x >> 5], __ballot_sync(kWarp, apart), value, scale, acc);
         };
         const int cnt = warp_neighbors(C, slots, cell_of(pi, C), P, grid_view(C, scene_index(C, i), off),
                                        hits[threadIdx.x >> 5], test, batch);
@@ -1124,6 +1130,66 @@ __global__ void __launch_bounds__(kQueueThreads) k_post_a_queued(SimConsts C, co
         const float3 zero = make_float3(0.f, 0.f, 0.f);
         finish_post_a(C, slots, i, t, C.use_vort ? make_float3(sum[0], sum[1], sum[2]) : zero,
                       C.use_akinci ? make_float3(sum[3], sum[4], sum[5]) : zero, rho, Om, Nm);
+    }
+}
+
+// Pass C alone after the commit, over the substep lists: without pass A to ask
+// which lists still hold, it asks itself, and its own queue follows.
+// 65,536 particles, a launch: 46 us recording and summing its own walk, 15 us
+// over the lists and 10 us for the queue.
+__global__ void __launch_bounds__(kScanThreads, BP_POSTBC_MIN_BLOCKS) k_post_c_lists(
+    SimConsts C, const float4 *__restrict__ P, const float4 *__restrict__ V, const int *__restrict__ off,
+    const float *__restrict__ mass, const float *__restrict__ rho, float4 *__restrict__ Vout)
+{
+    k_post_c_tile<true, false, true>(C, P, V, off, mass, rho, Vout, blockIdx.x * blockDim.x);
+}
+
+__global__ void __launch_bounds__(kQueueThreads) k_post_c_queued(SimConsts C, const float4 *__restrict__ P,
+                                                                const float4 *__restrict__ V,
+                                                                const int *__restrict__ off,
+                                                                const float *__restrict__ mass,
+                                                                const float *__restrict__ rho,
+                                                                float4 *__restrict__ Vout)
+{
+    __shared__ WarpRows rows[kQueueThreads / 32];
+    __shared__ WarpHits hits[kQueueThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int queued = C.sl_count[C.sl_pass];
+    adapt_skin(C);
+    const bool slots = post_slots(C, false);
+    const float4 *__restrict__ vs = slots ? C.cls_vel : V;
+    const float *__restrict__ ms = slots ? C.cls_mass : mass;
+    const float *__restrict__ rs = slots ? C.cls_rho : rho;
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) / 32; k < queued; k += gridDim.x * blockDim.x / 32) {
+        const int t = C.sl_queue[k];
+        const int i = slots ? __ldg(C.cls_perm + t) : t;
+        const float4 pi4 = slots ? C.cls_pos[t] : P[i];
+        const int phi = phase_of(pi4);
+        const float4 vi4 = V[i];
+        const float3 pi = f3(pi4), vi = f3(vi4);
+        if (C.nl_stats && slots && lane == 0) atomicAdd(C.nl_stats + 4, 1u);
+        float acc = 0.f;  // lanes 0..2: the weighted velocity differences
+        auto test = [&](int q, float4 pj) { return q != t && phase_of(pj) == phi && len2(pi - f3(pj)) <= C.h2; };
+        auto batch = [&](int, int n, int q, float4 pj) {
+            const bool in = lane < n;
+            float value[3] = {0.f, 0.f, 0.f};
+            float wgt = 0.f;
+            if (in) {
+                wgt = poly6(C, len2(pi - f3(pj)));
+                if (C.textbook) wgt = __fmul_rn(wgt, __fdiv_rn(__ldg(ms + q), __ldg(rs + q)));
+                const float3 dv = f3(vs[q]) - vi;
+                value[0] = dv.x;
+                value[1] = dv.y;
+                value[2] = dv.z;
+            }
+            warp_add<3, 0>(rows[threadIdx.x >> 5], __ballot_sync(kWarp, in), value, wgt, acc);
+        };
+        warp_neighbors(C, slots, cell_of(pi, C), P, grid_view(C, scene_index(C, i), off), hits[threadIdx.x >> 5], test,
+                       batch);
+        const float3 vn = make_float3(__shfl_sync(kWarp, acc, 0), __shfl_sync(kWarp, acc, 1), __shfl_sync(kWarp, acc, 2));
+        if (lane != 0) continue;
+        const float3 v = vi + C.xsph_c * vn;
+        Vout[i] = make_float4(v.x, v.y, v.z, vi4.w);
     }
 }
 
@@ -1555,6 +1621,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_post_b_group(SimConsts C, con
                   make_float3(acc[3], acc[4], acc[5]), Om, Vout);
 }
 
+template <bool First>  // as k_post_c_tile
 __global__ void __launch_bounds__(kGroupThreads) k_post_c_group(SimConsts C, const float4 *__restrict__ P,
                                                                 const float4 *__restrict__ V,
                                                                 const int *__restrict__ off,
@@ -1567,7 +1634,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_post_c_group(SimConsts C, con
     const float3 pi = f3(me.p4);
     const float4 vi4 = V[me.i];
     const float3 vi = f3(vi4);
-    const int listed = phi < 0 ? __ldg(C.nbr_count + me.t) : 0;
+    const GridView gv = grid_view(C, scene_index(C, me.i), off);
+    const bool reads = First ? group_reads(C, me, phi < 0, cell_of(pi, C), gv) : phi < 0;
+    const int listed = reads ? __ldg(C.nbr_count + me.t) : 0;
     const int own = me.slots ? me.t : me.i;
     struct Nb {
         float3 v;
@@ -1591,7 +1660,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_post_c_group(SimConsts C, con
         out.v[2] = dv.z;
         return phase_of(pj) == phi && d2 <= C.h2;
     };
-    const float4 *__restrict__ vs = me.slots ? C.cls_vb : V;
+    const float4 *__restrict__ vs = me.slots ? (First ? C.cls_vel : C.cls_vb) : V;
     const float *__restrict__ ms = me.slots ? C.cls_mass : mass;
     const float *__restrict__ rs = me.slots ? C.cls_rho : rho;
     float acc[3] = {0.f, 0.f, 0.f};
@@ -1603,9 +1672,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_post_c_group(SimConsts C, con
         Vout[me.i] = vi4;
         return;
     }
+    if (First && !reads) return;  // queued
     if (listed < 0)  // overflowed
         walk_neighbors<true>(
-            me.i, pi, 0, P, grid_view(C, scene_index(C, me.i), off), C, nullptr, -1,
+            me.i, pi, 0, P, gv, C, nullptr, -1,
             [&](int j, float4 pj) { return j != me.i && phase_of(pj) == phi && len2(pi - f3(pj)) <= C.h2; },
             [&](int j, float4 pj) {
                 GroupTerm<3> out;
@@ -1685,11 +1755,21 @@ void launch_post_b(cudaStream_t st, const SimConsts &C, const float4 *P, const f
     else BP_LAUNCH_SPLIT(k_post_b, st, C, P, V, Om, Nm, off, Vout);
     L->done(__func__);
 }
+void launch_post_c_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const int *off,
+                         const float *mass, const float *rho, float4 *Vout, LaunchLog *L)
+{
+    if (C.n <= 0) return;
+    if (use_groups(C)) k_post_c_group<true><<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, V, off, mass, rho, Vout);
+    else k_post_c_lists<<<(C.n + C.scan_block - 1) / C.scan_block, C.scan_block, 0, st>>>(C, P, V, off, mass, rho, Vout);
+    L->done("launch_post_c_lists");
+    k_post_c_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, V, off, mass, rho, Vout);
+    L->done("launch_post_c_queued");
+}
 void launch_post_c(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const int *off,
                    const float *mass, const float *rho, float4 *Vout, LaunchLog *L)
 {
     if (C.n <= 0) return;
-    if (use_groups(C) && C.nbr_count) k_post_c_group<<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, V, off, mass, rho, Vout);
+    if (use_groups(C) && C.nbr_count) k_post_c_group<false><<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, V, off, mass, rho, Vout);
     else BP_LAUNCH_SPLIT(k_post_c, st, C, P, V, off, mass, rho, Vout);
     L->done(__func__);
 }

@@ -167,10 +167,11 @@ __device__ __forceinline__ void warp_walk(const SimConsts &C, bool slots, int3 c
 constexpr int kWarpTerms = 7;  // odd: a warp's rows fall into different banks
 using WarpRows = float[32][kWarpTerms];
 // The lanes of `take` add value[0..N) to acc of lanes 0..N, in lane order;
-// lanes 3..5 add scale * value with one rounding where Scaled.
-template <int N, bool Scaled = false>
+// lanes From and up add scale * value with one rounding.
+template <int N, int From = N>
 __device__ __forceinline__ void warp_add(WarpRows &rows, unsigned take, const float (&value)[N], float scale, float &acc)
 {
+    constexpr bool Scaled = From < N;
     static_assert(N + (Scaled ? 1 : 0) <= kWarpTerms, "a row holds kWarpTerms quantities");
     const int lane = threadIdx.x & 31;
     if ((take >> lane) & 1u) {
@@ -184,7 +185,7 @@ __device__ __forceinline__ void warp_add(WarpRows &rows, unsigned take, const fl
         const int n = __popc(take);
 #pragma unroll 4
         for (int r = 0; r < n; ++r)
-            acc = (Scaled && lane >= 3) ? __fmaf_rn(rows[r][N], rows[r][lane], acc) : __fadd_rn(acc, rows[r][lane]);
+            acc = (Scaled && lane >= From) ? __fmaf_rn(rows[r][N], rows[r][lane], acc) : __fadd_rn(acc, rows[r][lane]);
     }
     __syncwarp();
 }

@@ -838,7 +838,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // fluid: 14 % of the particles displaced past the skin when recorded ahead
     // of it, 1 % behind it).  Contacts alone search ahead of their first pass.
     const bool shared = C.sl_pos != nullptr && s->nbr && iterations > 0 &&
-                        ((fluid && (iterations > 1 || post_ab)) || (pcoll && iterations > 1));
+                        ((fluid && (iterations > 1 || post_ab || C.use_xsph)) || (pcoll && iterations > 1));
     const bool listed_contacts = shared && pcoll && iterations > 1;
     const bool walked_contacts = pcoll && (!shared || fluid);  // in the first iteration at least
     ra.tile_solid = walked_contacts ? s->tile_solid : nullptr;
@@ -1021,7 +1021,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             if (verlet && it == 0)
                 cudaMemsetAsync(s->nl_outlier, 0, (size_t)C.D * C.D * C.nl_zwords * sizeof(unsigned long long), st);
             if (shared) {
-                next_list_pass(Cf, !record && it == iterations - 1 && !post_ab);
+                next_list_pass(Cf, !record && it == iterations - 1 && !post_ab && !C.use_xsph);
                 if (record) cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), st);
                 launch_lambda_lists(st, Cf, record, cur, s->mass, s->off, s->lam, s->rho, L);
             } else {
@@ -1123,8 +1123,8 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // The post passes keep class positions in their lists where lambda left
     // its densities in class order (SimConsts::cls_post); the velocities are
     // gathered into class order with the positions.
-    const bool post_slots = classes && lists && post_ab && fluid && iterations > 0 && !verlet;
     const bool post_lists = shared && fluid;
+    const bool post_slots = classes && lists && (post_ab || post_lists) && fluid && iterations > 0 && !verlet;
     const bool post_planes = walk_planes && post_ab && !post_lists;
     if ((post_ab || C.use_xsph) && classes)  // the post passes read the same positions
         launch_class_refresh(st, s->n, cur, ca, L, post_slots ? s->Vc : nullptr, post_planes ? s->walk_xyz : nullptr,
@@ -1160,13 +1160,19 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         }
         if (C.use_xsph) launch_post_c(st, Cl, cur, s->Vs, s->off, s->mass, s->rho, s->Vc, L);
     } else if (C.use_xsph) {
-        SimConsts Cx = Cpost;  // records its own pairs, then sums over them
+        SimConsts Cx = Cpost;
         if (lists) {
             Cx.nbr = s->nbr;
-            Cx.nbr_count = nullptr;
+            Cx.nbr_count = post_lists ? s->nbr_count : nullptr;
             Cx.nbr_cap = kPostListCap;
         }
-        launch_post_c(st, Cx, cur, s->Vc, s->off, s->mass, s->rho, s->Vs, L);
+        if (post_lists) {
+            Cx.cls_post = post_slots ? 1 : 0;
+            next_list_pass(Cx, true);
+            launch_post_c_lists(st, Cx, cur, s->Vc, s->off, s->mass, s->rho, s->Vs, L);
+        } else {  // records its own pairs, then sums over them
+            launch_post_c(st, Cx, cur, s->Vc, s->off, s->mass, s->rho, s->Vs, L);
+        }
         cudaMemcpyAsync(s->Vc, s->Vs, (size_t)s->n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
     }
 }

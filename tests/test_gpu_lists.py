@@ -127,3 +127,31 @@ def test_lists_of_particles_far_from_their_stored_cells(bp, gpu, n, grid_dim, mo
         g.close()
     for a, b in zip(*outs):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("mode", ["reference", "textbook"])
+@pytest.mark.parametrize("skin,iterations", [(0.0, 3), (0.0, 1), (0.004, 2)])
+@pytest.mark.parametrize("name", ["one_particle", "packed", "mixed_aliased", "large", "large_aliased"])
+def test_viscosity_alone_over_the_lists_is_bit_identical_to_walks(bp, gpu, name, skin, iterations, mode):
+    """Pass C without the passes before it: four lanes a particle and a thread
+    each, with alias classes and without, listed and queued."""
+    abi = bp.abi
+    m = abi.BP_MODE_TEXTBOOK if mode == "textbook" else abi.BP_MODE_REFERENCE
+    if name.startswith("large"):
+        scene = fluid_scene(bp, (40, 36, 34), seed=8, grid_dim=16 if name.endswith("aliased") else 64)
+    else:
+        scene = SCENES[name](bp)
+    stages = (abi.BP_STAGE_FLUID | abi.BP_STAGE_PLANES | abi.BP_STAGE_XSPH | abi.BP_STAGE_PARTICLE_COLLISION)
+    outs = []
+    for walk, sk in ((abi.BP_WALK_NO_STAGING, skin), (abi.BP_WALK_NO_STAGING | abi.BP_WALK_NO_LISTS, 0.0)):
+        g = bp.ParticleSolver(scene, bp.make_params(scene, mode=m, walk_options=walk, neighbor_skin=sk,
+                                                    stage_mask=stages, xsph_c=0.1))
+        if not walk & abi.BP_WALK_NO_LISTS and sk == 0.0:
+            assert g.walk_stats(2, DT, iterations)["listed"] > 0
+        else:
+            g.update(2, DT, iterations)
+        g.update(2, DT, iterations)
+        outs.append((g.positions(), g.velocities(), g.field(abi.BP_FIELD_DENSITIES)))
+        g.close()
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
