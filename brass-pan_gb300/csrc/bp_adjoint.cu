@@ -18,6 +18,7 @@
 
 #include "bp_dual.cuh"
 #include "bp_internal.h"
+#include "bp_lists.cuh"
 #include "bp_walk.cuh"
 
 namespace bp {
@@ -451,6 +452,10 @@ __device__ __forceinline__ float3 poly6_grad(const SimConsts &C, float3 r, float
     const float t = C.h2 - r2;
     return mul3(r, -6.f * C.c_poly6 * t * t);
 }
+__device__ __forceinline__ float3 fma_to(float3 acc, float s, float3 v)
+{
+    return make_float3(__fmaf_rn(s, v.x, acc.x), __fmaf_rn(s, v.y, acc.y), __fmaf_rn(s, v.z, acc.z));
+}
 // J^T g of the per-pair clamp u -> u (|u| < c) or c u / |u|
 __device__ __forceinline__ float3 clamp_vjp(const SimConsts &C, float3 u, float3 g)
 {
@@ -505,9 +510,82 @@ __device__ __forceinline__ void record_then_sum(const SimConsts &C, int k, float
     record_then_sum(C, k, pk, P, v, S, g, record, test, none, term3);
 }
 
+// One pair of walk A: what particle k at pk adds for a neighbour.
+struct DeltapPair {
+    const SimConsts &C;
+    int k, phk;
+    float3 pk, gk;
+    float lk, mk, inv_rho0;
+    // a neighbour's lambda, mass and incoming gradient
+    struct Nb {
+        float lam, mass;
+        float4 g;
+    };
+    __device__ __forceinline__ DeltapPair(const SimConsts &C_, int k_, float4 pk4, int sc,
+                                          const float *__restrict__ mass, const float *__restrict__ lam,
+                                          const float4 *__restrict__ gOut)
+        : C(C_), k(k_), phk(phase_of(pk4)), pk(f3(pk4)), gk(ld3(gOut, k_)), lk(lam[k_]), mk(mass[k_]),
+          inv_rho0(inv_rest_density(C_, sc))
+    {
+    }
+    // reference mode: the pair counts for both ends when its lower index is
+    // fluid; textbook mode: every fluid particle gathers over all neighbours
+    __device__ __forceinline__ bool counts(int j, float4 pj4) const
+    {
+        const float3 r = sub3(pk, f3(pj4));
+        const float d2 = dotf(r, r);
+        const bool fj = phase_of(pj4) < 0;
+        const bool inc = C.textbook ? (phk < 0 || fj) : ((j > k) ? (phk < 0) : fj);
+        return j != k && d2 <= C.h2 && d2 > 0.f && inc;
+    }
+    __device__ __forceinline__ bool within(int j, float4 pj4) const
+    {
+        const float3 r = sub3(pk, f3(pj4));
+        return j != k && dotf(r, r) <= C.h2;
+    }
+    // the addends of the position gradient and (w) of lambda-bar
+    __device__ __forceinline__ float4 term(float4 pj4, const Nb &nb) const
+    {
+        const float3 r = sub3(pk, f3(pj4));
+        const float d2 = dotf(r, r);
+        const float rl = sqrtf(d2);
+        const bool own = !C.textbook || phk < 0;              // dp_k has the pair
+        const bool other = !C.textbook || phase_of(pj4) < 0;  // dp_j has the pair
+        const SpikyD sp = spiky_d(C, r, rl);
+        float s = lk + nb.lam;
+        float3 dsc = make_float3(0.f, 0.f, 0.f);  // d scorr / d r
+        if (C.scorr_on) {
+            const float x = poly6(C, d2) * C.scorr_inv_wq;
+            s -= C.scorr_k * ipowf(x, C.scorr_ni);
+            if (C.scorr_ni > 0)
+                dsc = mul3(poly6_grad(C, r, d2), C.scorr_k * C.scorr_ni * ipowf(x, C.scorr_ni - 1) * C.scorr_inv_wq);
+        }
+        // term of dp_k: (m_j / rho0) clamp(s gradW(r))
+        const float3 u1b = own ? mul3(clamp_vjp(C, mul3(sp.g, s), gk), nb.mass * inv_rho0) : make_float3(0.f, 0.f, 0.f);
+        const float sb1 = dotf(u1b, sp.g);
+        const float3 rb1 = sub3(mul3(spiky_hess_mul(sp, r, rl, u1b), s), mul3(dsc, sb1));
+        // term of dp_j: (m_k / rho0) clamp(s gradW(-r))
+        const float3 g_neg = mul3(sp.g, -1.f);
+        const float3 u2b = other ? mul3(clamp_vjp(C, mul3(g_neg, s), f3(nb.g)), mk * inv_rho0)
+                                 : make_float3(0.f, 0.f, 0.f);
+        const float sb2 = dotf(u2b, g_neg);
+        // gradient w.r.t. r_jk = -r: H(-r) = H(r), dscorr(-r) = -dscorr(r)
+        const float3 rb2 = add3(mul3(spiky_hess_mul(sp, r, rl, u2b), s), mul3(dsc, sb2));
+        return f4(sub3(rb1, rb2), sb1 + sb2);
+    }
+};
+
 // Walk A: lambda-bar and the position gradient of the correction terms.  It
 // records every j != k within h (the pairs of the density terms, a superset
 // of its own), so that pass B sums over the same list instead of walking.
+// Lists: over the lists of the substep's adjoint (k_adj_record_lists); those
+// that may not read theirs are queued for k_adj_deltap_queued, which leaves
+// pass B the list of this iteration.
+// 65,536 particles, a launch: 63 us with its own walk, 35 us over the lists and
+// 9 us for the queue.  The terms' square root and divisions bound it; without
+// the branch on each entry, four terms at a time, it takes 37 us (entries that
+// do not count replaced by an ordinary pair) or 75 us (their divisions by zero).
+template <bool Lists>
 __global__ void __launch_bounds__(kWalkThreads) k_adj_deltap(SimConsts C, const float4 *__restrict__ P,
                                                              const float *__restrict__ mass,
                                                              const float *__restrict__ lam, const int *__restrict__ off,
@@ -515,75 +593,116 @@ __global__ void __launch_bounds__(kWalkThreads) k_adj_deltap(SimConsts C, const 
                                                              float *__restrict__ gLam, float4 *__restrict__ gPart)
 {
     StageShared &S = stage_shared();
-    const int g = stage_block(C, P, off, blockIdx.x * kWalkThreads, S);
+    const int g = Lists ? -1 : stage_block(C, P, off, blockIdx.x * kWalkThreads, S);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (Lists && k == 0) C.sl_count[C.sl_pass ^ 1] = 0;  // the next pass's queue
     if (k >= C.n) return;
     const float4 pk4 = P[k];
-    const int phk = phase_of(pk4);
-    const float3 pk = f3(pk4);
     const int sc = scene_index(C, k);
-    const float inv_rho0 = inv_rest_density(C, sc);
-    const float lk = lam[k], mk = mass[k];
-    const float3 gk = ld3(gOut, k);
+    const GridView v = grid_view(C, sc, off);
+    if (Lists && !reads_substep_list(C, k, k, f3(pk4), cell_of(f3(pk4), C), v)) return;
+    const DeltapPair pair(C, k, pk4, sc, mass, lam, gOut);
     float lb = 0.f;
     float3 pb = make_float3(0.f, 0.f, 0.f);
-    // reference mode: the pair counts for both ends when its lower index is
-    // fluid; textbook mode: every fluid particle gathers over all neighbours
-    auto test = [&](int j, float4 pj4) {
-        const float3 r = sub3(pk, f3(pj4));
-        const float d2 = dotf(r, r);
-        const bool fj = phase_of(pj4) < 0;
-        const bool inc = C.textbook ? (phk < 0 || fj) : ((j > k) ? (phk < 0) : fj);
-        return j != k && d2 <= C.h2 && d2 > 0.f && inc;
+    auto test = [&](int j, float4 pj4) { return pair.counts(j, pj4); };
+    auto fetch = [&](int j) { return DeltapPair::Nb{__ldg(lam + j), __ldg(mass + j), gOut[j]}; };
+    auto term = [&](int, float4 pj4, const DeltapPair::Nb &nb) {
+        const float4 t = pair.term(pj4, nb);
+        lb = __fadd_rn(lb, t.w);
+        pb = add3(pb, f3(t));
     };
-    // a neighbour's lambda, mass and incoming gradient
-    struct Nb {
-        float lam, mass;
-        float4 g;
-    };
-    auto fetch = [&](int j) { return Nb{__ldg(lam + j), __ldg(mass + j), gOut[j]}; };
-    auto term = [&](int j, float4 pj4, const Nb &nb) {
-            const float3 r = sub3(pk, f3(pj4));
-            const float d2 = dotf(r, r);
-            const float rl = sqrtf(d2);
-            const bool own = !C.textbook || phk < 0;               // dp_k has the pair
-            const bool other = !C.textbook || phase_of(pj4) < 0;  // dp_j has the pair
-            const SpikyD sp = spiky_d(C, r, rl);
-            float s = lk + nb.lam;
-            float3 dsc = make_float3(0.f, 0.f, 0.f);  // d scorr / d r
-            if (C.scorr_on) {
-                const float x = poly6(C, d2) * C.scorr_inv_wq;
-                s -= C.scorr_k * ipowf(x, C.scorr_ni);
-                if (C.scorr_ni > 0)
-                    dsc = mul3(poly6_grad(C, r, d2), C.scorr_k * C.scorr_ni * ipowf(x, C.scorr_ni - 1) * C.scorr_inv_wq);
-            }
-            // term of dp_k: (m_j / rho0) clamp(s gradW(r))
-            const float3 u1b = own ? mul3(clamp_vjp(C, mul3(sp.g, s), gk), nb.mass * inv_rho0)
-                                   : make_float3(0.f, 0.f, 0.f);
-            const float sb1 = dotf(u1b, sp.g);
-            const float3 rb1 = sub3(mul3(spiky_hess_mul(sp, r, rl, u1b), s), mul3(dsc, sb1));
-            // term of dp_j: (m_k / rho0) clamp(s gradW(-r))
-            const float3 g_neg = mul3(sp.g, -1.f);
-            const float3 u2b = other ? mul3(clamp_vjp(C, mul3(g_neg, s), f3(nb.g)), mk * inv_rho0)
-                                     : make_float3(0.f, 0.f, 0.f);
-            const float sb2 = dotf(u2b, g_neg);
-            // gradient w.r.t. r_jk = -r: H(-r) = H(r), dscorr(-r) = -dscorr(r)
-            const float3 rb2 = add3(mul3(spiky_hess_mul(sp, r, rl, u2b), s), mul3(dsc, sb2));
-            lb += sb1 + sb2;
-            pb = add3(pb, sub3(rb1, rb2));
-    };
-    auto within = [&](int j, float4 pj4) {
-        const float3 r = sub3(pk, f3(pj4));
-        return j != k && dotf(r, r) <= C.h2;
-    };
-    record_then_sum(C, k, pk, P, grid_view(C, sc, off), &S, g, within, test, fetch, term);
+    if (Lists) {
+        for_each_padded(C.nbr, C.n, k, __ldg(C.nbr_count + k) & 0xffff, P, fetch,
+                        [&](int j, float4 pj4, const DeltapPair::Nb &nb) {
+                            if (test(j, pj4)) term(j, pj4, nb);
+                        });
+    } else {
+        auto within = [&](int j, float4 pj4) { return pair.within(j, pj4); };
+        record_then_sum(C, k, pair.pk, P, v, &S, g, within, test, fetch, term);
+    }
     gLam[k] = lb;
     gPart[k] = f4(pb);
 }
 
+// The queued particles' walk A, a warp per particle (warp_walk), the terms
+// added in walk order.
+constexpr int kAdjQueueThreads = 128;
+__global__ void __launch_bounds__(kAdjQueueThreads) k_adj_deltap_queued(
+    SimConsts C, const float4 *__restrict__ P, const float *__restrict__ mass, const float *__restrict__ lam,
+    const int *__restrict__ off, const float4 *__restrict__ gOut, float *__restrict__ gLam, float4 *__restrict__ gPart)
+{
+    __shared__ WarpRows rows[kAdjQueueThreads / 32];
+    __shared__ WarpHits hits[kAdjQueueThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int queued = C.sl_count[C.sl_pass];
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) / 32; q < queued; q += gridDim.x * blockDim.x / 32) {
+        const int k = C.sl_queue[q];
+        const float4 pk4 = P[k];
+        const int sc = scene_index(C, k);
+        const DeltapPair pair(C, k, pk4, sc, mass, lam, gOut);
+        float acc = 0.f;  // lanes 0..2: the position gradient, 3: lambda-bar
+        auto batch = [&](int k0, int n, int j, float4 pj4) {
+            const bool in = lane < n;
+            if (in) put_entry(C, k, k0 + lane, j);
+            const bool take = in && pair.counts(j, pj4);
+            float value[4] = {0.f, 0.f, 0.f, 0.f};
+            if (take) {
+                const float4 t = pair.term(pj4, DeltapPair::Nb{__ldg(lam + j), __ldg(mass + j), gOut[j]});
+                value[0] = t.x;
+                value[1] = t.y;
+                value[2] = t.z;
+                value[3] = t.w;
+            }
+            warp_add(rows[threadIdx.x >> 5], __ballot_sync(kWarp, take), value, 1.f, acc);
+        };
+        const int cnt = warp_neighbors(C, false, cell_of(pair.pk, C), P, grid_view(C, sc, off),
+                                       hits[threadIdx.x >> 5],
+                                       [&](int j, float4 pj4) { return pair.within(j, pj4); }, batch);
+        const float3 pb = make_float3(__shfl_sync(kWarp, acc, 0), __shfl_sync(kWarp, acc, 1), __shfl_sync(kWarp, acc, 2));
+        const float lb = __shfl_sync(kWarp, acc, 3);
+        if (lane != 0) continue;
+        C.nbr_count[k] = cnt <= C.nbr_cap ? cnt : -1;
+        gLam[k] = lb;
+        gPart[k] = f4(pb);
+    }
+}
+
+// The lists of a substep's adjoint (SimConsts::sl_pos, recorded over the
+// sorted indices): one search for every walk its stages would take.  Recorded
+// at the positions P of the first of those stages, in the order the adjoint
+// undoes them; before each later one k_adj_track flags what its positions
+// differ by.  Iterations move particles by less than the skin, so few are
+// queued.  65,536 particles: 30 us a substep, and 6 us to flag a stage's.
+__global__ void __launch_bounds__(kWalkThreads) k_adj_record_lists(SimConsts C, const float4 *__restrict__ P,
+                                                                   const int *__restrict__ off)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) {
+        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = 0;
+        C.sl_count[kSlMoved] = 0;
+    }
+    if (k >= C.n) return;
+    const float4 pk4 = P[k];
+    const float3 pk = f3(pk4);
+    const GridView v = grid_view(C, scene_index(C, k), off);
+    const int3 c = cell_of(pk, C);
+    const float reach = C.h + substep_skin(C);
+    const int packed = record_substep_list(C, P, false, k, k, pk, c, __fmul_rn(reach, reach), v);
+    C.sl_pos[k] = pk4;
+    C.nbr_count[k] = packed;
+    C.sl_cell[k] = (packed >= 0 && near_stored_cell(C, k, c, v)) ? v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask) : kListNone;
+}
+
+__global__ void k_adj_track(SimConsts C, const float4 *__restrict__ P)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < C.n) track_displacement(C, k, f3(P[k]), true);
+}
+
 // Pass B: the density gradient; gP (in) = gOut + gPart + density terms.  It
-// sums over the list pass A recorded at the same positions (every j != k
-// within h, in walk order) and walks only where that list overflowed.
+// sums over the list pass A recorded at the same positions or read (a superset
+// of every j != k within h, in walk order) and walks only where that list
+// overflowed.
 __global__ void __launch_bounds__(kWalkThreads, 3) k_adj_lambda(SimConsts C, const float4 *__restrict__ P,
                                                              const float *__restrict__ mass,
                                                              const float *__restrict__ rho, const int *__restrict__ off,
@@ -616,22 +735,27 @@ __global__ void __launch_bounds__(kWalkThreads, 3) k_adj_lambda(SimConsts C, con
         float gl, gr, rh, m;
     };
     auto fetch = [&](int j) { return Nb{gLam[j], gRho ? gRho[j] : 0.f, rho[j], mass[j]}; };
+    // rounded explicitly: a listed and a walked particle get the same bits
     auto term = [&](int j, float4 pj4, const Nb &nb) {
         const int phj = phase_of(pj4);
         const float3 r = sub3(pk, f3(pj4));
-        const float3 gw = poly6_grad(C, r, dotf(r, r));
+        const float d2 = __fmaf_rn(r.z, r.z, __fmaf_rn(r.y, r.y, __fmul_rn(r.x, r.x)));
+        float s;
         if (j > k) {
-            pb = add3(pb, mul3(gw, rbk * nb.m * (phj < 0 ? 1.f : C.solid_scale)));
+            s = rbk * nb.m * (phj < 0 ? 1.f : C.solid_scale);
         } else {
             // rho_bar(j, phj) from the loaded values
             float rb = 0.f;
             if (phj <= 0) rb = (C.clamp_c && !(nb.rh / rho0 - 1.0f > 0.f)) ? nb.gr : nb.gr - nb.gl / (C.lambda_den * rho0);
-            pb = add3(pb, mul3(gw, rb * mk));
+            s = rb * mk;
         }
+        pb = fma_to(pb, s, poly6_grad(C, r, d2));
     };
     const int cnt = (C.nbr && C.nbr_count) ? __ldg(C.nbr_count + k) : -1;
-    if (cnt >= 0)  // pass A's list: exactly test's pairs
-        for_each_in_list_with(C.nbr, C.n, k, cnt, P, fetch, term);
+    if (cnt >= 0)  // pass A's list, or the substep's: there its index of the own entry above the count
+        for_each_in_list_with(C.nbr, C.n, k, cnt & 0xffff, P, fetch, [&](int j, float4 pj4, const Nb &nb) {
+            if (test(j, pj4)) term(j, pj4, nb);
+        });
     else
         walk_neighbors<true>(k, pk, 0, P, grid_view(C, sc, off), C, &S, g, test,
                              [&](int j, float4 pj4) { term(j, pj4, fetch(j)); });
@@ -742,6 +866,69 @@ __global__ void __launch_bounds__(kWalkThreads) k_adj_lambda_tb(SimConsts C, con
 // gradient is added to gRho).  Positions are the committed ones; gX receives
 // their gradient.
 
+struct XsphPair {
+    const SimConsts &C;
+    int i, phi;
+    float3 pi, vi, go;
+    float bi;
+    // a neighbour's velocity, incoming gradient, mass and density
+    struct Nb {
+        float4 v, g;
+        float mass, rho;
+    };
+    __device__ __forceinline__ XsphPair(const SimConsts &C_, int i_, float4 pi4, const float4 *__restrict__ V,
+                                        const float *__restrict__ mass, const float *__restrict__ rho,
+                                        const float4 *__restrict__ gVout)
+        : C(C_), i(i_), phi(phase_of(pi4)), pi(f3(pi4)), vi(ld3(V, i_)), go(ld3(gVout, i_)),
+          bi(C_.textbook ? mass[i_] / rho[i_] : 1.f)
+    {
+    }
+    __device__ __forceinline__ bool counts(int j, float4 pj4) const
+    {
+        const float3 r = sub3(pi, f3(pj4));
+        return j != i && phase_of(pj4) == phi && dotf(r, r) <= C.h2;
+    }
+    // The gradients grow by scale times value: gv of the velocity, gp of the
+    // position, rb (textbook) of b_i.
+    struct Term {
+        float3 gv, gp;
+        float gv_scale, gp_scale, rb;
+    };
+    __device__ __forceinline__ Term term(float4 pj4, const Nb &nb) const
+    {
+        const float3 r = sub3(pi, f3(pj4));
+        const float d2 = dotf(r, r);
+        const float bj = C.textbook ? nb.mass / nb.rho : 1.f;
+        const float3 gj = f3(nb.g), dv = sub3(f3(nb.v), vi);
+        Term t;
+        t.gv_scale = C.xsph_c * poly6(C, d2);
+        t.gv = sub3(mul3(gj, bi), mul3(go, bj));
+        t.gp_scale = C.xsph_c * (bj * dotf(dv, go) - bi * dotf(dv, gj));
+        t.gp = poly6_grad(C, r, d2);
+        t.rb = -dotf(dv, gj);  // j's sum: c W b_i (v_i - v_j) . g_j
+        return t;
+    }
+};
+__device__ __forceinline__ XsphPair::Nb xsph_neighbour(const SimConsts &C, const float4 *__restrict__ V,
+                                                       const float *__restrict__ mass, const float *__restrict__ rho,
+                                                       const float4 *__restrict__ gVout, int j)
+{
+    return XsphPair::Nb{V[j], gVout[j], C.textbook ? mass[j] : 1.f, C.textbook ? rho[j] : 1.f};
+}
+__device__ __forceinline__ void finish_xsph(const SimConsts &C, const XsphPair &pair, const float *__restrict__ rho,
+                                            float3 gv, float3 gp, float rb, float4 *__restrict__ gVin,
+                                            float4 *__restrict__ gX, float *__restrict__ gRho)
+{
+    const int i = pair.i;
+    gVin[i] = f4(gv);
+    gX[i] = f4(add3(ld3(gX, i), gp));
+    if (C.textbook) gRho[i] -= rb * pair.bi / rho[i];  // d b_i / d rho_i = -b_i / rho_i
+}
+
+// Lists: as k_adj_deltap, over the lists of the substep's adjoint.
+// 65,536 particles, a launch: 46 us with its own walk, 19 us over the lists and
+// 3 us for the queue.
+template <bool Lists>
 __global__ void __launch_bounds__(kWalkThreads) k_adj_xsph(SimConsts C, const float4 *__restrict__ P,
                                                            const float4 *__restrict__ V, const int *__restrict__ off,
                                                            const float *__restrict__ mass,
@@ -750,39 +937,70 @@ __global__ void __launch_bounds__(kWalkThreads) k_adj_xsph(SimConsts C, const fl
                                                            float4 *__restrict__ gX, float *__restrict__ gRho)
 {
     StageShared &S = stage_shared();
-    const int g = stage_block(C, P, off, blockIdx.x * kWalkThreads, S);
+    const int g = Lists ? -1 : stage_block(C, P, off, blockIdx.x * kWalkThreads, S);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (Lists && i == 0) C.sl_count[C.sl_pass ^ 1] = 0;  // the next pass's queue
     if (i >= C.n) return;
     const float4 pi4 = P[i];
-    const int phi = phase_of(pi4);
-    const float3 go = ld3(gVout, i);
-    if (phi >= 0) {
-        gVin[i] = f4(go);
+    if (phase_of(pi4) >= 0) {
+        gVin[i] = f4(ld3(gVout, i));
         return;
     }
-    const float3 pi = f3(pi4), vi = ld3(V, i);
-    const float bi = C.textbook ? mass[i] / rho[i] : 1.f;
-    float3 gv = go, gp = make_float3(0.f, 0.f, 0.f);
+    const GridView v = grid_view(C, scene_index(C, i), off);
+    if (Lists && !reads_substep_list(C, i, i, f3(pi4), cell_of(f3(pi4), C), v)) return;
+    const XsphPair pair(C, i, pi4, V, mass, rho, gVout);
+    float3 gv = pair.go, gp = make_float3(0.f, 0.f, 0.f);
     float rb = 0.f;
-    auto test = [&](int j, float4 pj4) {
-        const float3 r = sub3(pi, f3(pj4));
-        return j != i && phase_of(pj4) == phi && dotf(r, r) <= C.h2;
+    auto test = [&](int j, float4 pj4) { return pair.counts(j, pj4); };
+    auto fetch = [&](int j) { return xsph_neighbour(C, V, mass, rho, gVout, j); };
+    auto term = [&](int, float4 pj4, const XsphPair::Nb &nb) {
+        const XsphPair::Term t = pair.term(pj4, nb);
+        gv = fma_to(gv, t.gv_scale, t.gv);
+        gp = fma_to(gp, t.gp_scale, t.gp);
+        if (C.textbook) rb = __fmaf_rn(t.gv_scale, t.rb, rb);
     };
-    auto term = [&](int j, float4 pj4) {
-        const float3 r = sub3(pi, f3(pj4));
-        const float d2 = dotf(r, r);
-        const float w = poly6(C, d2);
-        const float bj = C.textbook ? mass[j] / rho[j] : 1.f;
-        const float3 gj = ld3(gVout, j);
-        gv = add3(gv, mul3(sub3(mul3(gj, bi), mul3(go, bj)), C.xsph_c * w));
-        const float3 dv = sub3(ld3(V, j), vi);
-        gp = add3(gp, mul3(poly6_grad(C, r, d2), C.xsph_c * (bj * dotf(dv, go) - bi * dotf(dv, gj))));
-        if (C.textbook) rb -= C.xsph_c * w * dotf(dv, gj);  // j's sum: c W b_i (v_i - v_j) . g_j
-    };
-    record_then_sum(C, i, pi, P, grid_view(C, scene_index(C, i), off), &S, g, test, test, term);
-    gVin[i] = f4(gv);
-    gX[i] = f4(add3(ld3(gX, i), gp));
-    if (C.textbook) gRho[i] -= rb * bi / rho[i];  // d b_i / d rho_i = -b_i / rho_i
+    if (Lists)
+        for_each_padded(C.nbr, C.n, i, __ldg(C.nbr_count + i) & 0xffff, P, fetch,
+                        [&](int j, float4 pj4, const XsphPair::Nb &nb) {
+                            if (test(j, pj4)) term(j, pj4, nb);
+                        });
+    else
+        record_then_sum(C, i, pair.pi, P, v, &S, g, test, test, fetch, term);
+    finish_xsph(C, pair, rho, gv, gp, rb, gVin, gX, gRho);
+}
+
+// The queued particles' XSPH gradient, a warp per particle.
+__global__ void __launch_bounds__(kAdjQueueThreads) k_adj_xsph_queued(
+    SimConsts C, const float4 *__restrict__ P, const float4 *__restrict__ V, const int *__restrict__ off,
+    const float *__restrict__ mass, const float *__restrict__ rho, const float4 *__restrict__ gVout,
+    float4 *__restrict__ gVin, float4 *__restrict__ gX, float *__restrict__ gRho)
+{
+    __shared__ WarpRows rows[kAdjQueueThreads / 32];
+    __shared__ WarpHits hits[kAdjQueueThreads / 32];
+    const int lane = threadIdx.x & 31;
+    const int queued = C.sl_count[C.sl_pass];
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) / 32; q < queued; q += gridDim.x * blockDim.x / 32) {
+        const int i = C.sl_queue[q];
+        const XsphPair pair(C, i, P[i], V, mass, rho, gVout);
+        WarpRows &row = rows[threadIdx.x >> 5];
+        // lanes 0..2
+        float gv = lane == 0 ? pair.go.x : (lane == 1 ? pair.go.y : pair.go.z), gp = 0.f, rb = 0.f;
+        auto batch = [&](int, int n, int j, float4 pj4) {
+            const bool in = lane < n;
+            const unsigned take = __ballot_sync(kWarp, in);
+            XsphPair::Term t = {};
+            if (in) t = pair.term(pj4, xsph_neighbour(C, V, mass, rho, gVout, j));
+            const float dv[3] = {t.gv.x, t.gv.y, t.gv.z}, dp[3] = {t.gp.x, t.gp.y, t.gp.z}, db[1] = {t.rb};
+            warp_add<3, 0>(row, take, dv, t.gv_scale, gv);
+            warp_add<3, 0>(row, take, dp, t.gp_scale, gp);
+            if (C.textbook) warp_add<1, 0>(row, take, db, t.gv_scale, rb);
+        };
+        warp_neighbors(C, false, cell_of(pair.pi, C), P, grid_view(C, scene_index(C, i), off), hits[threadIdx.x >> 5],
+                       [&](int j, float4 pj4) { return pair.counts(j, pj4); }, batch);
+        const float3 v = make_float3(__shfl_sync(kWarp, gv, 0), __shfl_sync(kWarp, gv, 1), __shfl_sync(kWarp, gv, 2));
+        const float3 p = make_float3(__shfl_sync(kWarp, gp, 0), __shfl_sync(kWarp, gp, 1), __shfl_sync(kWarp, gp, 2));
+        if (lane == 0) finish_xsph(C, pair, rho, v, p, rb, gVin, gX, gRho);
+    }
 }
 
 // ---- shape matching (alpha = 1): g_i = R q_i + cm ----
@@ -1392,13 +1610,25 @@ void adj_wind(cudaStream_t st, const SimConsts &C, const WindArgs &a, const floa
                                                           FG, FV, to_new, gP, gVs);
     k_adj_sum4<<<1, 1024, 0, st>>>(a.num_faces, FW, g_wind);
 }
+void adj_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const int *off)
+{
+    if (C.n <= 0) return;
+    if (record) k_adj_record_lists<<<blocks(C.n, kWalkThreads), kWalkThreads, 0, st>>>(C, P, off);
+    else k_adj_track<<<blocks(C.n), 256, 0, st>>>(C, P);
+}
 void adj_fluid(cudaStream_t st, const SimConsts &C, const float4 *Pin, const float *mass, const float *lam,
                const float *rho, const int *off, const float4 *gOut, const float *gRho, float *gLam, float4 *gPart,
                float4 *GD, float *rhob, float4 *gIn)
 {
     if (C.n <= 0) return;
     const int b = blocks(C.n, kWalkThreads);
-    k_adj_deltap<<<b, kWalkThreads, stage_bytes(C), st>>>(C, Pin, mass, lam, off, gOut, gLam, gPart);
+    if (C.sl_pos) {
+        k_adj_deltap<true><<<b, kWalkThreads, 0, st>>>(C, Pin, mass, lam, off, gOut, gLam, gPart);
+        k_adj_deltap_queued<<<queue_blocks(C.n, kAdjQueueThreads), kAdjQueueThreads, 0, st>>>(C, Pin, mass, lam, off,
+                                                                                            gOut, gLam, gPart);
+    } else {
+        k_adj_deltap<false><<<b, kWalkThreads, stage_bytes(C), st>>>(C, Pin, mass, lam, off, gOut, gLam, gPart);
+    }
     if (C.textbook) {
         k_adj_lambda_tb_prep<<<b, kWalkThreads, 0, st>>>(C, Pin, mass, off, gLam, gRho, GD, rhob);
         k_adj_lambda_tb<<<b, kWalkThreads, 0, st>>>(C, Pin, mass, off, GD, rhob, gPart, gOut, gIn);
@@ -1416,8 +1646,14 @@ void adj_xsph(cudaStream_t st, const SimConsts &C, const float4 *P, const float4
               const float *mass, const float *rho, const float4 *gVout, float4 *gVin, float4 *gX, float *gRho)
 {
     if (C.n <= 0) return;
-    k_adj_xsph<<<blocks(C.n, kWalkThreads), kWalkThreads, stage_bytes(C), st>>>(C, P, V, off, mass, rho, gVout,
-                                                                               gVin, gX, gRho);
+    const int b = blocks(C.n, kWalkThreads);
+    if (C.sl_pos) {
+        k_adj_xsph<true><<<b, kWalkThreads, 0, st>>>(C, P, V, off, mass, rho, gVout, gVin, gX, gRho);
+        k_adj_xsph_queued<<<queue_blocks(C.n, kAdjQueueThreads), kAdjQueueThreads, 0, st>>>(C, P, V, off, mass, rho,
+                                                                                          gVout, gVin, gX, gRho);
+    } else {
+        k_adj_xsph<false><<<b, kWalkThreads, stage_bytes(C), st>>>(C, P, V, off, mass, rho, gVout, gVin, gX, gRho);
+    }
 }
 
 void adj_contacts(cudaStream_t st, const SimConsts &C, const float4 *Pin, const float4 *Xs, const float *w,

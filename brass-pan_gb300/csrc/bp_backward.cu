@@ -37,6 +37,7 @@ void adj_distance_step(cudaStream_t st, const SimConsts &C, const DistanceStep &
 void adj_wind(cudaStream_t st, const SimConsts &C, const WindArgs &a, const float4 *Pin, const float4 *Vs,
               const float *mass, const int *to_new, float4 *gP, float4 *gVs, float4 *FG, float4 *FV, float4 *FW,
               float4 *g_wind);
+void adj_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const int *off);
 void adj_fluid(cudaStream_t st, const SimConsts &C, const float4 *Pin, const float *mass, const float *lam,
                const float *rho, const int *off, const float4 *gOut, const float *gRho, float *gLam, float4 *gPart,
                float4 *GD, float *rhob, float4 *gIn);
@@ -399,6 +400,32 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
         C.nbr_count = s->nbr_count;  // the fluid adjoint's pass A leaves its lists for pass B
         C.nbr_cap = kPostListCap;
     }
+    // One search for the stages that walk (k_adj_record_lists) where the update
+    // itself takes its lists so and two of them read them: the density passes,
+    // and XSPH alone after the commit (the post passes record their own).
+    SimConsts Cl = C;
+    bool listed = false;
+    int list_passes = 0;
+    int readers = 0;
+    for (const TapeRec &rec : T.recs) readers += rec.stage == TS_FLUID || rec.stage == TS_XSPH;
+    const bool shared = u.C.sl_pos && C.nbr && s->walk_xyz && readers > 1;
+    if (shared) {
+        Cl.sl_pos = u.C.sl_pos;
+        Cl.walk_xyz = s->walk_xyz;
+        Cl.walk_stride = s->walk_stride;
+    }
+    auto lists_at = [&](const float4 *P) -> const SimConsts & {
+        if (!shared) return C;
+        if (!listed) {
+            LaunchLog L;
+            launch_walk_planes(st, s->n, P, s->walk_xyz, s->walk_stride, &L);
+            clear_list_bits(s);
+        }
+        Cl.sl_pass = list_passes++ & 1;
+        adj_lists(st, Cl, !listed, P, s->off);
+        listed = true;
+        return Cl;
+    };
     const bp_params &p = u.prm;
     const bool planes = stage_on(p, BP_STAGE_PLANES) && s->nplanes > 0;
     const bool distance = stage_on(p, BP_STAGE_DISTANCE) && s->dist.num_edges > 0;
@@ -454,7 +481,8 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
         case TS_XSPH: {  // velocities before XSPH in the slot; positions: the commit's input
             int c = r - 1;
             while (c >= 0 && T.recs[c].stage != TS_COMMIT) --c;
-            adj_xsph(st, C, T.pool4[T.recs[c].slot], T.pool4[rec.slot], s->off, s->mass, T.pool1[rec.aux1], gV,
+            const float4 *Pc = T.pool4[T.recs[c].slot];
+            adj_xsph(st, lists_at(Pc), Pc, T.pool4[rec.slot], s->off, s->mass, T.pool1[rec.aux1], gV,
                      gVn, t.gX, t.gRho);
             std::swap(gV, gVn);
             break;
@@ -470,7 +498,7 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
                          t.g_rest);
             break;
         case TS_FLUID:
-            adj_fluid(st, C, T.pool4[rec.slot], s->mass, T.pool1[rec.aux], T.pool1[rec.aux + 1], s->off, gP,
+            adj_fluid(st, lists_at(T.pool4[rec.slot]), T.pool4[rec.slot], s->mass, T.pool1[rec.aux], T.pool1[rec.aux + 1], s->off, gP,
                       last_fluid ? t.gRho : nullptr, t.gLam, t.gPart, t.GD, t.rhob, gP2);
             last_fluid = false;
             std::swap(gP, gP2);

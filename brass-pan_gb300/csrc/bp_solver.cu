@@ -356,6 +356,11 @@ struct BatchSpec {
 // Words of SimConsts::sl_near and sl_far.
 static size_t sl_bit_words(const bp_solver *s) { return (kSlLevels + 4) * s->sl_words; }
 
+void bp::clear_list_bits(bp_solver *s)
+{
+    cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), s->stream);
+}
+
 // The Verlet lists' buffers (1 KB a particle), for parameters that ask for
 // them; single scenes only.
 static bp_status verlet_buffers(bp_solver *s, const bp_params &p)
@@ -986,7 +991,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         if (listed_contacts && !(fluid && it == 0)) {
             if (it == 0) {
                 refresh_planes(cur);
-                cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), st);
+                clear_list_bits(s);
                 launch_lambda_lists(st, Cf, true, cur, s->mass, s->off, s->lam, s->rho, L);
             }
             if (tape) tape->push(TS_PCOLL, slot);
@@ -1022,7 +1027,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
                 cudaMemsetAsync(s->nl_outlier, 0, (size_t)C.D * C.D * C.nl_zwords * sizeof(unsigned long long), st);
             if (shared) {
                 next_list_pass(Cf, !record && it == iterations - 1 && !post_ab && !C.use_xsph);
-                if (record) cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), st);
+                if (record) clear_list_bits(s);
                 launch_lambda_lists(st, Cf, record, cur, s->mass, s->off, s->lam, s->rho, L);
             } else {
                 launch_lambda(st, it == 0 ? Cbuild : Cf, cur, s->mass, s->off, s->lam, s->rho, L);

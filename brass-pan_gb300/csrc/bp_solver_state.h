@@ -223,6 +223,8 @@ struct bp_solver {
 namespace bp {
 // Substep constants of solver s for substep length sdt.
 SimConsts make_consts(const bp_solver *s, float sdt);
+// Clears the displacement bits of the substep lists.
+void clear_list_bits(bp_solver *s);
 // Records an update about to be enqueued while s->tape is open.
 bp_status tape_record_update(bp_solver *s, int nsub, float dt, int iterations, int picked, float3 ppos, float3 pvel);
 // Enqueues one substep on s->stream.  With a tape, the fused epilogues are
