@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_adj_record_lists(SimConsts C, 
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k == 0) {
-        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = 0;
+        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = C.sl_count[kSlWalks] = 0;
         C.sl_count[kSlMoved] = 0;
     }
     if (k >= C.n) return;

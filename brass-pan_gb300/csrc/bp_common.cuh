@@ -184,9 +184,12 @@ struct SimConsts {
     int *sl_queue;
     // [0], [1]: queue lengths, by the parity of the pass (a list pass clears the
     // other one); [kSlMoved]; [kSlDisplaced]: particles that the last list pass
-    // of a substep queued because something near them moved
+    // of a substep queued because something near them moved, [kSlWalks]: those
+    // of the passes before it
     int *sl_count;
-    float *sl_skin;   // [0] the skin in use, adapted after each substep (adapt_skin), [1] the last that was too small
+    // [0] the skin in use, adapted after each substep (adapt_skin), [1] the last
+    // that was too small, [2] such walks a particle of the last substeps
+    float *sl_skin;
     float sl_fixed;   // > 0: this skin instead
     int sl_pass;      // parity of this list pass
     int sl_adapt;     // this pass is the substep's last over the lists
@@ -201,9 +204,10 @@ struct SimConsts {
 };
 constexpr int kContactCap = 32;
 constexpr int kSlLevels = 3;
-constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlCounts = 4;
-// Bounds of the adapted skin and where it starts, as fractions of h.
-constexpr float kMinSkin = 0.02f, kMaxSkin = 0.1f, kStartSkin = 0.09f;
+constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlWalks = 4, kSlCounts = 5;
+// Bounds of the adapted skin and where it starts, as fractions of h: up to
+// kMaxSkin as a rule, up to kWideSkin where walks go on at that (adapt_skin).
+constexpr float kMinSkin = 0.02f, kMaxSkin = 0.1f, kWideSkin = 0.2f, kStartSkin = 0.09f;
 // sl_cell where there is no list to read: something near moved, or another reason.
 constexpr int kListMoved = -1, kListNone = -2;
 

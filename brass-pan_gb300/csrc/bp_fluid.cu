@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kScanThreads, BP_SCAN_MIN_BLOCKS) k_lambda_lis
         C.sl_count[C.sl_pass ^ 1] = 0;  // the next pass's queue
         if (Pass == kRecordLists) {
             C.sl_count[C.sl_pass] = 0;
-            C.sl_count[kSlDisplaced] = 0;
+            C.sl_count[kSlDisplaced] = C.sl_count[kSlWalks] = 0;
             C.sl_count[kSlMoved] = C.cls_perm ? *C.cls_moved : 0;
         }
     }
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(kQueueThreads) k_lambda_record(SimConsts C, co
     const int lane = threadIdx.x & 31;
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = 0;
+        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = C.sl_count[kSlWalks] = 0;
         C.sl_count[kSlMoved] = C.cls_perm ? *C.cls_moved : 0;
     }
     if (t >= C.n) return;  // whole warps

@@ -145,7 +145,7 @@ static bool planes_confine(const bp_solver *s, int D, float cell)
 // iterations and 3 post passes: 4.73 -> 3.04 ms a frame of 2 substeps; mixed
 // scene late 12.4 -> 8.85 ms; 1,728 particles 0.45 -> 0.32 ms).  The lists
 // come from the split, unstaged recording walk.  neighbor_skin sets the skin;
-// with 0 it adapts (adapt_skin), up to the kMaxSkin of h returned.
+// with 0 it adapts (adapt_skin), up to the kWideSkin of h returned.
 static float largest_skin(const bp_solver *s)
 {
     const bp_params &p = s->prm;
@@ -153,7 +153,7 @@ static float largest_skin(const bp_solver *s)
     if (!(p.walk_options & BP_WALK_NO_STAGING) || (p.walk_options & other) || p.scan_persistent ||
         !((p.stage_mask & BP_STAGE_FLUID) || ((p.stage_mask & BP_STAGE_PARTICLE_COLLISION) && s->has_solid)))
         return 0.f;
-    return p.kernel_radius * (p.neighbor_skin > 0.f ? p.neighbor_skin : kMaxSkin);
+    return p.kernel_radius * (p.neighbor_skin > 0.f ? p.neighbor_skin : kWideSkin);
 }
 
 static float class_reach(const bp_solver *s)
@@ -425,7 +425,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         (st = s->alloc(&s->off, ncells + 1)) || (st = s->alloc(&s->mass, N)) || (st = s->alloc(&s->lam, N)) || (st = s->alloc(&s->lm, N)) ||
         (st = s->alloc(&s->rho, N)) || (st = s->alloc(&s->w, N)) || (st = s->alloc(&s->err, 1)) ||
         (st = s->alloc(&s->staging, 6 * N)) || (st = s->alloc(&s->nl_pos, N)) || (st = s->alloc(&s->sl_cell, N)) ||
-        (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 2)) ||
+        (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 3)) ||
         (st = s->alloc(&s->sl_bits, sl_bit_words(s))) ||
         (st = s->alloc(&s->nl_stats, 5)) || (!batch && (st = verlet_buffers(s, *prm))))
         return bail(st);
@@ -499,7 +499,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         BP_CUDA_BAIL(cudaMemcpy(s->mass, m.data(), n * sizeof(float), cudaMemcpyHostToDevice));
     }
     s->Pcur = s->Pa;
-    const float skin0[2] = {kStartSkin * prm->kernel_radius, 0.f};
+    const float skin0[3] = {kStartSkin * prm->kernel_radius, 0.f, 0.f};
     BP_CUDA_BAIL(cudaMemcpy(s->sl_skin, skin0, sizeof(skin0), cudaMemcpyHostToDevice));
     BP_CUDA_BAIL(cudaMemset(s->lam, 0, N * sizeof(float)));
     BP_CUDA_BAIL(cudaMemset(s->rho, 0, N * sizeof(float)));

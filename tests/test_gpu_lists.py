@@ -155,3 +155,24 @@ def test_viscosity_alone_over_the_lists_is_bit_identical_to_walks(bp, gpu, name,
         g.close()
     for a, b in zip(*outs):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("solids", [False, True])
+def test_adapted_skins_of_a_bursting_block_are_bit_identical_to_walks(bp, gpu, solids):
+    """A squeezed block bursting apart, where the skin grows to its widest and
+    shrinks again: after every update the bits of walks without lists."""
+    abi = bp.abi
+    scene = (small_mixed_scene(bp, seed=7, fluid=(16, 12, 16), grid_dim=32) if solids
+             else fluid_scene(bp, (16, 14, 15), seed=7, grid_dim=32, box=(3.0, 3.0, 3.0)))
+    fluid = scene.phases < 0
+    low = scene.positions[fluid].min(axis=0)
+    scene.positions[fluid] = low + (scene.positions[fluid] - low) / np.float32(1.25)
+    ways = (abi.BP_WALK_NO_STAGING, abi.BP_WALK_NO_STAGING | abi.BP_WALK_NO_LISTS)
+    a, b = (bp.ParticleSolver(scene, bp.make_params(scene, mode=abi.BP_MODE_TEXTBOOK, walk_options=w)) for w in ways)
+    for _ in range(12):
+        for s in (a, b):
+            s.update(2, DT, 3)
+        np.testing.assert_array_equal(a.positions(), b.positions())
+        np.testing.assert_array_equal(a.velocities(), b.velocities())
+    a.close()
+    b.close()
