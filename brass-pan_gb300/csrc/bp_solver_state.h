@@ -88,12 +88,15 @@ struct SubstepTape {
 };
 }  // namespace bp
 
-// Recorded neighbours per particle for the post passes: about 33 at rest
-// density with h = 2 spacings, well over 128 in fluid compressed 2.5-fold
-// (particles beyond the cap walk their cells; 64 / 128 / 192 measured
-// 73.6 / 77.7 / 84.0 M particle-substeps/s over the mixed 200 frames).
+// Recorded neighbours per particle: about 33 within h at rest density with h =
+// 2 spacings, 130 in fluid settled to 2.5 times that and 220 with the substep
+// lists' widest skin, 300 while a dam break's front is compressed.  Particles
+// beyond the cap walk their cells, a warp each with the substep lists: 192 took
+// 44 ms a frame 50 frames into the mixed scene (80 % of the reads past the cap)
+// and 17.5 ms 200 frames in, 384 takes 21.7 and 15.4 ms.  Only records in use
+// are touched.
 #ifndef BP_POST_LIST_CAP
-#define BP_POST_LIST_CAP 192
+#define BP_POST_LIST_CAP 384
 #endif
 constexpr int kPostListCap = BP_POST_LIST_CAP;
 static_assert(kPostListCap % 4 == 0, "lists are stored as records of four entries");

@@ -25,13 +25,13 @@ def grains(bp, grid_dim=16):
 
 
 def packed(bp):
-    """A core at half spacing: its lists overflow (about 270 neighbours within
-    h), and those around it hold up to their capacity."""
+    """A core at 0.4 of the spacing: its lists overflow (about 500 neighbours
+    within h), and those around it hold up to their capacity."""
     s = fluid_scene(bp, (12, 12, 12), seed=41, grid_dim=16)
     x = s.positions.copy()
     c = x.mean(axis=0)
     core = np.all(np.abs(x - c) < 0.35, axis=1)
-    x[core] = c + (x[core] - c) * np.float32(0.5)
+    x[core] = c + (x[core] - c) * np.float32(0.4)
     s.positions = x.astype(np.float32)
     return s
 
@@ -176,3 +176,23 @@ def test_adapted_skins_of_a_bursting_block_are_bit_identical_to_walks(bp, gpu, s
         np.testing.assert_array_equal(a.velocities(), b.velocities())
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("mode", ["reference", "textbook"])
+@pytest.mark.parametrize("grid_dim", [8, 32])
+def test_overflowing_lists_recorded_by_each_pass(bp, gpu, grid_dim, mode):
+    """The lists that every pass records for the next one (walks over the
+    position records), past their capacity: the bits of walks without lists."""
+    abi = bp.abi
+    m = abi.BP_MODE_TEXTBOOK if mode == "textbook" else abi.BP_MODE_REFERENCE
+    scene = packed(bp)
+    scene.grid_dim = grid_dim
+    outs = []
+    for walk in (abi.BP_WALK_NO_STAGING | abi.BP_WALK_NO_PLANES, abi.BP_WALK_NO_STAGING | abi.BP_WALK_NO_LISTS):
+        g = bp.ParticleSolver(scene, bp.make_params(scene, mode=m, walk_options=walk))
+        for _ in range(3):
+            g.update(2, DT, 4)
+        outs.append((g.positions(), g.velocities(), g.field(abi.BP_FIELD_DENSITIES)))
+        g.close()
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
