@@ -410,7 +410,7 @@ __device__ __forceinline__ int list_state(const SimConsts &C, int i, int3 c, flo
 // Substep lists: particle i moved more than `level` quarters of the skin.
 // In a pile of tumbling bodies every particle does, in every iteration: one
 // read or atomic then settles all levels (a bit set per level: shape matching
-// of 1 M such particles 584 us a frame, one word a cell 546 us).
+// of 2.09 M such particles 584 us a frame, one word a cell 546 us).
 __device__ __forceinline__ void flag_moved(const SimConsts &C, int i, int level)
 {
     const unsigned key = (unsigned)__ldg(C.cell_keys + i);
