@@ -260,14 +260,18 @@ __device__ __forceinline__ void warp_pad(const SimConsts &C, int t, int cnt, int
 }
 
 // CTAs of `threads` for a launch over the queue, a warp per entry, whose length
-// only the device knows.
+// only the device knows.  32 of them an SM: walks differ tenfold in length, and
+// CTAs that start as others end even that out, where 8 resident ones that each
+// took every 8th share left SMs idle (mixed scene 6098 -> 6002 us a frame, 200
+// frames in 15.4 -> 14.9 ms; 16: 6043 us and 15.0 ms, 64 as 32); CTAs that find
+// no entry cost nothing measurable (1M fluid 4112 and 4121 us).
 inline int queue_blocks(int n, int threads)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int per = threads / 32;
-    return std::min((n + per - 1) / per, std::max(sms, 1) * 8);
+    return std::min((n + per - 1) / per, std::max(sms, 1) * 32);
 }
 
 }  // namespace bp
