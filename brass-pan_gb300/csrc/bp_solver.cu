@@ -1139,6 +1139,9 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     if (post_ab) {
         // pass A records each fluid particle's neighbours for passes B and C
         SimConsts Cl = Cpost;
+        // contacts alone: pass A leaves lists of its own in the walkers' slots,
+        // which the readers of the substep lists would take for theirs
+        if (!post_lists) Cl.sl_pos = nullptr;
         if (lists) {
             Cl.nbr = s->nbr;
             Cl.nbr_count = s->nbr_count;
@@ -1166,6 +1169,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         if (C.use_xsph) launch_post_c(st, Cl, cur, s->Vs, s->off, s->mass, s->rho, s->Vc, L);
     } else if (C.use_xsph) {
         SimConsts Cx = Cpost;
+        if (!post_lists) Cx.sl_pos = nullptr;
         if (lists) {
             Cx.nbr = s->nbr;
             Cx.nbr_count = post_lists ? s->nbr_count : nullptr;
