@@ -297,6 +297,19 @@ __device__ __forceinline__ void finish_lambda(const SimConsts &C, bool slots, in
     rho[i] = density;
 }
 
+// A solid's lambda, 0, and its pair for the position pass's gathers.  Later
+// passes of the substep leave solids out, so the pair goes to both orders: the
+// classes may close in between (k_class_refresh), and the lists then hold
+// sorted indices.
+__device__ __forceinline__ void record_solid(const SimConsts &C, bool slots, int i, int t,
+                                             const float *__restrict__ mass, float *__restrict__ lam)
+{
+    const float2 lm = make_float2(0.f, __ldg(mass + i));
+    lam[i] = 0.f;
+    C.lm[i] = lm;
+    if (slots) C.cls_lm[t] = lm;
+}
+
 // Records slot t's contact partners (SimConsts::cl_list) from its list just
 // recorded.
 __device__ __forceinline__ void record_contacts(const SimConsts &C, const float4 *__restrict__ P, bool slots, int t,
@@ -335,10 +348,7 @@ __device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const fl
     const bool solid = phase_of(pi4) > 0;
     if (Pass == kRecordLists) {
         C.sl_pos[i] = pi4;
-        if (solid && C.sl_fluid) {  // solids carry lambda 0 (read by the position pass)
-            lam[i] = 0.f;
-            (slots ? C.cls_lm[t] : C.lm[i]) = make_float2(0.f, __ldg(mass + i));
-        }
+        if (solid && C.sl_fluid) record_solid(C, slots, i, t, mass, lam);
     }
     // textbook mode: no pass but the contacts moves a solid by its neighbours
     if (solid && C.textbook && !(Pass == kRecordLists && C.cl_list)) return;
@@ -1224,10 +1234,7 @@ __global__ void __launch_bounds__(kQueueThreads) k_lambda_record(SimConsts C, co
     const bool solid = phi > 0;
     if (lane == 0) {
         C.sl_pos[i] = pi4;
-        if (solid && C.sl_fluid) {  // solids carry lambda 0 (read by the position pass)
-            lam[i] = 0.f;
-            (slots ? C.cls_lm[t] : C.lm[i]) = make_float2(0.f, __ldg(mass + i));
-        }
+        if (solid && C.sl_fluid) record_solid(C, slots, i, t, mass, lam);
     }
     if (solid && C.textbook && !C.cl_list) return;  // as lambda_substep_list
     const int sc = scene_index(C, i);
