@@ -187,8 +187,9 @@ struct SimConsts {
     // of a substep queued because something near them moved, [kSlWalks]: those
     // of the passes before it
     int *sl_count;
-    // [0] the skin in use, adapted after each substep (adapt_skin), [1] the last
-    // that was too small, [2] such walks a particle of the last substeps
+    // [0] the skin in use, as a fraction of h (a radius set later keeps it within
+    // kWideSkin), adapted after each substep (adapt_skin), [1] the last that was
+    // too small, [2] such walks a particle of the last substeps
     float *sl_skin;
     float sl_fixed;   // > 0: this skin instead
     int sl_pass;      // parity of this list pass
@@ -211,7 +212,10 @@ constexpr float kMinSkin = 0.02f, kMaxSkin = 0.1f, kWideSkin = 0.2f, kStartSkin 
 // sl_cell where there is no list to read: something near moved, or another reason.
 constexpr int kListMoved = -1, kListNone = -2;
 
-__device__ __forceinline__ float substep_skin(const SimConsts &C) { return C.sl_fixed > 0.f ? C.sl_fixed : __ldg(C.sl_skin); }
+__device__ __forceinline__ float substep_skin(const SimConsts &C)
+{
+    return C.sl_fixed > 0.f ? C.sl_fixed : __fmul_rn(C.h, __ldg(C.sl_skin));
+}
 // The square of a quarter of the skin, less what the rounding of the distance
 // tests may take (k quarters: k * k times it).
 __device__ __forceinline__ float substep_quarter2(const SimConsts &C)

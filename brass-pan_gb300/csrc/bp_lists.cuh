@@ -66,14 +66,14 @@ __device__ __forceinline__ void adapt_skin(const SimConsts &C)
     const long long moved = C.sl_count[kSlDisplaced];
     float skin = C.sl_skin[0], bad = C.sl_skin[1] * 0.998f;
     const float walks = 0.5f * (C.sl_skin[2] + (float)(moved + C.sl_count[kSlWalks]) / (float)C.n);
-    const bool wide = skin >= 0.999f * (C.h * kMaxSkin);
+    const bool wide = skin >= 0.999f * kMaxSkin;
     if (wide && walks > kWideWalks) {
-        skin = fminf(skin * 1.3f, C.h * kWideSkin);
+        skin = fminf(skin * 1.3f, kWideSkin);
     } else if (!wide && moved * 25 > C.n) {
         bad = skin;
-        skin = fminf(skin * 1.3f, C.h * kMaxSkin);
+        skin = fminf(skin * 1.3f, kMaxSkin);
     } else if (wide ? walks < kWideRest : moved * 100 < C.n) {
-        skin = fmaxf(skin * 0.9f, fmaxf(fminf(bad * 1.15f, skin), C.h * kMinSkin));
+        skin = fmaxf(skin * 0.9f, fmaxf(fminf(bad * 1.15f, skin), kMinSkin));
     }
     C.sl_skin[0] = skin;
     C.sl_skin[1] = bad;

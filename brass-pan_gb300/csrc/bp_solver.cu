@@ -499,7 +499,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         BP_CUDA_BAIL(cudaMemcpy(s->mass, m.data(), n * sizeof(float), cudaMemcpyHostToDevice));
     }
     s->Pcur = s->Pa;
-    const float skin0[3] = {kStartSkin * prm->kernel_radius, 0.f, 0.f};
+    const float skin0[3] = {kStartSkin, 0.f, 0.f};
     BP_CUDA_BAIL(cudaMemcpy(s->sl_skin, skin0, sizeof(skin0), cudaMemcpyHostToDevice));
     BP_CUDA_BAIL(cudaMemset(s->lam, 0, N * sizeof(float)));
     BP_CUDA_BAIL(cudaMemset(s->rho, 0, N * sizeof(float)));
