@@ -59,20 +59,30 @@ namespace {
 
 // Device buffers owned by a tape (freed with it).
 struct DevPool {
-    std::vector<void *> ptrs;
+    std::vector<std::pair<void *, size_t>> bufs;  // buffer, bytes
     size_t bytes = 0;
-    ~DevPool()
-    {
-        for (void *p : ptrs) cudaFree(p);
-    }
+    bool failed = false;  // an allocation did
+    ~DevPool() { give_back(0); }
     template <class T>
     T *get(size_t count)
     {
         void *p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        bytes += std::max<size_t>(count, 1) * sizeof(T);
+        const size_t size = std::max<size_t>(count, 1) * sizeof(T);
+        if (device_malloc(nullptr, &p, size) != cudaSuccess) {
+            failed = true;
+            return nullptr;
+        }
+        bufs.push_back({p, size});
+        bytes += size;
         return (T *)p;
+    }
+    // frees all but the first `count` buffers (those of a set that did not fit)
+    void give_back(size_t count)
+    {
+        for (; bufs.size() > count; bufs.pop_back()) {
+            cudaFree(bufs.back().first);
+            bytes -= bufs.back().second;
+        }
     }
 };
 
@@ -137,6 +147,20 @@ struct Tape {
     float *rhob = nullptr;
 };
 
+cudaError_t device_malloc(bp_solver *s, void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && s && s->spare) {
+        cudaStreamSynchronize(s->stream);
+        destroy_tape(s->spare);
+        s->spare = nullptr;
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
 void destroy_tape(Tape *t)
 {
     if (!t) return;
@@ -156,8 +180,8 @@ void destroy_tape(Tape *t)
 // and freeing the buffers and capturing the graphs again took 4.4 of 11.6 ms
 // (128 x 128 flag, 10 frames, on the host while the GPU waits) and 4.8 of
 // 11.7 ms (65,536 particles of fluid, 3 frames).  Buffers beyond this many
-// bytes are given back at the end of the recording, as every buffer is when
-// the solver is destroyed.
+// bytes are given back at the end of the recording, as those of one that ran
+// out of memory are, and as every buffer is when the solver is destroyed.
 constexpr size_t kSpareTapeBytes = size_t(512) << 20;
 
 void retire_tape(bp_solver *s)
@@ -169,7 +193,9 @@ void retire_tape(bp_solver *s)
     for (const SubstepTape *st : t->tapes)
         bytes += (st->pool4.size() * sizeof(float4) + st->pool1.size() * sizeof(float)) * (size_t)std::max(s->n, 1);
     for (const auto &b : t->snap.bufs) bytes += b.second;
-    if (bytes > kSpareTapeBytes) {
+    bool failed = t->pool.failed || t->snap.copies.size() < t->snap.bufs.size();
+    for (const SubstepTape *st : t->tapes) failed = failed || !st->ok;
+    if (failed || bytes > kSpareTapeBytes) {
         destroy_tape(t);
         return;
     }
@@ -184,7 +210,7 @@ int SubstepTape::fresh4()
 {
     if (used4 == (int)pool4.size()) {
         void *p = nullptr;
-        if (cudaMalloc(&p, (size_t)std::max(s->n, 1) * sizeof(float4)) != cudaSuccess) {
+        if (device_malloc(s, &p, (size_t)std::max(s->n, 1) * sizeof(float4)) != cudaSuccess) {
             ok = false;
             return -1;
         }
@@ -206,7 +232,7 @@ int SubstepTape::snap1(const float *src)
 {
     if (used1 == (int)pool1.size()) {
         void *p = nullptr;
-        if (cudaMalloc(&p, (size_t)std::max(s->n, 1) * sizeof(float)) != cudaSuccess) {
+        if (device_malloc(s, &p, (size_t)std::max(s->n, 1) * sizeof(float)) != cudaSuccess) {
             ok = false;
             return -1;
         }
@@ -221,13 +247,16 @@ namespace {
 bool alloc_state(Tape &t, const bp_solver *s, StateBuf &b)
 {
     const int nb = s->rigid.num_bodies;
+    const size_t before = t.pool.bufs.size();
     b.X = t.pool.get<float4>(s->n);
     b.V = t.pool.get<float4>(s->n);
     b.orig = t.pool.get<int>(s->n);
     b.to_new = t.pool.get<int>(s->n);
     b.rot = t.pool.get<float4>(nb);
     b.cm = t.pool.get<float4>(nb);
-    return b.X && b.V && b.orig && b.to_new && b.rot && b.cm;
+    const bool ok = b.X && b.V && b.orig && b.to_new && b.rot && b.cm;
+    if (!ok) t.pool.give_back(before);
+    return ok;
 }
 
 void save_state(const bp_solver *s, const StateBuf &b)
@@ -266,7 +295,7 @@ void load_state(bp_solver *s, const StateBuf &c, const StateBuf &first)
 
 bool alloc_ctx(Tape &t, const bp_solver *s, SubCtx &c)
 {
-    const size_t n = (size_t)s->n;
+    const size_t n = (size_t)s->n, before = t.pool.bufs.size();
     c.Xs = t.pool.get<float4>(n);
     c.order = t.pool.get<int>(n);
     c.to_new = t.pool.get<int>(n);
@@ -274,7 +303,9 @@ bool alloc_ctx(Tape &t, const bp_solver *s, SubCtx &c)
     c.off = t.pool.get<int>(s->ncells + 1);
     c.mass = t.pool.get<float>(n);
     c.w = t.pool.get<float>(n);
-    return c.Xs && c.order && c.to_new && c.keys && c.off && c.mass && c.w;
+    const bool ok = c.Xs && c.order && c.to_new && c.keys && c.off && c.mass && c.w;
+    if (!ok) t.pool.give_back(before);
+    return ok;
 }
 
 // The solver's buffers that a substep leaves for its adjoint.
@@ -339,7 +370,7 @@ bool stage_on(const bp_params &p, int bit) { return (p.stage_mask & bit) != 0; }
 bp_status ensure_grads(Tape &t, const bp_solver *s)
 {
     if (t.grads_ready) return BP_OK;
-    const size_t n = (size_t)s->n;
+    const size_t n = (size_t)s->n, before = t.pool.bufs.size();
     const size_t m = (size_t)s->dist.num_edges, f = (size_t)s->wind.num_faces;
     t.gX = t.pool.get<float4>(n);
     t.gV = t.pool.get<float4>(n);
@@ -369,8 +400,10 @@ bp_status ensure_grads(Tape &t, const bp_solver *s)
     t.rhob = t.pool.get<float>(n);
     if (!(t.gX && t.gV && t.gVn && t.gP && t.gP2 && t.gXs && t.gVs && t.gPart && t.gW && t.gLam && t.G1 &&
           t.G2 && t.FG && t.FV && t.FW && t.g_wind && t.g_stiff && t.g_rest && t.contacts && t.gRho && t.etab &&
-          t.omb && t.ombo && t.nmb && t.GD && t.rhob))
+          t.omb && t.ombo && t.nmb && t.GD && t.rhob)) {
+        t.pool.give_back(before);
         return fail_with(BP_ERR_OUT_OF_MEMORY, "backward: gradient buffers");
+    }
     t.grads_ready = true;
     return BP_OK;
 }

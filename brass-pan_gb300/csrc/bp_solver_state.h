@@ -31,6 +31,10 @@ inline bp_status fail_with(bp_status st, const std::string &msg)
 using namespace bp;
 
 namespace bp {
+// cudaMalloc on behalf of s (nullptr: of no solver).  Where memory is short it
+// first gives back what s keeps of an ended recording, and a failure leaves no
+// error behind for a later call to report.
+cudaError_t device_malloc(bp_solver *s, void **p, size_t bytes);
 void destroy_tape(Tape *t);  // frees a recording (bp_backward.cu)
 void retire_tape(bp_solver *s);  // ends s->tape; its buffers and graphs wait in s->spare for the next recording
 
@@ -70,13 +74,14 @@ struct SubstepTape {
     int used4 = 0, used1 = 0;
     std::vector<TapeRec> recs;
     int vs_slot = -1;  // velocities after the reorder (wind reads them)
-    bool ok = true;    // false after a failed allocation
+    bool ok = true;    // false after a failed allocation, until the next run
     // where the substep's committed state goes (nullptr: back into the solver's buffers)
     float4 *next_X = nullptr, *next_V = nullptr;
     int *next_orig = nullptr;
     void reset()
     {
         used4 = used1 = 0;
+        ok = true;
         recs.clear();
         vs_slot = -1;
     }
@@ -205,7 +210,7 @@ struct bp_solver {
     {
         void *p = nullptr;
         const size_t bytes = count * sizeof(T) > 0 ? count * sizeof(T) : 16;
-        cudaError_t e = cudaMalloc(&p, bytes);
+        cudaError_t e = bp::device_malloc(this, &p, bytes);
         if (e != cudaSuccess)
             return bp::fail_with(BP_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         allocs.push_back(p);
@@ -272,7 +277,7 @@ struct StateSnapshot {
         for (size_t k = 0; k < bufs.size(); ++k) {
             if (k == copies.size()) {
                 void *p = nullptr;
-                if (cudaMalloc(&p, bufs[k].second) != cudaSuccess)
+                if (bp::device_malloc(s, &p, bufs[k].second) != cudaSuccess)
                     return bp::fail_with(BP_ERR_OUT_OF_MEMORY, "state snapshot");
                 copies.push_back(p);
             }
