@@ -181,7 +181,8 @@ void destroy_tape(Tape *t)
 // (128 x 128 flag, 10 frames, on the host while the GPU waits) and 4.8 of
 // 11.7 ms (65,536 particles of fluid, 3 frames).  Buffers beyond this many
 // bytes are given back at the end of the recording, as those of one that ran
-// out of memory are, and as every buffer is when the solver is destroyed.
+// out of memory are; the kept ones by an end without a recording, where memory
+// runs short (device_malloc) and with the solver.
 constexpr size_t kSpareTapeBytes = size_t(512) << 20;
 
 void retire_tape(bp_solver *s)
@@ -644,7 +645,12 @@ extern "C" bp_status bp_solver_tape_end(bp_solver *s)
 {
     if (!s) return fail_with(BP_ERR_INVALID_ARGUMENT, "solver is NULL");
     if (s->stream) cudaStreamSynchronize(s->stream);
-    retire_tape(s);
+    if (s->tape) {
+        retire_tape(s);
+    } else {
+        destroy_tape(s->spare);
+        s->spare = nullptr;
+    }
     return BP_OK;
 }
 

@@ -187,6 +187,8 @@ class ParticleSolver:
         abi.check(self.lib, self.lib.bp_solver_tape_begin(self.handle, checkpoint_every))
 
     def tape_end(self):
+        """Ends the recording.  The solver keeps up to 512 MiB of its device buffers
+        for the next one; a second call gives them back."""
         abi.check(self.lib, self.lib.bp_solver_tape_end(self.handle))
 
     def backward(self, grad_positions=None, grad_velocities=None) -> dict[str, np.ndarray]:

@@ -351,6 +351,9 @@ typedef struct bp_gradients {
 bp_status bp_solver_tape_begin(bp_solver *s, int32_t checkpoint_every);
 bp_status bp_solver_backward(bp_solver *s, const float *grad_positions, const float *grad_velocities,
                              bp_gradients *out);
+/* Ends the recording.  Up to 512 MiB of its device buffers, and its graphs, stay
+ * with the solver for the next recording; another call, without a recording
+ * open, gives them back (as bp_solver_destroy does). */
 bp_status bp_solver_tape_end(bp_solver *s);
 
 /* ---- Batched ensembles ----------------------------------------------------

@@ -10,7 +10,10 @@ import sys
 import textwrap
 from pathlib import Path
 
+import numpy as np
 import pytest
+
+from conftest import fluid_scene
 
 pytestmark = pytest.mark.gpu
 
@@ -125,3 +128,30 @@ def test_gradients_after_a_failed_allocation(bp, gpu, tmp_path, kind):
         print("failed", failed)
         """)
     assert "failed" in out
+
+
+def test_a_second_end_gives_the_kept_buffers_back(bp, gpu):
+    """An ended recording's buffers stay for the next one until tape_end() is
+    called without a recording, which a recording after it does not notice."""
+    torch, abi = gpu, bp.abi
+    scene = fluid_scene(bp, (32, 32, 32), seed=2, grid_dim=32, box=(4.0, 4.0, 4.0))
+    p = bp.make_params(scene, stage_mask=abi.BP_STAGE_FLUID | abi.BP_STAGE_PLANES | abi.BP_STAGE_XSPH)
+    s = bp.ParticleSolver(scene, p)
+    begin = s.snapshot()
+    weights = np.random.default_rng(1).normal(size=(scene.num_particles, 3)).astype(np.float32)
+    grads, free = [], []
+    for _ in range(2):
+        s.restore(begin)
+        s.tape_begin(10)
+        s.update(2, 1.0 / 60.0, 2)
+        grads.append(s.backward(weights, 0.1 * weights))
+        s.tape_end()
+        free.append(torch.cuda.mem_get_info()[0])
+        s.tape_end()
+        free.append(torch.cuda.mem_get_info()[0])
+    # the adjoint's 13 buffers of 16 bytes a particle are the least it holds
+    least = 13 * 16 * scene.num_particles
+    assert free[1] - free[0] >= least and free[3] - free[2] >= least, free
+    for k, v in grads[0].items():
+        np.testing.assert_array_equal(grads[1][k], v, err_msg=k)
+    s.close()
