@@ -146,9 +146,8 @@ static bool planes_confine(const bp_solver *s, int D, float cell)
 // scene late 12.4 -> 8.85 ms; 1,728 particles 0.45 -> 0.32 ms).  The lists
 // come from the split, unstaged recording walk.  neighbor_skin sets the skin;
 // with 0 it adapts (adapt_skin), up to the kWideSkin of h returned.
-static float largest_skin(const bp_solver *s)
+static float largest_skin(const bp_solver *s, const bp_params &p)
 {
-    const bp_params &p = s->prm;
     const int32_t other = BP_WALK_NO_SPLIT | BP_WALK_NO_LISTS | BP_WALK_NO_PLANES;
     if (!(p.walk_options & BP_WALK_NO_STAGING) || (p.walk_options & other) || p.scan_persistent ||
         !((p.stage_mask & BP_STAGE_FLUID) || ((p.stage_mask & BP_STAGE_PARTICLE_COLLISION) && s->has_solid)))
@@ -166,7 +165,7 @@ static float class_reach(const bp_solver *s)
     if (s->n <= (1 << 16) && 4 * (size_t)s->n <= s->ncells) return 0.f;
     if (!s->cls.perm || s->tape || (p.walk_options & BP_WALK_NO_ALIAS_CLASSES)) return 0.f;
     const float reach = (float)(s->cls_dmin - 2) * p.cell_size - p.kernel_radius - (0.02f + 1e-3f * p.kernel_radius) -
-                        largest_skin(s);  // the walk that records the substep lists reaches h + skin
+                        largest_skin(s, p);  // the walk that records the substep lists reaches h + skin
     return reach > 0.f ? reach : 0.f;
 }
 
@@ -231,7 +230,7 @@ SimConsts bp::make_consts(const bp_solver *s, float sdt)
     C.split = (p.walk_options & BP_WALK_NO_SPLIT) ? 0 : 1;
     C.scan_block = p.scan_block > 0 ? p.scan_block : 256;
     C.scan_persist = p.scan_persistent ? 1 : 0;
-    const float skin = largest_skin(s);
+    const float skin = largest_skin(s, p);
     if (skin > 0.f) {  // substep lists (enqueue_substep decides per launch)
         C.sl_cell = s->sl_cell;
         C.sl_pos = s->nl_pos;
@@ -361,11 +360,12 @@ void bp::clear_list_bits(bp_solver *s)
     cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), s->stream);
 }
 
-// The Verlet lists' buffers (1 KB a particle), for parameters that ask for
-// them; single scenes only.
+// The Verlet lists' buffers (1 KB a particle), for parameters whose fluid
+// passes read them (a skin asked of walks without substep lists); single scenes
+// only.
 static bp_status verlet_buffers(bp_solver *s, const bp_params &p)
 {
-    if (!(p.neighbor_skin > 0.f) || s->vl) return BP_OK;
+    if (!(p.neighbor_skin > 0.f) || largest_skin(s, p) > 0.f || !(p.stage_mask & BP_STAGE_FLUID) || s->vl) return BP_OK;
     const size_t N = (size_t)std::max(s->n, 1), D = (size_t)p.grid_dim;
     bp_status st;
     int *lists = nullptr;
@@ -427,7 +427,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         (st = s->alloc(&s->staging, 6 * N)) || (st = s->alloc(&s->nl_pos, N)) || (st = s->alloc(&s->sl_cell, N)) ||
         (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 3)) ||
         (st = s->alloc(&s->sl_bits, sl_bit_words(s))) ||
-        (st = s->alloc(&s->nl_stats, 5)) || (!batch && (st = verlet_buffers(s, *prm))))
+        (st = s->alloc(&s->nl_stats, 5)))
         return bail(st);
     {
         char *scratch = nullptr;
@@ -467,6 +467,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
         if (sc->group_ids) grp[i] = sc->group_ids[i];
     }
     s->has_solid = has_solid;
+    if (!batch && (st = verlet_buffers(s, *prm))) return bail(st);
     s->num_solids = 0;
     for (int i = 0; i < n; ++i) s->num_solids += sc->phases[i] > 0;
     if ((st = s->alloc(&s->tile_solid, (N + 255) / 256)) || (st = s->alloc(&s->solid_prefix, N + 1)) ||

@@ -24,13 +24,16 @@ SHIM = r"""
 #include <stddef.h>
 static long calls, fail_at;  /* the fail_at-th call from now fails; 0: none does */
 static size_t above;         /* calls for more bytes than this fail; 0: none does */
-void shim_arm(long at, size_t bytes) { calls = 0; fail_at = at; above = bytes; }
+static size_t total;         /* bytes asked for since */
+void shim_arm(long at, size_t bytes) { calls = 0; total = 0; fail_at = at; above = bytes; }
 long shim_calls(void) { return calls; }
+size_t shim_bytes(void) { return total; }
 int cudaMalloc(void **p, size_t bytes)
 {
     static int (*real)(void **, size_t);
     if (!real) real = (int (*)(void **, size_t))dlsym(dlopen("libcudart.so.13", RTLD_LAZY), "cudaMalloc");
     ++calls;
+    total += bytes;
     if (calls == fail_at || (above && bytes > above)) bytes = (size_t)1 << 50;
     return real(p, bytes);
 }
@@ -38,7 +41,7 @@ int cudaMalloc(void **p, size_t bytes)
 
 
 def run_child(tmp_path, body):
-    """Runs body (python, with bp, abi, np, scenes of conftest and arm(at, bytes)) under the shim."""
+    """Runs body (python, with bp, abi, np, scenes of conftest, shim and arm(at, above)) under the shim."""
     lib = tmp_path / "shim.so"
     (tmp_path / "shim.c").write_text(SHIM)
     subprocess.run(["gcc", "-shared", "-fPIC", "-O1", str(tmp_path / "shim.c"), "-o", str(lib), "-ldl"], check=True)
@@ -52,6 +55,7 @@ abi = bp.abi
 shim = ctypes.CDLL({str(lib)!r})
 shim.shim_arm.argtypes = [ctypes.c_long, ctypes.c_size_t]
 shim.shim_calls.restype = ctypes.c_long
+shim.shim_bytes.restype = ctypes.c_size_t
 arm = lambda at=0, above=0: shim.shim_arm(at, above)
 """
     code = textwrap.dedent(head) + textwrap.dedent(body)
