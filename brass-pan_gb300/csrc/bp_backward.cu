@@ -432,7 +432,7 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
     if (!(u.prm.walk_options & BP_WALK_NO_LISTS)) {
         C.nbr = s->nbr;
         C.nbr_count = s->nbr_count;  // the fluid adjoint's pass A leaves its lists for pass B
-        C.nbr_cap = kPostListCap;
+        C.nbr_cap = s->nbr_cap;
     }
     // One search for the stages that walk (k_adj_record_lists) where the update
     // itself takes its lists so and two of them read them: the density passes,

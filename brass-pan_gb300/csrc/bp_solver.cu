@@ -376,8 +376,8 @@ static bp_status verlet_buffers(bp_solver *s, const bp_params &p)
     return BP_OK;
 }
 
-static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, void *stream, const BatchSpec *batch,
-                               bp_solver **out)
+static bp_status create_solver_with(int nbr_cap, const bp_scene_desc *sc, const bp_params *prm, void *stream,
+                                    const BatchSpec *batch, bp_solver **out)
 {
     if (!out) return fail(BP_ERR_INVALID_ARGUMENT, "out is NULL");
     *out = nullptr;
@@ -397,6 +397,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
     };
     const int n = sc->num_particles;
     s->n = n;
+    s->nbr_cap = nbr_cap;
     s->prm = *prm;
     s->nplanes = sc->num_planes;
     for (int k = 0; k < s->nplanes; ++k)
@@ -473,7 +474,7 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
     if ((st = s->alloc(&s->tile_solid, (N + 255) / 256)) || (st = s->alloc(&s->solid_prefix, N + 1)) ||
         (st = s->alloc(&s->solid_pos, N + 1)) ||  // phases may change after creation: room for every particle
         (st = s->alloc(&s->solid_list, N)) || (st = s->alloc(&s->solid_totals, (N + 1023) / 1024)) ||
-        (st = s->alloc(&s->nbr, N * kPostListCap)) ||
+        (st = s->alloc(&s->nbr, N * s->nbr_cap)) ||
         (st = s->alloc(&s->walk_xyz, 4 * (((N + 3) & ~(size_t)3) + kPlanePad))) ||
         (st = s->alloc(&s->nbr_count, N)))
         return bail(st);
@@ -621,6 +622,17 @@ static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, vo
     BP_CUDA_BAIL(cudaDeviceSynchronize());
     *out = s;
     return BP_OK;
+}
+
+static bp_status create_solver(const bp_scene_desc *sc, const bp_params *prm, void *stream, const BatchSpec *batch,
+                               bp_solver **out)
+{
+    bp_status st = BP_OK;
+    for (const int cap : kListCaps) {
+        st = create_solver_with(cap, sc, prm, stream, batch, out);
+        if (st != BP_ERR_OUT_OF_MEMORY) break;
+    }
+    return st;
 }
 
 extern "C" bp_status bp_solver_create(const bp_scene_desc *sc, const bp_params *prm, void *stream, bp_solver **out)
@@ -933,7 +945,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     if (lists) {
         Cf.nbr = s->nbr;
         Cf.nbr_count = s->nbr_count;
-        Cf.nbr_cap = kPostListCap;
+        Cf.nbr_cap = s->nbr_cap;
         Cf.lm = s->lm;
     }
     if (walk_planes) {
@@ -1146,7 +1158,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         if (lists) {
             Cl.nbr = s->nbr;
             Cl.nbr_count = s->nbr_count;
-            Cl.nbr_cap = kPostListCap;
+            Cl.nbr_cap = s->nbr_cap;
         }
         if (post_planes) {
             Cl.walk_xyz = s->walk_xyz;
@@ -1174,7 +1186,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         if (lists) {
             Cx.nbr = s->nbr;
             Cx.nbr_count = post_lists ? s->nbr_count : nullptr;
-            Cx.nbr_cap = kPostListCap;
+            Cx.nbr_cap = s->nbr_cap;
         }
         if (post_lists) {
             Cx.cls_post = post_slots ? 1 : 0;

@@ -99,12 +99,17 @@ struct SubstepTape {
 // beyond the cap walk their cells, a warp each with the substep lists: 192 took
 // 44 ms a frame 50 frames into the mixed scene (80 % of the reads past the cap)
 // and 17.5 ms 200 frames in, 384 takes 21.7 and 15.4 ms.  Only records in use
-// are touched.
+// are touched.  A solver whose buffers do not fit with lists of 384 (1.5 KB a
+// particle) is created with the next of kListCaps, with the same results: 192
+// entries, and 144, with which a batch takes what lists of 192 took alone (24
+// dam breaks, 850,986 particles, 120 frames: 831 ms with 384, 888 with 192).
 #ifndef BP_POST_LIST_CAP
 #define BP_POST_LIST_CAP 384
 #endif
 constexpr int kPostListCap = BP_POST_LIST_CAP;
-static_assert(kPostListCap % 4 == 0, "lists are stored as records of four entries");
+constexpr int kListCaps[] = {kPostListCap, 192, 144};
+static_assert(kPostListCap % 4 == 0 && kListCaps[1] % 4 == 0 && kListCaps[2] % 4 == 0,
+              "lists are stored as records of four entries");
 
 // Entries of a Verlet list (candidates within h + skin): about 1.3x the
 // neighbours within h at a skin of 0.1 h (particles beyond it walk their cells).
@@ -148,7 +153,8 @@ struct bp_solver {
     float4 *hash_pos = nullptr;
     unsigned *contact_reach = nullptr;
     int *solid_walk = nullptr;
-    int *nbr = nullptr, *nbr_count = nullptr;  // post-pass neighbour lists [kPostListCap][N], counts
+    int *nbr = nullptr, *nbr_count = nullptr;  // neighbour lists [nbr_cap][N], counts
+    int nbr_cap = kPostListCap;
     float2 *lm = nullptr;  // (lambda, mass) per sorted particle (SimConsts::lm)
     float *walk_xyz = nullptr;  // walk planes (SimConsts::walk_xyz): 4 planes of walk_stride floats
     int walk_stride = 0;
