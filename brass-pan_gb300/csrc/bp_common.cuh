@@ -193,7 +193,8 @@ struct SimConsts {
     float *sl_skin;
     float sl_fixed;   // > 0: this skin instead
     int sl_pass;      // parity of this list pass
-    int sl_adapt;     // this pass is the substep's last over the lists
+    int sl_last;      // this pass is the substep's last over the lists: what it moves is not tracked
+    int sl_adapt;     // and it adapts the skin
     int sl_fluid;     // the lists reach h + skin (the fluid passes read them)
     // Contact partners of slot t (nullptr: off), the candidates within two radii
     // + skin when the lists were recorded: cl_count[t] of them (-1: more than
@@ -476,6 +477,7 @@ __device__ __forceinline__ bool near_stored_cell(const SimConsts &C, int i, int3
 __device__ __forceinline__ void track_displacement(const SimConsts &C, int i, float3 p, bool active)
 {
     if (C.sl_pos) {
+        if (C.sl_last) return;  // nobody reads the flags any more (and adapt_skin may be writing the skin)
         const float d2 = len2(p - f3(C.sl_pos[i])), q2 = substep_quarter2(C);
         if (!(d2 <= q2)) flag_moved(C, i, d2 <= 4.0f * q2 ? 1 : (d2 <= 9.0f * q2 ? 2 : 3));  // NaN counts as moved
         return;

@@ -980,9 +980,12 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     bool planes_done = fuse_first_planes;
     bool committed = false;
     int list_passes = 0;  // over the substep lists
+    const SimConsts *Cw = &Cpost;  // of the stages that only move particles: they track them up to the last such pass
     auto next_list_pass = [&](SimConsts &K, bool last) {
         K.sl_pass = list_passes++ & 1;
+        K.sl_last = last ? 1 : 0;
         K.sl_adapt = last && C.sl_fixed == 0.f;
+        if (last) Cw = &Cpre;
     };
     for (int it = 0; it < iterations; ++it) {
         const SimConsts &Cit = it == 0 ? Cpre : Cpost;  // stages before lambda
@@ -1099,37 +1102,37 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
                 planes_done = true;
             }
             float4 *out = stage_out();
-            launch_distance_step(st, Cpost, ds, cur, out, L);
+            launch_distance_step(st, *Cw, ds, cur, out, L);
             stage_done(out);
             continue;
         }
         if (distance) {
             if (tape) tape->push(TS_DISTANCE, slot);
             in_place();
-            launch_distance(st, Cpost, s->dist, cur, s->w, s->to_new, s->err, L);
+            launch_distance(st, *Cw, s->dist, cur, s->w, s->to_new, s->err, L);
         }
         if (bending) {  // PS:956-969
             if (tape) tape->push(TS_BENDING, slot);
             in_place();
             BendingArgs ba = s->bend;
             ba.stiffness = s->prm.bending_stiffness;
-            launch_bending(st, Cpost, ba, cur, s->w, s->to_new, L);
+            launch_bending(st, *Cw, ba, cur, s->w, s->to_new, L);
         }
         if (rigid) {
             if (tape) tape->push(TS_SHAPE, slot);
             in_place();
-            launch_shape_matching(st, Cpost, s->rigid, cur, s->to_new, L);
+            launch_shape_matching(st, *Cw, s->rigid, cur, s->to_new, L);
             if (tape) tape->recs.back().aux = tape->snap4(s->rigid.rot, (size_t)s->rigid.num_bodies);
         }
         if (immov) {
             if (tape) tape->push(TS_IMMOVABLE, slot);
             in_place();
-            launch_immovable(st, Cpost, s->nimm, s->imm, s->to_new, s->Xs, cur, L);
+            launch_immovable(st, *Cw, s->nimm, s->imm, s->to_new, s->Xs, cur, L);
         }
     }
     if (!committed) {
         if (tape) tape->push(TS_COMMIT, slot);
-        launch_commit(st, Cpost, cur, s->Xs, s->Vs, s->orig_s, s->Xc, s->Vc, s->orig_c, L);
+        launch_commit(st, *Cw, cur, s->Xs, s->Vs, s->orig_s, s->Xc, s->Vc, s->orig_c, L);
     }
     s->Pcur = cur;
 
