@@ -1782,24 +1782,27 @@ void launch_post_c(cudaStream_t st, const SimConsts &C, const float4 *P, const f
 }
 
 // Same count on caller buffers in the reference's start/end format.  The three
-// cells of a column that do not wrap around the table are one run of sorted
-// positions (their keys are consecutive), from the first occupied one's start
-// to the last one's end: two loads find it where both ends are occupied, and
-// its positions are read in order, the twelve floats of four at a time.  Bound
-// by the latency and number of those loads (1,000,003 points, 128^3 table: 87
-// us; cell by cell, 27 pairs of loads a point, 154 us; three 16-byte loads for
-// four positions from the boundary below the run, 97 us).
+// cells of a column are one run of sorted positions (their keys are
+// consecutive), from the first occupied one's start to the last one's end: two
+// loads find it where both ends are occupied, and its positions are read in
+// order, Ahead of them (3 floats each) at a time.  Where the column wraps
+// around the table, two of its cells are a run and the third follows alone.
+// Bound by the latency and number of those loads (1,000,003 points, 128^3
+// table: 92 us; cell by cell, 27 pairs of loads a point, 153 us; three 16-byte
+// loads for four positions from the boundary below the run, 97 us).
+template <int Ahead>
 __device__ __forceinline__ int count_run(int b, int e, const float *__restrict__ pos3, float3 pi, float h2)
 {
     int cnt = 0;
-    for (; b + 4 <= e; b += 4) {
-        float v[12];
+    for (; b + Ahead <= e; b += Ahead) {
+        float v[3 * Ahead];
 #pragma unroll
-        for (int k = 0; k < 12; ++k) v[k] = __ldg(pos3 + 3 * (size_t)b + k);
+        for (int k = 0; k < 3 * Ahead; ++k) v[k] = __ldg(pos3 + 3 * (size_t)b + k);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < Ahead; ++k)
             cnt += len2(pi - make_float3(v[3 * k], v[3 * k + 1], v[3 * k + 2])) <= h2 ? 1 : 0;
     }
+    if constexpr (Ahead > 4) return cnt + count_run<4>(b, e, pos3, pi, h2);
     for (; b < e; ++b) {
         const float *p = pos3 + 3 * (size_t)b;
         cnt += len2(pi - make_float3(__ldg(p), __ldg(p + 1), __ldg(p + 2))) <= h2 ? 1 : 0;
@@ -1807,6 +1810,26 @@ __device__ __forceinline__ int count_run(int b, int e, const float *__restrict__
     return cnt;
 }
 
+// The `cells` consecutive cells from a on (2 or 3).
+template <int Ahead>
+__device__ __forceinline__ int count_cells(int a, int cells, const int *__restrict__ start,
+                                           const int *__restrict__ end, const float *__restrict__ pos3, float3 pi,
+                                           float h2)
+{
+    const int last = a + cells - 1;
+    int b = __ldg(start + a), e = __ldg(end + last);
+    if (b < 0) {
+        b = __ldg(start + a + 1);
+        if (b < 0) b = __ldg(start + last);
+    }
+    if (e < 0) {
+        e = __ldg(end + last - 1);
+        if (e < 0) e = __ldg(end + a);
+    }
+    return b >= 0 ? count_run<Ahead>(b, e, pos3, pi, h2) : 0;
+}
+
+template <int Ahead>
 __global__ void __launch_bounds__(128) k_neighbor_counts_f3(int n, const float *__restrict__ pos3, float cell, int D,
                                                             float h2, const int *__restrict__ start,
                                                             const int *__restrict__ end, int *__restrict__ counts)
@@ -1818,36 +1841,39 @@ __global__ void __launch_bounds__(128) k_neighbor_counts_f3(int n, const float *
     const unsigned m = (unsigned)D - 1u;
     const int cx = cell_coord(pi.x, cell), cy = cell_coord(pi.y, cell), cz = cell_coord(pi.z, cell);
     const unsigned z = (unsigned)cz & m;
+    const bool wraps = z == 0u || z == m;
     int cnt = 0;
-    for (int col = 0; col < 9; ++col) {
-        const int x = cx + col / 3 - 1, y = cy + col % 3 - 1;
-        if (z != 0u && z != m) {
-            const int a = cell_addr(x, y, cz - 1, D, m);
-            int b = __ldg(start + a), e = __ldg(end + a + 2);
-            if (b < 0) {
-                b = __ldg(start + a + 1);
-                if (b < 0) b = __ldg(start + a + 2);
-            }
-            if (e < 0) {
-                e = __ldg(end + a + 1);
-                if (e < 0) e = __ldg(end + a);
-            }
-            if (b >= 0) cnt += count_run(b, e, pos3, pi, h2);
-        } else {
-            for (int dz = -1; dz <= 1; ++dz) {
-                const int a = cell_addr(x, y, cz + dz, D, m);
-                cnt += count_run(__ldg(start + a), __ldg(end + a), pos3, pi, h2);
-            }
+    // a loop of its own for most warps; not worth its registers with the longer trips (1556 -> 1613 us below)
+    if (Ahead == 4 && !__any_sync(__activemask(), wraps)) {
+        for (int col = 0; col < 9; ++col)
+            cnt += count_cells<Ahead>(cell_addr(cx + col / 3 - 1, cy + col % 3 - 1, cz - 1, D, m), 3, start, end, pos3,
+                                      pi, h2);
+    } else {  // a warp takes both kinds of column together: each lane its run, then those that wrap the cell left
+        const int lo = z == 0u ? 0 : (int)z - 1, alone = z == 0u ? (int)m : 0;
+        for (int col = 0; col < 9; ++col) {
+            const int base = cell_addr(cx + col / 3 - 1, cy + col % 3 - 1, 0, D, m);
+            cnt += count_cells<Ahead>(base + lo, wraps ? 2 : 3, start, end, pos3, pi, h2);
+            if (wraps) cnt += count_run<Ahead>(__ldg(start + base + alone), __ldg(end + base + alone), pos3, pi, h2);
         }
     }
     counts[i] = cnt;
 }
 
+// Eight positions at a time where cells hold six points on average, and runs
+// twice as many as a trip takes (2,000,000 points, a call: 32^3 table, 61 a
+// cell, 1637 -> 1556 us, 64^3, 7.6 a cell, 360 -> 352; 128^3, 1.0 a cell, 173
+// -> 183; 1,000,003 on 64^3, 3.8 a cell, 106 -> 112).
+constexpr long long kDenseCell = 6;
+
 void launch_neighbor_counts_f3(cudaStream_t st, int n, const float *pos3, float cell, int D, float h,
                                const int *start, const int *end, int *counts)
 {
     if (n <= 0) return;
-    k_neighbor_counts_f3<<<(n + 127) / 128, 128, 0, st>>>(n, pos3, cell, D, h * h, start, end, counts);
+    const int grid = (n + 127) / 128;
+    if (n >= kDenseCell * D * D * D)
+        k_neighbor_counts_f3<8><<<grid, 128, 0, st>>>(n, pos3, cell, D, h * h, start, end, counts);
+    else
+        k_neighbor_counts_f3<4><<<grid, 128, 0, st>>>(n, pos3, cell, D, h * h, start, end, counts);
 }
 
 }  // namespace bp
