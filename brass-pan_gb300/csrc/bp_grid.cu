@@ -320,10 +320,10 @@ void launch_hash_state(cudaStream_t st, const SimConsts &C, const float4 *X, con
 // CTAs: the same 9-bit digits, tiles, warp segments and ranks as the
 // hash / upsweep / scan / downsweep chain, with the tiles' digit counts
 // exchanged through distributed shared memory and cluster barriers in place of
-// the launches between.  Such sorts are bound by those launches: a substep's
-// hash and sort on a 64^3 table took 6 of them, 33 us and the gaps between
-// them for 32,768 particles, now one of 22 us (1,728 particles: 9 us; 128 x
-// 128 flag, a frame 219 -> 188 us).  Above it a cluster's 8 SMs are too few.
+// the launches between.  Such sorts are bound by those launches: hash and sort
+// of 32,768 keys on a 64^3 table take 6 of them, and a build of the grid in a
+// graph 34.1 us, in one launch 26.7 (8,192 keys 31.2 and 12.8; 128 x 128 flag, a
+// frame 219 -> 188 us).  With more keys a cluster's 8 SMs are too few.
 constexpr int kClusterSortCtas = 8;  // the portable cluster size
 
 template <int Items, class KeyOf>
@@ -466,6 +466,14 @@ static void launch_cluster(void (*kernel)(K...), int n, int items, cudaStream_t 
 // its keys one after another (16,384 particles: 8 keys a thread in 4 CTAs 197
 // us a flag frame, 4 keys in 8 CTAs 188 us).
 constexpr int kClusterSortMax = kClusterSortCtas * kSortThreads * 16;
+// A solver's sort of at most two passes goes back to the chain above 8 keys a
+// thread: in its graph 16 cost more than the launches (fluid, a frame in one
+// launch and in the chain: 64^3 table, 32,768 particles 316 and 331 us, 35,937
+// 342 and 339, 64,000 372 and 367; 16^3, 35,937 425 and 422; with three passes,
+// 128^3, 35,937 368 and 373, 64,000 394 and 400).  A build on a caller's stream
+// stays at 16, as the host's launches bound its chain (50,000 points, 32^3 47.1
+// and 48.3 us, 64^3 49.1 and 49.2, 128^3 53.3 and 65.5).
+constexpr int kClusterSortTwoPasses = kClusterSortMax / 2;
 template <class F>
 static void with_cluster_items(int n, F &&f)
 {
@@ -481,12 +489,12 @@ void hash_sort_state(cudaStream_t st, const SimConsts &C, int dim, const float4 
                      int *keys_out, int *vals_out, const SortScratch &s, LaunchLog *L)
 {
     if (C.n <= 0) return;
-    if (C.n > kClusterSortMax) {
+    const int passes = sort_passes(dim);
+    if (C.n > (passes > 2 ? kClusterSortMax : kClusterSortTwoPasses)) {
         launch_hash_state(st, C, X, V, keys, s.hist, L);
         radix_sort_pairs(st, C.n, dim, keys, nullptr, keys_out, vals_out, s, true, L);
         return;
     }
-    const int passes = sort_passes(dim);
     with_cluster_items(C.n, [&](auto items) {
         launch_cluster(k_sort_state<items.value>, C.n, items.value, st, C, X, V, passes, keys, keys_out, vals_out, s);
     });
