@@ -185,14 +185,25 @@ struct SimConsts {
     // [0], [1]: queue lengths, by the parity of the pass (a list pass clears the
     // other one); [kSlMoved]; [kSlDisplaced]: particles that the last list pass
     // of a substep queued because something near them moved, [kSlWalks]: those
-    // of the passes before it
+    // of the fluid passes before it, [kSlContactWalks]: of the contact passes;
+    // [kSlWalkMode]: substeps left in walk mode; [kSlPairs], [kSlEntries]: a
+    // sample of the recorded entries, those within h and all
     int *sl_count;
     // [0] the skin in use, as a fraction of h (a radius set later keeps it within
     // kWideSkin), adapted after each substep (adapt_skin), [1] the last that was
-    // too small, [2] such walks a particle of the last substeps
+    // too small, [2] such walks a particle of the last substeps, [4] of their
+    // fluid passes; [3] entries recorded for a pair within h, over (1 + skin)^3
     float *sl_skin;
     float sl_fixed;   // > 0: this skin instead
     int sl_pass;      // parity of this list pass
+    // Walk mode (sl_may_walk: the solver's substeps may take it; sl_count[
+    // kSlWalkMode] > 0: this one does): where the lists would not pay, the fluid
+    // passes walk for every particle, as without substep lists.  Decided after
+    // each substep from the passes' costs (choose_mode).  sl_planes: where the
+    // position pass leaves the walk planes of the next walks (nullptr: nowhere).
+    int sl_may_walk;
+    float *sl_planes;
+    float sl_read_cost, sl_walk_cost;
     int sl_last;      // this pass is the substep's last over the lists: what it moves is not tracked
     int sl_adapt;     // and it adapts the skin
     int sl_fluid;     // the lists reach h + skin (the fluid passes read them)
@@ -206,7 +217,8 @@ struct SimConsts {
 };
 constexpr int kContactCap = 32;
 constexpr int kSlLevels = 3;
-constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlWalks = 4, kSlCounts = 5;
+constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlWalks = 4, kSlContactWalks = 5, kSlWalkMode = 6, kSlPairs = 7,
+              kSlEntries = 8, kSlCounts = 9;
 // Bounds of the adapted skin and where it starts, as fractions of h: up to
 // kMaxSkin as a rule, up to kWideSkin where walks go on at that (adapt_skin).
 constexpr float kMinSkin = 0.02f, kMaxSkin = 0.1f, kWideSkin = 0.2f, kStartSkin = 0.09f;
@@ -217,6 +229,12 @@ __device__ __forceinline__ float substep_skin(const SimConsts &C)
 {
     return C.sl_fixed > 0.f ? C.sl_fixed : __fmul_rn(C.h, __ldg(C.sl_skin));
 }
+__device__ __forceinline__ bool walk_mode(const SimConsts &C)
+{
+    return C.sl_may_walk && __ldg(C.sl_count + kSlWalkMode) != 0;
+}
+// The last substep in walk mode tracks displacements, to find whether lists would pay again.
+__device__ __forceinline__ bool walk_probe(const SimConsts &C) { return __ldg(C.sl_count + kSlWalkMode) == 1; }
 // The square of a quarter of the skin, less what the rounding of the distance
 // tests may take (k quarters: k * k times it).
 __device__ __forceinline__ float substep_quarter2(const SimConsts &C)
@@ -248,6 +266,17 @@ __device__ __forceinline__ int walk_planes_order(const SimConsts &C)
     if (!C.cls_perm) return 1;
     const int m = __ldg(C.cls_moved);
     return m == 0 ? 2 : (m == 1 ? 1 : 0);
+}
+
+// Writes particle p's x, y, z and phase bits to slot q of the walk planes
+// (SimConsts::walk_xyz).
+__device__ __forceinline__ void put_planes(float *planes, int stride, int q, float4 p)
+{
+    const size_t st = (size_t)stride;
+    planes[q] = p.x;
+    planes[st + q] = p.y;
+    planes[2 * st + q] = p.z;
+    planes[3 * st + q] = p.w;
 }
 
 // Class (0..7) of real cell c on a table of D cells per axis (D a power of two).
@@ -477,6 +506,7 @@ __device__ __forceinline__ bool near_stored_cell(const SimConsts &C, int i, int3
 __device__ __forceinline__ void track_displacement(const SimConsts &C, int i, float3 p, bool active)
 {
     if (C.sl_pos) {
+        if (walk_mode(C) && !walk_probe(C) && !C.cl_list) return;  // contacts read their lists in any mode
         if (C.sl_last) return;  // nobody reads the flags any more (and adapt_skin may be writing the skin)
         const float d2 = len2(p - f3(C.sl_pos[i])), q2 = substep_quarter2(C);
         if (!(d2 <= q2)) flag_moved(C, i, d2 <= 4.0f * q2 ? 1 : (d2 <= 9.0f * q2 ? 2 : 3));  // NaN counts as moved

@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(256) k_contacts_lists(SimConsts C, const float
     const int addr = cell_addr(c.x, c.y, c.z, v.D, v.mask);
     const bool alone = phi < 0 && C.cl_near && !((__ldg(C.cl_near + (addr >> 6)) >> (addr & 63)) & 1ull);
     const int cnt = alone ? 0 : __ldg(C.cl_count + t);
-    if (!alone && !reads_substep_list(C, t, i, xip, c, v, cnt >= 0)) return;
+    if (!alone && !reads_substep_list(C, t, i, xip, c, v, cnt >= 0, kSlContactWalks)) return;
     Contacts s{make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), 0};
     if (cnt > 0) {
         const float3 xi = f3(Xs[i]);

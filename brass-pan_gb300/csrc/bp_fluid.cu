@@ -332,53 +332,22 @@ __device__ __forceinline__ void record_contacts(const SimConsts &C, const float4
     C.cl_count[t] = n <= kContactCap ? n : -1;
 }
 
-// The lambda pass over the substep lists: the density (and, in textbook mode,
-// the denominator) of k_lambda, from the same pairs in the same order.
-// What bounds it: a list read is latency-bound on its gathers, like k_deltap;
-// the recording walk is issue-bound, like k_lambda.
-template <ListPass Pass>
-__device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const float4 *__restrict__ P,
-                                                    const float *__restrict__ mass, const int *__restrict__ off,
-                                                    float *__restrict__ lam, float *__restrict__ rho, int t)
+// The density (and, in textbook mode, the denominator) of fluid particle i of
+// slot t over its list (packed: what nbr_count holds), as k_lambda sums it over
+// the same pairs in the same order.  ReadOnly: the calling thread did not write
+// the list.  pairs (textbook mode): grows by the entries within h.
+template <bool ReadOnly>
+__device__ __forceinline__ void lambda_over_list(const SimConsts &C, const float4 *__restrict__ P,
+                                                 const float *__restrict__ mass, float *__restrict__ lam,
+                                                 float *__restrict__ rho, bool slots, int i, int t, float4 pi4, int sc,
+                                                 int3 c, const GridView &v, int packed, int &pairs)
 {
-    const bool slots = classes_on(C);
-    const int i = slots ? __ldg(C.cls_perm + t) : t;
-    const float4 pi4 = slots ? C.cls_pos[t] : P[i];
     const float3 pi = f3(pi4);
-    const bool solid = phase_of(pi4) > 0;
-    if (Pass == kRecordLists) {
-        C.sl_pos[i] = pi4;
-        if (solid && C.sl_fluid) record_solid(C, slots, i, t, mass, lam);
-    }
-    // textbook mode: no pass but the contacts moves a solid by its neighbours
-    if (solid && C.textbook && !(Pass == kRecordLists && C.cl_list)) return;
-    const int sc = scene_index(C, i);
-    const GridView v = grid_view(C, sc, off);
-    const int3 c = cell_of(pi, C);
-    int packed;
-    if (Pass == kReadLists) {
-        if (!reads_substep_list(C, t, i, pi, c, v) || solid) return;
-        packed = __ldg(C.nbr_count + t);
-    } else {
-        const float skin = substep_skin(C), touch = 2.0f * C.radius + skin;
-        const float reach = fmaxf(C.sl_fluid ? C.h + skin : 0.f, C.cl_list ? touch : 0.f);
-        packed = record_substep_list(C, P, slots, t, i, pi, c, __fmul_rn(reach, reach), v);
-        const bool fits = packed >= 0;
-        if (C.cl_list) record_contacts(C, P, slots, t, i, pi4, c, v, packed, __fmul_rn(touch, touch));
-        // the neighbours within h alone may still fit; later passes then walk
-        if (!fits && C.sl_fluid) packed = record_substep_list(C, P, slots, t, i, pi, c, C.h2, v);
-        C.nbr_count[t] = packed;
-        C.sl_cell[t] = (fits && near_stored_cell(C, i, c, v)) ? v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask) : kListNone;
-        if (!C.sl_fluid) return;
-    }
-    if (solid) return;
     const int cnt = packed & 0xffff, self = packed >> 16;
     const float4 *__restrict__ src = slots ? C.cls_pos : P;
     const float *__restrict__ ms = slots ? C.cls_mass : mass;
     const float rho0 = rest_density(C, sc);
     float density = 0.f, den = C.lambda_den;
-    // the records were written by the calling thread, except in a reading pass
-    constexpr bool kReadOnly = Pass == kReadLists;
     auto fetch = [&](int j) { return __ldg(ms + j); };
     if (!C.textbook) {
         auto add = [&](float mj, float4 pj, float d2) {
@@ -395,7 +364,7 @@ __device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const fl
             const bool ascending = self != kNoOwnEntry && inner(c.x) && inner(c.y) && inner(c.z);
             int e = ascending ? (self & ~3) : 0;
             const int first = e;
-            for_each_padded<kReadOnly>(C.nbr, C.n, t, cnt, src, fetch, [&](int j, float4 pj, float mj) {
+            for_each_padded<ReadOnly>(C.nbr, C.n, t, cnt, src, fetch, [&](int j, float4 pj, float mj) {
                 const float d2 = len2(pi - f3(pj));
                 bool take = d2 <= C.h2;
                 if (ascending) take = take && (unsigned)(e - self) < (unsigned)(cnt - self);
@@ -426,7 +395,10 @@ __device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const fl
         };
         if (packed >= 0) {
             int e = 0;
-            for_each_padded<kReadOnly>(C.nbr, C.n, t, cnt, src, fetch, [&](int, float4 pj, float mj) {
+            for_each_padded<ReadOnly>(C.nbr, C.n, t, cnt, src, fetch, [&](int, float4 pj, float mj) {
+                // (counted here, the terms' distances are free of the branch: 85.8 ->
+                // 79.6 us a reading pass of 829,440 particles)
+                pairs += len2(pi - f3(pj)) <= C.h2 ? 1 : 0;
                 if (e++ < cnt) term(mj, pj);
             });
         } else {
@@ -440,7 +412,70 @@ __device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const fl
     finish_lambda(C, slots, i, t, density, rho0, den, mass, lam, rho);
 }
 
-template <ListPass Pass>
+// The lambda pass over the substep lists: the density (and, in textbook mode,
+// the denominator) of k_lambda, from the same pairs in the same order.
+// What bounds it: a list read is latency-bound on its gathers, like k_deltap;
+// the recording walk is issue-bound, like k_lambda.
+// Walks: the substeps may be in walk mode; the recording pass then counts, over
+// every kSampleBlocks-th CTA, the entries it sums over and the pairs among them
+// (choose_mode).  Instances of their own: the mode costs the reading one 4 %.
+constexpr int kSampleBlocks = 64;
+template <ListPass Pass, bool Walks>
+__device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const float4 *__restrict__ P,
+                                                    const float *__restrict__ mass, const int *__restrict__ off,
+                                                    float *__restrict__ lam, float *__restrict__ rho, int t)
+{
+    const bool walking = Walks && walk_mode(C);  // loaded along with the particle
+    const bool slots = classes_on(C);
+    const int i = slots ? __ldg(C.cls_perm + t) : t;
+    const float4 pi4 = slots ? C.cls_pos[t] : P[i];
+    const float3 pi = f3(pi4);
+    const bool solid = phase_of(pi4) > 0;
+    if (Pass == kRecordLists) {
+        C.sl_pos[i] = pi4;
+        if (solid && C.sl_fluid) record_solid(C, slots, i, t, mass, lam);
+    }
+    // textbook mode: no pass but the contacts moves a solid by its neighbours
+    if (solid && C.textbook && !(Pass == kRecordLists && C.cl_list)) return;
+    const int sc = scene_index(C, i);
+    const GridView v = grid_view(C, sc, off);
+    const int3 c = cell_of(pi, C);
+    int packed;
+    if (Pass == kReadLists && walking) {
+        note_substep_list(C, t, i, pi, c, v);
+        packed = record_substep_list(C, P, slots, t, i, pi, c, C.h2, v);
+        C.nbr_count[t] = packed;
+    } else if (Pass == kReadLists) {
+        if (!reads_substep_list(C, t, i, pi, c, v) || solid) return;
+        packed = __ldg(C.nbr_count + t);
+    } else {
+        const float skin = substep_skin(C), touch = 2.0f * C.radius + skin;
+        const float reach = fmaxf(C.sl_fluid ? (walking ? C.h : C.h + skin) : 0.f, C.cl_list ? touch : 0.f);
+        packed = record_substep_list(C, P, slots, t, i, pi, c, __fmul_rn(reach, reach), v);
+        const bool fits = packed >= 0;
+        if (C.cl_list) record_contacts(C, P, slots, t, i, pi4, c, v, packed, __fmul_rn(touch, touch));
+        // the neighbours within h alone may still fit; later passes then walk
+        if (!fits && C.sl_fluid) packed = record_substep_list(C, P, slots, t, i, pi, c, C.h2, v);
+        C.nbr_count[t] = packed;
+        C.sl_cell[t] = (fits && near_stored_cell(C, i, c, v)) ? v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask) : kListNone;
+        if (!C.sl_fluid) return;
+    }
+    if (solid) return;
+    int pairs = 0;
+    // a pass that may walk reads its lists past the read-only path
+    lambda_over_list<Pass == kReadLists && !Walks>(C, P, mass, lam, rho, slots, i, t, pi4, sc, c, v, packed, pairs);
+    if (Pass == kRecordLists && Walks && blockIdx.x % kSampleBlocks == 0 && packed >= 0) {
+        const unsigned m = __activemask();
+        pairs = __reduce_add_sync(m, pairs);
+        const int entries = __reduce_add_sync(m, packed & 0xffff);
+        if ((threadIdx.x & 31) == __ffs(m) - 1) {
+            atomicAdd(C.sl_count + kSlPairs, pairs);
+            atomicAdd(C.sl_count + kSlEntries, entries);
+        }
+    }
+}
+
+template <ListPass Pass, bool Walks>
 __global__ void __launch_bounds__(kScanThreads, BP_SCAN_MIN_BLOCKS) k_lambda_lists(
     SimConsts C, const float4 *__restrict__ P, const float *__restrict__ mass, const int *__restrict__ off,
     float *__restrict__ lam, float *__restrict__ rho)
@@ -450,11 +485,11 @@ __global__ void __launch_bounds__(kScanThreads, BP_SCAN_MIN_BLOCKS) k_lambda_lis
         C.sl_count[C.sl_pass ^ 1] = 0;  // the next pass's queue
         if (Pass == kRecordLists) {
             C.sl_count[C.sl_pass] = 0;
-            C.sl_count[kSlDisplaced] = C.sl_count[kSlWalks] = 0;
+            C.sl_count[kSlDisplaced] = C.sl_count[kSlWalks] = C.sl_count[kSlContactWalks] = 0;
             C.sl_count[kSlMoved] = C.cls_perm ? *C.cls_moved : 0;
         }
     }
-    if (t < C.n) lambda_substep_list<Pass>(C, P, mass, off, lam, rho, t);
+    if (t < C.n) lambda_substep_list<Pass, Walks>(C, P, mass, off, lam, rho, t);
 }
 
 // The queued particles' lambda pass, a warp per particle: walks the
@@ -540,6 +575,7 @@ __device__ __forceinline__ void finish_deltap(const SimConsts &C, const DeltaArg
         a.orig_c[k] = a.orig_s[k];
     }
     a.Pout[k] = make_float4(p.x, p.y, p.z, pk4.w);
+    if (C.sl_planes && walk_mode(C)) put_planes(C.sl_planes, C.walk_stride, k, make_float4(p.x, p.y, p.z, pk4.w));
     track_displacement(C, k, p, true);
 }
 
@@ -951,8 +987,13 @@ __device__ __forceinline__ void k_post_c_tile(
     const float3 pi = f3(pi4), vi = f3(vi4);
     const GridView gv = grid_view(C, scene_index(C, i), off);
     if constexpr (First) {
-        if (!reads_substep_list(C, t, i, pi, cell_of(pi, C), gv)) return;
-        cnt = __ldg(C.nbr_count + t) & 0xffff;
+        if (walk_mode(C)) {
+            note_substep_list(C, t, i, pi, cell_of(pi, C), gv);
+            cnt = kWalkCells;
+        } else {
+            if (!reads_substep_list(C, t, i, pi, cell_of(pi, C), gv)) return;
+            cnt = __ldg(C.nbr_count + t) & 0xffff;
+        }
     }
     float3 vn = make_float3(0.f, 0.f, 0.f);
     auto body_at = [&](const float4 *__restrict__ Vp, const float *__restrict__ mp, const float *__restrict__ rp,
@@ -986,7 +1027,7 @@ __device__ __forceinline__ void k_post_c_tile(
         for_each_in_list(C.nbr, C.n, t, cnt, P, [&](int j, float4 pj4) {
             if (keep(j, pj4, len2(pi - f3(pj4)))) body(j, pj4);
         });
-    } else if (C.nbr && !C.nbr_count) {
+    } else if (C.nbr && (First || !C.nbr_count)) {
         // no pass A before it: record the walk's pairs, then sum over them
         ListWriter list(C.nbr, C.nbr_cap, C.n, t);
         walk_neighbors<Split>(i, pi, 0, P, gv, C, Stage ? &S : nullptr, g, test, [&](int j, float4) { list.push(j); });
@@ -1061,6 +1102,10 @@ __global__ void __launch_bounds__(kScanThreads, BP_POSTBC_MIN_BLOCKS) k_post_a_l
     const int phi = phase_of(pi4);
     if (phi >= 0) return;
     const float3 pi = f3(pi4);
+    if (walk_mode(C)) {  // k_post_a_walks follows
+        note_substep_list(C, t, i, pi, cell_of(pi, C), grid_view(C, scene_index(C, i), off));
+        return;
+    }
     if (!reads_substep_list(C, t, i, pi, cell_of(pi, C), grid_view(C, scene_index(C, i), off))) return;
     const int cnt = __ldg(C.nbr_count + t) & 0xffff;
     const float4 *__restrict__ src = slots ? C.cls_pos : P;
@@ -1080,6 +1125,16 @@ __global__ void __launch_bounds__(kScanThreads, BP_POSTBC_MIN_BLOCKS) k_post_a_l
             if (ok && C.use_akinci) nn = fma3(__frcp_rn(nb.rho), g, nn);
         });
     finish_post_a(C, slots, i, t, om, nn, rho, Om, Nm);
+}
+
+// Pass A in walk mode, a launch of its own: k_post_a_lists' 3 CTAs an SM cost the
+// walk 16 % (829,440 squeezed particles, 288 and 249 us), and where lists are
+// read its early exit takes 2 us.
+__global__ void __launch_bounds__(kScanThreads, BP_SCAN_MIN_BLOCKS) k_post_a_walks(
+    SimConsts C, const float4 *__restrict__ P, const float4 *__restrict__ V, const float *__restrict__ rho,
+    const int *__restrict__ off, float4 *__restrict__ Om, float4 *__restrict__ Nm)
+{
+    if (walk_mode(C)) k_post_a_tile<true, false>(C, P, V, rho, off, Om, Nm, blockIdx.x * blockDim.x);
 }
 
 // The queued particles' pass A, as k_lambda_queued: a queued particle leaves
@@ -1222,7 +1277,7 @@ __global__ void __launch_bounds__(kQueueThreads) k_lambda_record(SimConsts C, co
     const int lane = threadIdx.x & 31;
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = C.sl_count[kSlWalks] = 0;
+        C.sl_count[0] = C.sl_count[1] = C.sl_count[kSlDisplaced] = C.sl_count[kSlWalks] = C.sl_count[kSlContactWalks] = 0;
         C.sl_count[kSlMoved] = C.cls_perm ? *C.cls_moved : 0;
     }
     if (t >= C.n) return;  // whole warps
@@ -1694,10 +1749,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_post_c_group(SimConsts C, con
     Vout[me.i] = make_float4(v.x, v.y, v.z, vi4.w);
 }
 
-static bool use_groups(const SimConsts &C)
-{
-    return C.sl_pos && C.n <= (C.textbook ? kGroupMaxTextbook : kGroupMax);
-}
+bool reads_in_groups(int n, bool textbook) { return n <= (textbook ? kGroupMaxTextbook : kGroupMax); }
+static bool use_groups(const SimConsts &C) { return C.sl_pos && reads_in_groups(C.n, C.textbook != 0); }
 static unsigned group_blocks(const SimConsts &C)
 {
     return (unsigned)(((long long)C.n * kGroupLanes + kGroupThreads - 1) / kGroupThreads);
@@ -1716,8 +1769,10 @@ void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const
         L->done("launch_lambda");
         return;
     }
+    const bool walks = C.sl_may_walk != 0;
     if (record) {
-        k_lambda_lists<kRecordLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+        if (walks) k_lambda_lists<kRecordLists, true><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+        else k_lambda_lists<kRecordLists, false><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
         L->done("launch_lambda");
         return;
     }
@@ -1725,7 +1780,8 @@ void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const
         k_lambda_group<true><<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, mass, off, lam, rho);
     else if (use_groups(C))
         k_lambda_group<false><<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, mass, off, lam, rho);
-    else k_lambda_lists<kReadLists><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+    else if (walks) k_lambda_lists<kReadLists, true><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
+    else k_lambda_lists<kReadLists, false><<<grid, C.scan_block, 0, st>>>(C, P, mass, off, lam, rho);
     L->done("launch_lambda_lists");
     k_lambda_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, mass, off, lam, rho);
     L->done("launch_lambda_queued");
@@ -1744,6 +1800,10 @@ void launch_post_a_lists(cudaStream_t st, const SimConsts &C, const float4 *P, c
     if (use_groups(C)) k_post_a_group<<<group_blocks(C), kGroupThreads, 0, st>>>(C, P, V, rho, off, Om, Nm);
     else k_post_a_lists<<<(C.n + C.scan_block - 1) / C.scan_block, C.scan_block, 0, st>>>(C, P, V, rho, off, Om, Nm);
     L->done("launch_post_a_lists");
+    if (C.sl_may_walk) {
+        k_post_a_walks<<<(C.n + C.scan_block - 1) / C.scan_block, C.scan_block, 0, st>>>(C, P, V, rho, off, Om, Nm);
+        L->done("launch_post_a_walks");
+    }
     k_post_a_queued<<<queue_blocks(C.n, kQueueThreads), kQueueThreads, 0, st>>>(C, P, V, rho, off, Om, Nm);
     L->done("launch_post_a_queued");
 }

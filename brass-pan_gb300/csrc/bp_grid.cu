@@ -757,27 +757,18 @@ void launch_class_order(cudaStream_t st, int n, const int *sorted_keys, const in
     launch_cell_offsets(st, n, 8 * a.T, a.keys, a.off, L, gate);
 }
 
-// Writes particle p's x, y, z and phase bits to slot q of the walk planes
-// (SimConsts::walk_xyz).
-__device__ __forceinline__ void put_planes(float *planes, int stride, int q, float4 p)
-{
-    const size_t st = (size_t)stride;
-    planes[q] = p.x;
-    planes[st + q] = p.y;
-    planes[2 * st + q] = p.z;
-    planes[3 * st + q] = p.w;
-}
-
 // Walks use the classes while at least 1/32 of the particles sit in a cell
 // holding another class (below that the extra indirection costs more than
 // the skipped candidates save) and no particle has left the reach.
 // *moved: 1 where the gate is closed, 2 where a particle left the reach.
-// planes != nullptr: also writes the walk planes, in sorted order where the
-// gate is closed and in class order where it is open.
+// planes != nullptr: also writes the walk planes (wanted: where it is not 0), in
+// sorted order where the gate is closed and in class order where it is open.
 __global__ void __launch_bounds__(256) k_class_refresh(int n, const float4 *__restrict__ P,
                                                        const float4 *__restrict__ V, ClassArrays a, Gate gate,
-                                                       float *__restrict__ planes, int stride)
+                                                       float *__restrict__ planes, int stride,
+                                                       const int *__restrict__ wanted)
 {
+    if (wanted && __ldg(wanted) == 0) planes = nullptr;
     if (gate_closed(gate)) {  // uniform: written by an earlier kernel
         if (blockIdx.x == 0 && threadIdx.x == 0) *a.moved = 1;
         if (planes)
@@ -812,28 +803,30 @@ static int wave_blocks(int n)
 }
 
 void launch_class_refresh(cudaStream_t st, int n, const float4 *P, const ClassArrays &a, LaunchLog *L,
-                          const float4 *V, float *planes, int stride)
+                          const float4 *V, float *planes, int stride, const int *wanted)
 {
     if (n <= 0) return;
     // the common case without planes is the gate's early exit (one wave);
     // with planes, a thread per particle
-    const int blocks = planes ? (n + 255) / 256 : wave_blocks(n);
-    k_class_refresh<<<blocks, 256, 0, st>>>(n, P, V, a, class_gate(n, a), planes, stride);
+    const int blocks = planes && !wanted ? (n + 255) / 256 : wave_blocks(n);
+    k_class_refresh<<<blocks, 256, 0, st>>>(n, P, V, a, class_gate(n, a), planes, stride, wanted);
     L->done(__func__);
 }
 
 // The walk planes in sorted order (scenes without alias classes).
 __global__ void __launch_bounds__(256) k_walk_planes(int n, const float4 *__restrict__ P, float *__restrict__ planes,
-                                                     int stride)
+                                                     int stride, const int *__restrict__ wanted)
 {
+    if (wanted && __ldg(wanted) == 0) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         put_planes(planes, stride, i, P[i]);
 }
 
-void launch_walk_planes(cudaStream_t st, int n, const float4 *P, float *planes, int stride, LaunchLog *L)
+void launch_walk_planes(cudaStream_t st, int n, const float4 *P, float *planes, int stride, LaunchLog *L,
+                        const int *wanted)
 {
     if (n <= 0) return;
-    k_walk_planes<<<(n + 255) / 256, 256, 0, st>>>(n, P, planes, stride);
+    k_walk_planes<<<wanted ? wave_blocks(n) : (n + 255) / 256, 256, 0, st>>>(n, P, planes, stride, wanted);
     L->done(__func__);
 }
 

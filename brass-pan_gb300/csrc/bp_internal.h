@@ -127,11 +127,14 @@ void launch_class_order(cudaStream_t st, int n, const int *sorted_keys, const in
 // Gathers P into class order and flags particles beyond the reach.
 // V != nullptr: also gathers V into a.vel (before the post passes).
 // planes != nullptr: also writes the walk planes (SimConsts::walk_xyz), in
-// class order where the classes are open and in sorted order where not.
+// class order where the classes are open and in sorted order where not
+// (wanted: only where it is not 0 on the device).
 void launch_class_refresh(cudaStream_t st, int n, const float4 *P, const ClassArrays &a, LaunchLog *L,
-                          const float4 *V = nullptr, float *planes = nullptr, int stride = 0);
+                          const float4 *V = nullptr, float *planes = nullptr, int stride = 0,
+                          const int *wanted = nullptr);
 // The walk planes in sorted order (scenes without alias classes).
-void launch_walk_planes(cudaStream_t st, int n, const float4 *P, float *planes, int stride, LaunchLog *L);
+void launch_walk_planes(cudaStream_t st, int n, const float4 *P, float *planes, int stride, LaunchLog *L,
+                        const int *wanted = nullptr);
 
 // ---- fluid kernels ----
 void launch_lambda(cudaStream_t st, const SimConsts &C, const float4 *P, const float *mass, const int *off,
@@ -142,6 +145,7 @@ void launch_lambda(cudaStream_t st, const SimConsts &C, const float4 *P, const f
 void launch_lambda_lists(cudaStream_t st, const SimConsts &C, bool record, const float4 *P, const float *mass,
                          const int *off, float *lam, float *rho, LaunchLog *L);
 bool records_from_planes(int n);  // the recording launch reads the walk planes
+bool reads_in_groups(int n, bool textbook);  // the readers take four lanes a particle (no walk_mode)
 void launch_post_a_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,
                          const int *off, float4 *Om, float4 *Nm, LaunchLog *L);
 void launch_contacts_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *Xs, const float *w,

@@ -31,9 +31,10 @@ __device__ __forceinline__ void append_to(int *count, int *queue, int t)
 
 // May the particle of slot t, at pi, read its list in this pass?  Queues it
 // where not.
-// (fits: its list holds all it should.)
+// (fits: its list holds all it should.  walks: where those that something near
+// them keeps from it are counted, except in a substep's last pass.)
 __device__ __forceinline__ bool reads_substep_list(const SimConsts &C, int t, int i, float3 p, int3 c,
-                                                   const GridView &v, bool fits = true)
+                                                   const GridView &v, bool fits = true, int walks = kSlWalks)
 {
     int state = substep_list_state(C, t, i, p, v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask));
     if (state != 0) C.sl_cell[t] = state == 3 ? kListMoved : kListNone;
@@ -41,8 +42,57 @@ __device__ __forceinline__ bool reads_substep_list(const SimConsts &C, int t, in
     if (C.nl_stats) atomicAdd(C.nl_stats + state, 1u);
     if (state == 0) return true;
     append_to(C.sl_count + C.sl_pass, C.sl_queue, t);
-    if (state == 3) append_to(C.sl_count + (C.sl_adapt ? kSlDisplaced : kSlWalks), nullptr, t);
+    if (state == 3) append_to(C.sl_count + (C.sl_adapt ? kSlDisplaced : walks), nullptr, t);
     return false;
+}
+
+// In walk mode's last substep: counts the particle of slot t among those that
+// something near them would have kept from reading their lists.
+__device__ __forceinline__ void note_substep_list(const SimConsts &C, int t, int i, float3 p, int3 c, const GridView &v)
+{
+    if (!walk_probe(C)) return;
+    const int state = substep_list_state(C, t, i, p, v.base + cell_addr(c.x, c.y, c.z, v.D, v.mask));
+    if (state == 0) return;
+    C.sl_cell[t] = state == 3 ? kListMoved : kListNone;
+    if (state == 3) append_to(C.sl_count + (C.sl_adapt ? kSlDisplaced : kSlWalks), nullptr, t);
+}
+
+// Whether the next substep's fluid passes walk, from what its passes would cost,
+// in units of one over lists of a particle's pairs alone: lists cost their
+// entries for a pair (sampled as they are recorded) times sl_read_cost, and a
+// queued walk kQueueCost more; walks cost sl_walk_cost.  The coefficients are
+// the times of the passes of 314,432 particles (SimConsts::sl_read_cost).
+// Textbook corrections move particles further than the skin in fluid denser than
+// at rest (reference mode: 3 % of them at most, and lists win at every density),
+// and there the wider skin's entries and the queue cost more than the searches.
+// A frame without substep lists, with lists only, with both: 314,432 particles
+// squeezed 1.0, 1.1, 1.2 and 1.3 times 1692, 1803, 2496, 3146 us; 1344, 1986,
+// 2893, 4859; 1340, 1769, 2423, 3039; 829,440: 4001, 4235, 5869, 7341; 3196, 4414,
+// 6510, 11368; 3171, 4104, 5660, 7080.  210 frames of the mixed scene, a frame
+// 8.77, 7.93 and 7.91 ms.  With a queue cost of 5, 829,440 squeezed 1.141 times
+// took 5502 us (8 and 15: 5162); with 15 the mixed scene 7.97 ms.
+// Walk mode lasts kWalkSubsteps at a time; the last one counts who would have
+// walked, at a skin that shrinks faster than by the substep (adapt_skin), and
+// takes the entries from the last sample by the lists' volume.  The two lines
+// lie apart so that noise does not change the mode.
+constexpr float kQueueCost = 8.f, kWalkAbove = 1.03f, kListsBelow = 0.95f;
+constexpr int kWalkSubsteps = 8;
+// False: nothing was counted in this substep.
+__device__ __forceinline__ bool choose_mode(const SimConsts &C, float fluid_walks)
+{
+    int &left = C.sl_count[kSlWalkMode];
+    const int pairs = C.sl_count[kSlPairs], entries = C.sl_count[kSlEntries];
+    C.sl_count[kSlPairs] = C.sl_count[kSlEntries] = 0;
+    if (left > 1) {
+        --left;
+        return false;
+    }
+    const float wider = 1.0f + C.sl_skin[0], volume = wider * wider * wider;
+    if (left == 0 && pairs > 0) C.sl_skin[3] = (float)entries / ((float)pairs * volume);
+    C.sl_skin[4] = 0.5f * (C.sl_skin[4] + fluid_walks);
+    const float lists = C.sl_skin[3] * volume * C.sl_read_cost + kQueueCost * C.sl_skin[4];
+    left = lists > (left == 0 ? kWalkAbove : kListsBelow) * C.sl_walk_cost ? kWalkSubsteps : 0;
+    return true;
 }
 
 // The skin of the next substep's lists, from how many particles the last pass
@@ -56,16 +106,19 @@ __device__ __forceinline__ bool reads_substep_list(const SimConsts &C, int t, in
 // a particle's worth or more: a spike in one pass, as where a cloth lands, is
 // cheaper walked (150k particles with solids: 1730 us a frame, 1800 us wide).
 // Squeezed fluid bursting apart, textbook mode, kWideSkin 0.1, 0.15, 0.2 and
-// 0.3 of h: 38,850 particles 1031, 909, 853 and 902 us, 800,000 8898, 7763,
-// 7564 and 8208 us.
+// 0.3 of h: 38,850 particles 1031, 909, 853 and 902 us (larger scenes walk there:
+// choose_mode).
 // The results do not depend on the skin.
 constexpr float kWideWalks = 0.5f, kWideRest = 0.05f;
 __device__ __forceinline__ void adapt_skin(const SimConsts &C)
 {
     if (!C.sl_adapt || blockIdx.x != 0 || threadIdx.x != 0) return;
     const long long moved = C.sl_count[kSlDisplaced];
+    const float fluid_walks = (float)(moved + C.sl_count[kSlWalks]) / (float)C.n;
+    const bool walked = C.sl_may_walk && C.sl_count[kSlWalkMode] > 0;
+    if (C.sl_may_walk && !choose_mode(C, fluid_walks)) return;
     float skin = C.sl_skin[0], bad = C.sl_skin[1] * 0.998f;
-    const float walks = 0.5f * (C.sl_skin[2] + (float)(moved + C.sl_count[kSlWalks]) / (float)C.n);
+    const float walks = 0.5f * (C.sl_skin[2] + fluid_walks + (float)C.sl_count[kSlContactWalks] / (float)C.n);
     const bool wide = skin >= 0.999f * kMaxSkin;
     if (wide && walks > kWideWalks) {
         skin = fminf(skin * 1.3f, kWideSkin);
@@ -73,7 +126,7 @@ __device__ __forceinline__ void adapt_skin(const SimConsts &C)
         bad = skin;
         skin = fminf(skin * 1.3f, kMaxSkin);
     } else if (wide ? walks < kWideRest : moved * 100 < C.n) {
-        skin = fmaxf(skin * 0.9f, fmaxf(fminf(bad * 1.15f, skin), kMinSkin));
+        skin = fmaxf(skin * (walked ? 0.8f : 0.9f), fmaxf(fminf(bad * 1.15f, skin), kMinSkin));
     }
     C.sl_skin[0] = skin;
     C.sl_skin[1] = bad;
@@ -91,7 +144,7 @@ __device__ __forceinline__ int record_substep_list(const SimConsts &C, const flo
     int self = kNoOwnEntry;
     const int me = slots ? t : i;
     // the walk planes hold the order this walk reads, except where a particle
-    // left the classes' reach after they were written
+    // left the classes' reach after they were written, or without planes
     const int planes = walk_planes_order(C);
     if (planes == (slots ? 2 : 1)) {
         record_walk_planes(planes, pi, r2, v, C, [&](int c0, unsigned bits) {
@@ -106,7 +159,8 @@ __device__ __forceinline__ int record_substep_list(const SimConsts &C, const flo
             list.push(j);
         };
         auto test = [&](int, float4 pj) { return len2(pi - f3(pj)) <= r2; };
-        walk_table<true>(c, 0, P, v, nullptr, -1, test, push);
+        if (slots) walk_classes<true, true>(i, c, 0, v, C, test, push);
+        else walk_table<true>(c, 0, P, v, nullptr, -1, test, push);
     }
     const int cnt = list.finish(me);
     return cnt < 0 ? -1 : cnt | (self << 16);

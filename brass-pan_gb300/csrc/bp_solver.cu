@@ -426,7 +426,7 @@ static bp_status create_solver_with(int nbr_cap, const bp_scene_desc *sc, const 
         (st = s->alloc(&s->off, ncells + 1)) || (st = s->alloc(&s->mass, N)) || (st = s->alloc(&s->lam, N)) || (st = s->alloc(&s->lm, N)) ||
         (st = s->alloc(&s->rho, N)) || (st = s->alloc(&s->w, N)) || (st = s->alloc(&s->err, 1)) ||
         (st = s->alloc(&s->staging, 6 * N)) || (st = s->alloc(&s->nl_pos, N)) || (st = s->alloc(&s->sl_cell, N)) ||
-        (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 3)) ||
+        (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 5)) ||
         (st = s->alloc(&s->sl_bits, sl_bit_words(s))) ||
         (st = s->alloc(&s->nl_stats, 5)))
         return bail(st);
@@ -501,8 +501,9 @@ static bp_status create_solver_with(int nbr_cap, const bp_scene_desc *sc, const 
         BP_CUDA_BAIL(cudaMemcpy(s->mass, m.data(), n * sizeof(float), cudaMemcpyHostToDevice));
     }
     s->Pcur = s->Pa;
-    const float skin0[3] = {kStartSkin, 0.f, 0.f};
+    const float skin0[5] = {kStartSkin, 0.f, 0.f, 1.f, 0.f};
     BP_CUDA_BAIL(cudaMemcpy(s->sl_skin, skin0, sizeof(skin0), cudaMemcpyHostToDevice));
+    BP_CUDA_BAIL(cudaMemset(s->sl_count, 0, kSlCounts * sizeof(int)));
     BP_CUDA_BAIL(cudaMemset(s->lam, 0, N * sizeof(float)));
     BP_CUDA_BAIL(cudaMemset(s->rho, 0, N * sizeof(float)));
     BP_CUDA_BAIL(cudaMemset(s->Om, 0, N * sizeof(float4)));
@@ -923,6 +924,27 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         Csl.cl_count = s->cl_count;
         Csl.cl_near = fluid ? s->solid_near : nullptr;
     }
+    // Walk mode (choose_mode): textbook mode, one thread a particle (smaller scenes
+    // read lists at every density: 32,768 particles squeezed to 1.3 of their rest
+    // spacing 880 us a frame, 1011 walking).  The walk planes of its passes come
+    // with the class refresh, from the position pass where nothing moves
+    // particles behind it, or, where its 2 us do not count, in a launch of their
+    // own; otherwise the walks read the position records.
+    const bool may_walk = shared && fluid && C.textbook && C.sl_fixed == 0.f && !reads_in_groups(s->n, true);
+    const bool walk_refresh = may_walk && classes;
+    const bool deltap_planes = may_walk && !classes && fuse && !tail && !pcoll && !picking;
+    const bool plane_launch = may_walk && !classes && !deltap_planes && s->n > 200000;
+    const int *walk_wanted = s->sl_count + kSlWalkMode;
+    if (may_walk) {
+        Csl.sl_may_walk = 1;
+        Csl.sl_planes = deltap_planes ? s->walk_xyz : nullptr;
+        // A delta-p pass over the pairs alone is 1 (314,432 particles at rest: 39
+        // us).  Over lists of the pairs lambda takes 0.8, passes A, B, C 1.25, 1.45,
+        // 1.4; walking 2.4 and 3.4 for lambda and A, XSPH alone 3.5.
+        const float r = (float)(iterations - 1), xsph = C.use_xsph ? 1.4f : 0.f;
+        Csl.sl_read_cost = 0.8f * r + (r + 1.f) + (post_ab ? 1.25f + 1.45f + xsph : xsph);
+        Csl.sl_walk_cost = 2.4f * r + (r + 1.f) + (post_ab ? 3.4f + 1.45f + xsph : 2.5f * xsph);
+    }
     const SimConsts &Cpost = (verlet || shared) ? Csl : Cpre;
     // Without them lambda records each particle's neighbours within h for the
     // position pass (the same positions), which then reads them instead of
@@ -1038,7 +1060,13 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             // lambda and delta-p read the same positions
             const bool record = shared && it == 0;
             if (walk_planes && (!shared || record)) refresh_planes(cur);
+            else if (walk_refresh)
+                launch_class_refresh(st, s->n, cur, ca, L, nullptr, s->walk_xyz, s->walk_stride, walk_wanted);
             else refresh(cur);
+            if (shared && !record && plane_launch)
+                launch_walk_planes(st, s->n, cur, s->walk_xyz, s->walk_stride, L, walk_wanted);
+            else if (shared && !record && !walk_refresh && !deltap_planes)
+                Cf.walk_xyz = nullptr;  // the planes are of other positions
             if (verlet && it == 0)
                 cudaMemsetAsync(s->nl_outlier, 0, (size_t)C.D * C.D * C.nl_zwords * sizeof(unsigned long long), st);
             if (shared) {
@@ -1147,11 +1175,15 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     const bool post_lists = shared && fluid;
     const bool post_slots = classes && lists && (post_ab || post_lists) && fluid && iterations > 0 && !verlet;
     const bool post_planes = walk_planes && post_ab && !post_lists;
+    const bool post_walks = post_ab && (walk_refresh || deltap_planes || plane_launch);  // pass A's walks read planes
     if ((post_ab || C.use_xsph) && classes)  // the post passes read the same positions
-        launch_class_refresh(st, s->n, cur, ca, L, post_slots ? s->Vc : nullptr, post_planes ? s->walk_xyz : nullptr,
-                             s->walk_stride);
+        launch_class_refresh(st, s->n, cur, ca, L, post_slots ? s->Vc : nullptr,
+                             post_planes || post_walks ? s->walk_xyz : nullptr, s->walk_stride,
+                             post_walks ? walk_wanted : nullptr);
     else if (post_planes)
         launch_walk_planes(st, s->n, cur, s->walk_xyz, s->walk_stride, L);
+    else if (post_ab && plane_launch)
+        launch_walk_planes(st, s->n, cur, s->walk_xyz, s->walk_stride, L, walk_wanted);
     if (post_ab) {
         // pass A records each fluid particle's neighbours for passes B and C
         SimConsts Cl = Cpost;
@@ -1163,7 +1195,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             Cl.nbr_count = s->nbr_count;
             Cl.nbr_cap = s->nbr_cap;
         }
-        if (post_planes) {
+        if (post_planes || post_walks) {
             Cl.walk_xyz = s->walk_xyz;
             Cl.walk_stride = s->walk_stride;
         }
