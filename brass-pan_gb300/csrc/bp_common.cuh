@@ -186,13 +186,14 @@ struct SimConsts {
     // other one); [kSlMoved]; [kSlDisplaced]: particles that the last list pass
     // of a substep queued because something near them moved, [kSlWalks]: those
     // of the fluid passes before it, [kSlContactWalks]: of the contact passes;
-    // [kSlWalkMode]: substeps left in walk mode; [kSlPairs], [kSlEntries]: a
-    // sample of the recorded entries, those within h and all
+    // [kSlWalkMode]: substeps left in walk mode; [kSlSample]: particles whose list
+    // was sampled, with its pairs within h, entries and the walk's candidates
     int *sl_count;
     // [0] the skin in use, as a fraction of h (a radius set later keeps it within
     // kWideSkin), adapted after each substep (adapt_skin), [1] the last that was
     // too small, [2] such walks a particle of the last substeps, [4] of their
-    // fluid passes; [3] entries recorded for a pair within h, over (1 + skin)^3
+    // fluid passes; [3] entries recorded for a pair within h, over (1 + skin)^3;
+    // [5] the lists' cost over the walks'
     float *sl_skin;
     float sl_fixed;   // > 0: this skin instead
     int sl_pass;      // parity of this list pass
@@ -203,7 +204,9 @@ struct SimConsts {
     // position pass leaves the walk planes of the next walks (nullptr: nowhere).
     int sl_may_walk;
     float *sl_planes;
-    float sl_read_cost, sl_walk_cost;
+    // what choose_mode weighs: the passes that read lists after the first, pass A (or
+    // XSPH alone) or not, passes B and C, and 1 where walks have their planes
+    float sl_reads, sl_post_a, sl_post_bc, sl_search_cost;
     int sl_last;      // this pass is the substep's last over the lists: what it moves is not tracked
     int sl_adapt;     // and it adapts the skin
     int sl_fluid;     // the lists reach h + skin (the fluid passes read them)
@@ -217,8 +220,8 @@ struct SimConsts {
 };
 constexpr int kContactCap = 32;
 constexpr int kSlLevels = 3;
-constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlWalks = 4, kSlContactWalks = 5, kSlWalkMode = 6, kSlPairs = 7,
-              kSlEntries = 8, kSlCounts = 9;
+constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlWalks = 4, kSlContactWalks = 5, kSlWalkMode = 6, kSlSample = 7,
+              kSlPairs = 8, kSlEntries = 9, kSlCandidates = 10, kSlCounts = 11;
 // Bounds of the adapted skin and where it starts, as fractions of h: up to
 // kMaxSkin as a rule, up to kWideSkin where walks go on at that (adapt_skin).
 constexpr float kMinSkin = 0.02f, kMaxSkin = 0.1f, kWideSkin = 0.2f, kStartSkin = 0.09f;

@@ -465,12 +465,14 @@ __device__ __forceinline__ void lambda_substep_list(const SimConsts &C, const fl
     // a pass that may walk reads its lists past the read-only path
     lambda_over_list<Pass == kReadLists && !Walks>(C, P, mass, lam, rho, slots, i, t, pi4, sc, c, v, packed, pairs);
     if (Pass == kRecordLists && Walks && blockIdx.x % kSampleBlocks == 0 && packed >= 0) {
+        const int found[3] = {pairs, packed & 0xffff, walk_candidates(C, slots, i, c, v)};
         const unsigned m = __activemask();
-        pairs = __reduce_add_sync(m, pairs);
-        const int entries = __reduce_add_sync(m, packed & 0xffff);
-        if ((threadIdx.x & 31) == __ffs(m) - 1) {
-            atomicAdd(C.sl_count + kSlPairs, pairs);
-            atomicAdd(C.sl_count + kSlEntries, entries);
+        const bool first = (threadIdx.x & 31) == __ffs(m) - 1;
+        if (first) atomicAdd(C.sl_count + kSlSample, __popc(m));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int sum = __reduce_add_sync(m, found[k]);
+            if (first) atomicAdd(C.sl_count + kSlPairs + k, sum);
         }
     }
 }

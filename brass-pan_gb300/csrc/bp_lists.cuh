@@ -57,41 +57,66 @@ __device__ __forceinline__ void note_substep_list(const SimConsts &C, int t, int
     if (state == 3) append_to(C.sl_count + (C.sl_adapt ? kSlDisplaced : kSlWalks), nullptr, t);
 }
 
-// Whether the next substep's fluid passes walk, from what its passes would cost,
-// in units of one over lists of a particle's pairs alone: lists cost their
-// entries for a pair (sampled as they are recorded) times sl_read_cost, and a
-// queued walk kQueueCost more; walks cost sl_walk_cost.  The coefficients are
-// the times of the passes of 314,432 particles (SimConsts::sl_read_cost).
+// The candidates that the walk of particle i in cell c meets, but for the cells
+// past the table's end (slots: of its own class alone).
+__device__ __forceinline__ int walk_candidates(const SimConsts &C, bool slots, int i, int3 c, const GridView &v)
+{
+    const unsigned m = v.mask, D = (unsigned)v.D, z = min(max((unsigned)c.z & m, 1u), m - 1u);
+    const int *__restrict__ off = slots ? C.cls_off + v.base + (size_t)__ldg(C.cls_of + i) * (size_t)C.cls_T : v.off;
+    int n = 0;
+    for (int col = 0; col < 9; ++col) {
+        const unsigned a = ((unsigned)(c.x + col / 3 - 1) & m) * D * D + ((unsigned)(c.y + col % 3 - 1) & m) * D + z;
+        n += __ldg(off + a + 2) - __ldg(off + a - 1);
+    }
+    return n;
+}
+
+// Whether the next substep's fluid passes walk (walk mode), from what they would
+// cost, in units of a delta-p pass over lists of the pairs alone (1.18 us a pair
+// and particle for 314,432 of them): the lists' entries for a pair, sampled as
+// they are recorded, times the readers' shares (lambda 0.8, delta-p 1, pass A
+// 1.1, B 1.3, C 1.4), and the queued walks, kQueueSearch searches each; or a
+// search in each lambda pass and 1.4 in pass A, from the pairs and candidates of
+// a particle (measured at 33 to 67 pairs and 216 to 475 candidates: 97 to 177 us).
 // Textbook corrections move particles further than the skin in fluid denser than
-// at rest (reference mode: 3 % of them at most, and lists win at every density),
-// and there the wider skin's entries and the queue cost more than the searches.
+// at rest, and there the entries of a wide skin and the queue cost more than the
+// searches; in reference mode lists win at every density.
 // A frame without substep lists, with lists only, with both: 314,432 particles
-// squeezed 1.0, 1.1, 1.2 and 1.3 times 1692, 1803, 2496, 3146 us; 1344, 1986,
-// 2893, 4859; 1340, 1769, 2423, 3039; 829,440: 4001, 4235, 5869, 7341; 3196, 4414,
-// 6510, 11368; 3171, 4104, 5660, 7080.  210 frames of the mixed scene, a frame
-// 8.77, 7.93 and 7.91 ms.  With a queue cost of 5, 829,440 squeezed 1.141 times
-// took 5502 us (8 and 15: 5162); with 15 the mixed scene 7.97 ms.
-// Walk mode lasts kWalkSubsteps at a time; the last one counts who would have
-// walked, at a skin that shrinks faster than by the substep (adapt_skin), and
-// takes the entries from the last sample by the lists' volume.  The two lines
-// lie apart so that noise does not change the mode.
-constexpr float kQueueCost = 8.f, kWalkAbove = 1.03f, kListsBelow = 0.95f;
-constexpr int kWalkSubsteps = 8;
+// squeezed 1.0, 1.1, 1.2 and 1.3 times 1693, 1806, 2499, 3151 us; 1346, 1990,
+// 2899, 4861; 1347, 1782, 2435, 3060; 829,440: 4005, 4233, 5865, 7334; 3198, 4415,
+// 6510, 11365; 3183, 4376, 5681, 7117.  Twelve frames of 50 bursting scenes 1.00,
+// 1.06 and 1.08 times as fast, the slowest 0.85 and 0.98; 210 frames of the mixed
+// scene 8.77, 7.93 and 7.80 ms each.
+// The ratio is averaged while lists are read, as a burst is over in a few frames;
+// walk mode lasts kWalkSubsteps at a time, whose last one counts who would have
+// been queued, at a skin that shrinks faster than by the substep (adapt_skin).
+constexpr float kQueueSearch = 4.f, kWalkAbove = 1.05f, kListsBelow = 1.0f;
+constexpr int kWalkSubsteps = 4;
 // False: nothing was counted in this substep.
 __device__ __forceinline__ bool choose_mode(const SimConsts &C, float fluid_walks)
 {
     int &left = C.sl_count[kSlWalkMode];
-    const int pairs = C.sl_count[kSlPairs], entries = C.sl_count[kSlEntries];
-    C.sl_count[kSlPairs] = C.sl_count[kSlEntries] = 0;
+    const float sample = (float)C.sl_count[kSlSample], pairs = (float)C.sl_count[kSlPairs];
+    const float entries = (float)C.sl_count[kSlEntries], candidates = (float)C.sl_count[kSlCandidates];
+    for (int k = kSlSample; k <= kSlCandidates; ++k) C.sl_count[k] = 0;
     if (left > 1) {
         --left;
         return false;
     }
-    const float wider = 1.0f + C.sl_skin[0], volume = wider * wider * wider;
-    if (left == 0 && pairs > 0) C.sl_skin[3] = (float)entries / ((float)pairs * volume);
     C.sl_skin[4] = 0.5f * (C.sl_skin[4] + fluid_walks);
-    const float lists = C.sl_skin[3] * volume * C.sl_read_cost + kQueueCost * C.sl_skin[4];
-    left = lists > (left == 0 ? kWalkAbove : kListsBelow) * C.sl_walk_cost ? kWalkSubsteps : 0;
+    if (!(pairs > 0.f)) {
+        left = 0;
+        return true;
+    }
+    const float wider = 1.0f + C.sl_skin[0], volume = wider * wider * wider;
+    if (left == 0) C.sl_skin[3] = entries / (pairs * volume);
+    const float search = (0.042f * candidates + 1.7f * pairs + 15.f * sample) / pairs * C.sl_search_cost;
+    const float lists = C.sl_skin[3] * volume * (1.8f * C.sl_reads + 1.f + 1.1f * C.sl_post_a + C.sl_post_bc) +
+                        kQueueSearch * search * C.sl_skin[4];
+    const float walks = (1.f + search) * C.sl_reads + 1.f + 1.4f * search * C.sl_post_a + C.sl_post_bc;
+    const float ratio = lists / walks;
+    C.sl_skin[5] = left > 0 ? ratio : 0.75f * C.sl_skin[5] + 0.25f * fminf(ratio, 1.5f);
+    left = C.sl_skin[5] > (left > 0 ? kListsBelow : kWalkAbove) ? kWalkSubsteps : 0;
     return true;
 }
 

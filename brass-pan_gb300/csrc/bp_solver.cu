@@ -426,7 +426,7 @@ static bp_status create_solver_with(int nbr_cap, const bp_scene_desc *sc, const 
         (st = s->alloc(&s->off, ncells + 1)) || (st = s->alloc(&s->mass, N)) || (st = s->alloc(&s->lam, N)) || (st = s->alloc(&s->lm, N)) ||
         (st = s->alloc(&s->rho, N)) || (st = s->alloc(&s->w, N)) || (st = s->alloc(&s->err, 1)) ||
         (st = s->alloc(&s->staging, 6 * N)) || (st = s->alloc(&s->nl_pos, N)) || (st = s->alloc(&s->sl_cell, N)) ||
-        (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 5)) ||
+        (st = s->alloc(&s->sl_queue, N)) || (st = s->alloc(&s->sl_count, kSlCounts)) || (st = s->alloc(&s->sl_skin, 6)) ||
         (st = s->alloc(&s->sl_bits, sl_bit_words(s))) ||
         (st = s->alloc(&s->nl_stats, 5)))
         return bail(st);
@@ -501,7 +501,7 @@ static bp_status create_solver_with(int nbr_cap, const bp_scene_desc *sc, const 
         BP_CUDA_BAIL(cudaMemcpy(s->mass, m.data(), n * sizeof(float), cudaMemcpyHostToDevice));
     }
     s->Pcur = s->Pa;
-    const float skin0[5] = {kStartSkin, 0.f, 0.f, 1.f, 0.f};
+    const float skin0[6] = {kStartSkin, 0.f, 0.f, 1.f, 0.f, 1.f};
     BP_CUDA_BAIL(cudaMemcpy(s->sl_skin, skin0, sizeof(skin0), cudaMemcpyHostToDevice));
     BP_CUDA_BAIL(cudaMemset(s->sl_count, 0, kSlCounts * sizeof(int)));
     BP_CUDA_BAIL(cudaMemset(s->lam, 0, N * sizeof(float)));
@@ -938,12 +938,10 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     if (may_walk) {
         Csl.sl_may_walk = 1;
         Csl.sl_planes = deltap_planes ? s->walk_xyz : nullptr;
-        // A delta-p pass over the pairs alone is 1 (314,432 particles at rest: 39
-        // us).  Over lists of the pairs lambda takes 0.8, passes A, B, C 1.25, 1.45,
-        // 1.4; walking 2.4 and 3.4 for lambda and A, XSPH alone 3.5.
-        const float r = (float)(iterations - 1), xsph = C.use_xsph ? 1.4f : 0.f;
-        Csl.sl_read_cost = 0.8f * r + (r + 1.f) + (post_ab ? 1.25f + 1.45f + xsph : xsph);
-        Csl.sl_walk_cost = 2.4f * r + (r + 1.f) + (post_ab ? 3.4f + 1.45f + xsph : 2.5f * xsph);
+        Csl.sl_reads = (float)(iterations - 1);
+        Csl.sl_post_a = post_ab || C.use_xsph ? 1.f : 0.f;
+        Csl.sl_post_bc = post_ab ? 1.3f + (C.use_xsph ? 1.4f : 0.f) : 0.f;
+        Csl.sl_search_cost = walk_refresh || deltap_planes || plane_launch ? 1.f : 1.2f;
     }
     const SimConsts &Cpost = (verlet || shared) ? Csl : Cpre;
     // Without them lambda records each particle's neighbours within h for the
