@@ -148,8 +148,9 @@ bool records_from_planes(int n);  // the recording launch reads the walk planes
 bool reads_in_groups(int n, bool textbook);  // the readers take four lanes a particle (no walk_mode)
 void launch_post_a_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *V, const float *rho,
                          const int *off, float4 *Om, float4 *Nm, LaunchLog *L);
+// solid_prefix, solid_list: launch_solid_list's, or nullptr.
 void launch_contacts_lists(cudaStream_t st, const SimConsts &C, const float4 *P, const float4 *Xs, const float *w,
-                           const int *off, float4 *Pout, LaunchLog *L);
+                           const int *off, const int *solid_prefix, const int *solid_list, float4 *Pout, LaunchLog *L);
 struct DeltaArgs {
     const float4 *P;
     const float *mass, *lam;

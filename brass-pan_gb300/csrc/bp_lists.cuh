@@ -253,6 +253,36 @@ __device__ __forceinline__ void warp_walk(const SimConsts &C, bool slots, int3 c
     }
 }
 
+// The solids among the candidates of the table walk of cell c, in walk order, 32
+// at a time as warp_walk's: prefix[j] solids lie before sorted index j, list
+// holds theirs.
+template <class F>
+__device__ __forceinline__ void warp_walk_solids(int3 c, const float4 *__restrict__ P, const GridView &v,
+                                                 const int *__restrict__ prefix, const int *__restrict__ list, F &&chunk)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned m = v.mask, D = (unsigned)v.D;
+    const unsigned z0 = (unsigned)(c.z - 1) & m, z2 = (unsigned)(c.z + 1) & m;
+    const bool wrap = !(z0 < z2);
+    const int runs = wrap ? 18 : 9;
+    int rb = 0, re = 0;  // lane r finds the ends of run r
+    if (lane < runs) {
+        const int col = wrap ? lane >> 1 : lane, piece = wrap ? lane & 1 : 0;
+        const unsigned base = ((unsigned)(c.x + col / 3 - 1) & m) * D * D + ((unsigned)(c.y + col % 3 - 1) & m) * D;
+        rb = __ldg(prefix + __ldg(v.off + base + (piece ? 0u : z0)));
+        re = __ldg(prefix + __ldg(v.off + base + (wrap ? (piece ? z2 : D - 1u) : z2) + 1));
+    }
+#pragma unroll 1
+    for (int r = 0; r < runs; ++r) {
+        const int b = __shfl_sync(0xffffffffu, rb, r), e = __shfl_sync(0xffffffffu, re, r);
+#pragma unroll 1
+        for (int k = b + lane; k - lane < e; k += 32) {
+            const int q = k < e ? __ldg(list + k) : 0;
+            chunk(q, k < e ? P[q] : make_float4(0.f, 0.f, 0.f, 0.f), k < e);
+        }
+    }
+}
+
 // Sums of up to kWarpTerms quantities over a warp walk's pairs, in walk order:
 // lane c adds quantity c of each pair of a chunk from a row in shared memory
 // (a load and an add a pair for all of them together, instead of a shuffle a
@@ -293,13 +323,12 @@ struct WarpHits {
     float4 p[64];
     int q[64];
 };
-template <class T, class B>
-__device__ __forceinline__ int warp_neighbors(const SimConsts &C, bool slots, int3 c, const float4 *__restrict__ P,
-                                              const GridView &v, WarpHits &buf, T &&test, B &&batch)
+template <class W, class T, class B>
+__device__ __forceinline__ int warp_collect(WarpHits &buf, W &&walk, T &&test, B &&batch)
 {
     const int lane = threadIdx.x & 31;
     int done = 0, held = 0;
-    warp_walk(C, slots, c, P, v, [&](int q, float4 p, bool in) {
+    walk([&](int q, float4 p, bool in) {
         const bool hit = in && test(q, p);
         const unsigned hits = __ballot_sync(0xffffffffu, hit);
         if (!hits) return;
@@ -324,6 +353,12 @@ __device__ __forceinline__ int warp_neighbors(const SimConsts &C, bool slots, in
     if (held) batch(done, held, buf.q[lane], buf.p[lane]);
     __syncwarp();
     return done + held;
+}
+template <class T, class B>
+__device__ __forceinline__ int warp_neighbors(const SimConsts &C, bool slots, int3 c, const float4 *__restrict__ P,
+                                              const GridView &v, WarpHits &buf, T &&test, B &&batch)
+{
+    return warp_collect(buf, [&](auto &&chunk) { warp_walk(C, slots, c, P, v, chunk); }, test, batch);
 }
 
 // Writes entry k of slot t's list (layout of ListWriter) where it fits.

@@ -1034,7 +1034,8 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             SimConsts Cc = Cpost;
             next_list_pass(Cc, !fluid && it == iterations - 1);
             float4 *out = stage_out();
-            launch_contacts_lists(st, Cc, cur, s->Xs, s->w, s->off, out, L);
+            launch_contacts_lists(st, Cc, cur, s->Xs, s->w, s->off, walked_contacts ? s->solid_prefix : nullptr,
+                                  s->solid_list, out, L);
             stage_done(out);
         } else if (pcoll) {
             if (tape) tape->push(TS_PCOLL, slot);
