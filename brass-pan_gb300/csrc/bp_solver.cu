@@ -855,11 +855,17 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // contact pass before it walks, and the displacements it causes, the
     // largest of the substep, come before the lists (mixed scene, cloth on
     // fluid: 14 % of the particles displaced past the skin when recorded ahead
-    // of it, 1 % behind it).  Contacts alone search ahead of their first pass.
+    // of it, 1 % behind it).  Contacts alone search ahead of their first pass; so
+    // they do in a scene of solids, whose fluid passes find nothing to do: their
+    // lists of h + skin cost more than those passes' own walks (97,336 grains, all
+    // stages, 2 iterations, textbook mode 403 -> 260 us a frame, 340 without lists;
+    // reference mode 451 -> 382), but for the few in reference mode whose walks
+    // are bound by their latency (1,728 grains, 8 iterations 429 and 559 us).
+    const bool fluid_lists = fluid && (s->num_solids < s->n || (!C.textbook && !records_from_planes(s->n)));
     const bool shared = C.sl_pos != nullptr && s->nbr && iterations > 0 &&
-                        ((fluid && (iterations > 1 || post_ab || C.use_xsph)) || (pcoll && iterations > 1));
+                        ((fluid_lists && (iterations > 1 || post_ab || C.use_xsph)) || (pcoll && iterations > 1));
     const bool listed_contacts = shared && pcoll && iterations > 1;
-    const bool walked_contacts = pcoll && (!shared || fluid);  // in the first iteration at least
+    const bool walked_contacts = pcoll && (!shared || fluid_lists);  // in the first iteration at least
     ra.tile_solid = walked_contacts ? s->tile_solid : nullptr;
     if (walked_contacts) cudaMemsetAsync(s->tile_solid, 0, ((s->n + 255) / 256) * sizeof(int), st);
     const bool classes = C.cls_perm != nullptr;
@@ -918,11 +924,11 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     Cpre.nl_pos = nullptr;
     Cpre.sl_pos = nullptr;
     SimConsts Csl = C;
-    Csl.sl_fluid = fluid ? 1 : 0;
+    Csl.sl_fluid = fluid_lists ? 1 : 0;
     if (listed_contacts) {
         Csl.cl_list = s->cl_list;
         Csl.cl_count = s->cl_count;
-        Csl.cl_near = fluid ? s->solid_near : nullptr;
+        Csl.cl_near = fluid_lists ? s->solid_near : nullptr;
     }
     // Walk mode (choose_mode): textbook mode, one thread a particle (smaller scenes
     // read lists at every density: 32,768 particles squeezed to 1.3 of their rest
@@ -930,7 +936,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // with the class refresh, from the position pass where nothing moves
     // particles behind it, or, where its 2 us do not count, in a launch of their
     // own; otherwise the walks read the position records.
-    const bool may_walk = shared && fluid && C.textbook && C.sl_fixed == 0.f && !reads_in_groups(s->n, true);
+    const bool may_walk = shared && fluid_lists && C.textbook && C.sl_fixed == 0.f && !reads_in_groups(s->n, true);
     const bool walk_refresh = may_walk && classes;
     const bool deltap_planes = may_walk && !classes && fuse && !tail && !pcoll && !picking;
     const bool plane_launch = may_walk && !classes && !deltap_planes && s->n > 200000;
@@ -957,7 +963,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     const bool walk_planes = lists && !verlet && s->walk_xyz && C.split && !C.stage &&
                         !(s->prm.walk_options & BP_WALK_NO_PLANES);
     auto refresh_planes = [&](const float4 *P) {
-        if (shared && !records_from_planes(s->n)) refresh(P);
+        if (shared && fluid_lists && !records_from_planes(s->n)) refresh(P);
         else if (classes) launch_class_refresh(st, s->n, P, ca, L, nullptr, s->walk_xyz, s->walk_stride);
         else launch_walk_planes(st, s->n, P, s->walk_xyz, s->walk_stride, L);
     };
@@ -1024,7 +1030,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             }
         }
         planes_done = false;
-        if (listed_contacts && !(fluid && it == 0)) {
+        if (listed_contacts && !(fluid_lists && it == 0)) {
             if (it == 0) {
                 refresh_planes(cur);
                 clear_list_bits(s);
@@ -1032,7 +1038,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
             }
             if (tape) tape->push(TS_PCOLL, slot);
             SimConsts Cc = Cpost;
-            next_list_pass(Cc, !fluid && it == iterations - 1);
+            next_list_pass(Cc, !fluid_lists && it == iterations - 1);
             float4 *out = stage_out();
             launch_contacts_lists(st, Cc, cur, s->Xs, s->w, s->off, walked_contacts ? s->solid_prefix : nullptr,
                                   s->solid_list, out, L);
@@ -1057,18 +1063,18 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
         }
         if (fluid) {
             // lambda and delta-p read the same positions
-            const bool record = shared && it == 0;
-            if (walk_planes && (!shared || record)) refresh_planes(cur);
+            const bool reads = shared && fluid_lists, record = reads && it == 0;
+            if (walk_planes && (!reads || record)) refresh_planes(cur);
             else if (walk_refresh)
                 launch_class_refresh(st, s->n, cur, ca, L, nullptr, s->walk_xyz, s->walk_stride, walk_wanted);
             else refresh(cur);
-            if (shared && !record && plane_launch)
+            if (reads && !record && plane_launch)
                 launch_walk_planes(st, s->n, cur, s->walk_xyz, s->walk_stride, L, walk_wanted);
-            else if (shared && !record && !walk_refresh && !deltap_planes)
+            else if (reads && !record && !walk_refresh && !deltap_planes)
                 Cf.walk_xyz = nullptr;  // the planes are of other positions
             if (verlet && it == 0)
                 cudaMemsetAsync(s->nl_outlier, 0, (size_t)C.D * C.D * C.nl_zwords * sizeof(unsigned long long), st);
-            if (shared) {
+            if (reads) {
                 next_list_pass(Cf, !record && it == iterations - 1 && !post_ab && !C.use_xsph);
                 if (record) clear_list_bits(s);
                 launch_lambda_lists(st, Cf, record, cur, s->mass, s->off, s->lam, s->rho, L);
@@ -1171,7 +1177,7 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // The post passes keep class positions in their lists where lambda left
     // its densities in class order (SimConsts::cls_post); the velocities are
     // gathered into class order with the positions.
-    const bool post_lists = shared && fluid;
+    const bool post_lists = shared && fluid_lists;
     const bool post_slots = classes && lists && (post_ab || post_lists) && fluid && iterations > 0 && !verlet;
     const bool post_planes = walk_planes && post_ab && !post_lists;
     const bool post_walks = post_ab && (walk_refresh || deltap_planes || plane_launch);  // pass A's walks read planes
