@@ -856,12 +856,15 @@ void bp::enqueue_substep(bp_solver *s, const SimConsts &C, int iterations, int p
     // largest of the substep, come before the lists (mixed scene, cloth on
     // fluid: 14 % of the particles displaced past the skin when recorded ahead
     // of it, 1 % behind it).  Contacts alone search ahead of their first pass; so
-    // they do in a scene of solids, whose fluid passes find nothing to do: their
-    // lists of h + skin cost more than those passes' own walks (97,336 grains, all
-    // stages, 2 iterations, textbook mode 403 -> 260 us a frame, 340 without lists;
-    // reference mode 451 -> 382), but for the few in reference mode whose walks
-    // are bound by their latency (1,728 grains, 8 iterations 429 and 559 us).
-    const bool fluid_lists = fluid && (s->num_solids < s->n || (!C.textbook && !records_from_planes(s->n)));
+    // they do in a scene of solids in textbook mode, whose fluid passes walk for
+    // none of them: lists of h + skin cost more than those passes (97,336 grains,
+    // all stages, 2 iterations 403 -> 260 us a frame, 340 without lists).  In
+    // reference mode they walk for solids too: so do packed ones (the same 451 ->
+    // 382 us, 460 without), but not cloth, whose lists are short (200 x 200, 442 us
+    // and 467), nor few, whose walks are bound by their latency (1,728 grains, 8
+    // iterations 429 and 559 us).
+    const bool packed_solids = s->num_solids == s->n && !s->dist_step.range && records_from_planes(s->n);
+    const bool fluid_lists = fluid && !(packed_solids || (C.textbook && s->num_solids == s->n));
     const bool shared = C.sl_pos != nullptr && s->nbr && iterations > 0 &&
                         ((fluid_lists && (iterations > 1 || post_ab || C.use_xsph)) || (pcoll && iterations > 1));
     const bool listed_contacts = shared && pcoll && iterations > 1;
