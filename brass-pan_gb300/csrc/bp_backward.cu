@@ -424,6 +424,7 @@ void adjoint_substep(bp_solver *s, Tape &t, const Tape::Sub &u, const StateBuf &
     C.nl_pos = nullptr;
     C.sl_pos = nullptr;
     C.cell_keys = s->sorted_keys;
+    if (C.sl_first) C.sl_first = s->off;
     C.nl_stats = nullptr;
     // nor the alias classes: their class-order positions are gathered only
     // for the forward walks (the same candidates in the same order remain)
@@ -737,6 +738,7 @@ extern "C" bp_status bp_solver_backward(bp_solver *s, const float *grad_position
                     T.next_V = to.V;
                     T.next_orig = to.orig;
                     C.cell_keys = s->sorted_keys;
+                    if (C.sl_first) C.sl_first = s->off;
                     enqueue_substep(s, C, u.iterations, u.picked, u.ppos, &L, &T);
                     return;
                 }

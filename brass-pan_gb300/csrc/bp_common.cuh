@@ -179,8 +179,13 @@ struct SimConsts {
     // Over the cell keys: four bits a cell, bit k - 1 set where it stores a
     // particle that moved more than k quarters of the skin, and kSlLevels bit
     // sets of sl_words words, the k-th holding the cells with one among their 27
+    // (sl_first != nullptr, the cell offsets: tables above kSlBitCells cells, of
+    // which each substep would clear seven bits a cell.  sl_far is then indexed by
+    // the first particle of a cell, and sl_near holds kSlBitCells bits a set, which
+    // cells share: a shared bit queues a particle that could have read its list.)
     unsigned *sl_far, *sl_near;
     int sl_words;
+    const int *sl_first;
     int *sl_queue;
     // [0], [1]: queue lengths, by the parity of the pass (a list pass clears the
     // other one); [kSlMoved]; [kSlDisplaced]: particles that the last list pass
@@ -220,6 +225,7 @@ struct SimConsts {
 };
 constexpr int kContactCap = 32;
 constexpr int kSlLevels = 3;
+constexpr unsigned kSlBitCells = 1u << 22;
 constexpr int kSlMoved = 2, kSlDisplaced = 3, kSlWalks = 4, kSlContactWalks = 5, kSlWalkMode = 6, kSlSample = 7,
               kSlPairs = 8, kSlEntries = 9, kSlCandidates = 10, kSlCounts = 11;
 // Bounds of the adapted skin and where it starts, as fractions of h: up to
@@ -444,6 +450,12 @@ __device__ __forceinline__ int list_state(const SimConsts &C, int i, int3 c, flo
     return 0;
 }
 
+// The bit of cell a in a set of sl_near; the cells of a word stay together.
+__device__ __forceinline__ unsigned near_bit(const SimConsts &C, unsigned a)
+{
+    return C.sl_first ? (a ^ ((a / kSlBitCells) * 0x9e3779b1u & ~31u)) & (kSlBitCells - 1u) : a;
+}
+
 // Substep lists: particle i moved more than `level` quarters of the skin.
 // In a pile of tumbling bodies every particle does, in every iteration: one
 // read or atomic then settles all levels (a bit set per level: shape matching
@@ -452,8 +464,9 @@ __device__ __forceinline__ void flag_moved(const SimConsts &C, int i, int level)
 {
     const unsigned key = (unsigned)__ldg(C.cell_keys + i);
     // the first particle of a cell to move that far flags the cells around it
-    const unsigned want = (1u << level) - 1u, shift = (key & 7u) * 4u;
-    unsigned *far = C.sl_far + (key >> 3);
+    const unsigned slot = C.sl_first ? (unsigned)__ldg(C.sl_first + key) : key;
+    const unsigned want = (1u << level) - 1u, shift = (slot & 7u) * 4u;
+    unsigned *far = C.sl_far + (slot >> 3);
     unsigned fresh = want & ~(*far >> shift);
     if (fresh) fresh = want & ~(atomicOr(far, want << shift) >> shift);
     if (!fresh) return;
@@ -466,8 +479,8 @@ __device__ __forceinline__ void flag_moved(const SimConsts &C, int i, int level)
         unsigned *near = C.sl_near + (size_t)k * C.sl_words;
 #pragma unroll 1
         for (unsigned q = 0; q < 27u; ++q) {
-            const unsigned a = base + ((x + q / 9u - 1u) & m) * D * D + ((y + (q / 3u) % 3u - 1u) & m) * D +
-                               ((z + q % 3u - 1u) & m);
+            const unsigned a = near_bit(C, base + ((x + q / 9u - 1u) & m) * D * D + ((y + (q / 3u) % 3u - 1u) & m) * D +
+                                               ((z + q % 3u - 1u) & m));
             atomicOr(near + (a >> 5), 1u << (a & 31u));
         }
     }
@@ -482,8 +495,9 @@ __device__ __forceinline__ int substep_list_state(const SimConsts &C, int t, int
     const int built = C.sl_cell[t];
     if (built < 0) return built == kListMoved ? 3 : 1;
     if (built != key) return 2;
-    const unsigned *near = C.sl_near + (key >> 5);
-    auto moved = [&](int k) { return ((__ldg(near + (size_t)(k - 1) * C.sl_words) >> (key & 31)) & 1u) != 0u; };
+    const unsigned bit = near_bit(C, (unsigned)key);
+    const unsigned *near = C.sl_near + (bit >> 5);
+    auto moved = [&](int k) { return ((__ldg(near + (size_t)(k - 1) * C.sl_words) >> (bit & 31u)) & 1u) != 0u; };
     // nothing near (itself included) moved more than a quarter, or it moved
     // one quarter at most and the others three, or each two
     if (!moved(1)) return 0;

@@ -169,6 +169,14 @@ static float class_reach(const bp_solver *s)
     return reach > 0.f ? reach : 0.f;
 }
 
+// Words of SimConsts::sl_near and sl_far.  On a 512^3 table, 7 bits a cell took
+// 117 MB to clear, 20 us a substep; shared bits pay from where that is noticed.
+static bool shared_bits(const bp_solver *s) { return s->ncells > ((size_t)1 << 25); }
+static size_t sl_bit_words(const bp_solver *s)
+{
+    return kSlLevels * s->sl_words + (shared_bits(s) ? ((size_t)s->n + 7) / 8 : 4 * s->sl_words);
+}
+
 // Substep constants: SetKernelRadius (K/fluid.cuh:11-27) evaluated on the host.
 SimConsts bp::make_consts(const bp_solver *s, float sdt)
 {
@@ -237,6 +245,7 @@ SimConsts bp::make_consts(const bp_solver *s, float sdt)
         C.sl_near = s->sl_bits;
         C.sl_far = s->sl_bits + kSlLevels * s->sl_words;
         C.sl_words = (int)s->sl_words;
+        C.sl_first = shared_bits(s) ? s->off : nullptr;
         C.sl_queue = s->sl_queue;
         C.sl_count = s->sl_count;
         C.sl_skin = s->sl_skin;
@@ -352,9 +361,6 @@ struct BatchSpec {
     int max_planes = 0;
 };
 
-// Words of SimConsts::sl_near and sl_far.
-static size_t sl_bit_words(const bp_solver *s) { return (kSlLevels + 4) * s->sl_words; }
-
 void bp::clear_list_bits(bp_solver *s)
 {
     cudaMemsetAsync(s->sl_bits, 0, sl_bit_words(s) * sizeof(unsigned), s->stream);
@@ -417,7 +423,7 @@ static bp_status create_solver_with(int nbr_cap, const bp_scene_desc *sc, const 
     const size_t ncells = batch ? batch->ncells : (size_t)D * D * D;
     s->ncells = ncells;
     s->sort_dim = batch ? batch->sort_dim : D;
-    s->sl_words = (ncells + 31) / 32;
+    s->sl_words = ((shared_bits(s) ? (size_t)kSlBitCells : ncells) + 31) / 32;
     if ((st = s->alloc(&s->Xc, N)) || (st = s->alloc(&s->Vc, N)) || (st = s->alloc(&s->Xs, N)) ||
         (st = s->alloc(&s->Vs, N)) || (st = s->alloc(&s->Pa, N)) || (st = s->alloc(&s->Pb, N)) ||
         (st = s->alloc(&s->Om, N)) || (st = s->alloc(&s->Nm, N)) || (st = s->alloc(&s->orig_c, N)) ||
