@@ -272,14 +272,25 @@ __device__ __forceinline__ void warp_walk_solids(int3 c, const float4 *__restric
         rb = __ldg(prefix + __ldg(v.off + base + (piece ? 0u : z0)));
         re = __ldg(prefix + __ldg(v.off + base + (wrap ? (piece ? z2 : D - 1u) : z2) + 1));
     }
+    // mostly few in all: the runs' solids in one sequence, 32 at a time (six queues
+    // of the mixed scene's frame, a run after another 336 us, in sequence 330, all
+    // candidates 315, as most queued there are cloth; of its late frame, 360 us for
+    // all candidates and 345)
+    int upto = re - rb;  // solids in the runs up to this lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += t;
+    }
+    const int total = __shfl_sync(0xffffffffu, upto, 31), first = rb - (upto - (re - rb));
 #pragma unroll 1
-    for (int r = 0; r < runs; ++r) {
-        const int b = __shfl_sync(0xffffffffu, rb, r), e = __shfl_sync(0xffffffffu, re, r);
+    for (int k = lane; k - lane < total; k += 32) {
+        int r = 0;
 #pragma unroll 1
-        for (int k = b + lane; k - lane < e; k += 32) {
-            const int q = k < e ? __ldg(list + k) : 0;
-            chunk(q, k < e ? P[q] : make_float4(0.f, 0.f, 0.f, 0.f), k < e);
-        }
+        for (int u = 0; u < runs; ++u) r += k >= __shfl_sync(0xffffffffu, upto, u) ? 1 : 0;
+        const int at = k + __shfl_sync(0xffffffffu, first, r & 31);
+        const int q = k < total ? __ldg(list + at) : 0;
+        chunk(q, k < total ? P[q] : make_float4(0.f, 0.f, 0.f, 0.f), k < total);
     }
 }
 
