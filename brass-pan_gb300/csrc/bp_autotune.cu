@@ -2,11 +2,14 @@
 // solver's scene and step configuration.
 //
 // The walk variants (staging each CTA's neighbourhood in shared memory,
-// testing candidates in chunks before the pair terms, the post passes'
-// neighbour lists), the launch shapes of the unstaged scans (threads per
-// CTA, persistent CTAs), iteration fusion (plane collision and commit in the
-// reorder's and the position pass's epilogues) and the contact walks' cell
-// culling give bit-identical results, so the choice only affects speed.
+// testing candidates in chunks before the pair terms, neighbour lists), the
+// launch shapes of the unstaged scans (threads per CTA, persistent CTAs),
+// iteration fusion (plane collision and commit in the reorder's and the
+// position pass's epilogues) and the contact walks' cell culling give
+// bit-identical results, so the choice only affects speed.  The unstaged split
+// walks with lists take the substep lists; staged and persistent ones record
+// lists pass by pass.  Contact culling bears on the contact passes that walk: all
+// but those that read the substep lists.
 // Each candidate runs one update from the same state (the first call of a
 // configuration captures its CUDA graph; it is run once untimed), timed with
 // CUDA events on the solver's stream; the state is put back after every

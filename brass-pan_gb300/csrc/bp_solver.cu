@@ -81,7 +81,7 @@ extern "C" void bp_params_init(bp_params *p, float r)
     p->wind_drag = 10.0f;
     p->wind_lift = 100.0f;
     p->rotation_iterations = 20;
-    p->neighbor_skin = 0.0f;  // Verlet lists measured slower than the lambda-recorded lists (opt-in)
+    p->neighbor_skin = 0.0f;  // adapted; for walks without substep lists: no Verlet lists (measured no faster)
     // staging each CTA's neighbourhood in shared memory measured slower than
     // reading it through a full-size L1, and the contact walks' cell culling
     // pays only where solids dominate (both opt-in; bp_solver_autotune times them)

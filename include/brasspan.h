@@ -144,7 +144,8 @@ typedef struct bp_params {
     float neighbor_skin;         /* skin of the per-substep neighbour lists, as a fraction of h
                                     (results are identical under any): 0, which lets the unstaged
                                     split walks over the walk planes adapt it to the displacements
-                                    they meet and turns the lists off for the other walks */
+                                    they meet and turns the lists off for the other walks (which
+                                    take 1 KB a particle for theirs where it is above 0) */
     int32_t walk_options;        /* BP_WALK_* tuning switches of the neighbour walks:
                                     BP_WALK_NO_STAGING | BP_WALK_NO_CONTACT_CULLING */
     float bending_stiffness;     /* 0.8 (bending.cuh:71) */
@@ -297,9 +298,9 @@ bp_status bp_solver_profile(bp_solver *s, int32_t num_substeps, float dt, int32_
 
 /* One real update that also counts the neighbour walks of every scan pass:
  * out_walks[0] walks over the per-substep lists; 27-cell walks
- * because [1] there is no list for the particle (lists are off, the pass
- * builds them, its candidates did not fit, or an earlier pass found it had
- * left its cell), [2] the particle left the cell its list was built
+ * because [1] there is no list for the particle (lists are off or would not
+ * pay, the pass builds them, its candidates did not fit, or an earlier pass
+ * found it had left its cell), [2] the particle left the cell its list was built
  * for, [3] it and a particle stored in its 27 cells moved more than the
  * skin allows; [4] of the cell walks, those restricted to the alias classes. */
 bp_status bp_solver_walk_stats(bp_solver *s, int32_t num_substeps, float dt, int32_t iterations,
@@ -325,7 +326,7 @@ bp_status bp_solver_autotune(bp_solver *s, int32_t num_substeps, float dt, int32
 
 /* ---- Differentiable rollouts ------------------------------------------------
  * No counterpart in the reference.  bp_solver_tape_begin starts recording the
- * following bp_solver_update calls (no picking); the state is checkpointed at
+ * following bp_solver_update calls; the state is checkpointed at
  * the start of an update once `checkpoint_every` substeps have passed since
  * the last checkpoint.  bp_solver_backward then returns the gradient of a
  * scalar loss L(x_T, v_T) of the final state with respect to the state when
